@@ -1,9 +1,17 @@
 // Persistent one-sided Jacobi: all round-robin rounds of all sweeps in one
 // cooperative launch.  Every CTA walks the pairs of a round (k = blockIdx.x,
 // += gridDim.x), then waits at a grid barrier; after each sweep every CTA reads
-// the sweep's rotation count and leaves together when it is zero.  The barrier
+// the sweep's rotation flag and leaves together when it is zero.  The barrier
 // spins at most 2 s (then sets the status word and aborts), and cooperative
 // launch refuses grids that cannot be co-resident, so no wait is unbounded.
+//
+// What bounds it.  A warp issues one FP64 instruction every 64 cycles on this part
+// (measured: 65 cycles per dependent FMA, 514 for eight independent ones of one warp; the
+// four sub-partitions of an SM together one per 16), a division takes 660 cycles and a square
+// root ~900.  Per pair and round the three 256-thread block sums were 120 FP64 instructions
+// and nine barriers, the rotation's scalars ~4500 cycles in series.  Here the three sums
+// share their instructions (tri_sum: 48, two barriers, the same additions in the same order)
+// and the scalars take ~2300 cycles (rotation).
 #pragma once
 #include "ct_common.cuh"
 
@@ -19,41 +27,35 @@ __device__ __forceinline__ unsigned long long gtime() {
 }
 
 struct Sync {
-    unsigned* count;
-    unsigned* gen;
+    unsigned* count;   // arrivals of all barriers of the launch, zeroed before it
     int* abort_flag;
-    int* rot;        // [MAX_SWEEPS] rotation counts, zeroed before launch
-    int* sweeps;     // out: sweeps run
+    int* rot;          // [MAX_SWEEPS] nonzero: the sweep rotated; zeroed before launch
+    int* sweeps;       // out: sweeps run
     int* status;
 };
 
-__device__ __forceinline__ bool grid_barrier(const Sync& s) {
+// target: arrivals expected so far (per thread, starting at 0).  Data that crosses the
+// barrier is read with __ldcg (the L1 of another SM may hold an old copy).
+__device__ __forceinline__ bool grid_barrier(const Sync& s, unsigned& target) {
     __shared__ int ok;
+    target += gridDim.x;
     __syncthreads();
     if (threadIdx.x == 0) {
         ok = 1;
-        volatile unsigned* vgen = s.gen;
-        volatile int* vab = s.abort_flag;
-        const unsigned g0 = *vgen;
-        __threadfence();
-        const unsigned arrived = atomicAdd(s.count, 1u) + 1u;
-        if (arrived == gridDim.x) {
-            atomicExch(s.count, 0u);
-            __threadfence();
-            atomicAdd(s.gen, 1u);
-        } else {
-            const unsigned long long t0 = gtime();
-            while (*vgen == g0) {
-                if (*vab) { ok = 0; break; }
-                if (gtime() - t0 > 2000000000ull) {
-                    ok = 0;
-                    atomicExch(s.abort_flag, 1);
-                    ct_set_status(s.status, CT_ERR_CUDA);
-                    break;
-                }
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(s.count) : "memory");
+        const unsigned long long t0 = gtime();
+        for (;;) {
+            unsigned v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(s.count) : "memory");
+            if ((int)(v - target) >= 0) break;
+            if (*(volatile int*)s.abort_flag) { ok = 0; break; }
+            if (gtime() - t0 > 2000000000ull) {
+                ok = 0;
+                atomicExch(s.abort_flag, 1);
+                ct_set_status(s.status, CT_ERR_CUDA);
+                break;
             }
         }
-        __threadfence();
     }
     __syncthreads();
     return ok != 0;
@@ -69,23 +71,137 @@ __device__ __forceinline__ void pair_index(int P, int r, int k, int& p, int& q) 
     }
 }
 
-template <int N>
-__device__ __forceinline__ double block_sum(double v, double* sm) {
-    return ct_block_sum<N>(v, sm);
+// ---- FP64 scalars on the critical path -----------------------------------------------------
+// Biased exponent field of x.
+__device__ __forceinline__ int exp_field(double x) { return (int)((__double_as_longlong(x) >> 52) & 0x7ff); }
+// The mantissa of a normal x as a float in [1, 2), truncated, with x's sign: integer instructions.
+__device__ __forceinline__ float mant_f32(double x) {
+    const long long b = __double_as_longlong(x);
+    return __int_as_float((int)((b >> 63) & 1) << 31 | 127 << 23 | (int)((b >> 29) & 0x7fffff));
 }
+// A normal float as a double times 2^e, by its bits (the result must be normal).
+__device__ __forceinline__ double widen(float x, int e) {
+    const int b = __float_as_int(x);
+    const long long m = ((long long)(b & 0x7fffffff) << 29) + ((long long)(1023 - 127 + e) << 52);
+    return __longlong_as_double(m | ((long long)(b >> 31) << 63));
+}
+// exponent fields for which the scalings below and the residuals stay normal
+__device__ __forceinline__ bool mid_exp(int e) { return (unsigned)(e - 400) < 1248u; }
+
+// Correctly rounded n / d and sqrt(x) from FP32 estimates: one third-order Newton step (to the
+// last bit or so), then Markstein's correction with the exact residual (P. W. Markstein,
+// Computation of elementary functions on the IBM RISC System/6000 processor, IBM J. Res. Dev.
+// 34, 1990), in 6 and 7 dependent operations; outside the middle of the exponent range the
+// plain operators.  (390 and 455 cycles against 660 and ~870.)
+__device__ __forceinline__ double div_rn(double n, double d) {
+    const int en = exp_field(n), ed = exp_field(d);
+    if (!(mid_exp(en) && mid_exp(ed) && mid_exp(en - ed + 1023))) return n / d;
+    const double y0 = widen(__fdividef(1.0f, mant_f32(d)), 1023 - ed);
+    const double e = fma(-d, y0, 1.0);
+    const double y = fma(y0, fma(e, e, e), y0);
+    const double q = n * y;
+    return fma(fma(-d, q, n), y, q);
+}
+__device__ __forceinline__ double sqrt_rn(double x) {
+    const int ex = exp_field(x);
+    if (!mid_exp(ex) || x < 0.0) return sqrt(x);
+    // x = m 2^(2k), m in [1, 4)
+    const int k = (ex - 1023) >> 1;
+    const float mf = mant_f32(x) * (((ex - 1023) & 1) ? 2.0f : 1.0f);
+    const double y = widen(rsqrtf(mf), -k);
+    const double h = __longlong_as_double(__double_as_longlong(y) - (1ll << 52));   // y / 2
+    const double g = x * y;
+    const double r = fma(-g, h, 0.5);
+    const double p = fma(1.5 * r, r, r);
+    const double g1 = fma(g, p, g), h1 = fma(h, p, h);
+    return fma(fma(-g1, g1, x), h1, g1);
+}
+
+// Rotation that orthogonalises two vectors with |x_p|^2=a, |x_q|^2=b, <x_p,x_q>=c.
+// Vectors with |x|^2 <= floor (numerically zero next to |M|_F) are left alone:
+// rotating rounding noise never converges.  The threshold |c| > tol sqrt(a b) is decided in
+// FP32 on the mantissas and exponents unless the two sides agree to 1e-5.
+__device__ __forceinline__ bool rotation(double a, double b, double c, double tol, double floor, double& cs,
+                                         double& sn) {
+    if (!(a > floor && b > floor) || c == 0.0) return false;
+    {
+        const int ea = exp_field(a), eb = exp_field(b), ec = exp_field(c), et = exp_field(tol);
+        bool go;
+        const int de = 2 * (ec - 1023) - (ea - 1023) - (eb - 1023) - 2 * (et - 1023);
+        if (mid_exp(ea) && mid_exp(eb) && mid_exp(ec) && mid_exp(et)) {
+            const float fc = mant_f32(c), ft = mant_f32(tol);
+            // c^2 / (tol^2 a b) = ratio 2^de, ratio in (1/16, 4)
+            const float ratio = __fdividef(fc * fc, ft * ft * (mant_f32(a) * mant_f32(b)));
+            if (de > 6) go = true;
+            else if (de < -6) go = false;
+            else {
+                const float z = ratio * __int_as_float((127 + de) << 23);
+                go = z > 1.00001f;
+                if (!go && z > 0.99999f) go = fabs(c) > tol * sqrt(a * b);
+            }
+        } else {
+            go = fabs(c) > tol * sqrt(a * b);
+        }
+        if (!go) return false;
+    }
+    const double zeta = div_rn(b - a, 2.0 * c);
+    double t;
+    if (fabs(zeta) > 1e150) t = 0.5 / zeta;
+    else t = copysign(div_rn(1.0, fabs(zeta) + sqrt_rn(1.0 + zeta * zeta)), zeta);
+    cs = div_rn(1.0, sqrt_rn(1.0 + t * t));
+    sn = cs * t;
+    return true;
+}
+
+// Sums of a, b and c over the 256 threads of the CTA, each with the additions of ct_block_sum in
+// its order (a warp butterfly, then the eight warp sums by the first warp), the three sharing
+// instructions: per warp 6 FP64 additions instead of 15, then 3 instead of 15.  The results
+// are valid in the first 24 lanes of warp 0: lanes 0-7 hold a's sum, 8-15 b's, 16-23 c's.
+__device__ __forceinline__ double tri_sum(double a, double b, double c, double* sm) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    // offset 16: a in lanes 0-15, b in lanes 16-31 of y; c in both halves
+    const bool lo = lane < 16;
+    double y = (lo ? a : b) + __shfl_xor_sync(0xffffffffu, lo ? b : a, 16);
+    c += __shfl_xor_sync(0xffffffffu, c, 16);
+    // offset 8: lanes 0-7 a, 8-15 b, 16-23 c
+    const int src = lane < 8 ? lane : lane + 8;          // a: 0-7, b: 16-23
+    const double y1 = __shfl_sync(0xffffffffu, y, src & 31), y2 = __shfl_sync(0xffffffffu, y, (src + 8) & 31);
+    const double c2 = __shfl_xor_sync(0xffffffffu, c, 8);
+    y = lo ? y1 + y2 : c + c2;
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+    if (lane < 24 && (lane & 7) == 0) sm[(lane >> 3) * 8 + wid] = y;
+    __syncthreads();
+    if (wid == 0) {
+        y = lane < 24 ? sm[lane] : 0.0;
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+    }
+    return y;
+}
+
+// x' = cs x - sn y, y' = sn x + cs y, the multiply-adds fixed (the same bits in every kernel)
+template <typename T>
+__device__ __forceinline__ T rot_x(T cs, T sn, T x, T y) { return fma(cs, x, -(sn * y)); }
+template <typename T>
+__device__ __forceinline__ T rot_y(T cs, T sn, T x, T y) { return fma(sn, x, cs * y); }
 
 // T = float (mixed form: FP32 data, FP64 reductions) or double (plain form)
 template <typename T>
 __global__ void __launch_bounds__(NT) jacobi_coop_kernel(T* X, int64_t len, T* Q, int64_t nvec, double tol,
                                                         double floor_rel, const double* frob2, int max_sweeps,
                                                         Sync s) {
-    __shared__ double sm[32];
+    __shared__ double sm[24];
     __shared__ double rot_cs, rot_sn;
     __shared__ int do_rot;
     const int P = (int)(nvec + (nvec & 1));
     const double floor = floor_rel * (*frob2);
+    const int tid = threadIdx.x;
+    // vectors of up to 256 elements stay in a register between the sums and the rotation
+    const bool held = len <= NT && nvec <= NT;
+    unsigned target = 0;
     int sweep = 0;
-    bool ok = true;
+    bool ok = true, last_rot = true;
     for (; sweep < max_sweeps && ok; ++sweep) {
         for (int r = 0; r < P - 1 && ok; ++r) {
             for (int k = blockIdx.x; k < P / 2; k += gridDim.x) {
@@ -94,63 +210,98 @@ __global__ void __launch_bounds__(NT) jacobi_coop_kernel(T* X, int64_t len, T* Q
                 if (p >= nvec || q >= nvec) continue;
                 T* xp = X + (int64_t)p * len;
                 T* xq = X + (int64_t)q * len;
+                T* qp = Q + (int64_t)p * nvec;
+                T* qq = Q + (int64_t)q * nvec;
+                T x = 0, y = 0, g = 0, h = 0;
                 T fa = 0, fb = 0, fc = 0;
-                for (int64_t i = threadIdx.x; i < len; i += NT) {
-                    const T u = xp[i], v = xq[i];
-                    fa += u * u;
-                    fb += v * v;
-                    fc += u * v;
-                }
-                const double a = block_sum<NT>((double)fa, sm);
-                const double b = block_sum<NT>((double)fb, sm);
-                const double c = block_sum<NT>((double)fc, sm);
-                if (threadIdx.x == 0) {
-                    int go = 0;
-                    if (a > floor && b > floor && c != 0.0 && fabs(c) > tol * sqrt(a * b)) {
-                        const double zeta = (b - a) / (2.0 * c);
-                        const double t = (fabs(zeta) > 1e150)
-                                             ? 0.5 / zeta
-                                             : copysign(1.0, zeta) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
-                        const double cs = 1.0 / sqrt(1.0 + t * t);
-                        rot_cs = cs;
-                        rot_sn = cs * t;
-                        go = 1;
-                        atomicAdd(&s.rot[sweep], 1);
+                if (held) {
+                    if (tid < len) {
+                        x = __ldcg(xp + tid);
+                        y = __ldcg(xq + tid);
                     }
-                    do_rot = go;
+                    if (tid < nvec) {
+                        g = __ldcg(qp + tid);
+                        h = __ldcg(qq + tid);
+                    }
+                    if (tid < len) {
+                        fa += x * x;
+                        fb += y * y;
+                        fc += x * y;
+                    }
+                } else {
+                    for (int64_t i = tid; i < len; i += NT) {
+                        const T u = __ldcg(xp + i), v = __ldcg(xq + i);
+                        fa += u * u;
+                        fb += v * v;
+                        fc += u * v;
+                    }
+                }
+                const double sum = tri_sum((double)fa, (double)fb, (double)fc, sm);
+                if (tid < 32) {
+                    const double a = __shfl_sync(0xffffffffu, sum, 0), b = __shfl_sync(0xffffffffu, sum, 8),
+                                 c = __shfl_sync(0xffffffffu, sum, 16);
+                    double cs = 1.0, sn = 0.0;
+                    const bool go = rotation(a, b, c, tol, floor, cs, sn);
+                    if (tid == 0) {
+                        rot_cs = cs;
+                        rot_sn = sn;
+                        if (go) s.rot[sweep] = 1;
+                        do_rot = go ? 1 : 0;
+                    }
                 }
                 __syncthreads();
                 if (do_rot) {
                     const T cs = (T)rot_cs, sn = (T)rot_sn;
-                    for (int64_t i = threadIdx.x; i < len; i += NT) {
-                        const T u = xp[i], v = xq[i];
-                        xp[i] = cs * u - sn * v;
-                        xq[i] = sn * u + cs * v;
-                    }
-                    T* qp = Q + (int64_t)p * nvec;
-                    T* qq = Q + (int64_t)q * nvec;
-                    for (int64_t i = threadIdx.x; i < nvec; i += NT) {
-                        const T u = qp[i], v = qq[i];
-                        qp[i] = cs * u - sn * v;
-                        qq[i] = sn * u + cs * v;
+                    if (held) {
+                        if (tid < len) {
+                            xp[tid] = rot_x<T>(cs, sn, x, y);
+                            xq[tid] = rot_y<T>(cs, sn, x, y);
+                        }
+                        if (tid < nvec) {
+                            qp[tid] = rot_x<T>(cs, sn, g, h);
+                            qq[tid] = rot_y<T>(cs, sn, g, h);
+                        }
+                    } else {
+                        for (int64_t i = tid; i < len; i += NT) {
+                            const T u = __ldcg(xp + i), v = __ldcg(xq + i);
+                            xp[i] = rot_x<T>(cs, sn, u, v);
+                            xq[i] = rot_y<T>(cs, sn, u, v);
+                        }
+                        for (int64_t i = tid; i < nvec; i += NT) {
+                            const T u = __ldcg(qp + i), v = __ldcg(qq + i);
+                            qp[i] = rot_x<T>(cs, sn, u, v);
+                            qq[i] = rot_y<T>(cs, sn, u, v);
+                        }
                     }
                 }
                 __syncthreads();
             }
-            ok = grid_barrier(s);
+            ok = grid_barrier(s, target);
         }
         if (!ok) break;
-        const int rc = *(volatile int*)&s.rot[sweep];
-        if (rc == 0) {
+        last_rot = __ldcg(s.rot + sweep) != 0;
+        if (!last_rot) {
             ++sweep;
             break;
         }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         *s.sweeps = sweep;
-        if (ok && sweep >= max_sweeps && *(volatile int*)&s.rot[max_sweeps - 1] != 0)
-            ct_set_status(s.status, CT_ERR_NOCONV);
+        if (ok && sweep >= max_sweeps && last_rot) ct_set_status(s.status, CT_ERR_NOCONV);
     }
+}
+
+// Barrier and sweep scratch of a launch in d_flags: [16] count, [18] abort, [19] sweeps,
+// [32 .. 32 + max_sweeps) rotation flags; zeroed on the stream.
+inline int reset_sync(ct_handle* h, int max_sweeps, Sync& s) {
+    int* base = h->d_flags;
+    CT_CUDA(h, cudaMemsetAsync(base + 16, 0, (16 + max_sweeps) * sizeof(int), h->stream));
+    s.count = (unsigned*)(base + 16);
+    s.abort_flag = base + 18;
+    s.sweeps = base + 19;
+    s.rot = base + 32;
+    s.status = h->d_status;
+    return CT_OK;
 }
 
 // Launches the persistent Jacobi; sync scratch comes from h->d_flags.
@@ -161,16 +312,8 @@ int run(ct_handle* h, T* X, int64_t len, T* Q, int64_t nvec, double tol, double 
         if (sweeps_host) *sweeps_host = 0;
         return CT_OK;
     }
-    // scratch layout in d_flags: [16] count, [17] gen, [18] abort, [19] sweeps, [32..32+MAX_SWEEPS) rot
-    int* base = h->d_flags;
-    CT_CUDA(h, cudaMemsetAsync(base + 16, 0, (32 + MAX_SWEEPS - 16) * sizeof(int), h->stream));
     Sync s;
-    s.count = (unsigned*)(base + 16);
-    s.gen = (unsigned*)(base + 17);
-    s.abort_flag = base + 18;
-    s.sweeps = base + 19;
-    s.rot = base + 32;
-    s.status = h->d_status;
+    CT_TRY(reset_sync(h, MAX_SWEEPS, s));
     static int occ_dev = -1, occ = 0;
     if (occ_dev != h->device) {
         CT_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, jacobi_coop_kernel<T>, NT, 0));

@@ -10,44 +10,16 @@
 //                  accumulated rotations are V, the rotated columns are U S.
 // No division by a singular value is needed in either sweep direction.
 //
-// Small problems run in one CTA with everything in shared memory (no host
-// round trip); large ones run one launch per round-robin round, n/2 pairs in
-// parallel, with a rotation counter read back once per sweep.
+// Up to 200 KB of vectors and rotations run in one launch of four warps per
+// pair (ct_svd_small.cuh, no host round trip); large ones in one cooperative
+// launch, one CTA per pair, after a Householder QR.
 #include "ct_ops.cuh"
 #include "ct_jacobi_coop.cuh"
+#include "ct_svd_small.cuh"
 
 namespace {
 
-constexpr int SVD_NT = 256;
-constexpr int SVD_MAX_SWEEPS = 60;
-constexpr int FL_SVD_SWEEPS = 19;   // d_flags slot: sweeps of the last Jacobi (the cooperative one's too)
 constexpr double SVD_EPS2 = 2.2204460492503131e-16 * 2.2204460492503131e-16;
-
-__device__ __forceinline__ void tournament_pair(int P, int r, int k, int& p, int& q) {
-    if (k == 0) {
-        p = P - 1;
-        q = r;
-    } else {
-        p = (r + k) % (P - 1);
-        q = (r - k + (P - 1)) % (P - 1);
-    }
-}
-
-// Rotation that orthogonalises two vectors with |x_p|^2=a, |x_q|^2=b, <x_p,x_q>=c.
-// Vectors with |x|^2 <= floor (numerically zero next to |M|_F) are left alone:
-// rotating rounding noise never converges.
-__device__ __forceinline__ bool jacobi_rot(double a, double b, double c, double tol, double floor, double& cs,
-                                           double& sn) {
-    if (a <= floor || b <= floor) return false;
-    if (c == 0.0 || !(fabs(c) > tol * sqrt(a * b))) return false;
-    const double zeta = (b - a) / (2.0 * c);
-    double t;
-    if (fabs(zeta) > 1e150) t = 0.5 / zeta;
-    else t = copysign(1.0, zeta) / (fabs(zeta) + sqrt(1.0 + zeta * zeta));
-    cs = 1.0 / sqrt(1.0 + t * t);
-    sn = cs * t;
-    return true;
-}
 
 // ---- init: X (nvec x len) from M, Q = I ---------------------------------------
 __global__ void svd_init_kernel(const double* M, int64_t m, int64_t n, int cols, double* X, int64_t ldx,
@@ -61,78 +33,6 @@ __global__ void svd_init_kernel(const double* M, int64_t m, int64_t n, int cols,
     const int64_t tq = nvec * nvec;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < tq; t += (int64_t)gridDim.x * blockDim.x)
         Q[t] = ((t / nvec) == (t % nvec)) ? 1.0 : 0.0;
-}
-
-// ---- small path: whole Jacobi in one CTA, X and Q in shared memory ------------
-__global__ void __launch_bounds__(SVD_NT) svd_small_kernel(double* Xg, int64_t len, int64_t ldx, double* Qg,
-                                                           int nvec, double tol, int max_sweeps, int* status,
-                                                           int* sweeps_out) {
-    extern __shared__ double ssm[];
-    double* X = ssm;                         // nvec x len
-    double* Q = ssm + (int64_t)nvec * len;   // nvec x nvec
-    for (int64_t t = threadIdx.x; t < (int64_t)nvec * len; t += SVD_NT) X[t] = Xg[(t / len) * ldx + t % len];
-    for (int64_t t = threadIdx.x; t < (int64_t)nvec * nvec; t += SVD_NT) Q[t] = Qg[t];
-    __syncthreads();
-    __shared__ double red[32];
-    double f2 = 0.0;
-    for (int64_t t = threadIdx.x; t < (int64_t)nvec * len; t += SVD_NT) f2 = fma(X[t], X[t], f2);
-    const double floor = SVD_EPS2 * ct_block_sum<SVD_NT>(f2, red);
-    const int P = nvec + (nvec & 1);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = SVD_NT / 32;
-    bool converged = false;
-    int sweep = 0;
-    for (; sweep < max_sweeps; ++sweep) {
-        int rotated = 0;
-        for (int r = 0; r < P - 1; ++r) {
-            for (int k = warp; k < P / 2; k += nw) {
-                int p, q;
-                tournament_pair(P, r, k, p, q);
-                if (p >= nvec || q >= nvec) continue;
-                double* xp = X + (int64_t)p * len;
-                double* xq = X + (int64_t)q * len;
-                double a = 0.0, b = 0.0, c = 0.0;
-                for (int64_t i = lane; i < len; i += 32) {
-                    const double u = xp[i], v = xq[i];
-                    a = fma(u, u, a);
-                    b = fma(v, v, b);
-                    c = fma(u, v, c);
-                }
-                a = ct_warp_sum(a);
-                b = ct_warp_sum(b);
-                c = ct_warp_sum(c);
-                double cs, sn;
-                if (jacobi_rot(a, b, c, tol, floor, cs, sn)) {
-                    rotated = 1;
-                    for (int64_t i = lane; i < len; i += 32) {
-                        const double u = xp[i], v = xq[i];
-                        xp[i] = cs * u - sn * v;
-                        xq[i] = sn * u + cs * v;
-                    }
-                    double* qp = Q + (int64_t)p * nvec;
-                    double* qq = Q + (int64_t)q * nvec;
-                    for (int i = lane; i < nvec; i += 32) {
-                        const double u = qp[i], v = qq[i];
-                        qp[i] = cs * u - sn * v;
-                        qq[i] = sn * u + cs * v;
-                    }
-                }
-                __syncwarp();
-            }
-            __syncthreads();
-        }
-        if (!__syncthreads_or(rotated)) {
-            converged = true;
-            ++sweep;
-            break;
-        }
-    }
-    if (threadIdx.x == 0) {
-        *sweeps_out = sweep;
-        if (!converged) ct_set_status(status, CT_ERR_NOCONV);
-    }
-    __syncthreads();
-    for (int64_t t = threadIdx.x; t < (int64_t)nvec * len; t += SVD_NT) Xg[(t / len) * ldx + t % len] = X[t];
-    for (int64_t t = threadIdx.x; t < (int64_t)nvec * nvec; t += SVD_NT) Qg[t] = Q[t];
 }
 
 // sigma_j = |x_j|, one warp per vector
@@ -149,54 +49,66 @@ __global__ void svd_norms_kernel(const double* X, int64_t len, int64_t ldx, int6
     if (lane == 0) sig[v] = sqrt(a);
 }
 
-// descending order, ties by index: perm[rank(j)] = j
+// descending order, ties by index: perm[rank(j)] = j.  One warp per j; the comparisons on
+// the bit patterns (singular values are >= 0, so the integer order is theirs; NaN last):
+// FP64 compares share the slow FP64 pipe (256 values: 58 us with one thread per j and FP64
+// compares).
+__device__ __forceinline__ long long rank_bits(double s) { return isnan(s) ? -1ll : __double_as_longlong(s); }
 __global__ void svd_rank_kernel(const double* sig, int64_t nvec, int* perm) {
-    const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const int64_t j = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
+    const int lane = threadIdx.x & 31;
     if (j >= nvec) return;
-    const double sj = ct_rank_key(sig[j]);
-    int64_t rank = 0;
-    for (int64_t i = 0; i < nvec; ++i) {
-        const double si = ct_rank_key(sig[i]);
-        if (si > sj || (si == sj && i < j)) ++rank;
+    const long long sj = rank_bits(sig[j]);
+    int rank = 0;
+    for (int64_t i = lane; i < nvec; i += 32) {
+        const long long si = rank_bits(sig[i]);
+        rank += (si > sj || (si == sj && i < j)) ? 1 : 0;
     }
-    perm[rank] = (int)j;
+    rank = __reduce_add_sync(0xffffffffu, rank);
+    if (lane == 0) perm[rank] = (int)j;
 }
 
-// chi rule of dense_tensor.mojo:1528-1548, FP64, sequential sums in sorted order
+// chi rule of dense_tensor.mojo:1528-1548, FP64, sequential sums in sorted order.  One
+// warp: the lanes gather 32 weights at a time, the sums run over them in order.
 __global__ void svd_trunc_kernel(const double* sig, const int* perm, int64_t k, int64_t chi_max, double eps,
                                  double* scalars, int* flags) {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    const int lane = threadIdx.x;
+    auto weight = [&](int64_t i) {
+        const double s = i < k ? sig[perm[i]] : 0.0;
+        return s * s;
+    };
     int64_t chi = k < chi_max ? k : chi_max;
-    double total = 0.0, kept_at = 0.0;
-    for (int64_t i = 0; i < k; ++i) {
-        const double s = sig[perm[i]];
-        total += s * s;
+    double total = 0.0;
+    for (int64_t i0 = 0; i0 < k; i0 += 32) {
+        const double s2 = weight(i0 + lane);
+        const int n = (int)(k - i0 < 32 ? k - i0 : 32);
+        for (int l = 0; l < n; ++l) total += __shfl_sync(0xffffffffu, s2, l);
     }
-    if (eps > 0.0 && k > 0) {
-        if (total <= 0.0) {
-            chi = 0;
-        } else {
-            double kept = 0.0;
-            const int64_t limit = k < chi_max ? k : chi_max;
-            chi = limit;
-            for (int64_t t = 1; t <= limit; ++t) {
-                const double s = sig[perm[t - 1]];
-                kept += s * s;
-                if ((total - kept) / total <= eps) {
-                    chi = t;
+    double kept = 0.0;
+    if (eps > 0.0 && k > 0 && total <= 0.0) {
+        chi = 0;
+    } else {
+        const int64_t limit = chi;
+        bool done = false;
+        for (int64_t i0 = 0; i0 < limit && !done; i0 += 32) {
+            const double s2 = weight(i0 + lane);
+            const int n = (int)(limit - i0 < 32 ? limit - i0 : 32);
+            for (int l = 0; l < n; ++l) {
+                kept += __shfl_sync(0xffffffffu, s2, l);
+                if (eps > 0.0 && (total - kept) / total <= eps) {
+                    chi = i0 + l + 1;
+                    done = true;
                     break;
                 }
             }
         }
     }
-    for (int64_t i = 0; i < chi; ++i) {
-        const double s = sig[perm[i]];
-        kept_at += s * s;
+    if (lane == 0) {
+        scalars[SC_SVD_MINKEPT] = chi > 0 ? sig[perm[chi - 1]] : 0.0;
+        flags[FL_CHI] = (int)chi;
+        scalars[SC_TMP0] = total;
+        scalars[SC_TMP1] = kept;
     }
-    scalars[SC_SVD_MINKEPT] = chi > 0 ? sig[perm[chi - 1]] : 0.0;
-    flags[FL_CHI] = (int)chi;
-    scalars[SC_TMP0] = total;
-    scalars[SC_TMP1] = kept_at;
 }
 
 // outputs; vectors = rows (cols=0) or columns (cols=1) of M
@@ -301,12 +213,13 @@ __global__ void __launch_bounds__(QR_NT) qr_coop_kernel(double* T, int64_t len, 
     const int lane = threadIdx.x & 31;
     const int64_t nw = (int64_t)gridDim.x * (QR_NT / 32);
     const int64_t gw = (int64_t)blockIdx.x * (QR_NT / 32) + (threadIdx.x >> 5);
+    unsigned target = 0;
     for (int64_t j = 0; j < k; ++j) {
         const double* tj = T + j * nvec + j;
         const int64_t tl = nvec - j;
         double s2 = 0.0;
         for (int64_t i = threadIdx.x; i < tl; i += QR_NT) {
-            const double x = tj[i];
+            const double x = __ldcg(tj + i);
             u[i] = x;
             if (i > 0) s2 = fma(x, x, s2);
         }
@@ -338,7 +251,7 @@ __global__ void __launch_bounds__(QR_NT) qr_coop_kernel(double* T, int64_t len, 
                 for (int64_t i = lane; i < tl; i += 32) tr[i] = fma(-d, u[i], tr[i]);
             }
         }
-        if (j + 1 < k && !ct_jacobi::grid_barrier(s)) return;
+        if (j + 1 < k && !ct_jacobi::grid_barrier(s, target)) return;
     }
 }
 
@@ -443,16 +356,8 @@ static int svd_qr_jacobi(ct_handle* h, Arena& ar, const double* M, int64_t m, in
         const int64_t need = ct_cdiv(len > 1 ? len - 1 : 1, QR_NT / 32);
         if (grid > need) grid = need;
         if (grid < 1) grid = 1;
-        // grid barrier scratch in d_flags, as the Jacobi's: [16] count, [17] gen, [18] abort
-        int* base = h->d_flags;
-        CT_CUDA(h, cudaMemsetAsync(base + 16, 0, 4 * sizeof(int), h->stream));
         ct_jacobi::Sync sy;
-        sy.count = (unsigned*)(base + 16);
-        sy.gen = (unsigned*)(base + 17);
-        sy.abort_flag = base + 18;
-        sy.sweeps = base + 19;
-        sy.rot = base + 32;
-        sy.status = h->d_status;
+        CT_TRY(ct_jacobi::reset_sync(h, 0, sy));
         void* args[] = {&T, &len, &nvec, (void*)&k, &refl, &sy};
         CT_CUDA(h, cudaLaunchCooperativeKernel((const void*)qr_coop_kernel, dim3((unsigned)grid), dim3(QR_NT), args,
                                                smem, h->stream));
@@ -534,7 +439,20 @@ static int svd_run_geometry(ct_handle* h, Arena& ar, const double* M, int64_t m,
     const double* Qf = Q;
     bool small_run = false;
 
-    if (svd_uses_qr(nvec, len)) {
+    if (nvec >= 2 && (nvec * len + nvec * nvec) * (int64_t)sizeof(double) <= 200 * 1024) {
+        ct_svd_small::Args a{};
+        a.M = M;
+        a.n = n;
+        a.cols = cols;
+        a.nvec = (int)nvec;
+        a.len = (int)len;
+        a.X = X;
+        a.Q = Q;
+        a.nsq = sig;
+        a.tol = tol;
+        CT_TRY(ct_svd_small::run(h, a));
+        small_run = true;
+    } else if (svd_uses_qr(nvec, len)) {
         double* Qn = nullptr;
         CT_TRY(svd_qr_jacobi(h, ar, M, m, n, cols, nvec, len, tol, X, Q, &Qn));
         nv = k;
@@ -546,21 +464,7 @@ static int svd_run_geometry(ct_handle* h, Arena& ar, const double* M, int64_t m,
         if (g < 1) g = 1;
         svd_init_kernel<<<g, 256, 0, h->stream>>>(M, m, n, cols, X, ldx, Q, nvec); ct_note_launch();
         CT_LAUNCH_CHECK(h);
-        const size_t small_bytes = (size_t)(nvec * len + nvec * nvec) * sizeof(double);
-        if (nvec >= 2 && small_bytes <= 200 * 1024) {
-            static bool attr = false;
-            if (!attr) {
-                CT_CUDA(h, cudaFuncSetAttribute(svd_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                200 * 1024));
-                attr = true;
-            }
-            const int cap = (h->svd_max_sweeps > 0 && h->svd_max_sweeps < SVD_MAX_SWEEPS) ? h->svd_max_sweeps
-                                                                                            : SVD_MAX_SWEEPS;
-            svd_small_kernel<<<1, SVD_NT, small_bytes, h->stream>>>(X, len, ldx, Q, (int)nvec, tol, cap, h->d_status,
-                                                                    h->d_flags + FL_SVD_SWEEPS); ct_note_launch();
-            CT_LAUNCH_CHECK(h);
-            small_run = true;
-        } else if (nvec >= 2) {
+        if (nvec >= 2) {
             // beyond the QR's shared-memory limit: the Jacobi on the vectors themselves
             double* d_frob2 = h->d_scalars + SC_TMP0;
             CT_TRY(ct_reduce_nrm2sq(h, nvec * ldx, X, d_frob2, nullptr));
@@ -568,7 +472,7 @@ static int svd_run_geometry(ct_handle* h, Arena& ar, const double* M, int64_t m,
         }
     }
     svd_norms_kernel<<<(unsigned)ct_cdiv(nv * 32, 256), 256, 0, h->stream>>>(X, len, ldx, nv, sig); ct_note_launch();
-    svd_rank_kernel<<<(unsigned)ct_cdiv(nv, 256), 256, 0, h->stream>>>(sig, nv, perm); ct_note_launch();
+    svd_rank_kernel<<<(unsigned)ct_cdiv(nv * 32, 256), 256, 0, h->stream>>>(sig, nv, perm); ct_note_launch();
     svd_trunc_kernel<<<1, 32, 0, h->stream>>>(sig, perm, k, chi_max, eps_trunc, h->d_scalars, h->d_flags); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     int chi = 0;
@@ -579,7 +483,7 @@ static int svd_run_geometry(ct_handle* h, Arena& ar, const double* M, int64_t m,
                                h->stream));
     int small_sweeps = 0;
     if (small_run)
-        CT_CUDA(h, cudaMemcpyAsync(&small_sweeps, h->d_flags + FL_SVD_SWEEPS, sizeof(int), cudaMemcpyDeviceToHost,
+        CT_CUDA(h, cudaMemcpyAsync(&small_sweeps, h->d_flags + 19, sizeof(int), cudaMemcpyDeviceToHost,
                                    h->stream));
     CT_CUDA(h, cudaStreamSynchronize(h->stream));
     if (small_run) {
