@@ -162,6 +162,8 @@ int ct_destroy(ct_handle* h) {
     for (auto e : h->ktime_ev) cudaEventDestroy(e);
     cudaFree(h->splitk);
     cudaFree(h->oz_ws);
+    cudaFree(h->fm_ws);
+    for (void* p : h->fm_kept) cudaFree(p);
     cudaFree(h->tc_sk_part);
     cudaFree(h->tc_sk_flag);
     cudaFree(h->tc_hy_part);

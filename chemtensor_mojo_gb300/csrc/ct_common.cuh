@@ -51,6 +51,10 @@ struct ct_handle {
     size_t splitk_cap = 0;   // doubles
     void* oz_ws = nullptr;   // slices of the FP64 tensor-core GEMM (ct_ozaki.cu)
     size_t oz_ws_bytes = 0;
+    void* fm_ws = nullptr;   // residues of the FP64-form tensor-core GEMM (ct_f64mod.cu)
+    size_t fm_ws_bytes = 0;
+    bool fm_captured = false;        // fm_ws is in a captured graph
+    std::vector<void*> fm_kept;      // outgrown buffers of captured graphs, freed with the handle
     // allocation-free mode (the stack handle of ct_heff2_apply_noalloc): the
     // launchers never call cudaMalloc; split-K partials come from the fixed
     // region below, and K is split only as far as that region holds

@@ -53,7 +53,12 @@ int ct_heff1_run(ct_handle* h, Arena& ar, const double* L, const double* A, cons
     if (!T1 || !T2 || !Wt) return CT_ERR_OOM;
     CT_TRY(ct_build_wt_left(h, W, Wt, wl, d, wr));
     const int64_t n1 = d * Dr;
-    {   // T1[Dl', wl, (s Dr)] = sum_Dl L[wl, Dl, Dl'] A[Dl, (s Dr)]
+    if (ct_f64_route(h, wl * Dl, n1, Dl)) {
+        const OzMat a{L, Dl, Dl * Dl, 1, Dl};
+        const OzMat b{A, n1, 0, 1, n1};
+        const OzOut c{T1, Dl, n1, wl * n1};
+        CT_TRY(ct_f64_gemm(h, wl * Dl, n1, Dl, a, b, c));
+    } else {   // T1[Dl', wl, (s Dr)] = sum_Dl L[wl, Dl, Dl'] A[Dl, (s Dr)]
         GemmDesc g{};
         g.M = Dl; g.N = n1; g.K = Dl;
         g.A = L; g.sAm = 1; g.sAk = Dl;
@@ -70,7 +75,10 @@ int ct_heff1_run(ct_handle* h, Arena& ar, const double* L, const double* A, cons
         m.Wt = Wt;
         CT_TRY(ct_mpo_apply_f64_launch(h, m));
     }
-    {   // out[(Dl' s'), Dr'] = sum_(wr Dr) T2[(Dl' s'), (wr Dr)] R[(wr Dr), Dr']
+    if (ct_f64_route(h, Dl * d, Dr, wr * Dr)) {
+        CT_TRY(ct_f64_gemm(h, Dl * d, Dr, wr * Dr, OzMat{T2, Dl * d, 0, wr * Dr, 1}, OzMat{R, Dr, 0, 1, Dr},
+                           OzOut{out, Dl * d, 0, Dr}));
+    } else {   // out[(Dl' s'), Dr'] = sum_(wr Dr) T2[(Dl' s'), (wr Dr)] R[(wr Dr), Dr']
         GemmDesc g{};
         g.M = Dl * d; g.N = Dr; g.K = wr * Dr;
         g.A = T2; g.sAm = wr * Dr; g.sAk = 1;

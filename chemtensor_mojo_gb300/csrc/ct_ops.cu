@@ -13,8 +13,10 @@
 //     Ln[(wR Dr), Dr'] = sum_(Dl' s') T2[(Dl' s'),(wR Dr)] A[(Dl' s'),Dr'] GEMM
 //   right env (environments.mojo:309-417)
 //     T1[Dr', wR, s, Dl] = sum_Dr R[wR,Dr,Dr'] A[Dl,s,Dr]                  GEMM, batch (wR,s)
-//     T2[wL, Dl, s', Dr'] = sum_(wR s) W[wL,s,s',wR] T1                    MPO apply
-//     Rp[wL, Dl, Dl'] = sum_(s' Dr') T2[wL,Dl,(s' Dr')] A[Dl',(s' Dr')]    GEMM, batch wL
+//     T2[wL, s', Dr', Dl] = sum_(wR s) W[wL,s,s',wR] T1                    MPO apply
+//     Rp[wL, Dl, Dl'] = sum_(s' Dr') T2[wL,(s' Dr'),Dl] A[Dl',(s' Dr')]    GEMM, batch wL
+// FP64-form products that are faster on the BF16 tensor cores by residues run there as one
+// GEMM each (ct_f64mod.cu, ct_f64_route).
 #include <stdlib.h>
 
 #include "ct_ops.cuh"
@@ -47,7 +49,13 @@ int ct_heff_run(ct_handle* h, const HeffPlan& p, const double* theta, double* ou
     if (p.prec == CT_PREC_TF32X3) return ct_tc_heff_run(h, p, theta, out, skip);
     const int64_t Dl = p.Dl, d = p.d, Dr = p.Dr, wL = p.wL, wR = p.wR;
     const int64_t n1 = d * d * Dr;
-    {   // T1[Dl', wL, n1] = sum_Dl L[wL, Dl, Dl'] theta[Dl, n1]
+    if (ct_f64_route(h, wL * Dl, n1, Dl)) {
+        // the product below as one GEMM over rows (wL, Dl'): A(r, k) = L[wL][k][Dl']
+        const OzMat a{p.L, Dl, Dl * Dl, 1, Dl};
+        const OzMat b{theta, n1, 0, 1, n1};
+        const OzOut c{p.T1, Dl, n1, wL * n1};
+        CT_TRY(ct_f64_gemm(h, wL * Dl, n1, Dl, a, b, c, skip));
+    } else {   // T1[Dl', wL, n1] = sum_Dl L[wL, Dl, Dl'] theta[Dl, n1]
         GemmDesc g{};
         g.M = Dl; g.N = n1; g.K = Dl;
         g.A = p.L; g.sAm = 1; g.sAk = Dl;
@@ -67,7 +75,12 @@ int ct_heff_run(ct_handle* h, const HeffPlan& p, const double* theta, double* ou
         m.Wt = p.W12; m.skip = skip;
         CT_TRY(ct_mpo_apply_f64_launch(h, m));
     }
-    {   // out[(Dl' t1 t2), Dr'] = sum_(wR Dr) T3[.., (wR Dr)] R[(wR Dr), Dr']
+    if (ct_f64_route(h, Dl * d * d, Dr, wR * Dr)) {
+        const OzMat a{p.T3, Dl * d * d, 0, wR * Dr, 1};
+        const OzMat b{p.R, Dr, 0, 1, Dr};
+        const OzOut c{out, Dl * d * d, 0, Dr};
+        CT_TRY(ct_f64_gemm(h, Dl * d * d, Dr, wR * Dr, a, b, c, skip));
+    } else {   // out[(Dl' t1 t2), Dr'] = sum_(wR Dr) T3[.., (wR Dr)] R[(wR Dr), Dr']
         GemmDesc g{};
         g.M = Dl * d * d; g.N = Dr; g.K = wR * Dr;
         g.A = p.T3; g.sAm = wR * Dr; g.sAk = 1;
@@ -112,13 +125,13 @@ int ct_env_left2_run(ct_handle* h, Arena& ar, const double* Lp, const double* Ak
     const int64_t n1 = d * Drk;
     double* T1 = ar.take<double>(Dlb * wL * n1);
     if (!T1) return CT_ERR_OOM;
-    if (fp64_tc && ct_fp64_tc_enabled(h, wL * Dlb, n1, Dlk)) {
+    if (fp64_tc ? ct_fp64_tc_enabled(h, wL * Dlb, n1, Dlk) : ct_f64_route(h, wL * Dlb, n1, Dlk)) {
         // the same product as one GEMM over rows (wL, Dlb): A(r, k) = L[wL][k][Dlb],
         // B(n, k) = Ak[k][n], C row (wL, Dlb) at T1[Dlb][wL][.]
         const OzMat a{Lp, Dlb, Dlk * Dlb, 1, Dlb};
         const OzMat b{Ak, n1, 0, 1, n1};
         const OzOut c{T1, Dlb, n1, wL * n1};
-        CT_TRY(ct_oz_gemm_ex(h, wL * Dlb, n1, Dlk, a, b, 1.0, 0.0, c));
+        CT_TRY(fp64_tc ? ct_oz_gemm_ex(h, wL * Dlb, n1, Dlk, a, b, 1.0, 0.0, c) : ct_f64_gemm(h, wL * Dlb, n1, Dlk, a, b, c));
     } else {   // T1[Dlb, wL, (s Drk)] = sum_Dlk L[wL, Dlk, Dlb] Ak[Dlk, (s Drk)]; batch wL
         GemmDesc g{};
         g.M = Dlb; g.N = n1; g.K = Dlk;
@@ -143,12 +156,12 @@ int ct_env_left2_run(ct_handle* h, Arena& ar, const double* Lp, const double* Ak
         CT_TRY(ct_mpo_apply_f64_launch(h, m));
         T2 = T2w;
     }
-    if (fp64_tc && ct_fp64_tc_enabled(h, wR * Drk, Drb, Dlb * d)) {
+    if (fp64_tc ? ct_fp64_tc_enabled(h, wR * Drk, Drb, Dlb * d) : ct_f64_route(h, wR * Drk, Drb, Dlb * d)) {
         const int64_t M2 = wR * Drk;
         const OzMat a{T2, M2, 0, 1, M2};      // A(m, k) = T2[k][m]
         const OzMat b{Ab, Drb, 0, 1, Drb};    // B(n, k) = Ab[k][n]
         const OzOut c{Ln, M2, 0, Drb};
-        CT_TRY(ct_oz_gemm_ex(h, M2, Drb, Dlb * d, a, b, 1.0, 0.0, c));
+        CT_TRY(fp64_tc ? ct_oz_gemm_ex(h, M2, Drb, Dlb * d, a, b, 1.0, 0.0, c) : ct_f64_gemm(h, M2, Drb, Dlb * d, a, b, c));
     } else {   // Ln[(wR Drk), Drb] = sum_(Dlb s') T2[(Dlb s'), (wR Drk)] Ab[(Dlb s'), Drb]
         GemmDesc g{};
         g.M = wR * Drk; g.N = Drb; g.K = Dlb * d;
@@ -175,7 +188,13 @@ int ct_env_right_run(ct_handle* h, Arena& ar, int prec, const double* Rn, const 
     double* Wt = ar.take<double>((wL * d) * (wR * d));
     if (!T1 || !T2 || !Wt) return CT_ERR_OOM;
     CT_TRY(ct_build_wt_right(h, W, Wt, wL, d, wR));
-    {   // T1[Dr', wR, s, Dl] = sum_Dr R[wR, Dr, Dr'] A[Dl, s, Dr]; batch (wR, s)
+    if (ct_f64_route(h, wR * Dr, d * Dl, Dr)) {
+        // one GEMM over rows (wR, Dr') and columns (s, Dl)
+        const OzMat a{Rn, Dr, Dr * Dr, 1, Dr};
+        const OzMat b{A, Dl, Dr, d * Dr, 1};
+        const OzOut c{T1, Dr, d * Dl, wR * d * Dl};
+        CT_TRY(ct_f64_gemm(h, wR * Dr, d * Dl, Dr, a, b, c));
+    } else {   // T1[Dr', wR, s, Dl] = sum_Dr R[wR, Dr, Dr'] A[Dl, s, Dr]; batch (wR, s)
         GemmDesc g{};
         g.M = Dr; g.N = Dl; g.K = Dr;
         g.A = Rn; g.sAm = 1; g.sAk = Dr;
@@ -188,18 +207,23 @@ int ct_env_right_run(ct_handle* h, Arena& ar, int prec, const double* Rn, const 
         g.sC1 = d * Dl; g.sC0 = Dl;
         CT_TRY(ct_gemm_f64_launch(h, g));
     }
-    {   // T2[wL, Dl, s', Dr'] = sum_(wR s) Wt[(wL s'), (wR s)] T1[Dr', (wR s), Dl]
+    {   // T2[wL, s', Dr', Dl] = sum_(wR s) Wt[(wL s'), (wR s)] T1[Dr', (wR s), Dl]
         MpoDesc m{};
         m.O = Dr; m.K = wR * d; m.J = wL * d; m.I = Dl;
         m.in = T1; m.sIo = wR * d * Dl; m.sIk = Dl; m.sIi = 1;
-        m.out = T2; m.sOo = 1; m.sOi = d * Dr; m.J0 = d; m.sOj1 = Dl * d * Dr; m.sOj0 = Dr;
+        m.out = T2; m.sOo = Dl; m.sOi = 1; m.J0 = m.J; m.sOj1 = 0; m.sOj0 = Dr * Dl;
         m.Wt = Wt;
         CT_TRY(ct_mpo_apply_f64_launch(h, m));
     }
-    {   // Rp[wL, Dl, Dl'] = sum_(s' Dr') T2[wL, Dl, (s' Dr')] A[Dl', (s' Dr')]; batch wL
+    if (ct_f64_route(h, wL * Dl, Dl, d * Dr)) {
+        const OzMat a{T2, Dl, d * Dr * Dl, 1, Dl};
+        const OzMat b{A, Dl, 0, d * Dr, 1};
+        const OzOut c{Rp, wL * Dl, 0, Dl};
+        CT_TRY(ct_f64_gemm(h, wL * Dl, Dl, d * Dr, a, b, c));
+    } else {   // Rp[wL, Dl, Dl'] = sum_(s' Dr') T2[wL, (s' Dr'), Dl] A[Dl', (s' Dr')]; batch wL
         GemmDesc g{};
         g.M = Dl; g.N = Dl; g.K = d * Dr;
-        g.A = T2; g.sAm = d * Dr; g.sAk = 1;
+        g.A = T2; g.sAm = 1; g.sAk = Dl;
         g.B = A; g.sBk = 1; g.sBn = d * Dr;
         g.C = Rp; g.sCm = Dl; g.sCn = 1;
         g.alpha = 1.0; g.beta = 0.0; g.nb1 = wL; g.nb0 = 1;
@@ -223,6 +247,9 @@ int ct_theta_run(ct_handle* h, int prec, const double* Ai, const double* Aj, dou
         Arena ar(h);
         return ct_tc_gemm(h, ar, 0, 0, Dl * d, d * Dr, Dm, 1.0, Ai, Dm, Aj, d * Dr, 0.0, theta, d * Dr);
     }
+    if (ct_f64_route(h, Dl * d, d * Dr, Dm))
+        return ct_f64_gemm(h, Dl * d, d * Dr, Dm, OzMat{Ai, Dl * d, 0, Dm, 1}, OzMat{Aj, d * Dr, 0, 1, d * Dr},
+                           OzOut{theta, Dl * d, 0, d * Dr});
     GemmDesc g{};
     g.M = Dl * d; g.N = d * Dr; g.K = Dm;
     g.A = Ai; g.sAm = Dm; g.sAk = 1;

@@ -33,7 +33,8 @@ int ct_env_left_run(ct_handle* h, Arena& ar, int prec, const double* Lp, const d
 int ct_env_right_run(ct_handle* h, Arena& ar, int prec, const double* Rn, const double* A, const double* W,
                      double* Rp, int64_t Dl, int64_t d, int64_t Dr, int64_t wL, int64_t wR);
 size_t ct_env2_ws_bytes(int64_t Dlk, int64_t Dlb, int64_t d, int64_t Drk, int64_t Drb, int64_t wL, int64_t wR);
-// fp64_tc: the two large products on the BF16 tensor cores (ct_oz_gemm_ex, FP64-accurate)
+// fp64_tc: products from 2^21 multiply-adds on to the BF16 tensor cores (ct_oz_gemm_ex,
+// FP64-accurate), otherwise those that are faster there (ct_f64_route)
 int ct_env_left2_run(ct_handle* h, Arena& ar, const double* Lp, const double* Ak, const double* Ab,
                      const double* W, double* Ln, int64_t Dlk, int64_t Dlb, int64_t d, int64_t Drk, int64_t Drb,
                      int64_t wL, int64_t wR, bool fp64_tc = false);
@@ -93,6 +94,11 @@ struct OzOut {
 };
 int ct_oz_gemm_ex(ct_handle* h, int64_t M, int64_t N, int64_t K, const OzMat& A, const OzMat& B, double alpha,
                   double beta, const OzOut& C, int lower = 0);
+// FP64-form GEMM by residues (ct_f64mod.cu): whether a product of this size goes there (its
+// scratch is then in place), and the product
+bool ct_f64_route(ct_handle* h, int64_t M, int64_t N, int64_t K);
+int ct_f64_gemm(ct_handle* h, int64_t M, int64_t N, int64_t K, const OzMat& A, const OzMat& B, const OzOut& C,
+                const int* skip = nullptr);
 size_t ct_oz_gemm_ws_bytes(int64_t M, int64_t N, int64_t K);
 int ct_oz_gemm(ct_handle* h, int64_t M, int64_t N, int64_t K, const double* A, int64_t a_sr, int64_t a_sk,
                const double* B, int64_t b_sr, int64_t b_sk, double alpha, double beta, double* C, int64_t ldc,

@@ -16,7 +16,12 @@
  *     host scalar synchronise that stream.
  *
  * Precision forms (ct_prec):
- *   CT_PREC_FP64    plain form, FP64 everywhere.
+ *   CT_PREC_FP64    plain form, FP64 everywhere.  The contractions of H_eff,
+ *                   the environments, theta and the gradients form products
+ *                   that are large enough exactly, modulo 18 small integers on
+ *                   the BF16 tensor cores, from operands rounded to 2^-63 of
+ *                   each row's largest entry, and round them to FP64 once
+ *                   (CTDMRG_FP64_TC=0 keeps them on FP64 FMAs).
  *   CT_PREC_TF32X3  contractions on tcgen05 tensor cores in TF32 with
  *                   3xTF32 split compensation and FP32 accumulation; all
  *                   storage, Lanczos, eigensolve, SVD and reductions FP64.
@@ -233,8 +238,8 @@ CT_API int ct_mps_right_normalize(ct_handle* h, int nsites, int d, int64_t* bond
                            double* const* mps_sites);
 
 /* <psi|H|psi> and <psi|psi> through left environments on the device
- * (expectation_value, environments.mojo:475-532).  prec CT_PREC_FP64: SIMT
- * FP64 GEMMs; CT_PREC_FP64_TC: the environment GEMMs on the BF16 tensor
+ * (expectation_value, environments.mojo:475-532).  prec CT_PREC_FP64:
+ * FP64 products as above; CT_PREC_FP64_TC: the environment GEMMs on the BF16 tensor
  * cores with FP64-accurate slicing (the mixed form's final Rayleigh
  * quotient); CT_PREC_TF32X3 is taken as CT_PREC_FP64.                       */
 CT_API int ct_mps_expectation(ct_handle* h, int prec, int nsites, int d, const int64_t* mpo_dims,
