@@ -5,9 +5,13 @@
 // the path (dense_tensor_dot, dense_tensor.mojo:963-1328, and the permute +
 // GEMM chains of dmrg.mojo:254-374 / environments.mojo:99-417) is one launch
 // with the permutes folded into the operand addressing -- no physical
-// transposes.  FP64 on GB300 issues at a small fraction of the FP32 rate, so
-// a 64x64x16 smem tile with a 4x4 register block already saturates the FP64
-// pipe; the tensor-core path lives in ct_tc.cu.
+// transposes.  FP64 on GB300 issues at a small fraction of the FP32 rate (one
+// warp instruction per 64 clocks and SM quarter), so a 64x64x16 smem tile with
+// a 4x4 register block saturates the FP64 pipe of a product that fills the
+// GPU; the others are spread as thin as one warp per SM quarter.  The
+// tensor-core paths live in ct_tc.cu and ct_f64mod.cu.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 
 #include "ct_common.cuh"
@@ -17,9 +21,7 @@ namespace {
 constexpr int BK = 16;
 
 // One CTA computes a TBM x TBN tile of C with (TBM/4) x (TBN/4) threads, each
-// holding a 4 x 4 register block.  The 64 x 64 tile is the default; the
-// 32 x 32 tile gives small problems (the factorisation's panels) enough CTAs
-// to occupy every SM's FP64 pipe.
+// holding a 4 x 4 register block.
 template <int TBM, int TBN, bool A_K_CONTIG, bool B_N_CONTIG>
 __global__ void __launch_bounds__((TBM / 4) * (TBN / 4)) gemm_f64_kernel(GemmDesc g) {
     constexpr int NT = (TBM / 4) * (TBN / 4);
@@ -107,6 +109,116 @@ __global__ void __launch_bounds__((TBM / 4) * (TBN / 4)) gemm_f64_kernel(GemmDes
     }
 }
 
+// Products too small to fill the GPU with 64 x 64 tiles: an 8 x 16 tile per CTA, one element of
+// C per thread, four warps.  What bounds it is a thread's own chain of FMAs, which issue at one
+// per 64 clocks whether one element or sixteen are held per thread, so the elements go to as many
+// SM quarters as there are (32 x 32 tiles of two warps with 4 x 4 registers before: 16 elements
+// per thread in a row, on an eighth of the SMs).  The next K block is loaded to registers while
+// this one is computed.  Every element adds its products in the order of k, and the K pieces in
+// the order of the pieces, as the 64 x 64 kernel and splitk_reduce_kernel do; up to SP_MAXC
+// pieces are one cluster, whose first CTA adds them up, without scratch memory or a second launch.
+// Triangular forms keep the 32-wide granularity of what is skipped (TRI).
+// Measured (us per call, 32 x 32 tiles / here): 9x17x33 33 / 16, 128x32x96 27 / 16, 64x64x512
+// 29 / 20, 33x300x1000 84 / 33, 24x24x100000 414 / 152, 512x512x512 306 / 232, 1024x1024x64
+// 127 / 119.
+constexpr int SP_M = 8, SP_N = 16, SP_K = 32, SP_NT = SP_M * SP_N;
+constexpr int SP_MAXC = 8;
+constexpr int TRI = 32;
+
+template <bool A_K_CONTIG, bool B_N_CONTIG>
+__global__ void __launch_bounds__(SP_NT) gemm_f64_spread_kernel(GemmDesc g, int clustered) {
+    if (ct_skip(g.skip)) return;
+    __shared__ double As[SP_K][SP_M + 1];
+    __shared__ double Bs[SP_K][SP_N + 1];
+    __shared__ double piece[SP_MAXC][SP_NT];
+    const int ks = (int)((int64_t)blockIdx.z % g.ksplit);
+    const int64_t bz = (int64_t)blockIdx.z / g.ksplit;
+    const int64_t b1 = bz / g.nb0, b0 = bz % g.nb0;
+    const double* A = g.A + b1 * g.sA1 + b0 * g.sA0;
+    const double* B = g.B + b1 * g.sB1 + b0 * g.sB0;
+    const int64_t m0 = (int64_t)blockIdx.y * SP_M, n0 = (int64_t)blockIdx.x * SP_N;
+    const int64_t mt = m0 / TRI * TRI;
+    if (g.tri == 1 && n0 / TRI * TRI >= mt + TRI) return;   // the whole cluster
+    int64_t kend = (g.tri == 2 && mt + TRI < g.K) ? mt + TRI : g.K;
+    int64_t kbeg = 0;
+    if (g.ksplit > 1) {
+        const int64_t chunk = ((g.K + g.ksplit - 1) / g.ksplit + BK - 1) / BK * BK;
+        kbeg = ks * chunk;
+        if (kbeg + chunk < kend) kend = kbeg + chunk;
+    }
+    const int tid = threadIdx.x, tx = tid % SP_N, ty = tid / SP_N;
+    constexpr int NA = SP_M * SP_K / SP_NT, NB = SP_N * SP_K / SP_NT;
+    int am[NA], ak[NA], bn[NB], bk[NB];
+    const double *pa[NA], *pb[NB];
+#pragma unroll
+    for (int r = 0; r < NA; ++r) {
+        const int e = tid + SP_NT * r;
+        if (A_K_CONTIG) { ak[r] = e % SP_K; am[r] = e / SP_K; }
+        else            { am[r] = e % SP_M; ak[r] = e / SP_M; }
+        pa[r] = m0 + am[r] < g.M ? A + (m0 + am[r]) * g.sAm + (kbeg + ak[r]) * g.sAk : nullptr;
+    }
+#pragma unroll
+    for (int r = 0; r < NB; ++r) {
+        const int e = tid + SP_NT * r;
+        if (B_N_CONTIG) { bn[r] = e % SP_N; bk[r] = e / SP_N; }
+        else            { bk[r] = e % SP_K; bn[r] = e / SP_K; }
+        pb[r] = n0 + bn[r] < g.N ? B + (n0 + bn[r]) * g.sBn + (kbeg + bk[r]) * g.sBk : nullptr;
+    }
+    double ra[NA], rb[NB];
+    auto load = [&](int64_t k0) {
+#pragma unroll
+        for (int r = 0; r < NA; ++r) {
+            ra[r] = (pa[r] && k0 + ak[r] < kend) ? *pa[r] : 0.0;
+            if (pa[r]) pa[r] += SP_K * g.sAk;
+        }
+#pragma unroll
+        for (int r = 0; r < NB; ++r) {
+            rb[r] = (pb[r] && k0 + bk[r] < kend) ? *pb[r] : 0.0;
+            if (pb[r]) pb[r] += SP_K * g.sBk;
+        }
+    };
+    double acc = 0.0;
+    if (kbeg < kend) load(kbeg);
+    for (int64_t k0 = kbeg; k0 < kend; k0 += SP_K) {
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < NA; ++r) As[ak[r]][am[r]] = ra[r];
+#pragma unroll
+        for (int r = 0; r < NB; ++r) Bs[bk[r]][bn[r]] = rb[r];
+        __syncthreads();
+        if (k0 + SP_K < kend) load(k0 + SP_K);
+        const int kn = kend - k0 < SP_K ? (int)(kend - k0) : SP_K;
+#pragma unroll 1
+        for (int kk = 0; kk < kn; kk += 8) {
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                // (the rows from kn on hold zeros)
+                if (u < 4 || kk + u < kn) acc = fma(As[kk + u][ty], Bs[kk + u][tx], acc);
+            }
+        }
+    }
+    const int64_t gm = m0 + ty, gn = n0 + tx;
+    if (g.ksplit > 1) {
+        if (clustered) {
+            namespace cg = cooperative_groups;
+            cg::cluster_group cl = cg::this_cluster();
+            *cl.map_shared_rank(&piece[ks][tid], 0) = acc;
+            cl.sync();
+            if (ks != 0) return;
+            acc = 0.0;
+            for (int64_t i = 0; i < g.ksplit; ++i) acc += piece[i][tid];
+        } else if (gm < g.M && gn < g.N) {
+            g.part[(ks * g.M + gm) * g.N + gn] = acc;
+            return;
+        }
+    }
+    if (gm >= g.M || gn >= g.N) return;
+    double* c = g.C + b1 * g.sC1 + b0 * g.sC0 + gm * g.sCm + gn * g.sCn;
+    double v = g.alpha * acc;
+    if (g.beta != 0.0) v = fma(g.beta, *c, v);
+    *c = v;
+}
+
 // C = alpha * sum_ks part[ks] + beta * C, the partial sums added in a fixed
 // order (deterministic); tiles the GEMM kernel skips (tri == 1) stay untouched.
 __global__ void splitk_reduce_kernel(GemmDesc g, int tile) {
@@ -138,11 +250,37 @@ int launch_tiles(ct_handle* h, const GemmDesc& g, int64_t nb) {
     else if (bn) { gemm_f64_kernel<TBM, TBN, false, true><<<grid, nt, 0, h->stream>>>(g); ct_note_launch(); }
     else { gemm_f64_kernel<TBM, TBN, false, false><<<grid, nt, 0, h->stream>>>(g); ct_note_launch(); }
     CT_LAUNCH_CHECK(h);
-    if (g.ksplit > 1) {
+    return CT_OK;
+}
+
+int launch_spread(ct_handle* h, const GemmDesc& g, int64_t nb) {
+    // (the limits of 32 x 32 tiles)
+    const int64_t ym = ct_cdiv(g.M, SP_M), z = nb * g.ksplit;
+    if (ym > 65535 || z > 65535) {
+        ct_seterr(h, "gemm grid too large (M=%lld nb=%lld)", (long long)g.M, (long long)nb);
+        return CT_ERR_UNSUPPORTED;
+    }
+    const bool clustered = g.ksplit > 1 && g.ksplit <= SP_MAXC;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)ct_cdiv(g.N, SP_N), (unsigned)ym, (unsigned)z);
+    cfg.blockDim = dim3(SP_NT);
+    cfg.stream = h->stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim = {1, 1, (unsigned)g.ksplit};
+    if (clustered) {
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+    }
+    const bool ak = (g.sAk == 1), bn = (g.sBn == 1);
+    auto* f = ak ? (bn ? gemm_f64_spread_kernel<true, true> : gemm_f64_spread_kernel<true, false>)
+                 : (bn ? gemm_f64_spread_kernel<false, true> : gemm_f64_spread_kernel<false, false>);
+    CT_CUDA(h, cudaLaunchKernelEx(&cfg, f, g, (int)clustered)); ct_note_launch();
+    if (g.ksplit > 1 && !clustered) {
         const int64_t tot = g.M * g.N;
         int64_t blocks = ct_cdiv(tot, 256);
         if (blocks > 4 * (int64_t)h->num_sms) blocks = 4 * (int64_t)h->num_sms;
-        splitk_reduce_kernel<<<(unsigned)blocks, 256, 0, h->stream>>>(g, TBM); ct_note_launch();
+        splitk_reduce_kernel<<<(unsigned)blocks, 256, 0, h->stream>>>(g, TRI); ct_note_launch();
         CT_LAUNCH_CHECK(h);
     }
     return CT_OK;
@@ -159,9 +297,9 @@ int ct_gemm_f64_launch(ct_handle* h, const GemmDesc& g) {
     gg.ksplit = 1;
     gg.part = nullptr;
     const int64_t sms = h->num_sms;
-    // the FP64 pipe of one SM bounds a CTA here, so the launch needs at least
-    // one CTA per SM: 64 x 64 tiles when there are two per SM, else 32 x 32
-    // tiles, with K split over the idle SMs when even those are too few
+    // 64 x 64 tiles when there are two per SM: they fill the FP64 pipes (1024 x 1024 x 64 is the
+    // largest below, 127 us on 32 x 32 tiles and 119 spread); else the spread form, with K split
+    // over the idle SMs when there is less than one 32 x 32 block of C for each
     // tiles that do work (tri == 1 skips those strictly above the diagonal)
     auto active = [&](int64_t t) {
         const int64_t tm = ct_cdiv(g.M, t), tn = ct_cdiv(g.N, t);
@@ -170,8 +308,6 @@ int ct_gemm_f64_launch(ct_handle* h, const GemmDesc& g) {
         for (int64_t i = 0; i < tm; ++i) a += std::min<int64_t>(tn, i + 1);
         return a * nb;
     };
-    // (measured: 32 x 32 tiles, several CTAs per SM, beat 64 x 64 tiles with
-    // split K on a 1024 x 1024 x 2048 lower-only product, 2.7 vs 3.1 ms)
     if (active(64) >= 2 * sms) return launch_tiles<64, 64>(h, gg, nb);
     const int64_t tiles = active(32);
     if (nb == 1 && tiles < sms && g.K >= 64) {
@@ -186,7 +322,7 @@ int ct_gemm_f64_launch(ct_handle* h, const GemmDesc& g) {
                 gg.part = h->splitk_fixed;
             }
         } else if (ks > 1) {
-            const size_t need = (size_t)(ks * g.M * g.N);
+            const size_t need = ks > SP_MAXC ? (size_t)(ks * g.M * g.N) : 0;
             if (h->splitk_cap < need) {
                 if (h->splitk) cudaFree(h->splitk);
                 h->splitk = nullptr;
@@ -198,5 +334,5 @@ int ct_gemm_f64_launch(ct_handle* h, const GemmDesc& g) {
             gg.part = h->splitk;
         }
     }
-    return launch_tiles<32, 32>(h, gg, nb);
+    return launch_spread(h, gg, nb);
 }
