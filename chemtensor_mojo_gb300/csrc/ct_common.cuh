@@ -211,6 +211,26 @@ __device__ __forceinline__ double ct_block_sum(double v, double* sm) {
 // the same rank and parts of the permutation are never written.
 __device__ __forceinline__ double ct_rank_key(double s) { return isnan(s) ? -INFINITY : s; }
 
+// (float)x and (double)x, bit for bit, as integer work where the result and the operand are normal
+// or zero: the conversion instructions issue at the FP64 rate, 1/64 of the integer rate.
+__device__ __forceinline__ float ct_d2f(double x) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    const unsigned e = hi & 0x7ff00000u;
+    if (e - (897u << 20) <= (253u << 20)) {   // 2^-126 <= |x| < 2^128
+        unsigned u = __funnelshift_l(lo, hi, 3) - (384u << 23);          // 9 bits of exponent, 23 of mantissa
+        u += (((lo << 3) | (u & 1u)) > 0x80000000u) ? 1u : 0u;           // the other 29: to nearest, ties to even
+        return __uint_as_float(u | (hi & 0x80000000u));
+    }
+    if (((hi << 1) | lo) == 0) return __uint_as_float(hi);
+    return (float)x;
+}
+__device__ __forceinline__ double ct_f2d(float f) {
+    const unsigned u = __float_as_uint(f), a = u & 0x7fffffffu;
+    if (a - 0x00800000u < 0x7f000000u) return __hiloint2double((int)((u & 0x80000000u) | ((a >> 3) + (896u << 20))), (int)(u << 29));
+    if (a == 0) return __hiloint2double((int)u, 0);
+    return (double)f;
+}
+
 __device__ __forceinline__ void ct_set_status(int* st, int code) {
     if (st) atomicCAS(st, 0, code);
 }

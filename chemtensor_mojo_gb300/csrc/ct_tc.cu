@@ -21,6 +21,7 @@
 #include <stdlib.h>
 
 #include <algorithm>
+#include <initializer_list>
 #include <new>
 
 #include "ct_ops.cuh"
@@ -946,54 +947,88 @@ struct PackDesc {
     int64_t K1, K0, K0p, s_k1, s_k0;
     float* hi;
     float* lo;
-    int64_t ldk;   // = K1 * K0p rounded up to 32
-    double scale;
-    const double* scale_ptr;   // optional device scalar multiplier
+    int64_t ldk;      // = K1 * K0p rounded up to 32
+    int k_fast;       // source contiguous along k0, else along r0
+};
+constexpr int PACK_MAX = 3;
+struct PackBatch {
+    PackDesc d[PACK_MAX];
+    int64_t first[PACK_MAX + 1];   // first block of each operand
+    int n;
 };
 
-// 32 x 32 tiles through shared memory; K_FAST: source contiguous along k0.
-// The tile's 32 row offsets and 32 column offsets are computed once per block
-// (the 64-bit divisions of the index split would otherwise dominate).
-template <bool K_FAST>
-__global__ void __launch_bounds__(256) pack_split_kernel(PackDesc p, const int* skip) {
+// Up to PACK_MAX operands in one launch; 32 rows x 64 k per block.  What bounds it is memory:
+// 8 bytes in and 8 out per element.  Each thread has its 8 loads in flight at once, the rounding to
+// FP32 is integer work (a conversion instruction issues at the FP64 rate, 9 us of the 25 that
+// 5 x 1024 x 1024 took), and the planes are stored 16 bytes at a time.  The tile's row and column
+// offsets are computed once per block (the 64-bit divisions of the index split would otherwise
+// dominate).  Measured (us, 32 x 32 tiles, one launch per operand / here): L and R of H_eff
+// at chi 1024, d 2, w 5: 48 / 29 (5.8 TB/s), theta 19 / 13.
+__global__ void __launch_bounds__(256) pack_split_kernel(const __grid_constant__ PackBatch pb, const int* skip) {
     if (ct_skip(skip)) return;
-    __shared__ double tile[32][33];
-    __shared__ int64_t roff[32], koff[32];
-    const int64_t rb = (int64_t)blockIdx.y * 32;
-    const int64_t kb = (int64_t)blockIdx.x * 32;   // in padded k space
-    const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
-    if (ty == 0) {
-        const int64_t r = rb + tx;
-        roff[tx] = (r < p.rows) ? (r / p.R0) * p.s_r1 + (r % p.R0) * p.s_r0 : -1;
-    } else if (ty == 1) {
-        const int64_t k = kb + tx;
-        int64_t o = -1;
+    __shared__ float tile[64][33];
+    __shared__ int64_t roff[32], koff[64];
+    int o = 0;
+    while (o + 1 < pb.n && (int64_t)blockIdx.x >= pb.first[o + 1]) ++o;
+    const PackDesc& p = pb.d[o];
+    const int64_t blk = (int64_t)blockIdx.x - pb.first[o], nk = (p.ldk + 63) / 64;
+    const int64_t rb = blk / nk * 32, kb = blk % nk * 64;   // k in padded space
+    const int tid = threadIdx.x, lane = tid % 32, warp = tid / 32;
+    if (tid < 32) {
+        const int64_t r = rb + tid;
+        roff[tid] = (r < p.rows) ? (r / p.R0) * p.s_r1 + (r % p.R0) * p.s_r0 : -1;
+    } else if (tid < 96) {
+        const int64_t k = kb + tid - 32;
+        int64_t of = -1;
         if (k < p.ldk) {
             const int64_t k1 = k / p.K0p, k0 = k % p.K0p;
-            if (k1 < p.K1 && k0 < p.K0) o = k1 * p.s_k1 + k0 * p.s_k0;
+            if (k1 < p.K1 && k0 < p.K0) of = k1 * p.s_k1 + k0 * p.s_k0;
         }
-        koff[tx] = o;
-    }
-    double scd = p.scale;
-    if (p.scale_ptr) scd *= *p.scale_ptr;
-    const float sc = (float)scd;
-    __syncthreads();
-    for (int i = ty; i < 32; i += 8) {
-        const int ri = K_FAST ? i : tx, ki = K_FAST ? tx : i;
-        const int64_t ro = roff[ri], ko = koff[ki];
-        const double v = (ro >= 0 && ko >= 0) ? p.src[ro + ko] : 0.0;
-        if (K_FAST) tile[i][tx] = v;
-        else tile[tx][i] = v;
+        koff[tid - 32] = of;
     }
     __syncthreads();
-    for (int i = ty; i < 32; i += 8) {
-        const int64_t r = rb + i, k = kb + tx;
-        if (r < p.rows && k < p.ldk) {
-            float h, l;
-            split_tf32((float)tile[i][tx] * sc, h, l);
-            p.hi[r * p.ldk + k] = h;
-            p.lo[r * p.ldk + k] = l;
+    double v[8];
+    if (p.k_fast) {
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int64_t ro = roff[warp * 4 + u / 2], ko = koff[lane + 32 * (u & 1)];
+            v[u] = (ro >= 0 && ko >= 0) ? p.src[ro + ko] : 0.0;
         }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) tile[lane + 32 * (u & 1)][warp * 4 + u / 2] = ct_d2f(v[u]);
+    } else {
+        const int64_t ro = roff[lane];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const int64_t ko = koff[warp + 8 * u];
+            v[u] = (ro >= 0 && ko >= 0) ? p.src[ro + ko] : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) tile[warp + 8 * u][lane] = ct_d2f(v[u]);
+    }
+    __syncthreads();
+    // (ldk is a multiple of 32)
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+        const int r = (lane / 8) + 4 * warp, k = (lane % 8) * 4 + 32 * u;
+        if (rb + r >= p.rows || kb + k >= p.ldk) continue;
+        float4 hv, lv;
+        split_tf32(tile[k + 0][r], hv.x, lv.x);
+        split_tf32(tile[k + 1][r], hv.y, lv.y);
+        split_tf32(tile[k + 2][r], hv.z, lv.z);
+        split_tf32(tile[k + 3][r], hv.w, lv.w);
+        *reinterpret_cast<float4*>(p.hi + (rb + r) * p.ldk + kb + k) = hv;
+        *reinterpret_cast<float4*>(p.lo + (rb + r) * p.ldk + kb + k) = lv;
+    }
+}
+
+// zeros in columns [k0, k0 + n) of the 2 planes' rows (the MPO legs write the others)
+__global__ void __launch_bounds__(256) pad_zero_kernel(float* hi, float* lo, int64_t rows, int64_t ld, int64_t k0, int n) {
+    const int64_t total = rows * n;
+    for (int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x; t < total; t += (int64_t)gridDim.x * 256) {
+        const int64_t at = t / n * ld + k0 + t % n;
+        hi[at] = 0.f;
+        lo[at] = 0.f;
     }
 }
 
@@ -1469,27 +1504,53 @@ int tc_gemm_launch(ct_handle* h, const SplitOperand& A, const SplitOperand& B, i
     return CT_OK;
 }
 
-int pack_launch(ct_handle* h, const PackDesc& p, bool k_fast, const int* skip) {
-    if (p.rows <= 0 || p.ldk <= 0) return CT_OK;
-    dim3 grid((unsigned)ct_cdiv(p.ldk, 32), (unsigned)ct_cdiv(p.rows, 32));
-    if (grid.y > 65535) return CT_ERR_UNSUPPORTED;
-    dim3 block(32, 8);
-    if (k_fast) { pack_split_kernel<true><<<grid, block, 0, h->stream>>>(p, skip); ct_note_launch(); }
-    else { pack_split_kernel<false><<<grid, block, 0, h->stream>>>(p, skip); ct_note_launch(); }
+int pack_launch(ct_handle* h, std::initializer_list<PackDesc> ops, const int* skip) {
+    PackBatch pb{};
+    for (const PackDesc& p : ops) {
+        if (p.rows <= 0 || p.ldk <= 0) continue;
+        if (ct_cdiv(p.rows, 32) > 65535) return CT_ERR_UNSUPPORTED;
+        pb.d[pb.n] = p;
+        pb.first[pb.n + 1] = pb.first[pb.n] + ct_cdiv(p.rows, 32) * ct_cdiv(p.ldk, 64);
+        ++pb.n;
+    }
+    if (pb.n == 0) return CT_OK;
+    if (pb.first[pb.n] > 0x7fffffff) return CT_ERR_UNSUPPORTED;
+    pack_split_kernel<<<(unsigned)pb.first[pb.n], 256, 0, h->stream>>>(pb, skip); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }
 
-// Plain 2-level-row, 1-level-k pack helper.
+// Plain 2-level-row, 1-level-k pack.
 PackDesc pack_desc(const double* src, int64_t rows, int64_t R0, int64_t s_r1, int64_t s_r0, int64_t K, int64_t s_k,
-                   const SplitOperand& dst) {
+                   const SplitOperand& dst, bool k_fast) {
     PackDesc p{};
     p.src = src;
     p.rows = rows; p.R0 = R0; p.s_r1 = s_r1; p.s_r0 = s_r0;
     p.K1 = 1; p.K0 = K; p.K0p = dst.ldk; p.s_k1 = 0; p.s_k0 = s_k;
     p.hi = dst.hi; p.lo = dst.lo; p.ldk = dst.ldk;
-    p.scale = 1.0; p.scale_ptr = nullptr;
+    p.k_fast = k_fast;
     return p;
+}
+
+// R[wR, Dr, Dr'] -> rows Dr', k = (wR, Dr) with per-wR padding to Drp
+PackDesc pack_desc_r4(const double* R, int64_t Dr, int64_t wR, int64_t Drp, const SplitOperand& dst) {
+    PackDesc p{};
+    p.src = R;
+    p.rows = Dr; p.R0 = Dr; p.s_r1 = 0; p.s_r0 = 1;
+    p.K1 = wR; p.K0 = Dr; p.K0p = Drp; p.s_k1 = Dr * Dr; p.s_k0 = Dr;
+    p.hi = dst.hi; p.lo = dst.lo; p.ldk = dst.ldk;
+    return p;
+}
+
+// Zeros in an operand's padding columns, which the MPO legs do not write: columns [k0, period) of
+// every period (nothing when there are none).
+int pad_zero(ct_handle* h, const SplitOperand& s, int64_t period, int64_t k0) {
+    if (k0 >= period) return CT_OK;
+    const int64_t rows = s.rows * (s.ldk / period);
+    const int64_t blocks = std::min<int64_t>(ct_cdiv(rows * (period - k0), 256), 16 * (int64_t)h->num_sms);
+    pad_zero_kernel<<<(unsigned)blocks, 256, 0, h->stream>>>(s.hi, s.lo, rows, period, k0, (int)(period - k0)); ct_note_launch();
+    CT_LAUNCH_CHECK(h);
+    return CT_OK;
 }
 
 template <int JT>
@@ -1603,21 +1664,10 @@ int ct_tc_heff_prepare(ct_handle* h, Arena& ar, HeffPlan& p) {
     q.W12 = ar.take<double>((size_t)((d * d * wR) * (wL * d * d)));
     if (!q.Lp.lo || !q.R4.lo || !q.th.lo || !q.A4.lo || !q.T1 || !q.W12) return CT_ERR_OOM;
     CT_TRY(ct_build_w12(h, p.W1, p.W2, q.W12, wL, d, wM, wR));
-    // L[wL, Dl, Dl'] -> Lp[(wL, Dl')][Dl]
-    CT_TRY(pack_launch(h, pack_desc(p.L, wL * Dl, Dl, Dl * Dl, 1, Dl, Dl, q.Lp), false, nullptr));
-    // R[wR, Dr, Dr'] -> R4[Dr'][(wR, Dr)] with per-wR padding
-    {
-        PackDesc pd{};
-        pd.src = p.R;
-        pd.rows = Dr; pd.R0 = Dr; pd.s_r1 = 0; pd.s_r0 = 1;
-        pd.K1 = wR; pd.K0 = Dr; pd.K0p = q.Dr_pad; pd.s_k1 = Dr * Dr; pd.s_k0 = Dr;
-        pd.hi = q.R4.hi; pd.lo = q.R4.lo; pd.ldk = wR * q.Dr_pad;
-        pd.scale = 1.0;
-        CT_TRY(pack_launch(h, pd, false, nullptr));
-    }
-    // padding columns of A4 are never written by the MPO leg: zero them once
-    CT_CUDA(h, cudaMemsetAsync(q.A4.hi, 0, (size_t)(q.A4.rows * q.A4.ldk) * 4, h->stream));
-    CT_CUDA(h, cudaMemsetAsync(q.A4.lo, 0, (size_t)(q.A4.rows * q.A4.ldk) * 4, h->stream));
+    // L[wL, Dl, Dl'] -> Lp[(wL, Dl')][Dl], and R
+    CT_TRY(pack_launch(h, {pack_desc(p.L, wL * Dl, Dl, Dl * Dl, 1, Dl, Dl, q.Lp, false),
+                           pack_desc_r4(p.R, Dr, wR, q.Dr_pad, q.R4)}, nullptr));
+    CT_TRY(pad_zero(h, q.A4, q.Dr_pad, Dr));
     p.tc = &q;
     return CT_OK;
 }
@@ -1627,7 +1677,7 @@ int ct_tc_heff_run(ct_handle* h, const HeffPlan& p, const double* theta, double*
     const int64_t Dl = p.Dl, d = p.d, Dr = p.Dr, wL = p.wL, wR = p.wR;
     const int64_t n1 = d * d * Dr;
     // theta[Dl, n1] -> th[n1][Dl]
-    CT_TRY(pack_launch(h, pack_desc(theta, n1, n1, 0, 1, Dl, n1, q.th), false, skip));
+    CT_TRY(pack_launch(h, {pack_desc(theta, n1, n1, 0, 1, Dl, n1, q.th, false)}, skip));
     {   // T1[Dl'][wL][n1] (fp32) = Lp . th^T
         TcEpi e{};
         e.C = q.T1; e.out_fp64 = 0; e.M0 = Dl; e.sCm1 = n1; e.sCm0 = wL * n1; e.alpha = 1.0; e.beta = 0.0;
@@ -1673,26 +1723,15 @@ int ct_tc_heff1_run(ct_handle* h, Arena& ar, const double* L, const double* A, c
     double* Wt = ar.take<double>((size_t)((d * wr) * (wl * d)));
     if (!Lp.lo || !R4.lo || !th.lo || !A4.lo || !T1 || !Wt) return CT_ERR_OOM;
     CT_TRY(ct_build_wt_left(h, W, Wt, wl, d, wr));
-    // L[wl, Dl, Dl'] -> Lp[(wl, Dl')][Dl]
-    CT_TRY(pack_launch(h, pack_desc(L, wl * Dl, Dl, Dl * Dl, 1, Dl, Dl, Lp), false, nullptr));
-    {   // R[wr, Dr, Dr'] -> R4[Dr'][(wr, Dr)] with per-wr padding
-        PackDesc pd{};
-        pd.src = R;
-        pd.rows = Dr; pd.R0 = Dr; pd.s_r1 = 0; pd.s_r0 = 1;
-        pd.K1 = wr; pd.K0 = Dr; pd.K0p = Drp; pd.s_k1 = Dr * Dr; pd.s_k0 = Dr;
-        pd.hi = R4.hi; pd.lo = R4.lo; pd.ldk = K4;
-        pd.scale = 1.0;
-        CT_TRY(pack_launch(h, pd, false, nullptr));
-    }
-    // A[Dl, (s Dr)] -> th[(s Dr)][Dl]
-    CT_TRY(pack_launch(h, pack_desc(A, n1, n1, 0, 1, Dl, n1, th), false, nullptr));
+    // L[wl, Dl, Dl'] -> Lp[(wl, Dl')][Dl], R, A[Dl, (s Dr)] -> th[(s Dr)][Dl]
+    CT_TRY(pack_launch(h, {pack_desc(L, wl * Dl, Dl, Dl * Dl, 1, Dl, Dl, Lp, false), pack_desc_r4(R, Dr, wr, Drp, R4),
+                           pack_desc(A, n1, n1, 0, 1, Dl, n1, th, false)}, nullptr));
     {   // T1[Dl'][wl][(s Dr)] (fp32) = Lp . th^T
         TcEpi e{};
         e.C = T1; e.out_fp64 = 0; e.M0 = Dl; e.sCm1 = n1; e.sCm0 = wl * n1; e.alpha = 1.0; e.beta = 0.0;
         CT_TRY(tc_gemm_launch(h, Lp, th, wl * Dl, n1, e, nullptr));
     }
-    CT_CUDA(h, cudaMemsetAsync(A4.hi, 0, (size_t)(A4.rows * A4.ldk) * 4, h->stream));
-    CT_CUDA(h, cudaMemsetAsync(A4.lo, 0, (size_t)(A4.rows * A4.ldk) * 4, h->stream));
+    CT_TRY(pad_zero(h, A4, Drp, Dr));
     {   // A4[(Dl' s')][(wr, Dr)] = Wt . T1
         MpoTcDesc m{};
         m.O = Dl; m.K = wl * d; m.J = d * wr; m.I = Dr;
@@ -1732,15 +1771,16 @@ int ct_tc_env_left_run(ct_handle* h, Arena& ar, const double* Lp, const double* 
     double* Wt = ar.take<double>((size_t)((d * wR) * (wL * d)));
     if (!La.lo || !Ab.lo || !T1 || !A3.lo || !B3.lo || !Wt) return CT_ERR_OOM;
     CT_TRY(ct_build_wt_left(h, W, Wt, wL, d, wR));
-    CT_TRY(pack_launch(h, pack_desc(Lp, wL * Dl, Dl, Dl * Dl, 1, Dl, Dl, La), false, nullptr));
-    CT_TRY(pack_launch(h, pack_desc(A, n1, n1, 0, 1, Dl, n1, Ab), false, nullptr));
+    // with B3[Dr'][(Dl' s')] = A[Dl', s', Dr']
+    CT_TRY(pack_launch(h, {pack_desc(Lp, wL * Dl, Dl, Dl * Dl, 1, Dl, Dl, La, false),
+                           pack_desc(A, n1, n1, 0, 1, Dl, n1, Ab, false),
+                           pack_desc(A, Dr, Dr, 0, 1, Dl * d, Dr, B3, false)}, nullptr));
     {   // T1[Dl'][wL][(s Dr)]
         TcEpi e{};
         e.C = T1; e.out_fp64 = 0; e.M0 = Dl; e.sCm1 = n1; e.sCm0 = wL * n1; e.alpha = 1.0;
         CT_TRY(tc_gemm_launch(h, La, Ab, wL * Dl, n1, e, nullptr));
     }
-    CT_CUDA(h, cudaMemsetAsync(A3.hi, 0, (size_t)(A3.rows * A3.ldk) * 4, h->stream));
-    CT_CUDA(h, cudaMemsetAsync(A3.lo, 0, (size_t)(A3.rows * A3.ldk) * 4, h->stream));
+    CT_TRY(pad_zero(h, A3, K3, Dl * d));
     {   // A3[(wR Dr)][(Dl' s')] = Wt . T1
         MpoTcDesc m{};
         m.O = Dl; m.K = wL * d; m.J = d * wR; m.I = Dr;
@@ -1749,8 +1789,6 @@ int ct_tc_env_left_run(ct_handle* h, Arena& ar, const double* Lp, const double* 
         m.Wt = Wt;
         CT_TRY(mpo_tc_launch(h, m));
     }
-    // B3[Dr'][(Dl' s')] = A[Dl', s', Dr']
-    CT_TRY(pack_launch(h, pack_desc(A, Dr, Dr, 0, 1, Dl * d, Dr, B3), false, nullptr));
     TcEpi e{};
     e.C = Ln; e.out_fp64 = 1; e.M0 = wR * Dr; e.sCm1 = 0; e.sCm0 = Dr; e.alpha = 1.0;
     return tc_gemm_launch(h, A3, B3, wR * Dr, Dr, e, nullptr);
@@ -1769,16 +1807,17 @@ int ct_tc_env_right_run(ct_handle* h, Arena& ar, const double* Rn, const double*
     if (!Ra.lo || !Ab.lo || !T1 || !A3.lo || !B3.lo || !Wt) return CT_ERR_OOM;
     CT_TRY(ct_build_wt_right(h, W, Wt, wL, d, wR));
     // R[wR, Dr, Dr'] -> Ra[(wR, Dr')][Dr]
-    CT_TRY(pack_launch(h, pack_desc(Rn, wR * Dr, Dr, Dr * Dr, 1, Dr, Dr, Ra), false, nullptr));
     // A[Dl, s, Dr] -> Ab[(s, Dl)][Dr]   (row n' = s*Dl + Dl_idx)
-    CT_TRY(pack_launch(h, pack_desc(A, d * Dl, Dl, Dr, d * Dr, Dr, 1, Ab), true, nullptr));
+    // B3[Dl'][(s' Dr')] = A natural layout
+    CT_TRY(pack_launch(h, {pack_desc(Rn, wR * Dr, Dr, Dr * Dr, 1, Dr, Dr, Ra, false),
+                           pack_desc(A, d * Dl, Dl, Dr, d * Dr, Dr, 1, Ab, true),
+                           pack_desc(A, Dl, Dl, 0, d * Dr, d * Dr, 1, B3, true)}, nullptr));
     {   // T1[Dr'][wR][s][Dl]
         TcEpi e{};
         e.C = T1; e.out_fp64 = 0; e.M0 = Dr; e.sCm1 = d * Dl; e.sCm0 = wR * d * Dl; e.alpha = 1.0;
         CT_TRY(tc_gemm_launch(h, Ra, Ab, wR * Dr, d * Dl, e, nullptr));
     }
-    CT_CUDA(h, cudaMemsetAsync(A3.hi, 0, (size_t)(A3.rows * A3.ldk) * 4, h->stream));
-    CT_CUDA(h, cudaMemsetAsync(A3.lo, 0, (size_t)(A3.rows * A3.ldk) * 4, h->stream));
+    CT_TRY(pad_zero(h, A3, K3, d * Dr));
     {   // A3[(wL Dl)][(s' Dr')] = Wt . T1
         MpoTcDesc m{};
         m.O = Dr; m.K = wR * d; m.J = wL * d; m.I = Dl;
@@ -1787,8 +1826,6 @@ int ct_tc_env_right_run(ct_handle* h, Arena& ar, const double* Rn, const double*
         m.Wt = Wt;
         CT_TRY(mpo_tc_launch(h, m));
     }
-    // B3[Dl'][(s' Dr')] = A natural layout
-    CT_TRY(pack_launch(h, pack_desc(A, Dl, Dl, 0, d * Dr, d * Dr, 1, B3), true, nullptr));
     TcEpi e{};
     e.C = Rp; e.out_fp64 = 1; e.M0 = wL * Dl; e.sCm1 = 0; e.sCm0 = Dl; e.alpha = 1.0;
     return tc_gemm_launch(h, A3, B3, wL * Dl, Dl, e, nullptr);
@@ -1812,11 +1849,10 @@ int ct_tc_gemm_ex(ct_handle* h, Arena& ar, int trans_a, int trans_b, int64_t m, 
     SplitOperand b = take_split(ar, n, kp);
     if (!a.lo || !b.lo) return CT_ERR_OOM;
     // op(A)[i, p]: trans_a=0 -> A[i*lda + p] (k contiguous), 1 -> A[p*lda + i]
-    CT_TRY(pack_launch(h, trans_a ? pack_desc(A, m, m, 0, 1, k, lda, a) : pack_desc(A, m, m, 0, lda, k, 1, a),
-                       !trans_a, nullptr));
     // op(B)[p, j]: trans_b=0 -> B[p*ldb + j] -> rows j, k stride ldb; 1 -> B[j*ldb + p]
-    CT_TRY(pack_launch(h, trans_b ? pack_desc(B, n, n, 0, ldb, k, 1, b) : pack_desc(B, n, n, 0, 1, k, ldb, b),
-                       trans_b != 0, nullptr));
+    CT_TRY(pack_launch(h, {trans_a ? pack_desc(A, m, m, 0, 1, k, lda, a, false) : pack_desc(A, m, m, 0, lda, k, 1, a, true),
+                           trans_b ? pack_desc(B, n, n, 0, ldb, k, 1, b, true) : pack_desc(B, n, n, 0, 1, k, ldb, b, false)},
+                       nullptr));
     TcEpi e{};
     e.C = C; e.out_fp64 = out_fp64; e.M0 = m; e.sCm1 = 0; e.sCm0 = ldc; e.alpha = alpha; e.beta = beta;
     return tc_gemm_launch(h, a, b, m, n, e, nullptr);
