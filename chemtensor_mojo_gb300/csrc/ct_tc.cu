@@ -1143,6 +1143,242 @@ __global__ void __launch_bounds__(MPOT_NT) mpo_tc2_kernel(MpoTcDesc m) {
     }
 }
 
+// The weights of output rows [jbeg, jbeg + jn) in shared memory, as FP32: a list of the non-zero
+// ones of each row with their k (times kstep) when they are less than half, else all of them,
+// MPO_RB rows together ([row block][k][MPO_RB]).  Hamiltonians' weights are mostly zeros: 30 of
+// the 400 of the fused XXZ bulk pair are not, 119 of the 9216 of Fermi-Hubbard's.  `region` holds
+// MPO_RB ceil(jn / MPO_RB) K floats, start jn + 1 ints, joff jn output offsets, stage jn K floats
+// that are free again afterwards.
+constexpr int MPO_RB = 32;
+__device__ bool mpo_weights(const MpoTcDesc& m, int64_t jbeg, int jn, int kstep, float* stage, float* region, int* start,
+                            int64_t* joff) {
+    const int nt = blockDim.x, tid = threadIdx.x, warp = tid / 32, lane = tid % 32, K = (int)m.K;
+#pragma unroll 8
+    for (int t = tid; t < jn * K; t += nt) stage[t] = ct_d2f(m.Wt[jbeg * K + t]);
+    for (int j = tid; j < jn; j += nt) {
+        const int64_t jj = jbeg + j;
+        joff[j] = (jj / m.J0) * m.sOj1 + (jj % m.J0) * m.sOj0;
+    }
+    __syncthreads();
+    for (int j = warp; j < jn; j += nt / 32) {
+        int n = 0;
+        for (int k = lane; k < K; k += 32) n += (__float_as_uint(stage[j * K + k]) << 1) != 0;
+        n = __reduce_add_sync(0xffffffffu, n);
+        if (lane == 0) start[j + 1] = n;
+    }
+    __syncthreads();
+    if (warp == 0) {   // prefix sums of the rows' counts
+        int base = 0;
+        for (int j0 = 0; j0 < jn; j0 += 32) {
+            int v = j0 + lane < jn ? start[j0 + lane + 1] : 0;
+#pragma unroll
+            for (int off = 1; off < 32; off *= 2) {
+                const int u = __shfl_up_sync(0xffffffffu, v, off);
+                if (lane >= off) v += u;
+            }
+            if (j0 + lane < jn) start[j0 + lane + 1] = base + v;
+            base += __shfl_sync(0xffffffffu, v, 31);
+        }
+        if (lane == 0) start[0] = 0;
+    }
+    __syncthreads();
+    const bool sparse = 2 * start[jn] <= jn * K;
+    if (sparse) {
+        float2* list = reinterpret_cast<float2*>(region);
+        if (start[jn] == 0 && tid == 0) list[0] = make_float2(0.f, 0.f);   // (read, not used)
+        for (int j = warp; j < jn; j += nt / 32) {
+            int n = start[j];
+            for (int k0 = 0; k0 < K; k0 += 32) {
+                const float w = k0 + lane < K ? stage[j * K + k0 + lane] : 0.f;
+                const bool nz = (__float_as_uint(w) << 1) != 0;
+                const unsigned mask = __ballot_sync(0xffffffffu, nz);
+                if (nz) list[n + __popc(mask & ((1u << lane) - 1))] = make_float2(w, __int_as_float((k0 + lane) * kstep));
+                n += __popc(mask);
+            }
+        }
+    } else {
+        const int jp = (jn + MPO_RB - 1) / MPO_RB * MPO_RB;
+        for (int t = tid; t < jp * K; t += nt) {
+            const int jj = t % MPO_RB, k = t / MPO_RB % K, j = t / (MPO_RB * K) * MPO_RB + jj;
+            region[t] = j < jn ? stage[j * K + k] : 0.f;
+        }
+    }
+    __syncthreads();
+    return sparse;
+}
+
+__device__ __forceinline__ bool nonfinite(float x) { return (__float_as_uint(x) & 0x7f800000u) == 0x7f800000u; }
+
+// The leg where outputs are contiguous in i (H_eff): a column per thread, all of its K inputs
+// first (kept in shared memory, read by the thread that wrote them), then its rows.  What bounds it
+// is memory, 4 bytes in and 8 out per element, so a thread's loads are in flight together and
+// only non-zero weights are multiplied, in the order of k; a column with an infinity or a NaN,
+// where 0 * x counts, takes all.  With few zeros, two columns per thread and the rows by register
+// blocks.  A block does several tiles with one set of weights.  Measured (us,
+// the kernels before / here): H_eff's leg for Fermi-Hubbard (K = 96) at chi 128 38 / 16, 129
+// 118 / 16, 512 297 / 143, 211 x 163 127 / 25; XXZ chi 65 14 / 10; no zero weight, K = 96, chi 128
+// 39 / 37, 129 117 / 36.
+constexpr int MPOC_NT = 256;
+__global__ void __launch_bounds__(MPOC_NT) mpo_tc_cols_kernel(MpoTcDesc m, int jch) {
+    if (ct_skip(m.skip)) return;
+    extern __shared__ __align__(16) float msm[];
+    const int K = (int)m.K, tid = threadIdx.x;
+    const int64_t jbeg = (int64_t)blockIdx.y * jch;
+    const int jn = (int)((m.J - jbeg) < jch ? (m.J - jbeg) : jch);
+    float* xs = msm + tid;                                             // [K][MPOC_NT]
+    float* region = msm + (size_t)K * MPOC_NT;
+    int64_t* joff = reinterpret_cast<int64_t*>(region + (size_t)jch * K);
+    int* start = reinterpret_cast<int*>(joff + jch);
+    const bool sparse = mpo_weights(m, jbeg, jn, MPOC_NT, msm, region, start, joff);
+    const unsigned ni = (unsigned)m.I, cols = (unsigned)m.O * ni, step = gridDim.x * MPOC_NT;   // (cols < 2^31)
+    auto store = [&](int64_t at, float acc) {
+        float h, l;
+        split_tf32(acc, h, l);
+        m.hi[at] = h;
+        m.lo[at] = l;
+    };
+    if (!sparse) {
+        for (unsigned c = blockIdx.x * MPOC_NT + tid; c < cols; c += 2 * step) {
+            const unsigned c1 = c + step < cols ? c + step : c;
+            const unsigned oa = c / ni, ia = c - oa * ni, ob = c1 / ni, ib = c1 - ob * ni;
+            const float *pa = m.in + oa * m.sIo + ia, *pb = m.in + ob * m.sIo + ib;
+            const int64_t ba = oa * m.sOo + ia, bb = ob * m.sOo + ib;
+            for (int j0 = 0; j0 < jn; j0 += MPO_RB) {
+                float acc[MPO_RB][2];
+#pragma unroll
+                for (int j = 0; j < MPO_RB; ++j) acc[j][0] = acc[j][1] = 0.f;
+                const float4* w = reinterpret_cast<const float4*>(region + (size_t)j0 * K);
+#pragma unroll 2
+                for (int k = 0; k < K; ++k) {
+                    const float xa = pa[k * m.sIk], xb = pb[k * m.sIk];
+#pragma unroll
+                    for (int q = 0; q < MPO_RB / 4; ++q) {
+                        const float4 v = w[k * (MPO_RB / 4) + q];
+                        acc[4 * q + 0][0] = fmaf(v.x, xa, acc[4 * q + 0][0]);
+                        acc[4 * q + 0][1] = fmaf(v.x, xb, acc[4 * q + 0][1]);
+                        acc[4 * q + 1][0] = fmaf(v.y, xa, acc[4 * q + 1][0]);
+                        acc[4 * q + 1][1] = fmaf(v.y, xb, acc[4 * q + 1][1]);
+                        acc[4 * q + 2][0] = fmaf(v.z, xa, acc[4 * q + 2][0]);
+                        acc[4 * q + 2][1] = fmaf(v.z, xb, acc[4 * q + 2][1]);
+                        acc[4 * q + 3][0] = fmaf(v.w, xa, acc[4 * q + 3][0]);
+                        acc[4 * q + 3][1] = fmaf(v.w, xb, acc[4 * q + 3][1]);
+                    }
+                }
+#pragma unroll
+                for (int j = 0; j < MPO_RB; ++j) {
+                    if (j0 + j >= jn) break;
+                    store(ba + joff[j0 + j], acc[j][0]);
+                    if (c1 != c) store(bb + joff[j0 + j], acc[j][1]);
+                }
+            }
+        }
+        return;
+    }
+    const float2* list = reinterpret_cast<const float2*>(region);
+    for (unsigned c = blockIdx.x * MPOC_NT + tid; c < cols; c += step) {
+        const unsigned o = c / ni, i = c - o * ni;
+        const float* in = m.in + o * m.sIo + i;
+        const int64_t obase = o * m.sOo + i;
+        bool bad = false;
+#pragma unroll 12
+        for (int k = 0; k < K; ++k) {
+            const float x = in[k * m.sIk];
+            bad |= nonfinite(x);
+            xs[k * MPOC_NT] = x;
+        }
+        if (bad) {
+            for (int j = 0; j < jn; ++j) {
+                float acc = 0.f;
+                for (int k = 0; k < K; ++k) acc = fmaf(ct_d2f(m.Wt[(jbeg + j) * K + k]), xs[k * MPOC_NT], acc);
+                store(obase + joff[j], acc);
+            }
+            continue;
+        }
+        // four rows at a time, their first terms (most rows have one or none) side by side
+        for (int j0 = 0; j0 < jn; j0 += 4) {
+            int s[5];
+            float acc[4];
+#pragma unroll
+            for (int q = 0; q < 5; ++q) s[q] = start[min(j0 + q, jn)];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const bool any = s[q + 1] > s[q];
+                const float2 wk = list[any ? s[q] : 0];
+                acc[q] = any ? fmaf(wk.x, xs[__float_as_int(wk.y)], 0.f) : 0.f;
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                for (int e = s[q] + 1; e < s[q + 1]; ++e) {
+                    const float2 wk = list[e];
+                    acc[q] = fmaf(wk.x, xs[__float_as_int(wk.y)], acc[q]);
+                }
+                if (j0 + q < jn) store(obase + joff[j0 + q], acc[q]);
+            }
+        }
+    }
+}
+
+// The leg where outputs are contiguous in o (environments): tiles of 32 o x 8 i through shared
+// memory, read along i and written along o.  Otherwise as above.
+// Measured (us, the general kernel / here): left environment, XXZ chi 1024 134 / 40 (126 MB, 3.2
+// TB/s), 513 44 / 14, 65 8 / 6; Fermi-Hubbard chi 512 94 / 46; no zero weight, chi 1024, w 5 133 / 50.
+constexpr int MPOR_NT = 256, MPOR_LD = 33, MPOR_K = 8 * MPOR_LD;
+__global__ void __launch_bounds__(MPOR_NT) mpo_tc_rows_kernel(MpoTcDesc m, int jch) {
+    if (ct_skip(m.skip)) return;
+    extern __shared__ __align__(16) float msm[];
+    const int K = (int)m.K, tid = threadIdx.x;
+    const int64_t jbeg = (int64_t)blockIdx.y * jch;
+    const int jn = (int)((m.J - jbeg) < jch ? (m.J - jbeg) : jch);
+    float* xs = msm;                                                   // [K][8][MPOR_LD]
+    float* region = msm + (size_t)K * MPOR_K;
+    int64_t* joff = reinterpret_cast<int64_t*>(region + (size_t)jch * K);
+    int* start = reinterpret_cast<int*>(joff + jch);
+    const bool sparse = mpo_weights(m, jbeg, jn, MPOR_K, msm, region, start, joff);
+    const int64_t ti = (m.I + 7) / 8, tiles = ti * ((m.O + 31) / 32);
+    for (int64_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+        const int64_t o0 = t / ti * 32, i0 = t % ti * 8;
+        bool bad = false;
+        {
+            const int i = tid % 8, o = tid / 8;
+            const bool live = o0 + o < m.O && i0 + i < m.I;
+            const float* in = m.in + (o0 + o) * m.sIo + (i0 + i) * m.sIi;
+#pragma unroll 10
+            for (int k = 0; k < K; ++k) {
+                const float x = live ? in[k * m.sIk] : 0.f;
+                bad |= nonfinite(x);
+                xs[k * MPOR_K + i * MPOR_LD + o] = x;
+            }
+        }
+        const bool all = __syncthreads_or(bad) != 0;
+        const int64_t o = o0 + tid % 32, i = i0 + tid / 32;
+        const float* x = xs + (tid / 32) * MPOR_LD + tid % 32;
+        if (o < m.O && i < m.I) {
+            const int64_t obase = o * m.sOo + i * m.sOi;
+            const float2* list = reinterpret_cast<const float2*>(region);
+            for (int j = 0; j < jn; ++j) {
+                float acc = 0.f;
+                if (!sparse) {
+                    const float* w = region + (size_t)(j / MPO_RB) * MPO_RB * K + j % MPO_RB;
+                    for (int k = 0; k < K; ++k) acc = fmaf(w[MPO_RB * k], x[k * MPOR_K], acc);
+                } else if (all) {
+                    for (int k = 0; k < K; ++k) acc = fmaf(ct_d2f(m.Wt[(jbeg + j) * K + k]), x[k * MPOR_K], acc);
+                } else {
+                    const int end = start[j + 1];
+                    for (int e = start[j]; e < end; ++e) {
+                        const float2 wk = list[e];
+                        acc = fmaf(wk.x, x[__float_as_int(wk.y)], acc);
+                    }
+                }
+                float h, l;
+                split_tf32(acc, h, l);
+                m.hi[obase + joff[j]] = h;
+                m.lo[obase + joff[j]] = l;
+            }
+        }
+        __syncthreads();
+    }
+}
+
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
@@ -1568,20 +1804,65 @@ int mpo_tc2_launch(ct_handle* h, const MpoTcDesc& m) {
     return CT_OK;
 }
 
+// Launch of a leg kernel with xbytes of staged columns (256 per k at least) beside its weights;
+// false when they do not fit (nothing launched).
+template <auto kernel>
+bool mpo_leg_launch(ct_handle* h, const MpoTcDesc& m, int nt, size_t xbytes, int64_t tiles, int* rc) {
+    constexpr size_t kBudget = 200 * 1024;
+    const size_t block = MPO_RB * ((size_t)m.K * sizeof(float) + sizeof(int64_t) + sizeof(int));
+    *rc = CT_OK;
+    if (xbytes + block + 16 > kBudget) return false;
+    const int64_t fit = (int64_t)((kBudget - 16 - xbytes) / block) * MPO_RB;
+    // rows in several blocks where the tiles leave SMs idle
+    const int64_t split = std::max<int64_t>(1, std::min<int64_t>(ct_cdiv(m.J, MPO_RB), 2 * (int64_t)h->num_sms / tiles));
+    const int64_t jch = std::min<int64_t>({ct_round_up(ct_cdiv(m.J, split), MPO_RB), fit, 256}), nz = ct_cdiv(m.J, jch);
+    if (nz > 65535) return false;
+    const size_t smem = xbytes + (size_t)(jch / MPO_RB) * block + 16;
+    static int attr_dev = -1;
+    if (attr_dev != h->device) {
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBudget) != cudaSuccess) {
+            (void)cudaGetLastError();
+            return false;
+        }
+        attr_dev = h->device;
+    }
+    const int64_t per_sm = std::min<int64_t>((int64_t)(225 * 1024 / (smem + 1024)), 2048 / nt);
+    const dim3 grid((unsigned)std::min<int64_t>(tiles, per_sm * h->num_sms), (unsigned)nz);
+    kernel<<<grid, nt, smem, h->stream>>>(m, (int)jch); ct_note_launch();
+    *rc = [&]() -> int {
+        CT_LAUNCH_CHECK(h);
+        return CT_OK;
+    }();
+    return true;
+}
+
 int mpo_tc_launch(ct_handle* h, const MpoTcDesc& m) {
     if (m.O <= 0 || m.I <= 0 || m.J <= 0) return CT_OK;
-    // paired-column kernel when the layout allows float2 access and the weight
-    // chunk fits (K x 32 floats within 96 KB)
-    const bool even = m.sIi == 1 && m.sOi == 1 && (m.I % 2) == 0 && (m.sIo % 2) == 0 && (m.sIk % 2) == 0 &&
-                      (m.sOo % 2) == 0 && (m.sOj1 % 2) == 0 && (m.sOj0 % 2) == 0 &&
-                      (((uintptr_t)m.in | (uintptr_t)m.hi | (uintptr_t)m.lo) & 7) == 0;
-    if (even && m.O <= 65535 && (size_t)m.K * 32 * sizeof(float) + 256 <= 96 * 1024) {
-        if (m.J <= 8) return mpo_tc2_launch<8>(h, m);
-        if (m.J <= 12) return mpo_tc2_launch<12>(h, m);
-        if (m.J <= 16) return mpo_tc2_launch<16>(h, m);
-        if (m.J <= 20) return mpo_tc2_launch<20>(h, m);
-        if (m.J <= 24) return mpo_tc2_launch<24>(h, m);
-        return mpo_tc2_launch<32>(h, m);
+    if (m.O <= 65535 && m.K > 0) {
+        int rc = CT_OK;
+        const bool along_i = m.sIi == 1 && m.sOi == 1;
+        // Few weights and 8-byte aligned pairs of columns: memory bounds the leg with every weight
+        // multiplied too (XXZ, chi 1024: 54 us, 53 from the list; no zero weight: 54, 60), and
+        // without the list it starts sooner (chi 64: 8 us, 10).  With many (K = 96) the list saves
+        // more than it costs.
+        const bool even = along_i && (m.I % 2) == 0 && (m.sIo % 2) == 0 && (m.sIk % 2) == 0 && (m.sOo % 2) == 0 &&
+                          (m.sOj1 % 2) == 0 && (m.sOj0 % 2) == 0 &&
+                          (((uintptr_t)m.in | (uintptr_t)m.hi | (uintptr_t)m.lo) & 7) == 0;
+        if (even && m.K <= 32) {
+            if (m.J <= 8) return mpo_tc2_launch<8>(h, m);
+            if (m.J <= 12) return mpo_tc2_launch<12>(h, m);
+            if (m.J <= 16) return mpo_tc2_launch<16>(h, m);
+            if (m.J <= 20) return mpo_tc2_launch<20>(h, m);
+            if (m.J <= 24) return mpo_tc2_launch<24>(h, m);
+            return mpo_tc2_launch<32>(h, m);
+        }
+        if (along_i && m.O * m.I < (1ll << 31) &&
+            mpo_leg_launch<mpo_tc_cols_kernel>(h, m, MPOC_NT, (size_t)m.K * MPOC_NT * sizeof(float),
+                                               ct_cdiv(m.O * m.I, MPOC_NT), &rc))
+            return rc;
+        if (m.sOi != 1 && mpo_leg_launch<mpo_tc_rows_kernel>(h, m, MPOR_NT, (size_t)m.K * MPOR_K * sizeof(float),
+                                                             ct_cdiv(m.I, 8) * ct_cdiv(m.O, 32), &rc))
+            return rc;
     }
     // the whole of Wt in shared memory when it fits in 96 KB, else chunks of rows
     constexpr size_t kBudget = 96 * 1024;
