@@ -14,8 +14,11 @@
 // and the scalars take ~2300 cycles (rotation).
 #pragma once
 #include "ct_common.cuh"
+#include "ct_fp64.cuh"
 
 namespace ct_jacobi {
+
+using namespace ct_fp64;
 
 constexpr int NT = 256;
 constexpr int MAX_SWEEPS = 48;
@@ -69,52 +72,6 @@ __device__ __forceinline__ void pair_index(int P, int r, int k, int& p, int& q) 
         p = (r + k) % (P - 1);
         q = (r - k + (P - 1)) % (P - 1);
     }
-}
-
-// ---- FP64 scalars on the critical path -----------------------------------------------------
-// Biased exponent field of x.
-__device__ __forceinline__ int exp_field(double x) { return (int)((__double_as_longlong(x) >> 52) & 0x7ff); }
-// The mantissa of a normal x as a float in [1, 2), truncated, with x's sign: integer instructions.
-__device__ __forceinline__ float mant_f32(double x) {
-    const long long b = __double_as_longlong(x);
-    return __int_as_float((int)((b >> 63) & 1) << 31 | 127 << 23 | (int)((b >> 29) & 0x7fffff));
-}
-// A normal float as a double times 2^e, by its bits (the result must be normal).
-__device__ __forceinline__ double widen(float x, int e) {
-    const int b = __float_as_int(x);
-    const long long m = ((long long)(b & 0x7fffffff) << 29) + ((long long)(1023 - 127 + e) << 52);
-    return __longlong_as_double(m | ((long long)(b >> 31) << 63));
-}
-// exponent fields for which the scalings below and the residuals stay normal
-__device__ __forceinline__ bool mid_exp(int e) { return (unsigned)(e - 400) < 1248u; }
-
-// Correctly rounded n / d and sqrt(x) from FP32 estimates: one third-order Newton step (to the
-// last bit or so), then Markstein's correction with the exact residual (P. W. Markstein,
-// Computation of elementary functions on the IBM RISC System/6000 processor, IBM J. Res. Dev.
-// 34, 1990), in 6 and 7 dependent operations; outside the middle of the exponent range the
-// plain operators.  (390 and 455 cycles against 660 and ~870.)
-__device__ __forceinline__ double div_rn(double n, double d) {
-    const int en = exp_field(n), ed = exp_field(d);
-    if (!(mid_exp(en) && mid_exp(ed) && mid_exp(en - ed + 1023))) return n / d;
-    const double y0 = widen(__fdividef(1.0f, mant_f32(d)), 1023 - ed);
-    const double e = fma(-d, y0, 1.0);
-    const double y = fma(y0, fma(e, e, e), y0);
-    const double q = n * y;
-    return fma(fma(-d, q, n), y, q);
-}
-__device__ __forceinline__ double sqrt_rn(double x) {
-    const int ex = exp_field(x);
-    if (!mid_exp(ex) || x < 0.0) return sqrt(x);
-    // x = m 2^(2k), m in [1, 4)
-    const int k = (ex - 1023) >> 1;
-    const float mf = mant_f32(x) * (((ex - 1023) & 1) ? 2.0f : 1.0f);
-    const double y = widen(rsqrtf(mf), -k);
-    const double h = __longlong_as_double(__double_as_longlong(y) - (1ll << 52));   // y / 2
-    const double g = x * y;
-    const double r = fma(-g, h, 0.5);
-    const double p = fma(1.5 * r, r, r);
-    const double g1 = fma(g, p, g), h1 = fma(h, p, h);
-    return fma(fma(-g1, g1, x), h1, g1);
 }
 
 // Rotation that orthogonalises two vectors with |x_p|^2=a, |x_q|^2=b, <x_p,x_q>=c.
