@@ -150,6 +150,21 @@ static inline void ct_note_launch() { g_ct_launches.fetch_add(1, std::memory_ord
 
 #define CT_LAUNCH_CHECK(h) CT_CUDA(h, cudaGetLastError())
 
+template <typename... P, typename... A>
+void ct_launch(ct_handle* h, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = h->stream;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);   // (CT_LAUNCH_CHECK reads the error)
+}
+
 static inline int64_t ct_cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
 static inline int64_t ct_round_up(int64_t a, int64_t b) { return ct_cdiv(a, b) * b; }
 
@@ -233,6 +248,19 @@ __device__ __forceinline__ double ct_f2d(float f) {
 
 __device__ __forceinline__ void ct_set_status(int* st, int code) {
     if (st) atomicCAS(st, 0, code);
+}
+
+// Programmatic dependent launch.  Every kernel of the library opens with ct_pdl() and is launched
+// by ct_launch: the next kernel's blocks may then be set up while this one still runs, and wait
+// here until it has ended and its writes are visible.  No statement comes before it (an early
+// return without the wait would let a later kernel overtake an earlier one).  A launch in
+// stream order costs 2 to 3 us between two kernels, this way about 1: Lanczos at chi 32 (150
+// launches) 1023 -> 837 us, the 16-site Heisenberg run (19,000 launches) 187 -> 162 ms.
+__device__ __forceinline__ void ct_pdl_next() { asm volatile("griddepcontrol.launch_dependents;"); }
+__device__ __forceinline__ void ct_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void ct_pdl() {
+    ct_pdl_next();
+    ct_pdl_wait();
 }
 
 // kernels that belong to an early-terminating loop read this flag first

@@ -167,6 +167,7 @@ constexpr int FM_PK = 64;    // columns per block of the residue kernel
 // for a zero row).  Blocks [0, nba) take operand A's rows.  sk == 1: a warp per row; else
 // threads along the rows, which are contiguous then.
 __global__ void __launch_bounds__(256) fm_rowexp_kernel(FmSrc a, FmSrc b, int nba, const int* skip) {
+    ct_pdl();
     if (ct_skip(skip)) return;
     __shared__ unsigned long long part[8][FM_PR];
     const bool first = (int)blockIdx.x < nba;
@@ -241,6 +242,7 @@ __device__ __forceinline__ unsigned long long fm_fixed(double v, int e, int bits
 // along the rows.
 __global__ void __launch_bounds__(256) fm_residue_kernel(FmSrc a, FmSrc b, int nba, int bits, const ModTable tab,
                                                          const int* skip) {
+    ct_pdl();
     if (ct_skip(skip)) return;
     __shared__ double tile[FM_PK][FM_PR + 1];
     const bool first = (int)blockIdx.x < nba;
@@ -320,6 +322,7 @@ struct FmOut {
 __global__ void __launch_bounds__(FM_THREADS, 1)
     fm_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M, int N,
                    int Kpad, FmOut out, const ModTable tab, const int* skip, int* status) {
+    ct_pdl();
     if (ct_skip(skip)) return;
     extern __shared__ uint8_t fm_smem_raw[];
     uint8_t* smem = fm_smem_raw + ((1024u - (smem_u32(fm_smem_raw) & 1023u)) & 1023u);
@@ -502,6 +505,7 @@ struct FmC {
 // 2^26), so that the multi-word sums have six terms.  A thread takes four columns of a row.
 __global__ void __launch_bounds__(256) fm_crt_kernel(FmOut in, int M, int N, FmSrc a, FmSrc b, FmC c, int bits,
                                                      const CrtTable tab, const int* skip) {
+    ct_pdl();
     if (ct_skip(skip)) return;
     const int64_t n0 = 4 * ((int64_t)blockIdx.x * 64 + (threadIdx.x & 63));
     const int64_t m = (int64_t)blockIdx.y * 4 + (threadIdx.x >> 6);
@@ -709,14 +713,14 @@ int ct_f64_gemm(ct_handle* h, int64_t M, int64_t N, int64_t K, const OzMat& A, c
     const int nba = (int)ct_cdiv(M, FM_PR);
     const dim3 grid((unsigned)(nba + ct_cdiv(N, FM_PR)), (unsigned)ct_cdiv(q.ldk, FM_PK));
     if (grid.y > 65535) return CT_ERR_UNSUPPORTED;
-    fm_rowexp_kernel<<<grid.x, 256, 0, h->stream>>>(a, b, nba, skip); ct_note_launch();
-    fm_residue_kernel<<<grid, 256, 0, h->stream>>>(a, b, nba, bits, t.mod, skip); ct_note_launch();
+    ct_launch(h, fm_rowexp_kernel, grid.x, 256, 0, a, b, nba, skip); ct_note_launch();
+    ct_launch(h, fm_residue_kernel, grid, 256, 0, a, b, nba, bits, t.mod, skip); ct_note_launch();
     const int64_t items = q.tiles * MODS;
     const int64_t ctas = items < h->num_sms ? items : h->num_sms;
-    fm_gemm_kernel<<<(unsigned)ctas, FM_THREADS, FM_SMEM, h->stream>>>(ta, tb, (int)M, (int)N, (int)q.ldk, o, t.mod, skip,
+    ct_launch(h, fm_gemm_kernel, (unsigned)ctas, FM_THREADS, FM_SMEM, ta, tb, (int)M, (int)N, (int)q.ldk, o, t.mod, skip,
                                                                        h->d_status); ct_note_launch();
     const FmC c{Cout.p, Cout.M0 > 0 ? Cout.M0 : M, Cout.s1, Cout.s0};
-    fm_crt_kernel<<<dim3((unsigned)ct_cdiv(N, 256), (unsigned)ct_cdiv(M, 4)), 256, 0, h->stream>>>(
+    ct_launch(h, fm_crt_kernel, dim3((unsigned)ct_cdiv(N, 256), (unsigned)ct_cdiv(M, 4)), 256, 0, 
         o, (int)M, (int)N, a, b, c, bits, t.crt, skip); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;

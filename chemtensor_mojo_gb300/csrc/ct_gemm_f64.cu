@@ -24,6 +24,7 @@ constexpr int BK = 16;
 // holding a 4 x 4 register block.
 template <int TBM, int TBN, bool A_K_CONTIG, bool B_N_CONTIG>
 __global__ void __launch_bounds__((TBM / 4) * (TBN / 4)) gemm_f64_kernel(GemmDesc g) {
+    ct_pdl();
     constexpr int NT = (TBM / 4) * (TBN / 4);
     constexpr int TX = TBN / 4;
     if (ct_skip(g.skip)) return;
@@ -127,6 +128,7 @@ constexpr int TRI = 32;
 
 template <bool A_K_CONTIG, bool B_N_CONTIG>
 __global__ void __launch_bounds__(SP_NT) gemm_f64_spread_kernel(GemmDesc g, int clustered) {
+    ct_pdl();
     if (ct_skip(g.skip)) return;
     __shared__ double As[SP_K][SP_M + 1];
     __shared__ double Bs[SP_K][SP_N + 1];
@@ -222,6 +224,7 @@ __global__ void __launch_bounds__(SP_NT) gemm_f64_spread_kernel(GemmDesc g, int 
 // C = alpha * sum_ks part[ks] + beta * C, the partial sums added in a fixed
 // order (deterministic); tiles the GEMM kernel skips (tri == 1) stay untouched.
 __global__ void splitk_reduce_kernel(GemmDesc g, int tile) {
+    ct_pdl();
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < g.M * g.N;
          t += (int64_t)gridDim.x * blockDim.x) {
         const int64_t gm = t / g.N, gn = t % g.N;
@@ -245,10 +248,10 @@ int launch_tiles(ct_handle* h, const GemmDesc& g, int64_t nb) {
     constexpr int nt = (TBM / 4) * (TBN / 4);
     const bool ak = (g.sAk == 1);
     const bool bn = (g.sBn == 1);
-    if (ak && bn) { gemm_f64_kernel<TBM, TBN, true, true><<<grid, nt, 0, h->stream>>>(g); ct_note_launch(); }
-    else if (ak) { gemm_f64_kernel<TBM, TBN, true, false><<<grid, nt, 0, h->stream>>>(g); ct_note_launch(); }
-    else if (bn) { gemm_f64_kernel<TBM, TBN, false, true><<<grid, nt, 0, h->stream>>>(g); ct_note_launch(); }
-    else { gemm_f64_kernel<TBM, TBN, false, false><<<grid, nt, 0, h->stream>>>(g); ct_note_launch(); }
+    if (ak && bn) { ct_launch(h, gemm_f64_kernel<TBM, TBN, true, true>, grid, nt, 0, g); ct_note_launch(); }
+    else if (ak) { ct_launch(h, gemm_f64_kernel<TBM, TBN, true, false>, grid, nt, 0, g); ct_note_launch(); }
+    else if (bn) { ct_launch(h, gemm_f64_kernel<TBM, TBN, false, true>, grid, nt, 0, g); ct_note_launch(); }
+    else { ct_launch(h, gemm_f64_kernel<TBM, TBN, false, false>, grid, nt, 0, g); ct_note_launch(); }
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }
@@ -265,13 +268,13 @@ int launch_spread(ct_handle* h, const GemmDesc& g, int64_t nb) {
     cfg.gridDim = dim3((unsigned)ct_cdiv(g.N, SP_N), (unsigned)ym, (unsigned)z);
     cfg.blockDim = dim3(SP_NT);
     cfg.stream = h->stream;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim = {1, 1, (unsigned)g.ksplit};
-    if (clustered) {
-        cfg.attrs = &at;
-        cfg.numAttrs = 1;
-    }
+    cudaLaunchAttribute at[2]{};
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // (as ct_launch)
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim = {1, 1, (unsigned)g.ksplit};
+    cfg.attrs = at;
+    cfg.numAttrs = clustered ? 2 : 1;
     const bool ak = (g.sAk == 1), bn = (g.sBn == 1);
     auto* f = ak ? (bn ? gemm_f64_spread_kernel<true, true> : gemm_f64_spread_kernel<true, false>)
                  : (bn ? gemm_f64_spread_kernel<false, true> : gemm_f64_spread_kernel<false, false>);
@@ -280,7 +283,7 @@ int launch_spread(ct_handle* h, const GemmDesc& g, int64_t nb) {
         const int64_t tot = g.M * g.N;
         int64_t blocks = ct_cdiv(tot, 256);
         if (blocks > 4 * (int64_t)h->num_sms) blocks = 4 * (int64_t)h->num_sms;
-        splitk_reduce_kernel<<<(unsigned)blocks, 256, 0, h->stream>>>(g, TRI); ct_note_launch();
+        ct_launch(h, splitk_reduce_kernel, (unsigned)blocks, 256, 0, g, TRI); ct_note_launch();
         CT_LAUNCH_CHECK(h);
     }
     return CT_OK;

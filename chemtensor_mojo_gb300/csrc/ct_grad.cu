@@ -33,6 +33,7 @@ struct Buf {
 // g = fH hA - fN nA; the host folds 2/N, the energy and the environments'
 // power-of-two scales into the two factors
 __global__ void grad_combine_kernel(int64_t n, const double* hA, const double* nA, double fH, double fN, double* g) {
+    ct_pdl();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         g[i] = fH * hA[i] - fN * nA[i];
 }
@@ -258,7 +259,7 @@ int ct_energy_grad(ct_handle* h, int prec, int N, int d, const int64_t* mpo_dims
             // g = 2 (hA_true - E nA_true) / N_true with X_true = X 2^(left + right exponents)
             const double fH = ldexp(2.0 / Nsc, (int)(cumHL[i] + cumHR[i + 1] - eN));
             const double fNn = ldexp(2.0 * energy / Nsc, (int)(cumNL[i] + cumNR[i + 1] - eN));
-            grad_combine_kernel<<<g, 256, 0, h->stream>>>(ns, hA.p, nA.p, fH, fNn, grads[i]); ct_note_launch();
+            ct_launch(h, grad_combine_kernel, g, 256, 0, ns, hA.p, nA.p, fH, fNn, grads[i]); ct_note_launch();
             CT_LAUNCH_CHECK(h);
             if (i > 0) {
                 {

@@ -148,6 +148,7 @@ template <typename T>
 __global__ void __launch_bounds__(NT) jacobi_coop_kernel(T* X, int64_t len, T* Q, int64_t nvec, double tol,
                                                         double floor_rel, const double* frob2, int max_sweeps,
                                                         Sync s) {
+    ct_pdl();
     __shared__ double sm[24];
     __shared__ double rot_cs, rot_sn;
     __shared__ int do_rot;

@@ -27,6 +27,7 @@ constexpr int MPO_WARPS = MPO_NT / 32;
 // 15.8 / 5.2, Ising chi 32 11.9 / 3.9; H_eff with no
 // zero weight, chi 128, d 4, w 6 (K = 96): 1326 / 1042.
 __global__ void __launch_bounds__(MPO_NT) mpo_apply_f64_kernel(MpoDesc m, int jch) {
+    ct_pdl();
     if (ct_skip(m.skip)) return;
     extern __shared__ double msm[];
     const int K = (int)m.K;
@@ -98,6 +99,7 @@ __global__ void __launch_bounds__(MPO_NT) mpo_apply_f64_kernel(MpoDesc m, int jc
 // ([z * jch, z * jch + jch) of J); shared memory holds that chunk of Wt and
 // its output offsets.
 __global__ void __launch_bounds__(WIDE_NT) mpo_apply_f64_wide_kernel(MpoDesc m, int64_t jch) {
+    ct_pdl();
     if (ct_skip(m.skip)) return;
     extern __shared__ double wsm[];
     const int64_t jbeg = (int64_t)blockIdx.z * jch;
@@ -136,6 +138,7 @@ __global__ void __launch_bounds__(WIDE_NT) mpo_apply_f64_wide_kernel(MpoDesc m, 
 // W12t[(t1 t2 wR), (wL s1 s2)] = sum_wM W1[wL,s1,t1,wM] W2[wM,s2,t2,wR]
 __global__ void build_w12_kernel(const double* W1, const double* W2, double* W12t, int64_t wL,
                                  int64_t d, int64_t wM, int64_t wR) {
+    ct_pdl();
     const int64_t J = d * d * wR, K = wL * d * d;
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= J * K) return;
@@ -153,6 +156,7 @@ __global__ void build_w12_kernel(const double* W1, const double* W2, double* W12
 
 // Wt[(s' wR), (wL s)] = W[wL, s, s', wR]   (left environment)
 __global__ void build_wt_left_kernel(const double* W, double* Wt, int64_t wL, int64_t d, int64_t wR) {
+    ct_pdl();
     const int64_t J = d * wR, K = wL * d;
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= J * K) return;
@@ -163,6 +167,7 @@ __global__ void build_wt_left_kernel(const double* W, double* Wt, int64_t wL, in
 
 // Wt[(wL s'), (wR s)] = W[wL, s, s', wR]   (right environment)
 __global__ void build_wt_right_kernel(const double* W, double* Wt, int64_t wL, int64_t d, int64_t wR) {
+    ct_pdl();
     const int64_t J = wL * d, K = wR * d;
     const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= J * K) return;
@@ -174,6 +179,7 @@ __global__ void build_wt_right_kernel(const double* W, double* Wt, int64_t wL, i
 // W[(al, bl), i, o, (ar, br)] = sum_m Wa[al, i, m, ar] Wb[bl, m, o, br]   (MPO composition)
 __global__ void mpo_compose_kernel(const double* Wa, const double* Wb, double* W, int64_t wLa, int64_t d_in,
                                    int64_t d_mid, int64_t wRa, int64_t wLb, int64_t d_out, int64_t wRb) {
+    ct_pdl();
     const int64_t n = wLa * wLb * d_in * d_out * wRa * wRb;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
         int64_t q = t;
@@ -196,6 +202,7 @@ __global__ void mpo_compose_kernel(const double* Wa, const double* Wb, double* W
 __global__ void __launch_bounds__(256) apply_mpo_kernel(const double* __restrict__ A, const double* __restrict__ W,
                                                         double* __restrict__ out, int64_t Dl, int64_t d, int64_t Dr,
                                                         int64_t wL, int64_t d_out, int64_t wR) {
+    ct_pdl();
     const int64_t rows = wL * Dl * d_out * wR;
     for (int64_t row = blockIdx.y; row < rows; row += gridDim.y) {
         int64_t q = row;
@@ -220,7 +227,7 @@ int ct_mpo_compose_launch(ct_handle* h, const double* Wa, const double* Wb, doub
     const int64_t n = wLa * wLb * d_in * d_out * wRa * wRb;
     if (n <= 0) return CT_OK;
     const int64_t g = std::min<int64_t>(ct_cdiv(n, 256), (int64_t)h->num_sms * 8);
-    mpo_compose_kernel<<<(unsigned)g, 256, 0, h->stream>>>(Wa, Wb, Wout, wLa, d_in, d_mid, wRa, wLb, d_out, wRb);
+    ct_launch(h, mpo_compose_kernel, (unsigned)g, 256, 0, Wa, Wb, Wout, wLa, d_in, d_mid, wRa, wLb, d_out, wRb);
     ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
@@ -231,7 +238,7 @@ int ct_apply_mpo_launch(ct_handle* h, const double* A, const double* W, double* 
     const int64_t rows = wL * Dl * d_out * wR;
     if (rows <= 0 || Dr <= 0) return CT_OK;
     dim3 grid((unsigned)std::min<int64_t>(ct_cdiv(Dr, 256), 64), (unsigned)std::min<int64_t>(rows, 65535));
-    apply_mpo_kernel<<<grid, 256, 0, h->stream>>>(A, W, out, Dl, d, Dr, wL, d_out, wR);
+    ct_launch(h, apply_mpo_kernel, grid, 256, 0, A, W, out, Dl, d, Dr, wL, d_out, wR);
     ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
@@ -255,9 +262,9 @@ int ct_mpo_apply_f64_launch(ct_handle* h, const MpoDesc& m) {
         const int64_t jch = std::min<int64_t>(m.J, (int64_t)((kBudget - xbytes) / per_row));
         const int64_t nz = ct_cdiv(m.J, jch);
         if (m.O > 65535 || nz > 65535) return CT_ERR_UNSUPPORTED;
-        // up to eight blocks per SM, each over several tiles (its list is then made once)
-        dim3 grid((unsigned)std::min<int64_t>(ct_cdiv(m.O * m.I, 32), 8 * (int64_t)h->num_sms), (unsigned)nz);
-        mpo_apply_f64_kernel<<<grid, MPO_NT, (size_t)jch * per_row + xbytes, h->stream>>>(m, (int)jch); ct_note_launch();
+        // up to six blocks per SM (40 registers), each over several tiles (its list is then made once)
+        dim3 grid((unsigned)std::min<int64_t>(ct_cdiv(m.O * m.I, 32), 6 * (int64_t)h->num_sms), (unsigned)nz);
+        ct_launch(h, mpo_apply_f64_kernel, grid, MPO_NT, (size_t)jch * per_row + xbytes, m, (int)jch); ct_note_launch();
         CT_LAUNCH_CHECK(h);
         return CT_OK;
     }
@@ -275,7 +282,7 @@ int ct_mpo_apply_f64_launch(ct_handle* h, const MpoDesc& m) {
     const int64_t nz = ct_cdiv(m.J, jch);
     if (m.O > 65535 || nz > 65535) return CT_ERR_UNSUPPORTED;
     dim3 grid((unsigned)ct_cdiv(m.I, WIDE_NT), (unsigned)m.O, (unsigned)nz);
-    mpo_apply_f64_wide_kernel<<<grid, WIDE_NT, (size_t)jch * per_row, h->stream>>>(m, jch); ct_note_launch();
+    ct_launch(h, mpo_apply_f64_wide_kernel, grid, WIDE_NT, (size_t)jch * per_row, m, jch); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }
@@ -283,21 +290,21 @@ int ct_mpo_apply_f64_launch(ct_handle* h, const MpoDesc& m) {
 int ct_build_w12(ct_handle* h, const double* W1, const double* W2, double* W12t, int64_t wL,
                  int64_t d, int64_t wM, int64_t wR) {
     const int64_t n = (d * d * wR) * (wL * d * d);
-    build_w12_kernel<<<(unsigned)ct_cdiv(n, 256), 256, 0, h->stream>>>(W1, W2, W12t, wL, d, wM, wR); ct_note_launch();
+    ct_launch(h, build_w12_kernel, (unsigned)ct_cdiv(n, 256), 256, 0, W1, W2, W12t, wL, d, wM, wR); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }
 
 int ct_build_wt_left(ct_handle* h, const double* W, double* Wt, int64_t wL, int64_t d, int64_t wR) {
     const int64_t n = (d * wR) * (wL * d);
-    build_wt_left_kernel<<<(unsigned)ct_cdiv(n, 256), 256, 0, h->stream>>>(W, Wt, wL, d, wR); ct_note_launch();
+    ct_launch(h, build_wt_left_kernel, (unsigned)ct_cdiv(n, 256), 256, 0, W, Wt, wL, d, wR); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }
 
 int ct_build_wt_right(ct_handle* h, const double* W, double* Wt, int64_t wL, int64_t d, int64_t wR) {
     const int64_t n = (wL * d) * (wR * d);
-    build_wt_right_kernel<<<(unsigned)ct_cdiv(n, 256), 256, 0, h->stream>>>(W, Wt, wL, d, wR); ct_note_launch();
+    ct_launch(h, build_wt_right_kernel, (unsigned)ct_cdiv(n, 256), 256, 0, W, Wt, wL, d, wR); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }

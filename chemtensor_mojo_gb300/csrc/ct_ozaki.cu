@@ -125,6 +125,7 @@ struct OzEpi {
 __global__ void __launch_bounds__(OZ_THREADS, 1)
     oz_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M, int N,
                    int Mp, int Np, int Kpad, int lower, OzEpi epi, int* status) {
+    ct_pdl();
     extern __shared__ uint8_t oz_smem_raw[];
     uint8_t* smem = oz_smem_raw + ((1024u - (smem_u32(oz_smem_raw) & 1023u)) & 1023u);
     uint64_t* full = (uint64_t*)(smem + OZ_TILE_BYTES);
@@ -347,6 +348,7 @@ struct OzSrc {
 // ex[r]: 2^ex[r] > max_k |x[r][k]| >= 2^(ex[r] - 1); 0 for a zero row (and rows >= R).
 // One warp per row; lanes stride over k.
 __global__ void oz_rowexp_kernel(OzSrc a, int64_t Rp, int* ex) {
+    ct_pdl();
     const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
     const int lane = threadIdx.x & 31;
     if (r >= Rp) return;
@@ -368,6 +370,7 @@ __global__ void oz_rowexp_kernel(OzSrc a, int64_t Rp, int* ex) {
 template <bool K_FAST>
 __global__ void __launch_bounds__(256) oz_slice_kernel(OzSrc a, int64_t Rp, int64_t ldk, const int* ex,
                                                        __nv_bfloat16* out) {
+    ct_pdl();
     __shared__ double tile[32][33];
     __shared__ int64_t rbase[32];
     const int64_t r0 = (int64_t)blockIdx.y * 32, k0 = (int64_t)blockIdx.x * 32;
@@ -433,13 +436,13 @@ struct OzOperand {
 int oz_pack(ct_handle* h, const OzSrc& a, const OzOperand& op) {
     {
         const int64_t thr = op.rows_p * 32;
-        oz_rowexp_kernel<<<(unsigned)ct_cdiv(thr, 256), 256, 0, h->stream>>>(a, op.rows_p, op.ex);
+        ct_launch(h, oz_rowexp_kernel, (unsigned)ct_cdiv(thr, 256), 256, 0, a, op.rows_p, op.ex);
         ct_note_launch();
     }
     dim3 grid((unsigned)ct_cdiv(op.ldk, 32), (unsigned)ct_cdiv(op.rows_p, 32));
     if (grid.y > 65535) return CT_ERR_UNSUPPORTED;
-    if (a.sk == 1) oz_slice_kernel<true><<<grid, dim3(32, 8), 0, h->stream>>>(a, op.rows_p, op.ldk, op.ex, op.sl);
-    else oz_slice_kernel<false><<<grid, dim3(32, 8), 0, h->stream>>>(a, op.rows_p, op.ldk, op.ex, op.sl);
+    if (a.sk == 1) ct_launch(h, oz_slice_kernel<true>, grid, dim3(32, 8), 0, a, op.rows_p, op.ldk, op.ex, op.sl);
+    else ct_launch(h, oz_slice_kernel<false>, grid, dim3(32, 8), 0, a, op.rows_p, op.ldk, op.ex, op.sl);
     ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
@@ -567,7 +570,7 @@ int ct_oz_gemm_ex(ct_handle* h, int64_t M, int64_t N, int64_t K, const OzMat& A,
     const int64_t grid = tiles < h->num_sms ? tiles : h->num_sms;
     int slot = -1;
     CT_TRY(ct_ktime_begin(h, KT_OZ_GEMM, 2.0 * (double)M * (double)N * (double)K, &slot));
-    oz_gemm_kernel<<<(unsigned)grid, OZ_THREADS, OZ_SMEM, h->stream>>>(ta, tb, (int)M, (int)N, (int)Mp, (int)Np,
+    ct_launch(h, oz_gemm_kernel, (unsigned)grid, OZ_THREADS, OZ_SMEM, ta, tb, (int)M, (int)N, (int)Mp, (int)Np,
                                                                        (int)ldk, lower ? 1 : 0, e, h->d_status);
     ct_note_launch();
     CT_LAUNCH_CHECK(h);

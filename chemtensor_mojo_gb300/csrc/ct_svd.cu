@@ -24,6 +24,7 @@ constexpr double SVD_EPS2 = 2.2204460492503131e-16 * 2.2204460492503131e-16;
 // ---- init: X (nvec x len) from M, Q = I ---------------------------------------
 __global__ void svd_init_kernel(const double* M, int64_t m, int64_t n, int cols, double* X, int64_t ldx,
                                 double* Q, int64_t nvec) {
+    ct_pdl();
     const int64_t len = cols ? m : n;
     const int64_t tot = nvec * len;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += (int64_t)gridDim.x * blockDim.x) {
@@ -37,6 +38,7 @@ __global__ void svd_init_kernel(const double* M, int64_t m, int64_t n, int cols,
 
 // sigma_j = |x_j|, one warp per vector
 __global__ void svd_norms_kernel(const double* X, int64_t len, int64_t ldx, int64_t nvec, double* sig) {
+    ct_pdl();
     const int64_t v = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
     const int lane = threadIdx.x & 31;
     if (v >= nvec) return;
@@ -55,6 +57,7 @@ __global__ void svd_norms_kernel(const double* X, int64_t len, int64_t ldx, int6
 // compares).
 __device__ __forceinline__ long long rank_bits(double s) { return isnan(s) ? -1ll : __double_as_longlong(s); }
 __global__ void svd_rank_kernel(const double* sig, int64_t nvec, int* perm) {
+    ct_pdl();
     const int64_t j = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
     const int lane = threadIdx.x & 31;
     if (j >= nvec) return;
@@ -72,6 +75,7 @@ __global__ void svd_rank_kernel(const double* sig, int64_t nvec, int* perm) {
 // warp: the lanes gather 32 weights at a time, the sums run over them in order.
 __global__ void svd_trunc_kernel(const double* sig, const int* perm, int64_t k, int64_t chi_max, double eps,
                                  double* scalars, int* flags) {
+    ct_pdl();
     const int lane = threadIdx.x;
     auto weight = [&](int64_t i) {
         const double s = i < k ? sig[perm[i]] : 0.0;
@@ -115,6 +119,7 @@ __global__ void svd_trunc_kernel(const double* sig, const int* perm, int64_t k, 
 __global__ void svd_gather_kernel(const double* X, int64_t ldx, const double* Q, int64_t ldq, const double* sig,
                                   const int* perm, const int* flags, int64_t m, int64_t n, int cols, int mode,
                                   double* A, double* B, double* S) {
+    ct_pdl();
     const int64_t chi = flags[FL_CHI];
     // A: m x chi
     const int64_t totA = m * chi;
@@ -186,6 +191,7 @@ constexpr size_t QR_SMEM_CAP = 200 * 1024;
 // diag[i] for c == i, 0 for c < i.
 __global__ void transpose_kernel(const double* src, int64_t rows, int64_t cols, int64_t lds, double* dst,
                                  const double* diag) {
+    ct_pdl();
     __shared__ double tile[32][33];
     const int64_t r0 = (int64_t)blockIdx.y * 32, c0 = (int64_t)blockIdx.x * 32;
     for (int dy = threadIdx.y; dy < 32; dy += blockDim.y) {
@@ -208,6 +214,7 @@ __global__ void transpose_kernel(const double* src, int64_t rows, int64_t cols, 
 // barrier (bounded, as in the Jacobi) ends the step.
 __global__ void __launch_bounds__(QR_NT) qr_coop_kernel(double* T, int64_t len, int64_t nvec, int64_t k,
                                                         double* refl, ct_jacobi::Sync s) {
+    ct_pdl();
     extern __shared__ double u[];
     __shared__ double red[32];
     const int lane = threadIdx.x & 31;
@@ -260,6 +267,7 @@ __global__ void __launch_bounds__(QR_NT) qr_coop_kernel(double* T, int64_t len, 
 // reflector in shared memory; one warp per row.
 __global__ void __launch_bounds__(QR_NT) qr_form_kernel(const double* T, int64_t nvec, int64_t k,
                                                         const double* refl, const double* J, int rows, double* Qn) {
+    ct_pdl();
     extern __shared__ double sm[];
     double* u = sm;
     double* c = sm + nvec;
@@ -290,6 +298,7 @@ __global__ void __launch_bounds__(QR_NT) qr_form_kernel(const double* T, int64_t
 }
 
 __global__ void identity_kernel(double* Q, int64_t n) {
+    ct_pdl();
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n * n; t += (int64_t)gridDim.x * blockDim.x)
         Q[t] = (t / n == t % n) ? 1.0 : 0.0;
 }
@@ -324,7 +333,7 @@ size_t ct_svd_ws_bytes(int64_t m, int64_t n, int mode) {
 static void launch_transpose(ct_handle* h, const double* src, int64_t rows, int64_t cols, int64_t lds, double* dst,
                              const double* diag) {
     const dim3 grid((unsigned)ct_cdiv(cols, 32), (unsigned)ct_cdiv(rows, 32));
-    transpose_kernel<<<grid, dim3(32, 8), 0, h->stream>>>(src, rows, cols, lds, dst, diag); ct_note_launch();
+    ct_launch(h, transpose_kernel, grid, dim3(32, 8), 0, src, rows, cols, lds, dst, diag); ct_note_launch();
 }
 
 // QR-preconditioned Jacobi of the vectors of M (rows: cols = 0, columns: cols = 1).
@@ -365,8 +374,7 @@ static int svd_qr_jacobi(ct_handle* h, Arena& ar, const double* M, int64_t m, in
     }
     // R2 (k x len) into X, J = I
     launch_transpose(h, T, len, k, nvec, X, refl + 2 * k);
-    identity_kernel<<<(unsigned)std::min<int64_t>(ct_cdiv(k * k, 256), 4 * (int64_t)h->num_sms), 256, 0,
-                      h->stream>>>(J, k); ct_note_launch();
+    ct_launch(h, identity_kernel, (unsigned)std::min<int64_t>(ct_cdiv(k * k, 256), 4 * (int64_t)h->num_sms), 256, 0, J, k); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     double* d_frob2 = h->d_scalars + SC_TMP0;
     CT_TRY(ct_reduce_nrm2sq(h, k * len, X, d_frob2, nullptr));
@@ -376,7 +384,7 @@ static int svd_qr_jacobi(ct_handle* h, Arena& ar, const double* M, int64_t m, in
         if (rows > QR_NT / 32) rows = QR_NT / 32;
         if (rows < 1) rows = 1;
         const size_t smem = (size_t)(rows + 1) * nvec * sizeof(double);
-        qr_form_kernel<<<(unsigned)ct_cdiv(k, rows), QR_NT, smem, h->stream>>>(T, nvec, k, refl, J, (int)rows, Qn);
+        ct_launch(h, qr_form_kernel, (unsigned)ct_cdiv(k, rows), QR_NT, smem, T, nvec, k, refl, J, (int)rows, Qn);
         ct_note_launch();
         CT_LAUNCH_CHECK(h);
     }
@@ -462,7 +470,7 @@ static int svd_run_geometry(ct_handle* h, Arena& ar, const double* M, int64_t m,
         int g = (int)ct_cdiv(tot, 256);
         if (g > h->num_sms * 16) g = h->num_sms * 16;
         if (g < 1) g = 1;
-        svd_init_kernel<<<g, 256, 0, h->stream>>>(M, m, n, cols, X, ldx, Q, nvec); ct_note_launch();
+        ct_launch(h, svd_init_kernel, g, 256, 0, M, m, n, cols, X, ldx, Q, nvec); ct_note_launch();
         CT_LAUNCH_CHECK(h);
         if (nvec >= 2) {
             // beyond the QR's shared-memory limit: the Jacobi on the vectors themselves
@@ -471,9 +479,9 @@ static int svd_run_geometry(ct_handle* h, Arena& ar, const double* M, int64_t m,
             CT_TRY(ct_jacobi::run<double>(h, X, len, Q, nvec, tol, SVD_EPS2, d_frob2, nullptr));
         }
     }
-    svd_norms_kernel<<<(unsigned)ct_cdiv(nv * 32, 256), 256, 0, h->stream>>>(X, len, ldx, nv, sig); ct_note_launch();
-    svd_rank_kernel<<<(unsigned)ct_cdiv(nv * 32, 256), 256, 0, h->stream>>>(sig, nv, perm); ct_note_launch();
-    svd_trunc_kernel<<<1, 32, 0, h->stream>>>(sig, perm, k, chi_max, eps_trunc, h->d_scalars, h->d_flags); ct_note_launch();
+    ct_launch(h, svd_norms_kernel, (unsigned)ct_cdiv(nv * 32, 256), 256, 0, X, len, ldx, nv, sig); ct_note_launch();
+    ct_launch(h, svd_rank_kernel, (unsigned)ct_cdiv(nv * 32, 256), 256, 0, sig, nv, perm); ct_note_launch();
+    ct_launch(h, svd_trunc_kernel, 1, 32, 0, sig, perm, k, chi_max, eps_trunc, h->d_scalars, h->d_flags); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     int chi = 0;
     double sums[2];
@@ -505,7 +513,7 @@ static int svd_run_geometry(ct_handle* h, Arena& ar, const double* M, int64_t m,
         int g = (int)ct_cdiv(tot, 256);
         if (g > h->num_sms * 16) g = h->num_sms * 16;
         if (g < 1) g = 1;
-        svd_gather_kernel<<<g, 256, 0, h->stream>>>(X, ldx, Qf, ldq, sig, perm, h->d_flags, m, n, cols, mode, A, B,
+        ct_launch(h, svd_gather_kernel, g, 256, 0, X, ldx, Qf, ldq, sig, perm, h->d_flags, m, n, cols, mode, A, B,
                                                     S); ct_note_launch();
         CT_LAUNCH_CHECK(h);
     }

@@ -37,6 +37,7 @@ namespace {
 constexpr int NT = 256;
 
 __global__ void to_f32_kernel(const double* M, int64_t m, int64_t n, int cols, float* X, float* Q, int64_t nvec) {
+    ct_pdl();
     const int64_t len = cols ? m : n;
     const int64_t tot = nvec * len;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += (int64_t)gridDim.x * blockDim.x) {
@@ -49,6 +50,7 @@ __global__ void to_f32_kernel(const double* M, int64_t m, int64_t n, int cols, f
 }
 
 __global__ void norms32_kernel(const float* X, int64_t len, int64_t nvec, double* sig) {
+    ct_pdl();
     const int64_t v = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
     const int lane = threadIdx.x & 31;
     if (v >= nvec) return;
@@ -62,6 +64,7 @@ __global__ void norms32_kernel(const float* X, int64_t len, int64_t nvec, double
 }
 
 __global__ void rank_desc_kernel(const double* sig, int64_t n, int* perm) {
+    ct_pdl();
     const int64_t j = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     const double sj = ct_rank_key(sig[j]);
@@ -75,6 +78,7 @@ __global__ void rank_desc_kernel(const double* sig, int64_t n, int* perm) {
 
 // Qt[i][x] = (double) Q32[perm[i]][x]
 __global__ void lift_kernel(const float* Q, int64_t nvec, const int* perm, int64_t c, double* Qt) {
+    ct_pdl();
     const int64_t tot = c * nvec;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += (int64_t)gridDim.x * blockDim.x) {
         const int64_t i = t / nvec, x = t % nvec;
@@ -83,17 +87,20 @@ __global__ void lift_kernel(const float* Q, int64_t nvec, const int* perm, int64
 }
 
 __global__ void f32_to_f64_kernel(const float* a, double* b, int64_t n) {
+    ct_pdl();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         b[i] = (double)a[i];
 }
 
 __global__ void sub_identity_kernel(double* G, int64_t c) {
+    ct_pdl();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < c; i += (int64_t)gridDim.x * blockDim.x)
         G[i * c + i] -= 1.0;
 }
 
 // FP64 norms of the c projected vectors: rows of P[c][ld] (rows=1) or columns of P[len][c] (rows=0)
 __global__ void proj_norms_kernel(const double* P, int64_t c, int64_t len, int rows, double* sig) {
+    ct_pdl();
     const int64_t v = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
     const int lane = threadIdx.x & 31;
     if (v >= c) return;
@@ -109,6 +116,7 @@ __global__ void proj_norms_kernel(const double* P, int64_t c, int64_t len, int r
 // chi rule with the total weight |theta|^2 (dense_tensor.mojo:1528-1548)
 __global__ void trunc_kernel(const double* sig, const int* perm, int64_t limit, int64_t k, double eps,
                              const double* total_p, double* scalars, int* flags) {
+    ct_pdl();
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
     const double total = *total_p;
     int64_t chi = limit;
@@ -141,6 +149,7 @@ __global__ void trunc_kernel(const double* sig, const int* perm, int64_t limit, 
 __global__ void gather_kernel(const double* Qt, int64_t nvec, const double* P, int64_t c, const int* perm,
                               const int* flags, const double* sig, int64_t m, int64_t n, int mode, double* A,
                               double* B, double* S) {
+    ct_pdl();
     const int64_t chi = flags[FL_CHI];
     const int64_t totA = m * chi;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < totA; t += (int64_t)gridDim.x * blockDim.x) {
@@ -215,7 +224,7 @@ int ct_svd_mixed_run(ct_handle* h, Arena& ar, const double* M, int64_t m, int64_
         double* Qp64 = ar.take<double>(nvec * nvec);
         if (!Qp64) return CT_ERR_OOM;
         const size_t mark2 = ar.off;
-        f32_to_f64_kernel<<<grid_elems(h, nvec * nvec), 256, 0, h->stream>>>(qcache, Qp64, nvec * nvec); ct_note_launch();
+        ct_launch(h, f32_to_f64_kernel, grid_elems(h, nvec * nvec), 256, 0, qcache, Qp64, nvec * nvec); ct_note_launch();
         CT_LAUNCH_CHECK(h);
         if (!cols) CT_TRY(ct_tc_gemm_ex(h, ar, 0, 0, nvec, n, m, 1.0, Qp64, nvec, M, n, 0.0, X, 0, n));
         else CT_TRY(ct_tc_gemm_ex(h, ar, 0, 1, nvec, m, n, 1.0, Qp64, nvec, M, n, 0.0, X, 0, m));
@@ -223,7 +232,7 @@ int ct_svd_mixed_run(ct_handle* h, Arena& ar, const double* M, int64_t m, int64_
         CT_CUDA(h, cudaMemcpyAsync(Q, qcache, (size_t)(nvec * nvec) * sizeof(float), cudaMemcpyDeviceToDevice,
                                    h->stream));
     } else {
-        to_f32_kernel<<<grid_elems(h, nvec * (len > nvec ? len : nvec)), 256, 0, h->stream>>>(M, m, n, cols, X, Q, nvec); ct_note_launch();
+        ct_launch(h, to_f32_kernel, grid_elems(h, nvec * (len > nvec ? len : nvec)), 256, 0, M, m, n, cols, X, Q, nvec); ct_note_launch();
         CT_LAUNCH_CHECK(h);
     }
     // 1. FP32 one-sided Jacobi
@@ -235,9 +244,9 @@ int ct_svd_mixed_run(ct_handle* h, Arena& ar, const double* M, int64_t m, int64_
     if (qcache)
         CT_CUDA(h, cudaMemcpyAsync(qcache, Q, (size_t)(nvec * nvec) * sizeof(float), cudaMemcpyDeviceToDevice,
                                    h->stream));
-    norms32_kernel<<<(unsigned)ct_cdiv(nvec * 32, 256), 256, 0, h->stream>>>(X, len, nvec, sig32); ct_note_launch();
-    rank_desc_kernel<<<(unsigned)ct_cdiv(nvec, 256), 256, 0, h->stream>>>(sig32, nvec, perm32); ct_note_launch();
-    lift_kernel<<<grid_elems(h, c * nvec), 256, 0, h->stream>>>(Q, nvec, perm32, c, Qt); ct_note_launch();
+    ct_launch(h, norms32_kernel, (unsigned)ct_cdiv(nvec * 32, 256), 256, 0, X, len, nvec, sig32); ct_note_launch();
+    ct_launch(h, rank_desc_kernel, (unsigned)ct_cdiv(nvec, 256), 256, 0, sig32, nvec, perm32); ct_note_launch();
+    ct_launch(h, lift_kernel, grid_elems(h, c * nvec), 256, 0, Q, nvec, perm32, c, Qt); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     // 2. Newton-Schulz: Qt <- Qt - 1/2 (Qt Qt^T - I) Qt, Gram matrix in FP64
     for (int it = 0; it < 2; ++it) {
@@ -248,7 +257,7 @@ int ct_svd_mixed_run(ct_handle* h, Arena& ar, const double* M, int64_t m, int64_
         g.C = G; g.sCm = c; g.sCn = 1;
         g.alpha = 1.0; g.beta = 0.0; g.nb1 = 1; g.nb0 = 1;
         CT_TRY(ct_gemm_f64_launch(h, g));
-        sub_identity_kernel<<<grid_elems(h, c), 256, 0, h->stream>>>(G, c); ct_note_launch();
+        ct_launch(h, sub_identity_kernel, grid_elems(h, c), 256, 0, G, c); ct_note_launch();
         CT_LAUNCH_CHECK(h);
         ar.off = mark;
         CT_TRY(ct_tc_gemm(h, ar, 0, 0, c, nvec, c, -0.5, G, c, Qt, nvec, 1.0, Qt, nvec));
@@ -273,7 +282,7 @@ int ct_svd_mixed_run(ct_handle* h, Arena& ar, const double* M, int64_t m, int64_
         } else {
             CT_TRY(ct_tc_gemm(h, ar, 0, 0, c, n, m, 1.0, Qt, nvec, M, n, 0.0, Pj, n));
         }
-        proj_norms_kernel<<<(unsigned)ct_cdiv(c * 32, 256), 256, 0, h->stream>>>(Pj, c, n, 1, sig); ct_note_launch();
+        ct_launch(h, proj_norms_kernel, (unsigned)ct_cdiv(c * 32, 256), 256, 0, Pj, c, n, 1, sig); ct_note_launch();
     } else {
         // Pj[m][c] = M[m][n] . Qt[c][n]^T
         if (fp64_proj) {
@@ -287,10 +296,10 @@ int ct_svd_mixed_run(ct_handle* h, Arena& ar, const double* M, int64_t m, int64_
         } else {
             CT_TRY(ct_tc_gemm(h, ar, 0, 1, m, c, n, 1.0, M, n, Qt, nvec, 0.0, Pj, c));
         }
-        proj_norms_kernel<<<(unsigned)ct_cdiv(c * 32, 256), 256, 0, h->stream>>>(Pj, c, m, 0, sig); ct_note_launch();
+        ct_launch(h, proj_norms_kernel, (unsigned)ct_cdiv(c * 32, 256), 256, 0, Pj, c, m, 0, sig); ct_note_launch();
     }
-    rank_desc_kernel<<<(unsigned)ct_cdiv(c, 256), 256, 0, h->stream>>>(sig, c, perm); ct_note_launch();
-    trunc_kernel<<<1, 32, 0, h->stream>>>(sig, perm, c, k, eps_trunc, d_total, h->d_scalars, h->d_flags); ct_note_launch();
+    ct_launch(h, rank_desc_kernel, (unsigned)ct_cdiv(c, 256), 256, 0, sig, c, perm); ct_note_launch();
+    ct_launch(h, trunc_kernel, 1, 32, 0, sig, perm, c, k, eps_trunc, d_total, h->d_scalars, h->d_flags); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     int chi = 0;
     double sums[2];
@@ -307,7 +316,7 @@ int ct_svd_mixed_run(ct_handle* h, Arena& ar, const double* M, int64_t m, int64_
     out->sum_s2_all = sums[0];
     out->sum_s2_kept = sums[1];
     if (chi > 0) {
-        gather_kernel<<<grid_elems(h, (m > n ? m : n) * (int64_t)chi), 256, 0, h->stream>>>(
+        ct_launch(h, gather_kernel, grid_elems(h, (m > n ? m : n) * (int64_t)chi), 256, 0, 
             Qt, nvec, Pj, c, perm, h->d_flags, sig, m, n, mode, Aout, Bout, Sout); ct_note_launch();
         CT_LAUNCH_CHECK(h);
     }

@@ -45,6 +45,7 @@ __device__ __forceinline__ void team_sync(int team) {
 // vectors read twice instead of held.
 template <int E, bool CLUSTER>
 __global__ void __launch_bounds__(CLUSTER ? TEAM * MAX_TEAMS : TEAM) svd_small_kernel(Args a) {
+    ct_pdl();
     constexpr int R = E > 0 ? E : 1;
     constexpr double EPS = 2.2204460492503131e-16;
     __shared__ double dots[MAX_TEAMS][3];

@@ -92,6 +92,7 @@ __device__ __forceinline__ double randn_at(uint64_t seed, uint64_t t) {
 // rows[k] (k < count) of Y (rows x len) <- Gaussian rows; one block per listed row
 __global__ void replace_rows_kernel(double* Y, int64_t len, const int* rows, const int* count, int cap,
                                     uint64_t seed) {
+    ct_pdl();
     const int n = min(*count, cap);
     for (int k = blockIdx.x; k < n; k += gridDim.x) {
         const int64_t r = rows[k];
@@ -101,6 +102,7 @@ __global__ void replace_rows_kernel(double* Y, int64_t len, const int* rows, con
 }
 
 __global__ void row_normalize_kernel(double* Y, int64_t rows, int64_t len) {
+    ct_pdl();
     const int64_t r = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / 32;
     const int lane = threadIdx.x & 31;
     if (r >= rows) return;
@@ -113,6 +115,7 @@ __global__ void row_normalize_kernel(double* Y, int64_t rows, int64_t len) {
 }
 
 __global__ void transpose_copy_kernel(const double* src, int64_t rows, int64_t cols, double* dst) {
+    ct_pdl();
     // dst[c][r] = src[r][c]
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < rows * cols;
          t += (int64_t)gridDim.x * blockDim.x) {
@@ -123,6 +126,7 @@ __global__ void transpose_copy_kernel(const double* src, int64_t rows, int64_t c
 
 // G (cp x cp): the padding rows/columns >= c become the identity; Linv is cleared.
 __global__ void chol_prepare_kernel(double* G, double* Linv, int64_t c, int64_t cp) {
+    ct_pdl();
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < cp * cp;
          t += (int64_t)gridDim.x * blockDim.x) {
         const int64_t i = t / cp, j = t % cp;
@@ -221,6 +225,7 @@ __device__ __forceinline__ void chol_pivot(double p, int j, double* pv, long lon
 __global__ void __launch_bounds__(CH_THREADS) chol_diag_kernel(double* G, double* Linv, int64_t ld,
                                                         unsigned long long* minpiv, int* fail, int* defrows,
                                                         int* defcount, int64_t row0, double floor) {
+    ct_pdl();
     extern __shared__ __align__(16) unsigned char chol_smem_raw[];   // three CH_NB x (CH_NB + 1) tiles
     double(*R)[CH_NB + 1] = reinterpret_cast<double(*)[CH_NB + 1]>(chol_smem_raw);
     double(*Ls)[CH_NB + 1] = R + CH_NB;
@@ -317,11 +322,13 @@ __global__ void __launch_bounds__(CH_THREADS) chol_diag_kernel(double* G, double
 }
 
 __global__ void split_piv_set_kernel(unsigned long long* piv, double p) {
+    ct_pdl();
     if (threadIdx.x == 0) atomicMin(piv, (unsigned long long)__double_as_longlong(p < 0.0 ? 0.0 : p));
 }
 
 // running minima of the two passes' pivots start at 1e300; the failure flag at 0
 __global__ void split_flags_init_kernel(unsigned long long* piv, int* fail) {
+    ct_pdl();
     if (threadIdx.x < 2) piv[threadIdx.x] = (unsigned long long)__double_as_longlong(1.0e300);
     if (threadIdx.x == 0) *fail = 0;
 }
@@ -384,7 +391,7 @@ int chol_inv(ct_handle* h, double* G, double* Linv, int64_t ld, int64_t n, doubl
             CT_CUDA(h, cudaFuncSetAttribute(chol_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
             attr_dev = h->device;
         }
-        chol_diag_kernel<<<1, CH_THREADS, smem, h->stream>>>(G, Linv, ld, d_minpiv, d_fail, mk.rows, mk.count, row0,
+        ct_launch(h, chol_diag_kernel, 1, CH_THREADS, smem, G, Linv, ld, d_minpiv, d_fail, mk.rows, mk.count, row0,
                                                       mk.rows ? mk.floor : 0.0);
         ct_note_launch();
         CT_LAUNCH_CHECK(h);
@@ -414,6 +421,7 @@ int chol_inv(ct_handle* h, double* G, double* Linv, int64_t ld, int64_t n, doubl
 // a non-negative double, atomicMax; a NaN counts as 1e300).
 __global__ void orth_correction_kernel(const double* G, int64_t ldg, int64_t c, double* F,
                                        unsigned long long* emax) {
+    ct_pdl();
     double m = 0.0;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < c * c;
          t += (int64_t)gridDim.x * blockDim.x) {
@@ -455,7 +463,7 @@ int orth_correct(ct_handle* h, Arena& ar, const double* Q, double* out, int64_t 
     for (int step = 0; step < 2; ++step) {
         CT_CUDA(h, cudaMemsetAsync(d_emax, 0, sizeof(unsigned long long), h->stream));
         CT_TRY(fac_gemm(h, c, c, len, cur, len, cur, len, 1, ob.G, ob.cp, 1.0, 0.0, 1));   // lower tiles of Q Q^T
-        orth_correction_kernel<<<grid_n(h, c * c), 256, 0, h->stream>>>(ob.G, ob.cp, c, ob.Linv, d_emax);
+        ct_launch(h, orth_correction_kernel, grid_n(h, c * c), 256, 0, ob.G, ob.cp, c, ob.Linv, d_emax);
         ct_note_launch();
         CT_LAUNCH_CHECK(h);
         unsigned long long bits = 0;
@@ -466,7 +474,7 @@ int orth_correct(ct_handle* h, Arena& ar, const double* Q, double* out, int64_t 
         if (step == 0) {
             if (!(emax <= ORTH_CORR_MAX)) return CT_OK;
             const double p = 1.0 - emax;
-            split_piv_set_kernel<<<1, 32, 0, h->stream>>>(piv, p);
+            ct_launch(h, split_piv_set_kernel, 1, 32, 0, piv, p);
             ct_note_launch();
             CT_LAUNCH_CHECK(h);
         } else if (!(emax <= ORTH_CORR_MAX)) {
@@ -493,7 +501,7 @@ int orth_rows(ct_handle* h, Arena& ar, double* Z, double* W, int64_t c, int64_t 
               bool two_pass, unsigned long long* d_minpiv, int* d_fail, bool complete, uint64_t seed,
               int* replaced) {
     const int64_t cp = ob.cp;
-    row_normalize_kernel<<<(unsigned)ct_cdiv(c * 32, 256), 256, 0, h->stream>>>(Z, c, len); ct_note_launch();
+    ct_launch(h, row_normalize_kernel, (unsigned)ct_cdiv(c * 32, 256), 256, 0, Z, c, len); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     double* src = Z;
     double* dst = W;
@@ -508,7 +516,7 @@ int orth_rows(ct_handle* h, Arena& ar, double* Z, double* W, int64_t c, int64_t 
                 break;
             }
         }
-        chol_prepare_kernel<<<grid_n(h, cp * cp), 256, 0, h->stream>>>(ob.G, ob.Linv, c, cp); ct_note_launch();
+        ct_launch(h, chol_prepare_kernel, grid_n(h, cp * cp), 256, 0, ob.G, ob.Linv, c, cp); ct_note_launch();
         CT_LAUNCH_CHECK(h);
         CT_TRY(fac_gemm(h, c, c, len, src, len, src, len, 1, ob.G, cp, 1.0, 0.0, 1));
         CholMarks mk;
@@ -525,10 +533,10 @@ int orth_rows(ct_handle* h, Arena& ar, double* Z, double* W, int64_t c, int64_t 
             CT_CUDA(h, cudaStreamSynchronize(h->stream));
             if (nrep > 0) {
                 const unsigned g = (unsigned)std::min<int64_t>(nrep, (int64_t)h->num_sms * 4);
-                replace_rows_kernel<<<g, 256, 0, h->stream>>>(dst, len, ob.defrows, d_count, (int)cp, seed);
+                ct_launch(h, replace_rows_kernel, g, 256, 0, dst, len, ob.defrows, d_count, (int)cp, seed);
                 ct_note_launch();
                 CT_LAUNCH_CHECK(h);
-                row_normalize_kernel<<<(unsigned)ct_cdiv(c * 32, 256), 256, 0, h->stream>>>(dst, c, len);
+                ct_launch(h, row_normalize_kernel, (unsigned)ct_cdiv(c * 32, 256), 256, 0, dst, c, len);
                 ct_note_launch();
                 CT_LAUNCH_CHECK(h);
             }
@@ -589,7 +597,7 @@ int split_attempt(ct_handle* h, Arena& ar, const SplitBufs& sb, const double* M,
         return orth_rows(h, ar, Zr, Wr, c, len, ob, two, d_piv, d_fail, complete, seed + 0x9E37ull * ++call,
                          &replaced);
     };
-    split_flags_init_kernel<<<1, 32, 0, h->stream>>>(d_piv, d_fail); ct_note_launch();
+    ct_launch(h, split_flags_init_kernel, 1, 32, 0, d_piv, d_fail); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     // X: c rows over n (left-to-right) or over m (right-to-left).  The power
     // steps' intermediate bases need no second pass.
@@ -619,7 +627,7 @@ int split_attempt(ct_handle* h, Arena& ar, const SplitBufs& sb, const double* M,
         CT_TRY(orth(Z, basis_out, m, true));
         CT_TRY(ct_tc_gemm(h, ar, 0, 0, c, n, m, 1.0, basis_out, m, M, n, 0.0, Bout, n));
         ar.off = mark;
-        transpose_copy_kernel<<<grid_n(h, c * m), 256, 0, h->stream>>>(basis_out, c, m, Aout); ct_note_launch();
+        ct_launch(h, transpose_copy_kernel, grid_n(h, c * m), 256, 0, basis_out, c, m, Aout); ct_note_launch();
         CT_LAUNCH_CHECK(h);
     } else {
         // V = orth(X theta) -> B and basis_out; A = theta V^T
@@ -714,6 +722,7 @@ int ct_split_subspace(ct_handle* h, Arena& ar, const double* M, int64_t m, int64
 namespace {
 // Z[j][i] = A[i][j], j < k  (the first k columns of A[m,n] as rows)
 __global__ void cols_to_rows_kernel(const double* A, int64_t m, int64_t n, int64_t k, double* Z) {
+    ct_pdl();
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < k * m; t += (int64_t)gridDim.x * blockDim.x) {
         const int64_t j = t / m, i = t % m;
         Z[t] = A[i * n + j];
@@ -721,6 +730,7 @@ __global__ void cols_to_rows_kernel(const double* A, int64_t m, int64_t n, int64
 }
 // R[i][j] = 0 for j < i
 __global__ void zero_strict_lower_kernel(double* R, int64_t k, int64_t n) {
+    ct_pdl();
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < k * n; t += (int64_t)gridDim.x * blockDim.x) {
         const int64_t i = t / n, j = t % n;
         if (j < i) R[t] = 0.0;
@@ -748,16 +758,16 @@ int ct_qr_run(ct_handle* h, Arena& ar, const double* A, int64_t m, int64_t n, do
     if (!Z || !W || !ob.G || !ob.Linv || !ob.S || !ob.defrows) return CT_ERR_OOM;
     unsigned long long* d_piv = (unsigned long long*)(h->d_scalars + SC_SPLIT_PIV);
     int* d_fail = h->d_flags + FL_CHOL_FAIL;
-    split_flags_init_kernel<<<1, 32, 0, h->stream>>>(d_piv, d_fail); ct_note_launch();
+    ct_launch(h, split_flags_init_kernel, 1, 32, 0, d_piv, d_fail); ct_note_launch();
     CT_LAUNCH_CHECK(h);
-    cols_to_rows_kernel<<<grid_n(h, k * m), 256, 0, h->stream>>>(A, m, n, k, Z); ct_note_launch();
+    ct_launch(h, cols_to_rows_kernel, grid_n(h, k * m), 256, 0, A, m, n, k, Z); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     int nrep = 0;
     CT_TRY(orth_rows(h, ar, Z, W, k, m, ob, true, d_piv, d_fail, true, 0x51ED270B0ull, &nrep));
     CT_TRY(fac_gemm(h, k, n, m, W, m, A, n, 0, R, n, 1.0, 0.0, 0));   // R = Q^T A
-    transpose_copy_kernel<<<grid_n(h, k * m), 256, 0, h->stream>>>(W, k, m, Q); ct_note_launch();
+    ct_launch(h, transpose_copy_kernel, grid_n(h, k * m), 256, 0, W, k, m, Q); ct_note_launch();
     CT_LAUNCH_CHECK(h);
-    zero_strict_lower_kernel<<<grid_n(h, k * n), 256, 0, h->stream>>>(R, k, n); ct_note_launch();
+    ct_launch(h, zero_strict_lower_kernel, grid_n(h, k * n), 256, 0, R, k, n); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     int fail = 0;
     CT_CUDA(h, cudaMemcpyAsync(&fail, d_fail, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
@@ -772,6 +782,7 @@ int ct_qr_run(ct_handle* h, Arena& ar, const double* A, int64_t m, int64_t n, do
 
 namespace {
 __global__ void randn_fill_kernel(double* X, int64_t n, uint64_t seed) {
+    ct_pdl();
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x)
         X[t] = randn_at(seed, (uint64_t)t);
 }
@@ -789,7 +800,7 @@ int ct_cold_basis(ct_handle* h, const double* prev, int64_t c_prev, int64_t c, i
         c_prev = 0;
     const int64_t nr = (c - c_prev) * len;
     if (nr > 0) {
-        randn_fill_kernel<<<grid_n(h, nr), 256, 0, h->stream>>>(X + c_prev * len, nr, seed); ct_note_launch();
+        ct_launch(h, randn_fill_kernel, grid_n(h, nr), 256, 0, X + c_prev * len, nr, seed); ct_note_launch();
         CT_LAUNCH_CHECK(h);
     }
     return CT_OK;
@@ -800,7 +811,7 @@ int ct_cold_basis(ct_handle* h, const double* prev, int64_t c_prev, int64_t c, i
 int ct_basis_from_split(ct_handle* h, int mode, const double* Aout, const double* Bout, int64_t m, int64_t n,
                         int64_t c, double* basis) {
     if (mode == 0) {
-        transpose_copy_kernel<<<grid_n(h, m * c), 256, 0, h->stream>>>(Aout, m, c, basis); ct_note_launch();
+        ct_launch(h, transpose_copy_kernel, grid_n(h, m * c), 256, 0, Aout, m, c, basis); ct_note_launch();
         CT_LAUNCH_CHECK(h);
     } else {
         CT_CUDA(h, cudaMemcpyAsync(basis, Bout, (size_t)(c * n) * sizeof(double), cudaMemcpyDeviceToDevice,

@@ -82,6 +82,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     tc_gemm_kernel(const __grid_constant__ CUtensorMap tmAh, const __grid_constant__ CUtensorMap tmAl,
                    const __grid_constant__ CUtensorMap tmBh, const __grid_constant__ CUtensorMap tmBl, int M, int N,
                    int Kpad, TcEpi epi, const int* skip, int* status) {
+    ct_pdl();
     using L = TcSmem<BN, STAGES>;
     if (ct_skip(skip)) return;
     extern __shared__ uint8_t tc_smem_raw[];
@@ -285,6 +286,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     tc_gemm_persist_kernel(const __grid_constant__ CUtensorMap tmAh, const __grid_constant__ CUtensorMap tmAl,
                            const __grid_constant__ CUtensorMap tmBh, const __grid_constant__ CUtensorMap tmBl, int M,
                            int N, int Kpad, TcEpi epi, TcStreamK skd, int use_sk, const int* skip, int* status) {
+    ct_pdl();
     using L = TcSmem<BN, STAGES>;
     if (ct_skip(skip)) return;
     extern __shared__ uint8_t tc_smem_raw[];
@@ -644,6 +646,7 @@ __global__ void __launch_bounds__(tc_chunk_threads(BN), 1)
     tc_gemm_chunk_kernel(const __grid_constant__ CUtensorMap tmAh, const __grid_constant__ CUtensorMap tmAl,
                          const __grid_constant__ CUtensorMap tmBh, const __grid_constant__ CUtensorMap tmBl, int M,
                          int N, int Kpad, int kc, TcEpi epi, TcHybrid hy, const int* skip, int* status) {
+    ct_pdl_wait();
     using L = TcSmem<BN, STAGES>;
     constexpr int EPW = tc_chunk_epw(BN);
     constexpr int HC = BN / EPW;   // columns per epilogue warp
@@ -928,6 +931,7 @@ __global__ void __launch_bounds__(tc_chunk_threads(BN), 1)
             }
         }
     }
+    ct_pdl_next();
     __syncthreads();
     if (warp == 1) {
         tc_fence_after();
@@ -965,6 +969,7 @@ struct PackBatch {
 // dominate).  Measured (us, 32 x 32 tiles, one launch per operand / here): L and R of H_eff
 // at chi 1024, d 2, w 5: 48 / 29 (5.8 TB/s), theta 19 / 13.
 __global__ void __launch_bounds__(256) pack_split_kernel(const __grid_constant__ PackBatch pb, const int* skip) {
+    ct_pdl();
     if (ct_skip(skip)) return;
     __shared__ float tile[64][33];
     __shared__ int64_t roff[32], koff[64];
@@ -1024,6 +1029,7 @@ __global__ void __launch_bounds__(256) pack_split_kernel(const __grid_constant__
 
 // zeros in columns [k0, k0 + n) of the 2 planes' rows (the MPO legs write the others)
 __global__ void __launch_bounds__(256) pad_zero_kernel(float* hi, float* lo, int64_t rows, int64_t ld, int64_t k0, int n) {
+    ct_pdl();
     const int64_t total = rows * n;
     for (int64_t t = (int64_t)blockIdx.x * 256 + threadIdx.x; t < total; t += (int64_t)gridDim.x * 256) {
         const int64_t at = t / n * ld + k0 + t % n;
@@ -1047,6 +1053,7 @@ constexpr int MPOT_NT = 128, MPOT_JC = 32;
 // ([z * jch, z * jch + jch) of J).  Dynamic shared memory: that chunk of Wt as
 // FP32 [jch][K], then its jch output offsets (int64).
 __global__ void __launch_bounds__(MPOT_NT) mpo_tc_kernel(MpoTcDesc m, int64_t jch) {
+    ct_pdl();
     if (ct_skip(m.skip)) return;
     extern __shared__ float wsf[];
     const int64_t jbeg = (int64_t)blockIdx.z * jch;
@@ -1094,6 +1101,7 @@ __global__ void __launch_bounds__(MPOT_NT) mpo_tc_kernel(MpoTcDesc m, int64_t jc
 // Needs unit column strides and even I, sIo, sIk, sOo and output offsets.
 template <int JT>
 __global__ void __launch_bounds__(MPOT_NT) mpo_tc2_kernel(MpoTcDesc m) {
+    ct_pdl();
     if (ct_skip(m.skip)) return;
     extern __shared__ __align__(16) float wk[];   // [K][JT], then JT int64 offsets
     const int64_t jbeg = (int64_t)blockIdx.z * JT;
@@ -1220,6 +1228,7 @@ __device__ __forceinline__ bool nonfinite(float x) { return (__float_as_uint(x) 
 // 39 / 37, 129 117 / 36.
 constexpr int MPOC_NT = 256;
 __global__ void __launch_bounds__(MPOC_NT) mpo_tc_cols_kernel(MpoTcDesc m, int jch) {
+    ct_pdl();
     if (ct_skip(m.skip)) return;
     extern __shared__ __align__(16) float msm[];
     const int K = (int)m.K, tid = threadIdx.x;
@@ -1324,6 +1333,7 @@ __global__ void __launch_bounds__(MPOC_NT) mpo_tc_cols_kernel(MpoTcDesc m, int j
 // TB/s), 513 44 / 14, 65 8 / 6; Fermi-Hubbard chi 512 94 / 46; no zero weight, chi 1024, w 5 133 / 50.
 constexpr int MPOR_NT = 256, MPOR_LD = 33, MPOR_K = 8 * MPOR_LD;
 __global__ void __launch_bounds__(MPOR_NT) mpo_tc_rows_kernel(MpoTcDesc m, int jch) {
+    ct_pdl();
     if (ct_skip(m.skip)) return;
     extern __shared__ __align__(16) float msm[];
     const int K = (int)m.K, tid = threadIdx.x;
@@ -1637,7 +1647,7 @@ int tc_gemm_run(ct_handle* h, const SplitOperand& A, const SplitOperand& B, int6
             hy.cnt = h->tc_hy_cnt;
             grid = hy.tiles_dp > 0 ? h->num_sms : hy.gsk;
         }
-        tc_gemm_chunk_kernel<BN, STAGES><<<(unsigned)grid, tc_chunk_threads(BN), L::TOTAL, h->stream>>>(
+        ct_launch(h, tc_gemm_chunk_kernel<BN, STAGES>, (unsigned)grid, tc_chunk_threads(BN), L::TOTAL, 
             ta_h, ta_l, tb_h, tb_l, (int)M, (int)N, (int)A.ldk, kc, epi, hy, skip, h->d_status);
         ct_note_launch();
     } else if (tc_use_persistent()) {
@@ -1664,13 +1674,13 @@ int tc_gemm_run(ct_handle* h, const SplitOperand& A, const SplitOperand& B, int6
             sk.part = h->tc_sk_part;
             sk.flag = h->tc_sk_flag;
         }
-        tc_gemm_persist_kernel<BN, STAGES><<<(unsigned)grid, TC_THREADS, L::TOTAL, h->stream>>>(
+        ct_launch(h, tc_gemm_persist_kernel<BN, STAGES>, (unsigned)grid, TC_THREADS, L::TOTAL, 
             ta_h, ta_l, tb_h, tb_l, (int)M, (int)N, (int)A.ldk, epi, sk, use_sk ? 1 : 0, skip, h->d_status);
         ct_note_launch();
     } else {
         dim3 grid((unsigned)ct_cdiv(N, BN), (unsigned)ct_cdiv(M, TC_BM));
         if (grid.y > 65535) return CT_ERR_UNSUPPORTED;
-        tc_gemm_kernel<BN, STAGES><<<grid, TC_THREADS, L::TOTAL, h->stream>>>(
+        ct_launch(h, tc_gemm_kernel<BN, STAGES>, grid, TC_THREADS, L::TOTAL, 
             ta_h, ta_l, tb_h, tb_l, (int)M, (int)N, (int)A.ldk, epi, skip, h->d_status); ct_note_launch();
     }
     CT_LAUNCH_CHECK(h);
@@ -1751,7 +1761,7 @@ int pack_launch(ct_handle* h, std::initializer_list<PackDesc> ops, const int* sk
     }
     if (pb.n == 0) return CT_OK;
     if (pb.first[pb.n] > 0x7fffffff) return CT_ERR_UNSUPPORTED;
-    pack_split_kernel<<<(unsigned)pb.first[pb.n], 256, 0, h->stream>>>(pb, skip); ct_note_launch();
+    ct_launch(h, pack_split_kernel, (unsigned)pb.first[pb.n], 256, 0, pb, skip); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }
@@ -1784,7 +1794,7 @@ int pad_zero(ct_handle* h, const SplitOperand& s, int64_t period, int64_t k0) {
     if (k0 >= period) return CT_OK;
     const int64_t rows = s.rows * (s.ldk / period);
     const int64_t blocks = std::min<int64_t>(ct_cdiv(rows * (period - k0), 256), 16 * (int64_t)h->num_sms);
-    pad_zero_kernel<<<(unsigned)blocks, 256, 0, h->stream>>>(s.hi, s.lo, rows, period, k0, (int)(period - k0)); ct_note_launch();
+    ct_launch(h, pad_zero_kernel, (unsigned)blocks, 256, 0, s.hi, s.lo, rows, period, k0, (int)(period - k0)); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }
@@ -1799,7 +1809,7 @@ int mpo_tc2_launch(ct_handle* h, const MpoTcDesc& m) {
         attr_dev = h->device;
     }
     dim3 grid((unsigned)ct_cdiv(m.I / 2, MPOT_NT), (unsigned)m.O, (unsigned)ct_cdiv(m.J, JT));
-    mpo_tc2_kernel<JT><<<grid, MPOT_NT, smem, h->stream>>>(m); ct_note_launch();
+    ct_launch(h, mpo_tc2_kernel<JT>, grid, MPOT_NT, smem, m); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }
@@ -1828,7 +1838,11 @@ bool mpo_leg_launch(ct_handle* h, const MpoTcDesc& m, int nt, size_t xbytes, int
     }
     const int64_t per_sm = std::min<int64_t>((int64_t)(225 * 1024 / (smem + 1024)), 2048 / nt);
     const dim3 grid((unsigned)std::min<int64_t>(tiles, per_sm * h->num_sms), (unsigned)nz);
-    kernel<<<grid, nt, smem, h->stream>>>(m, (int)jch); ct_note_launch();
+    // (large legs in plain stream order: blocks set up beside the GEMM before made the left
+    // environment of chi 1024 slower, 324 us against 315; small ones gain)
+    if (tiles > grid.x) kernel<<<grid, nt, smem, h->stream>>>(m, (int)jch);
+    else ct_launch(h, kernel, grid, nt, smem, m, (int)jch);
+    ct_note_launch();
     *rc = [&]() -> int {
         CT_LAUNCH_CHECK(h);
         return CT_OK;
@@ -1882,7 +1896,7 @@ int mpo_tc_launch(ct_handle* h, const MpoTcDesc& m) {
         attr_dev = h->device;
     }
     dim3 grid((unsigned)ct_cdiv(m.I, MPOT_NT), (unsigned)m.O, (unsigned)nz);
-    mpo_tc_kernel<<<grid, MPOT_NT, smem, h->stream>>>(m, jch); ct_note_launch();
+    ct_launch(h, mpo_tc_kernel, grid, MPOT_NT, smem, m, jch); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }

@@ -24,6 +24,7 @@ template <int MODE>
 __global__ void __launch_bounds__(RT) partial_kernel(int64_t n, const double* __restrict__ x,
                                                      const double* __restrict__ y, double* partials,
                                                      const int* skip) {
+    ct_pdl();
     if (ct_skip(skip)) return;
     __shared__ double sm[32];
     double acc = 0.0;
@@ -68,6 +69,7 @@ __device__ double finish_sum(const double* partials, int np, double* sm) {
 // ---- phase 2 finishers ------------------------------------------------------
 __global__ void __launch_bounds__(RT) finish_store_kernel(const double* partials, int np, double* out,
                                                           const int* skip) {
+    ct_pdl();
     if (ct_skip(skip)) return;
     __shared__ double sm[32];
     const double s = finish_sum(partials, np, sm);
@@ -85,14 +87,17 @@ int grid_for(ct_handle* h, int64_t n) {
 
 // ---- elementwise -------------------------------------------------------------
 __global__ void axpy_kernel(int64_t n, double alpha, const double* x, double* y) {
+    ct_pdl();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         y[i] = fma(alpha, x[i], y[i]);
 }
 __global__ void scale_kernel(int64_t n, double alpha, double* x) {
+    ct_pdl();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         x[i] *= alpha;
 }
 __global__ void fill_kernel(double* x, int64_t n, double v) {
+    ct_pdl();
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         x[i] = v;
 }
@@ -110,6 +115,7 @@ __device__ __forceinline__ double block_reciprocal(double x) {
 // y = x / sqrt(*nsq); status zero_code when sqrt(nsq) < 1e-14 (dmrg.mojo:605-611)
 __global__ void scale_inv_sqrt_kernel(int64_t n, const double* x, double* y, const double* nsq,
                                       const int* skip, int* status, int zero_code) {
+    ct_pdl();
     if (ct_skip(skip)) return;
     __shared__ double nrm_s;
     if (threadIdx.x == 0) nrm_s = sqrt(*nsq);
@@ -126,11 +132,13 @@ __global__ void scale_inv_sqrt_kernel(int64_t n, const double* x, double* y, con
 }
 
 __global__ void check_finite_kernel(const double* x, int* status, const int* skip) {
+    ct_pdl();
     if (ct_skip(skip)) return;
     if (!isfinite(*x)) ct_set_status(status, CT_ERR_NONFINITE);
 }
 
 __global__ void identity_env_kernel(double* E, int64_t w, int64_t D) {
+    ct_pdl();
     const int64_t n = w * D * D;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
         const int64_t r = (t / D) % D, c = t % D;
@@ -139,6 +147,7 @@ __global__ void identity_env_kernel(double* E, int64_t w, int64_t D) {
 }
 
 __global__ void identity_env_rect_kernel(double* E, int64_t w, int64_t Dk, int64_t Db) {
+    ct_pdl();
     const int64_t n = w * Dk * Db;
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (int64_t)gridDim.x * blockDim.x) {
         const int64_t r = (t / Db) % Dk, c = t % Db;
@@ -153,6 +162,7 @@ struct PermArgs {
     int64_t in_stride_of_out_axis[6];
 };
 __global__ void permute_kernel(const double* in, double* out, PermArgs a) {
+    ct_pdl();
     for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < a.n; t += (int64_t)gridDim.x * blockDim.x) {
         int64_t rem = t, src = 0;
         for (int ax = a.rank - 1; ax >= 0; --ax) {
@@ -172,6 +182,7 @@ template <bool NORM>
 __global__ void __launch_bounds__(RT) lanczos_update_kernel(int64_t n, double* w, const double* vj,
                                                             const double* vjm1, const double* scalars,
                                                             int j, double* partials, const int* skip) {
+    ct_pdl();
     if (ct_skip(skip)) return;
     __shared__ double sm[32];
     const double a = scalars[SC_ALPHA + j];
@@ -220,6 +231,7 @@ __global__ void __launch_bounds__(RT) lanczos_update_kernel(int64_t n, double* w
 // beta_j = sqrt(sum); breakdown test beta < 100 n eps (dmrg.mojo:630-673)
 __global__ void __launch_bounds__(RT) lanczos_beta_finish(const double* partials, int np, double* scalars,
                                                           int* flags, int j, double thr, const int* skip) {
+    ct_pdl();
     if (ct_skip(skip)) return;
     __shared__ double sm[32];
     const double s = finish_sum(partials, np, sm);
@@ -236,6 +248,7 @@ __global__ void __launch_bounds__(RT) lanczos_beta_finish(const double* partials
 
 __global__ void lanczos_next_kernel(int64_t n, const double* w, double* vnext, const double* scalars, int j,
                                     const int* skip) {
+    ct_pdl();
     if (ct_skip(skip)) return;
     const double inv = block_reciprocal(scalars[SC_BETA + j]);
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
@@ -581,6 +594,7 @@ __global__ void __launch_bounds__(RT) lanczos_alpha_kernel(int64_t n, const doub
                                                            const double* __restrict__ w, double* partials,
                                                            unsigned* counter, double* scalars, int j,
                                                            const int* skip) {
+    ct_pdl();
     if (ct_skip(skip)) return;
     __shared__ double sm[32];
     double acc = 0.0;
@@ -616,6 +630,7 @@ __global__ void __launch_bounds__(RT) cgs_dots_kernel(int64_t n, const double* _
                                                       const double* __restrict__ V, int64_t ldv, int nvec, int vec2,
                                                       double* partials, unsigned* counter, double* coeff,
                                                       const int* skip) {
+    ct_pdl();
     if (ct_skip(skip)) return;
     cgs_dots_dev(n, w, V, ldv, nvec, vec2, partials, counter, coeff);
 }
@@ -624,6 +639,7 @@ __global__ void __launch_bounds__(RT) cgs_update_kernel(int64_t n, double* __res
                                                         const double* coeff, double* partials, unsigned* counter,
                                                         double* scalars, int* flags, int j, double thr,
                                                         const int* skip) {
+    ct_pdl();
     if (ct_skip(skip)) return;
     cgs_update_dev(n, w, V, ldv, nvec, vec2, coeff, partials, counter, scalars, flags, j, thr);
 }
@@ -633,6 +649,7 @@ __global__ void __launch_bounds__(RT) cgs32_dots_kernel(int64_t n, const double*
                                                         const float* __restrict__ V, int64_t ldv, int nvec, int vec4,
                                                         double* partials, unsigned* counter, double* coeff,
                                                         const int* skip) {
+    ct_pdl();
     if (ct_skip(skip)) return;
     cgs32_dots_dev(n, w, V, ldv, nvec, vec4, partials, counter, coeff);
 }
@@ -641,6 +658,7 @@ __global__ void __launch_bounds__(RT) cgs32_update_kernel(int64_t n, double* __r
                                                           const double* coeff, double* partials, unsigned* counter,
                                                           double* scalars, int* flags, int j, double thr,
                                                           const int* skip, double ratio64) {
+    ct_pdl();
     if (ct_skip(skip)) return;
     cgs32_update_dev(n, w, V, ldv, nvec, vec4, coeff, partials, counter, scalars, flags, j, thr, 0, ratio64);
 }
@@ -653,6 +671,7 @@ __global__ void __launch_bounds__(RT) cgs_redo_dots_kernel(int64_t n, const doub
                                                            int64_t ldv, int nvec, int vec2, int vec4,
                                                            double* partials, unsigned* counter, double* coeff,
                                                            const int* skip, const int* flags) {
+    ct_pdl();
     if (ct_skip(skip)) return;
     if (*(volatile const int*)(flags + FL_REDO64))
         cgs_dots_dev(n, w, V, ldv, nvec, vec2, partials, counter, coeff);
@@ -665,6 +684,7 @@ __global__ void __launch_bounds__(RT) cgs_redo_update_kernel(int64_t n, double* 
                                                              int vec2, int vec4, const double* coeff,
                                                              double* partials, unsigned* counter, double* scalars,
                                                              int* flags, int j, double thr, const int* skip) {
+    ct_pdl();
     if (ct_skip(skip)) return;
     if (*(volatile const int*)(flags + FL_REDO64))
         cgs_update_dev(n, w, V, ldv, nvec, vec2, coeff, partials, counter, scalars, flags, j, thr);
@@ -675,6 +695,7 @@ __global__ void __launch_bounds__(RT) cgs_redo_update_kernel(int64_t n, double* 
 // v_{j+1} = w / beta_j in FP64 and its FP32 copy
 __global__ void lanczos_next32_kernel(int64_t n, const double* w, double* vnext, float* vnext32,
                                       const double* scalars, int j, const int* skip) {
+    ct_pdl();
     if (ct_skip(skip)) return;
     const double inv = block_reciprocal(scalars[SC_BETA + j]);
     const int64_t stride = (int64_t)gridDim.x * blockDim.x;
@@ -705,6 +726,7 @@ __global__ void lanczos_next32_kernel(int64_t n, const double* w, double* vnext,
 }
 
 __global__ void f64_to_f32_copy_kernel(int64_t n, const double* x, float* y, const int* skip) {
+    ct_pdl();
     if (ct_skip(skip)) return;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
         y[i] = (float)x[i];
@@ -713,6 +735,7 @@ __global__ void f64_to_f32_copy_kernel(int64_t n, const double* x, float* y, con
 // Ritz vector: out = sum_{i < numiter} c_i V[i]
 __global__ void ritz_kernel(int64_t n, const double* V, int64_t ldv, const double* scalars, const int* flags,
                             double* out) {
+    ct_pdl();
     const int nk = flags[FL_NUMITER];
     for (int64_t x = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; x < n; x += (int64_t)gridDim.x * blockDim.x) {
         double acc = 0.0;
@@ -727,6 +750,7 @@ __global__ void ritz_kernel(int64_t n, const double* V, int64_t ldv, const doubl
 // strict '>' scan from (0,1).
 __global__ void tridiag_jacobi_kernel(double* scalars, int* flags, int* status, double tol, int max_rot,
                                       int converged_mode) {
+    ct_pdl();
     extern __shared__ double tsm[];
     const int n = flags[FL_NUMITER];
     const int lane = threadIdx.x;
@@ -894,6 +918,7 @@ __device__ void tridiag_narrow(bool below, double* lo, double* hi, unsigned* mas
 }
 
 __global__ void __launch_bounds__(TB_NT) tridiag_bisect_kernel(double* scalars, const int* flags, int* status) {
+    ct_pdl();
     __shared__ double a[CT_MAX_KRYLOV], b[CT_MAX_KRYLOV], x[CT_MAX_KRYLOV];
     __shared__ double as[CT_MAX_KRYLOV], b2s[CT_MAX_KRYLOV];   // T scaled; then the pivots and their reciprocals
     __shared__ double b2[CT_MAX_KRYLOV], l[CT_MAX_KRYLOV];
@@ -1059,6 +1084,7 @@ __global__ void __launch_bounds__(TB_NT) tridiag_bisect_kernel(double* scalars, 
 }
 
 __global__ void init_lanczos_flags(int* flags, int max_iter) {
+    ct_pdl();
     flags[FL_STOP] = 0;
     flags[FL_NUMITER] = max_iter;
 }
@@ -1075,36 +1101,36 @@ int elem_grid(ct_handle* h, int64_t n) {
 
 int ct_reduce_dot(ct_handle* h, int64_t n, const double* x, const double* y, double* d_out, const int* skip) {
     const int g = grid_for(h, n);
-    partial_kernel<0><<<g, RT, 0, h->stream>>>(n, x, y, h->d_partials, skip); ct_note_launch();
-    finish_store_kernel<<<1, RT, 0, h->stream>>>(h->d_partials, g, d_out, skip); ct_note_launch();
+    ct_launch(h, partial_kernel<0>, g, RT, 0, n, x, y, h->d_partials, skip); ct_note_launch();
+    ct_launch(h, finish_store_kernel, 1, RT, 0, h->d_partials, g, d_out, skip); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }
 
 int ct_reduce_nrm2sq(ct_handle* h, int64_t n, const double* x, double* d_out, const int* skip) {
     const int g = grid_for(h, n);
-    partial_kernel<1><<<g, RT, 0, h->stream>>>(n, x, nullptr, h->d_partials, skip); ct_note_launch();
-    finish_store_kernel<<<1, RT, 0, h->stream>>>(h->d_partials, g, d_out, skip); ct_note_launch();
+    ct_launch(h, partial_kernel<1>, g, RT, 0, n, x, nullptr, h->d_partials, skip); ct_note_launch();
+    ct_launch(h, finish_store_kernel, 1, RT, 0, h->d_partials, g, d_out, skip); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }
 
 int ct_scale_by_inv_sqrt(ct_handle* h, int64_t n, const double* x, double* y, const double* d_nsq,
                          const int* skip, int zero_code) {
-    scale_inv_sqrt_kernel<<<elem_grid(h, n), 256, 0, h->stream>>>(n, x, y, d_nsq, skip, h->d_status, zero_code); ct_note_launch();
+    ct_launch(h, scale_inv_sqrt_kernel, elem_grid(h, n), 256, 0, n, x, y, d_nsq, skip, h->d_status, zero_code); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }
 
 int ct_fill(ct_handle* h, double* x, int64_t n, double v) {
     if (n <= 0) return CT_OK;
-    fill_kernel<<<elem_grid(h, n), 256, 0, h->stream>>>(x, n, v); ct_note_launch();
+    ct_launch(h, fill_kernel, elem_grid(h, n), 256, 0, x, n, v); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }
 
 int ct_check_finite(ct_handle* h, const double* d_x, const int* skip) {
-    check_finite_kernel<<<1, 1, 0, h->stream>>>(d_x, h->d_status, skip); ct_note_launch();
+    ct_launch(h, check_finite_kernel, 1, 1, 0, d_x, h->d_status, skip); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }
@@ -1118,7 +1144,7 @@ int ct_copy(ct_handle* h, double* dst, const double* src, int64_t n) {
 int ct_identity_env(ct_handle* h, double* E, int64_t w, int64_t D) {
     const int64_t n = w * D * D;
     if (n <= 0) return CT_OK;
-    identity_env_kernel<<<elem_grid(h, n), 256, 0, h->stream>>>(E, w, D); ct_note_launch();
+    ct_launch(h, identity_env_kernel, elem_grid(h, n), 256, 0, E, w, D); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }
@@ -1126,7 +1152,7 @@ int ct_identity_env(ct_handle* h, double* E, int64_t w, int64_t D) {
 int ct_identity_env_rect(ct_handle* h, double* E, int64_t w, int64_t Dk, int64_t Db) {
     const int64_t n = w * Dk * Db;
     if (n <= 0) return CT_OK;
-    identity_env_rect_kernel<<<elem_grid(h, n), 256, 0, h->stream>>>(E, w, Dk, Db); ct_note_launch();
+    ct_launch(h, identity_env_rect_kernel, elem_grid(h, n), 256, 0, E, w, Dk, Db); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }
@@ -1152,24 +1178,24 @@ int ct_permute_launch(ct_handle* h, const double* in, double* out, int rank, con
         a.in_stride_of_out_axis[ax] = in_stride[p];
     }
     if (a.n == 0) return CT_OK;
-    permute_kernel<<<elem_grid(h, a.n), 256, 0, h->stream>>>(in, out, a); ct_note_launch();
+    ct_launch(h, permute_kernel, elem_grid(h, a.n), 256, 0, in, out, a); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }
 
 int ct_vec_axpy_launch(ct_handle* h, int64_t n, double alpha, const double* x, double* y) {
-    axpy_kernel<<<elem_grid(h, n), 256, 0, h->stream>>>(n, alpha, x, y); ct_note_launch();
+    ct_launch(h, axpy_kernel, elem_grid(h, n), 256, 0, n, alpha, x, y); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }
 int ct_vec_scale_launch(ct_handle* h, int64_t n, double alpha, double* x) {
-    scale_kernel<<<elem_grid(h, n), 256, 0, h->stream>>>(n, alpha, x); ct_note_launch();
+    ct_launch(h, scale_kernel, elem_grid(h, n), 256, 0, n, alpha, x); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }
 
 int ct_lanczos_init(ct_handle* h, int max_iter) {
-    init_lanczos_flags<<<1, 1, 0, h->stream>>>(h->d_flags, max_iter); ct_note_launch();
+    ct_launch(h, init_lanczos_flags, 1, 1, 0, h->d_flags, max_iter); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }
@@ -1177,7 +1203,7 @@ int ct_lanczos_init(ct_handle* h, int max_iter) {
 int ct_lanczos_alpha(ct_handle* h, int64_t n, const double* vj, const double* w, int j, const int* skip) {
     const int g = grid_for(h, n);
     unsigned* counter = reinterpret_cast<unsigned*>(h->d_flags + FL_CNT);
-    lanczos_alpha_kernel<<<g, RT, 0, h->stream>>>(n, vj, w, h->d_partials, counter, h->d_scalars, j, skip);
+    ct_launch(h, lanczos_alpha_kernel, g, RT, 0, n, vj, w, h->d_partials, counter, h->d_scalars, j, skip);
     ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
@@ -1186,8 +1212,8 @@ int ct_lanczos_alpha(ct_handle* h, int64_t n, const double* vj, const double* w,
 int ct_lanczos_update(ct_handle* h, int64_t n, double* w, const double* vj, const double* vjm1, int j,
                       double beta_threshold, const int* skip) {
     const int g = grid_for(h, n);
-    lanczos_update_kernel<true><<<g, RT, 0, h->stream>>>(n, w, vj, vjm1, h->d_scalars, j, h->d_partials, skip); ct_note_launch();
-    lanczos_beta_finish<<<1, RT, 0, h->stream>>>(h->d_partials, g, h->d_scalars, h->d_flags, j,
+    ct_launch(h, lanczos_update_kernel<true>, g, RT, 0, n, w, vj, vjm1, h->d_scalars, j, h->d_partials, skip); ct_note_launch();
+    ct_launch(h, lanczos_beta_finish, 1, RT, 0, h->d_partials, g, h->d_scalars, h->d_flags, j,
                                                  beta_threshold, skip); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
@@ -1205,9 +1231,9 @@ int ct_lanczos_reorth_pass(ct_handle* h, int64_t n, double* w, const double* V, 
     const int vec2 = ((n & 1) == 0 && (ldv & 1) == 0 && aligned16(w) && aligned16(V)) ? 1 : 0;
     unsigned* counter = reinterpret_cast<unsigned*>(h->d_flags + FL_CNT);
     double* coeff = h->d_scalars + SC_MISC;
-    cgs_dots_kernel<<<g, RT, 0, h->stream>>>(n, w, V, ldv, nvec, vec2, h->d_partials, counter, coeff, skip);
+    ct_launch(h, cgs_dots_kernel, g, RT, 0, n, w, V, ldv, nvec, vec2, h->d_partials, counter, coeff, skip);
     ct_note_launch();
-    cgs_update_kernel<<<g, RT, 0, h->stream>>>(n, w, V, ldv, nvec, vec2, coeff, h->d_partials, counter,
+    ct_launch(h, cgs_update_kernel, g, RT, 0, n, w, V, ldv, nvec, vec2, coeff, h->d_partials, counter,
                                                h->d_scalars, h->d_flags, j, beta_threshold, skip);
     ct_note_launch();
     CT_LAUNCH_CHECK(h);
@@ -1229,9 +1255,9 @@ int ct_lanczos_reorth_pass32(ct_handle* h, int64_t n, double* w, const float* V3
     // the dots: two blocks per SM keep ~150 KB of loads in flight per SM, and fewer blocks
     // mean fewer block reductions (FP64)
     const int gd = g < 2 * h->num_sms ? g : 2 * h->num_sms;
-    cgs32_dots_kernel<<<gd, RT, 0, h->stream>>>(n, w, V32, ldv, nvec, vec4, h->d_partials, counter, coeff, skip);
+    ct_launch(h, cgs32_dots_kernel, gd, RT, 0, n, w, V32, ldv, nvec, vec4, h->d_partials, counter, coeff, skip);
     ct_note_launch();
-    cgs32_update_kernel<<<g, RT, 0, h->stream>>>(n, w, V32, ldv, nvec, vec4, coeff, h->d_partials, counter,
+    ct_launch(h, cgs32_update_kernel, g, RT, 0, n, w, V32, ldv, nvec, vec4, coeff, h->d_partials, counter,
                                                  h->d_scalars, h->d_flags, j, beta_threshold, skip, ratio64);
     ct_note_launch();
     CT_LAUNCH_CHECK(h);
@@ -1250,10 +1276,10 @@ int ct_lanczos_reorth_redo(ct_handle* h, int64_t n, double* w, const double* V, 
     const int vec4 = ((n & 3) == 0 && (ldv & 3) == 0 && aligned16(w) && aligned16(V32)) ? 1 : 0;
     unsigned* counter = reinterpret_cast<unsigned*>(h->d_flags + FL_CNT);
     double* coeff = h->d_scalars + SC_MISC;
-    cgs_redo_dots_kernel<<<g, RT, 0, h->stream>>>(n, w, V, V32, ldv, nvec, vec2, vec4, h->d_partials, counter, coeff,
+    ct_launch(h, cgs_redo_dots_kernel, g, RT, 0, n, w, V, V32, ldv, nvec, vec2, vec4, h->d_partials, counter, coeff,
                                                   skip, h->d_flags);
     ct_note_launch();
-    cgs_redo_update_kernel<<<g, RT, 0, h->stream>>>(n, w, V, V32, ldv, nvec, vec2, vec4, coeff, h->d_partials,
+    ct_launch(h, cgs_redo_update_kernel, g, RT, 0, n, w, V, V32, ldv, nvec, vec2, vec4, coeff, h->d_partials,
                                                     counter, h->d_scalars, h->d_flags, j, beta_threshold, skip);
     ct_note_launch();
     CT_LAUNCH_CHECK(h);
@@ -1262,14 +1288,14 @@ int ct_lanczos_reorth_redo(ct_handle* h, int64_t n, double* w, const double* V, 
 
 int ct_lanczos_next32(ct_handle* h, int64_t n, const double* w, double* vnext, float* vnext32, int j,
                       const int* skip) {
-    lanczos_next32_kernel<<<elem_grid(h, n), 256, 0, h->stream>>>(n, w, vnext, vnext32, h->d_scalars, j, skip);
+    ct_launch(h, lanczos_next32_kernel, elem_grid(h, n), 256, 0, n, w, vnext, vnext32, h->d_scalars, j, skip);
     ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }
 
 int ct_f64_to_f32(ct_handle* h, int64_t n, const double* x, float* y, const int* skip) {
-    f64_to_f32_copy_kernel<<<elem_grid(h, n), 256, 0, h->stream>>>(n, x, y, skip); ct_note_launch();
+    ct_launch(h, f64_to_f32_copy_kernel, elem_grid(h, n), 256, 0, n, x, y, skip); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }
@@ -1279,14 +1305,14 @@ int ct_f64_to_f32(ct_handle* h, int64_t n, const double* x, float* y, const int*
 int ct_lanczos_update_nonorm(ct_handle* h, int64_t n, double* w, const double* vj, const double* vjm1, int j,
                              const int* skip) {
     const int g = grid_for(h, n);
-    lanczos_update_kernel<false><<<g, RT, 0, h->stream>>>(n, w, vj, vjm1, h->d_scalars, j, h->d_partials, skip);
+    ct_launch(h, lanczos_update_kernel<false>, g, RT, 0, n, w, vj, vjm1, h->d_scalars, j, h->d_partials, skip);
     ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }
 
 int ct_lanczos_next(ct_handle* h, int64_t n, const double* w, double* vnext, int j, const int* skip) {
-    lanczos_next_kernel<<<elem_grid(h, n), 256, 0, h->stream>>>(n, w, vnext, h->d_scalars, j, skip); ct_note_launch();
+    ct_launch(h, lanczos_next_kernel, elem_grid(h, n), 256, 0, n, w, vnext, h->d_scalars, j, skip); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }
@@ -1301,17 +1327,17 @@ int ct_tridiag_eig(ct_handle* h, int max_iter, double tol, int max_rotations) {
         attr = true;
     }
     if (max_rotations <= 0) {
-        tridiag_bisect_kernel<<<1, TB_NT, 0, h->stream>>>(h->d_scalars, h->d_flags, h->d_status); ct_note_launch();
+        ct_launch(h, tridiag_bisect_kernel, 1, TB_NT, 0, h->d_scalars, h->d_flags, h->d_status); ct_note_launch();
         CT_LAUNCH_CHECK(h);
         return CT_OK;
     }
-    tridiag_jacobi_kernel<<<1, 32, smem, h->stream>>>(h->d_scalars, h->d_flags, h->d_status, tol, max_rotations, 0); ct_note_launch();
+    ct_launch(h, tridiag_jacobi_kernel, 1, 32, smem, h->d_scalars, h->d_flags, h->d_status, tol, max_rotations, 0); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }
 
 int ct_ritz(ct_handle* h, int64_t n, const double* V, int64_t ldv, double* out) {
-    ritz_kernel<<<elem_grid(h, n), 256, 0, h->stream>>>(n, V, ldv, h->d_scalars, h->d_flags, out); ct_note_launch();
+    ct_launch(h, ritz_kernel, elem_grid(h, n), 256, 0, n, V, ldv, h->d_scalars, h->d_flags, out); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }

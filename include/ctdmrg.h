@@ -324,8 +324,8 @@ CT_API int ct_svd_split_warm(ct_handle* h, const double* theta, int64_t Dl, int6
 /* ---- allocation-free H_eff apply (no counterpart in the reference) --------
  * For callers that cannot let a library allocate device memory, e.g. a Mojo/MAX
  * host whose DeviceContext allocator owns every buffer, or a caller under a
- * fixed device-memory budget.  Same FP64 result as ct_heff2_apply (same
- * kernels), enqueued on `stream`; takes no handle and calls no cudaMalloc.
+ * fixed device-memory budget.  Same FP64 result as ct_heff2_apply to rounding
+ * (the same kernels, with every product on FP64 FMAs), enqueued on `stream`; takes no handle and calls no cudaMalloc.
  * Its intermediates live in one static device array of
  * CT_NOALLOC_SCRATCH_DOUBLES doubles (16 MiB) held by every GPU that loads the
  * library until exit; sizes that need more than that
