@@ -68,7 +68,7 @@ namespace {
 // per chi=1024 warm split, with the earlier three-barrier leaf): the extra
 // recursion level's small products cost more than the leaves saved.
 constexpr int CH_NB = 64;
-constexpr int CH_THREADS = 288;      // leaf: 8 row warps and the pivot warp
+constexpr int CH_THREADS = 384;      // leaf: the pivot warp, and nine row warps on the other SM quarters
 constexpr int FL_CHOL_FAIL = 100;    // d_flags slot: non-positive pivot seen
 constexpr int FL_DEF_COUNT = 101;    // d_flags slot: rows marked for replacement in a first pass
 // smallest accepted Cholesky pivot of a first pass (the squared share of a
@@ -212,24 +212,24 @@ __device__ __forceinline__ void chol_pivot(double p, int j, double* pv, long lon
 // where a_lj is column j of the trailing matrix, snapshotted when the step before
 // finished it (col[], double-buffered).  Column j of L is a_ij / sqrt(p_j) (stored
 // unscaled during the sweep, scaled once at the end), row j of L^{-1} is
-// R[j][k] / sqrt(p_j) (R[j][j] = 1).  A ninth warp forms the next pivot at the start
-// of each step, p_{j+1} = a_{j+1,j+1} - a_{j+1,j}^2 / p_j (the same arithmetic as the
-// row update, whose owner leaves that element unwritten: nothing reads it again), and
-// its 1/p, sqrt(p), 1/sqrt(p) (double-buffered), while warps 0..7 run the step's
-// multiply-adds: the pivot chain is no longer behind any row's.  Warp w < 8 owns the
-// rows i = w (mod 8), up to 8 per step, lane l the positions l and l + 32 of each; a
-// warp loads all its rows before its multiply-adds, so their latencies overlap.
-// On this part FP64 issues at ~1/64 of the FP32 rate: the sweep's cost is its FP64
-// instruction count (about 2.8k warp-instructions of multiply-adds) and one barrier
-// per column.
+// R[j][k] / sqrt(p_j) (R[j][j] = 1; both scaled at the end).  Warp 0 forms the next
+// pivot during each step, p_{j+1} = a_{j+1,j+1} - a_{j+1,j}^2 / p_j (the same arithmetic
+// as the row update, whose owner leaves that element unwritten: nothing reads it again),
+// and its 1/p, sqrt(p), 1/sqrt(p) (double-buffered).  Nine warps own the rows i = rw (mod
+// 9), up to 8 per step, lane l the positions l and l + 32 of each; a warp loads all its
+// rows before its multiply-adds, so their latencies overlap.
+// What bounds it: FP64 issues at one warp instruction per 64 clocks and SM quarter; the
+// pivot's eleven dependent ones take 700 clocks a step, the rows' multiply-adds 1100 on
+// three quarters.  The pivot has a quarter of the SM to itself (the row warps are those
+// with warp % 4 != 0): beside two row warps each of its instructions waits its turn,
+// which set the step (75 us a leaf so, 68 here).
 __global__ void __launch_bounds__(CH_THREADS) chol_diag_kernel(double* G, double* Linv, int64_t ld,
                                                         unsigned long long* minpiv, int* fail, int* defrows,
                                                         int* defcount, int64_t row0, double floor) {
     ct_pdl();
-    extern __shared__ __align__(16) unsigned char chol_smem_raw[];   // three CH_NB x (CH_NB + 1) tiles
+    extern __shared__ __align__(16) unsigned char chol_smem_raw[];   // two CH_NB x (CH_NB + 1) tiles
     double(*R)[CH_NB + 1] = reinterpret_cast<double(*)[CH_NB + 1]>(chol_smem_raw);
     double(*Ls)[CH_NB + 1] = R + CH_NB;
-    double(*Xs)[CH_NB + 1] = Ls + CH_NB;
     __shared__ double col[2][CH_NB];
     __shared__ double piv[2][3];
     __shared__ double dinv[CH_NB];
@@ -241,7 +241,6 @@ __global__ void __launch_bounds__(CH_THREADS) chol_diag_kernel(double* G, double
         const double g = (j <= i) ? G[i * ld + j] : 0.0;
         R[i][j] = g;
         Ls[i][j] = 0.0;
-        Xs[i][j] = 0.0;
         if (j == 0) col[0][i] = g;
     }
     if (t == 0) {
@@ -249,39 +248,38 @@ __global__ void __launch_bounds__(CH_THREADS) chol_diag_kernel(double* G, double
         chol_pivot(G[0], 0, piv[0], &mp, fail, defrows, defcount, row0, floor_bits);
     }
     __syncthreads();
+    if (t == 0) {
+        Ls[0][0] = piv[0][1];
+        dinv[0] = piv[0][2];
+    }
     const int k0 = lane, k1 = lane + 32;
+    const int rw = (warp & 3) ? (warp >> 2) * 3 + (warp & 3) - 1 : -1;   // row warp
     for (int j = 0; j < CH_NB; ++j) {
         const int b = j & 1;
         const double inv_p = piv[b][0];
-        if (warp == 8) {
+        if (rw < 0) {
             // the pivot of step j + 1 from a_{j+1,j} and a_{j+1,j+1}, both final since step j - 1
-            if (lane == 0 && j + 1 < CH_NB) {
+            if (t == 0 && j + 1 < CH_NB) {
                 const double a = col[b][j + 1];
                 const double v = fma(-(a * inv_p), a, R[j + 1][j + 1]);
-                chol_pivot(v, j + 1, piv[b ^ 1], &mp, fail, defrows, defcount, row0, floor_bits);
+                double* pv = piv[b ^ 1];
+                chol_pivot(v, j + 1, pv, &mp, fail, defrows, defcount, row0, floor_bits);
+                Ls[j + 1][j + 1] = pv[1];
+                dinv[j + 1] = pv[2];
             }
             __syncthreads();
             continue;
         }
-        // this warp's rows i > j, i = warp (mod 8); lane q < 8 forms row q's multiplier and
-        // keeps its entry of L's column j (unscaled)
-        const int i0 = j + 1 + ((warp - (j + 1)) & 7);
+        // this warp's rows i > j, i = rw (mod 9); lane q < 8 forms row q's multiplier and keeps
+        // its entry of L's column j (unscaled)
+        const int i0 = j + 1 + (rw + 72 - (j + 1)) % 9;
         double fq = 0.0;
         {
-            const int iq = i0 + 8 * lane;
+            const int iq = i0 + 9 * lane;
             if (lane < 8 && iq < CH_NB) {
                 const double a = col[b][iq];
                 fq = a * inv_p;
                 Ls[iq][j] = a;
-            }
-        }
-        if (warp == (j & 7)) {
-            // row j is final: its row of L^{-1} and the diagonal of L
-            const double inv_d = piv[b][2];
-            for (int k = lane; k <= j; k += 32) Xs[j][k] = (k == j ? 1.0 : R[j][k]) * inv_d;
-            if (lane == 0) {
-                Ls[j][j] = piv[b][1];
-                dinv[j] = inv_d;
             }
         }
         // the sources of positions k0, k1 are the same for every row
@@ -290,16 +288,16 @@ __global__ void __launch_bounds__(CH_THREADS) chol_diag_kernel(double* G, double
         double base0[8], base1[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-            const int i = i0 + 8 * q;
+            const int i = i0 + 9 * q;
             base0[q] = (i < CH_NB && k0 <= i && k0 != j) ? R[i][k0] : 0.0;
             base1[q] = (i < CH_NB && k1 <= i && k1 != j) ? R[i][k1] : 0.0;
         }
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-            const int i = i0 + 8 * q;
+            const int i = i0 + 9 * q;
             if (i >= CH_NB) break;   // warp-uniform
             const double f = __shfl_sync(0xffffffffu, fq, q);
-            // (the next pivot's element, i == k == j + 1, is warp 8's)
+            // (the next pivot's element, i == k == j + 1, is the pivot warp's)
             if (k0 <= i && !(i == j + 1 && k0 == j + 1)) {
                 const double v = fma(-f, s0, base0[q]);
                 R[i][k0] = v;
@@ -317,7 +315,7 @@ __global__ void __launch_bounds__(CH_THREADS) chol_diag_kernel(double* G, double
     for (int e = t; e < CH_NB * CH_NB; e += blockDim.x) {
         const int i = e / CH_NB, j = e % CH_NB;
         G[i * ld + j] = i > j ? Ls[i][j] * dinv[j] : Ls[i][j];
-        Linv[i * ld + j] = Xs[i][j];
+        Linv[i * ld + j] = j <= i ? (j < i ? R[i][j] : 1.0) * dinv[i] : 0.0;
     }
 }
 
@@ -385,7 +383,7 @@ struct CholMarks {
 int chol_inv(ct_handle* h, double* G, double* Linv, int64_t ld, int64_t n, double* S,
              unsigned long long* d_minpiv, int* d_fail, const CholMarks& mk, int64_t row0) {
     if (n <= CH_NB) {
-        constexpr int smem = 3 * CH_NB * (CH_NB + 1) * (int)sizeof(double);
+        constexpr int smem = 2 * CH_NB * (CH_NB + 1) * (int)sizeof(double);
         static int attr_dev = -1;
         if (attr_dev != h->device) {
             CT_CUDA(h, cudaFuncSetAttribute(chol_diag_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
