@@ -58,12 +58,10 @@ constexpr int LIMBS = 5;                                // 32-bit limbs of P (14
 // pairwise coprime, at most 256: P = 2^140.6
 constexpr int kMod[MODS] = {256, 253, 251, 249, 247, 245, 241, 239, 233, 229, 227, 223, 211, 199, 197, 193, 191, 181};
 
-// Constants of one modulus: 2^21 and 2^42 modulo m, the multiplier of the exact quotient
-// floor(x / m) = umulhi(x, magic) >> 7 for x < 2^31, 1 / m, and the inverse of P / m modulo m
-// (symmetric: at most m / 2 in magnitude).
+// Constants of one modulus: m, 1 / m, 2^(13 i) modulo m for i = 1 .. 4 and the inverse of P / m
+// modulo m (symmetric residues: at most m / 2 in magnitude).
 struct ModConst {
-    unsigned m, p21, p42, magic;
-    float mf, rcp, inv;
+    float mf, rcp, p[4], inv;
 };
 struct ModTable {
     ModConst c[MODS];
@@ -96,18 +94,19 @@ Tables make_tables() {
     };
     for (int i = 0; i < MODS; ++i) {
         ModConst& c = t.mod.c[i];
-        c.m = (unsigned)kMod[i];
-        c.mf = (float)kMod[i];
-        c.p21 = (unsigned)((1ull << 21) % c.m);
-        c.p42 = (unsigned)((1ull << 42) % c.m);
-        c.magic = (unsigned)(((1ull << 39) + c.m - 1) / c.m);
-        c.rcp = 1.0f / (float)c.m;
+        const int m = kMod[i];
+        c.mf = (float)m;
+        c.rcp = 1.0f / (float)m;
+        for (int j = 0; j < 4; ++j) {
+            const int v = (int)((1ull << (13 * (j + 1))) % (unsigned long long)m);
+            c.p[j] = (float)(2 * v > m ? v - m : v);
+        }
         unsigned r = 1;
         for (int j = 0; j < MODS; ++j)
-            if (j != i) r = r * (unsigned)kMod[j] % c.m;
+            if (j != i) r = r * (unsigned)kMod[j] % (unsigned)m;
         int inv = 1;
-        while (inv < (int)c.m && (unsigned)inv * r % c.m != 1) ++inv;
-        c.inv = (float)(2 * inv > (int)c.m ? inv - (int)c.m : inv);
+        while (inv < m && (unsigned)inv * r % (unsigned)m != 1) ++inv;
+        c.inv = (float)(2 * inv > m ? inv - m : inv);
     }
     CrtTable& q = t.crt;
     q.P[0] = 1;
@@ -155,7 +154,8 @@ struct FmSrc {
     const double* p;
     int64_t R, K, R0, s1, s0, sk;
     __nv_bfloat16* res;
-    int* ex;
+    int* ex;        // the rows' exponents, and those of their pieces of FM_XK columns
+    int* part;
     int64_t ldk;
     __host__ __device__ int64_t row(int64_t r) const { return (r / R0) * s1 + (r % R0) * s0; }
 };
@@ -163,65 +163,60 @@ struct FmSrc {
 constexpr int FM_PR = 8;     // rows per block of the two operand kernels
 constexpr int FM_PK = 64;    // columns per block of the residue kernel
 
-// Row exponents of both operands in one launch (ex[r]: 2^ex > max_k |x[r][k]| >= 2^(ex - 1), 0
-// for a zero row).  Blocks [0, nba) take operand A's rows.  sk == 1: a warp per row; else
-// threads along the rows, which are contiguous then.
+constexpr int FM_XK = 256;   // columns per block of the exponent kernel
+constexpr int FM_ZERO = -0x40000000;
+
+// Exponents of both operands' rows over FM_XK columns (part: 2^e > max |x[r][k]| >= 2^(e - 1),
+// FM_ZERO without a non-zero, FM_NONFINITE).  Blocks (x, y): 8 rows, x in [0, nba) operand A's,
+// columns [y FM_XK, +FM_XK); every thread has its 8 loads in flight at once (with whole rows per
+// block, the memory latency five times over and too few blocks: 12.5 us instead of 4 for the
+// H_eff products of chi 256).  sk == 1: a warp per row; else threads along the rows, which are
+// contiguous then.
 __global__ void __launch_bounds__(256) fm_rowexp_kernel(FmSrc a, FmSrc b, int nba, const int* skip) {
     ct_pdl();
     if (ct_skip(skip)) return;
     __shared__ unsigned long long part[8][FM_PR];
     const bool first = (int)blockIdx.x < nba;
     const FmSrc& x = first ? a : b;
-    const int64_t r0 = (int64_t)(first ? blockIdx.x : blockIdx.x - nba) * FM_PR;
+    const int64_t r0 = (int64_t)(first ? blockIdx.x : blockIdx.x - nba) * FM_PR, k0 = (int64_t)blockIdx.y * FM_XK;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // largest magnitude of each row, as bit patterns (their integer order is the order; a NaN
     // or infinity exceeds every finite value)
     constexpr unsigned long long ABS = 0x7fffffffffffffffull;
+    const bool along = x.sk == 1;
+    const int64_t r = r0 + (along ? warp : tid % FM_PR);
     unsigned long long m = 0;
-    if (x.sk == 1) {
-        const int64_t r = r0 + warp;
-        if (r < x.R) {
-            const double* p = x.p + x.row(r);
-#pragma unroll 8
-            for (int64_t k = lane; k < x.K; k += 32) {
-                const unsigned long long v = (unsigned long long)__double_as_longlong(p[k]) & ABS;
-                m = v > m ? v : m;
-            }
-        }
+    if (r < x.R) {
+        const double* p = x.p + x.row(r);
+        const int64_t k = k0 + (along ? lane : tid / FM_PR);
+        unsigned long long v[FM_XK / 32];
 #pragma unroll
-        for (int of = 16; of > 0; of >>= 1) {
-            const unsigned long long v = __shfl_xor_sync(0xffffffffu, m, of);
-            m = v > m ? v : m;
-        }
-        if (lane < 8) part[lane][warp] = lane == 0 ? m : 0;
-    } else {
-        const int r = tid % FM_PR;
-        if (r0 + r < x.R) {
-            const double* p = x.p + x.row(r0 + r);
-#pragma unroll 8
-            for (int64_t k = tid / FM_PR; k < x.K; k += 256 / FM_PR) {
-                const unsigned long long v = (unsigned long long)__double_as_longlong(p[k * x.sk]) & ABS;
-                m = v > m ? v : m;
-            }
-        }
+        for (int u = 0; u < FM_XK / 32; ++u)
+            v[u] = k + 32 * u < x.K ? (unsigned long long)__double_as_longlong(p[(k + 32 * u) * x.sk]) & ABS : 0ull;
 #pragma unroll
-        for (int of = 16; of >= FM_PR; of >>= 1) {
-            const unsigned long long v = __shfl_xor_sync(0xffffffffu, m, of);
-            m = v > m ? v : m;
-        }
-        if (lane < FM_PR) part[warp][lane] = m;
+        for (int u = 0; u < FM_XK / 32; ++u) m = v[u] > m ? v[u] : m;
     }
-    __syncthreads();
-    if (tid < FM_PR && r0 + tid < x.R) {
-        m = 0;
+#pragma unroll
+    for (int of = 16; of > 0; of >>= 1) {
+        if (!along && of < FM_PR) break;
+        const unsigned long long v = __shfl_xor_sync(0xffffffffu, m, of);
+        m = v > m ? v : m;
+    }
+    if (!along) {
+        if (lane < FM_PR) part[warp][lane] = m;
+        __syncthreads();
+        if (tid >= FM_PR) return;
 #pragma unroll
         for (int i = 0; i < 8; ++i) m = part[i][tid] > m ? part[i][tid] : m;
-        int e = 0;
-        if (m >= 0x7ff0000000000000ull) e = FM_NONFINITE;
-        else if (m > 0) frexp(__longlong_as_double((long long)m), &e);
-        x.ex[r0 + tid] = e;
+    } else if (lane != 0) {
+        return;
     }
+    if (r >= x.R) return;
+    const int field = (int)(m >> 52);
+    const int e = field == 0x7ff ? FM_NONFINITE : field ? field - 1022 : m ? -1010 - __clzll((long long)m) : FM_ZERO;
+    x.part[(int64_t)blockIdx.y * x.R + r] = e;
 }
+
 
 // |v| 2^(bits - e) rounded to an integer (e: the row's exponent), 0 in a non-finite row
 __device__ __forceinline__ unsigned long long fm_fixed(double v, int e, int bits) {
@@ -269,29 +264,41 @@ __global__ void __launch_bounds__(256) fm_residue_kernel(FmSrc a, FmSrc b, int n
         v0 = tile[2 * lane][warp];
         v1 = tile[2 * lane + 1][warp];
     }
-    if (k >= x.ldk || r0 + warp >= x.R) return;
-    const int e = x.ex[r0 + warp];
+    if (r0 + warp >= x.R) return;
+    int e = FM_ZERO;   // the row's exponent from its pieces'
+    for (int64_t c = lane; c * FM_XK < x.K; c += 32) e = max(e, x.part[c * x.R + r0 + warp]);
+    e = __reduce_max_sync(0xffffffffu, e);
+    if (e == FM_ZERO) e = 0;
+    if (blockIdx.y == 0 && lane == 0) x.ex[r0 + warp] = e;
     const unsigned long long u0 = fm_fixed(v0, e, bits), u1 = fm_fixed(v1, e, bits);
-    const float g0 = v0 < 0.0 ? -1.0f : 1.0f, g1 = v1 < 0.0 ? -1.0f : 1.0f;
-    // three 21-bit digits of each
-    constexpr unsigned D = (1u << 21) - 1;
-    const unsigned a0 = (unsigned)u0 & D, a1 = (unsigned)(u0 >> 21) & D, a2 = (unsigned)(u0 >> 42);
-    const unsigned b0 = (unsigned)u1 & D, b1 = (unsigned)(u1 >> 21) & D, b2 = (unsigned)(u1 >> 42);
+    // five 13-bit digits of each as floats with the value's sign (a digit in the low bits of
+    // 2^23 + digit)
+    float d[2][5];
+#pragma unroll
+    for (int i = 0; i < 5; ++i) {
+        const float x0 = __uint_as_float(0x4B000000u | ((unsigned)(u0 >> (13 * i)) & 8191u)) - 8388608.0f;
+        const float x1 = __uint_as_float(0x4B000000u | ((unsigned)(u1 >> (13 * i)) & 8191u)) - 8388608.0f;
+        d[0][i] = __double2hiint(v0) < 0 ? -x0 : x0;
+        d[1][i] = __double2hiint(v1) < 0 ? -x1 : x1;
+    }
     const int64_t plane = x.R * x.ldk;
     __nv_bfloat16* out = x.res + (r0 + warp) * x.ldk + k;
 #pragma unroll
     for (int i = 0; i < MODS; ++i) {
         const ModConst& c = tab.c[i];
-        const unsigned half = c.m >> 1;
-        const unsigned s0 = a2 * c.p42 + a1 * c.p21 + a0 + half, s1 = b2 * c.p42 + b1 * c.p21 + b0 + half;   // < 2^31
-        // x + half - m floor((x + half) / m) - half: in [-m/2, m/2]; integers to BF16 (exact: 8
-        // bits) through 1.5 2^23
-        const unsigned base = 0x4B400000u - half;
-        const unsigned d0 = s0 - (__umulhi(s0, c.magic) >> 7) * c.m + base;
-        const unsigned d1 = s1 - (__umulhi(s1, c.magic) >> 7) * c.m + base;
-        const uint32_t f0 = __float_as_uint((__uint_as_float(d0) - 12582912.0f) * g0);
-        const uint32_t f1 = __float_as_uint((__uint_as_float(d1) - 12582912.0f) * g1);
-        *reinterpret_cast<uint32_t*>(out + i * plane) = __byte_perm(f0, f1, 0x7632);
+        // sum of digit times 2^(13 i) mod m, below 2^23 and exact, minus m rint(sum / m): at most 128
+        // in magnitude, exact in BF16 (the upper half of the FP32 word)
+        constexpr float RND = 12582912.0f;   // 1.5 2^23
+        uint32_t f[2];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            float t = d[q][0];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) t = fmaf(d[q][j + 1], c.p[j], t);
+            const float n = __fsub_rn(fmaf(t, c.rcp, RND), RND);
+            f[q] = __float_as_uint(fmaf(-n, c.mf, t));
+        }
+        *reinterpret_cast<uint32_t*>(out + i * plane) = __byte_perm(f[0], f[1], 0x7632);
     }
 }
 
@@ -609,7 +616,7 @@ FmPlan fm_plan(int64_t M, int64_t N, int64_t K) {
     q.ldn = ct_round_up(N, FM_BN);
     q.tiles = ct_cdiv(M, FM_BM) * ct_cdiv(N, FM_BN);
     q.bytes = ct_bytes(MODS * M * q.ldk, 2) + ct_bytes(MODS * N * q.ldk, 2) + ct_bytes(MODS * M * q.ldn, 1) +
-              ct_bytes(M, 4) + ct_bytes(N, 4);
+              ct_bytes(M, 4) + ct_bytes(N, 4) + ct_bytes(ct_cdiv(K, FM_XK) * M, 4) + ct_bytes(ct_cdiv(K, FM_XK) * N, 4);
     return q;
 }
 
@@ -691,15 +698,19 @@ int ct_f64_gemm(ct_handle* h, int64_t M, int64_t N, int64_t K, const OzMat& A, c
     const FmPlan q = fm_plan(M, N, K);
     CT_TRY(fm_workspace(h, q.bytes));
     uint8_t* p = (uint8_t*)h->fm_ws;
-    FmSrc a{A.p, M, K, A.R0 > 0 ? A.R0 : M, A.s1, A.s0, A.sk, (__nv_bfloat16*)p, nullptr, q.ldk};
+    FmSrc a{A.p, M, K, A.R0 > 0 ? A.R0 : M, A.s1, A.s0, A.sk, (__nv_bfloat16*)p, nullptr, nullptr, q.ldk};
     p += ct_bytes(MODS * M * q.ldk, 2);
-    FmSrc b{B.p, N, K, B.R0 > 0 ? B.R0 : N, B.s1, B.s0, B.sk, (__nv_bfloat16*)p, nullptr, q.ldk};
+    FmSrc b{B.p, N, K, B.R0 > 0 ? B.R0 : N, B.s1, B.s0, B.sk, (__nv_bfloat16*)p, nullptr, nullptr, q.ldk};
     p += ct_bytes(MODS * N * q.ldk, 2);
     FmOut o{(unsigned char*)p, q.ldn};
     p += ct_bytes(MODS * M * q.ldn, 1);
     a.ex = (int*)p;
     p += ct_bytes(M, 4);
     b.ex = (int*)p;
+    p += ct_bytes(N, 4);
+    a.part = (int*)p;
+    p += ct_bytes(ct_cdiv(K, FM_XK) * M, 4);
+    b.part = (int*)p;
     CUtensorMap ta, tb;
     CT_TRY(fm_map(h, &ta, a, FM_BM));
     CT_TRY(fm_map(h, &tb, b, FM_BN));
@@ -713,7 +724,7 @@ int ct_f64_gemm(ct_handle* h, int64_t M, int64_t N, int64_t K, const OzMat& A, c
     const int nba = (int)ct_cdiv(M, FM_PR);
     const dim3 grid((unsigned)(nba + ct_cdiv(N, FM_PR)), (unsigned)ct_cdiv(q.ldk, FM_PK));
     if (grid.y > 65535) return CT_ERR_UNSUPPORTED;
-    ct_launch(h, fm_rowexp_kernel, grid.x, 256, 0, a, b, nba, skip); ct_note_launch();
+    ct_launch(h, fm_rowexp_kernel, dim3(grid.x, (unsigned)ct_cdiv(K, FM_XK)), 256, 0, a, b, nba, skip); ct_note_launch();
     ct_launch(h, fm_residue_kernel, grid, 256, 0, a, b, nba, bits, t.mod, skip); ct_note_launch();
     const int64_t items = q.tiles * MODS;
     const int64_t ctas = items < h->num_sms ? items : h->num_sms;
