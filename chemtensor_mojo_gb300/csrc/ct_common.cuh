@@ -340,6 +340,9 @@ int ct_lanczos_reorth_pass32(ct_handle* h, int64_t n, double* w, const float* V3
                              double beta_threshold, const int* skip, double ratio64);
 int ct_lanczos_reorth_redo(ct_handle* h, int64_t n, double* w, const double* V, const float* V32, int64_t ldv, int j,
                            double beta_threshold, const int* skip);
+bool ct_lanczos_step_fits(ct_handle* h, int64_t n);
+int ct_lanczos_step(ct_handle* h, int64_t n, double* w, double* V, float* V32, int j, bool reorth, double beta_threshold,
+                    double ratio64, const int* skip);
 int ct_lanczos_next32(ct_handle* h, int64_t n, const double* w, double* vnext, float* vnext32, int j,
                       const int* skip);
 int ct_f64_to_f32(ct_handle* h, int64_t n, const double* x, float* y, const int* skip);

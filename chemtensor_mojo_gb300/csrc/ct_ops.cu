@@ -314,6 +314,7 @@ int ct_lanczos_run(ct_handle* h, Arena& ar, int prec, const double* theta_in, do
     // algorithmic FLOPs of one apply (the reference's four contractions)
     const double heff_flops = 2.0 * (double)Dl * wL * d * d * Dr * Dl + 2.0 * (double)Dl * d * Dr * wL * d * d * wM +
                               2.0 * (double)Dl * Dr * d * wM * d * d * wR + 2.0 * (double)Dl * d * d * Dr * wR * Dr;
+    const bool short_step = ct_lanczos_step_fits(h, N);
     for (int j = 0; j < max_iter - 1; ++j) {
         double* vj = V + (int64_t)j * N;
         const double* vjm1 = (j > 0) ? V + (int64_t)(j - 1) * N : nullptr;
@@ -335,6 +336,11 @@ int ct_lanczos_run(ct_handle* h, Arena& ar, int prec, const double* theta_in, do
                                      : 8.0 * (double)N * (double)(2 + (j > 0 ? 4 : 3) + (j + 2) + (j + 3) + 2);
             int kv = -1;
             CT_TRY(ct_ktime_begin(h, KT_LANCZOS_VEC, bytes, &kv));
+            if (short_step) {
+                CT_TRY(ct_lanczos_step(h, N, w, V, V32, j, true, thr, ct_lanczos_redo32() ? 1e4 : 0.1, stop));
+                CT_TRY(ct_ktime_end(h, kv));
+                continue;
+            }
             CT_TRY(ct_lanczos_alpha(h, N, vj, w, j, stop));
             CT_TRY(ct_lanczos_update_nonorm(h, N, w, vj, vjm1, j, stop));
             if (V32) {
@@ -353,6 +359,10 @@ int ct_lanczos_run(ct_handle* h, Arena& ar, int prec, const double* theta_in, do
         }
         // the reference's recurrence (dmrg.mojo:612-689): alpha, w -= alpha v_j + beta v_{j-1},
         // beta = |w|, v_{j+1} = w / beta
+        if (short_step) {
+            CT_TRY(ct_lanczos_step(h, N, w, V, nullptr, j, false, thr, 0.0, stop));
+            continue;
+        }
         CT_TRY(ct_lanczos_alpha(h, N, vj, w, j, stop));
         CT_TRY(ct_lanczos_update(h, N, w, vj, vjm1, j, thr, stop));
         CT_TRY(ct_lanczos_next(h, N, w, V + (int64_t)(j + 1) * N, j, stop));

@@ -174,19 +174,10 @@ __global__ void permute_kernel(const double* in, double* out, PermArgs a) {
     }
 }
 
-// ---- Lanczos -------------------------------------------------------------------
-// w -= alpha_j v_j + beta_{j-1} v_{j-1}; partial |w|^2 when NORM (the mixed form's
-// reorthogonalisation measures the norm itself, and on this part FP64 issues at 1/64 of
-// the FP32 rate: the unused norm was a third of the kernel's FP64 work)
+// w -= a v_j + b v_{j-1} over this thread's elements, with their |w|^2
 template <bool NORM>
-__global__ void __launch_bounds__(RT) lanczos_update_kernel(int64_t n, double* w, const double* vj,
-                                                            const double* vjm1, const double* scalars,
-                                                            int j, double* partials, const int* skip) {
-    ct_pdl();
-    if (ct_skip(skip)) return;
-    __shared__ double sm[32];
-    const double a = scalars[SC_ALPHA + j];
-    const double b = (j > 0) ? scalars[SC_BETA + j - 1] : 0.0;
+__device__ __forceinline__ double recurrence(int64_t n, double* w, const double* vj, const double* vjm1, double a,
+                                             double b) {
     double acc = 0.0;
     const int64_t stride = (int64_t)gridDim.x * RT;
     if (aligned16(w) && aligned16(vj) && (!vjm1 || aligned16(vjm1))) {
@@ -222,8 +213,23 @@ __global__ void __launch_bounds__(RT) lanczos_update_kernel(int64_t n, double* w
             if (NORM) acc = fma(x, x, acc);
         }
     }
+    return acc;
+}
+
+// ---- Lanczos -------------------------------------------------------------------
+// w -= alpha_j v_j + beta_{j-1} v_{j-1}; partial |w|^2 when NORM (the mixed form's
+// reorthogonalisation measures the norm itself, and on this part FP64 issues at 1/64 of
+// the FP32 rate: the unused norm was a third of the kernel's FP64 work)
+template <bool NORM>
+__global__ void __launch_bounds__(RT) lanczos_update_kernel(int64_t n, double* w, const double* vj,
+                                                            const double* vjm1, const double* scalars,
+                                                            int j, double* partials, const int* skip) {
+    ct_pdl();
+    if (ct_skip(skip)) return;
+    __shared__ double sm[32];
+    const double acc0 = recurrence<NORM>(n, w, vj, vjm1, scalars[SC_ALPHA + j], (j > 0) ? scalars[SC_BETA + j - 1] : 0.0);
     if (NORM) {
-        acc = ct_block_sum<RT>(acc, sm);
+        const double acc = ct_block_sum<RT>(acc0, sm);
         if (threadIdx.x == 0) partials[blockIdx.x] = acc;
     }
 }
@@ -315,9 +321,8 @@ __device__ __forceinline__ void cgs_dots_group(int64_t n, const double* __restri
 }
 
 // pass A: coeff[v] = <V[v], w> for v < nvec
-__device__ __forceinline__ void cgs_dots_dev(int64_t n, const double* __restrict__ w, const double* __restrict__ V,
-                                             int64_t ldv, int nvec, int vec2, double* partials, unsigned* counter,
-                                             double* coeff) {
+__device__ __forceinline__ void cgs_dots_part(int64_t n, const double* __restrict__ w, const double* __restrict__ V,
+                                             int64_t ldv, int nvec, int vec2, double* partials) {
     __shared__ double sm[CGS_VB][RT / 32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     for (int v0 = 0; v0 < nvec; v0 += CGS_VB) {
@@ -351,23 +356,33 @@ __device__ __forceinline__ void cgs_dots_dev(int64_t n, const double* __restrict
         }
         __syncthreads();
     }
-    if (!last_block_arrived(counter)) return;
-    // last block: one warp per coefficient, lanes stride over the block partials
+}
+
+// the coefficients from the blocks' partial sums: one warp per coefficient, lanes stride over
+// the blocks
+__device__ __forceinline__ void cgs_coeffs(const double* partials, int nvec, double* coeff) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     for (int v = wid; v < nvec; v += RT / 32) {
         double r = 0.0;
         for (int b = lane; b < (int)gridDim.x; b += 32) r += __ldcg(partials + (int64_t)b * nvec + v);
         r = ct_warp_sum(r);
         if (lane == 0) coeff[v] = r;
     }
+}
+
+__device__ __forceinline__ void cgs_dots_dev(int64_t n, const double* __restrict__ w, const double* __restrict__ V,
+                                             int64_t ldv, int nvec, int vec2, double* partials, unsigned* counter,
+                                             double* coeff) {
+    cgs_dots_part(n, w, V, ldv, nvec, vec2, partials);
+    if (!last_block_arrived(counter)) return;
+    cgs_coeffs(partials, nvec, coeff);
     if (threadIdx.x == 0) *counter = 0u;
 }
 
 // pass B: w -= sum_v coeff[v] V[v] with |w|^2; the last block forms beta_j = |w|
 // and makes the breakdown test beta < thr (dmrg.mojo:630-673)
-__device__ __forceinline__ void cgs_update_dev(int64_t n, double* __restrict__ w, const double* __restrict__ V,
-                                               int64_t ldv, int nvec, int vec2, const double* coeff, double* partials,
-                                               unsigned* counter, double* scalars, int* flags, int j, double thr) {
-    __shared__ double sm[32];
+__device__ __forceinline__ double cgs_update_part(int64_t n, double* __restrict__ w, const double* __restrict__ V, int64_t ldv,
+                                                 int nvec, int vec2, const double* coeff) {
     __shared__ double c[CT_MAX_KRYLOV];
     for (int v = threadIdx.x; v < nvec; v += RT) c[v] = coeff[v];
     __syncthreads();
@@ -405,6 +420,14 @@ __device__ __forceinline__ void cgs_update_dev(int64_t n, double* __restrict__ w
             nn = fma(x, x, nn);
         }
     }
+    return nn;
+}
+
+__device__ __forceinline__ void cgs_update_dev(int64_t n, double* __restrict__ w, const double* __restrict__ V,
+                                               int64_t ldv, int nvec, int vec2, const double* coeff, double* partials,
+                                               unsigned* counter, double* scalars, int* flags, int j, double thr) {
+    __shared__ double sm[32];
+    double nn = cgs_update_part(n, w, V, ldv, nvec, vec2, coeff);
     nn = ct_block_sum<RT>(nn, sm);
     if (threadIdx.x == 0) partials[blockIdx.x] = nn;
     if (!last_block_arrived(counter)) return;
@@ -458,9 +481,8 @@ __device__ __forceinline__ void cgs32_dots_group(int64_t n, const double* __rest
     }
 }
 
-__device__ __forceinline__ void cgs32_dots_dev(int64_t n, const double* __restrict__ w, const float* __restrict__ V,
-                                               int64_t ldv, int nvec, int vec4, double* partials, unsigned* counter,
-                                               double* coeff) {
+__device__ __forceinline__ void cgs32_dots_part(int64_t n, const double* __restrict__ w, const float* __restrict__ V,
+                                               int64_t ldv, int nvec, int vec4, double* partials) {
     static_assert(RT == 256 && CGS_VB == 16, "the block reduction maps 256 threads onto 16 x 16");
     __shared__ float red[CGS_VB][RT + 1];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -500,21 +522,19 @@ __device__ __forceinline__ void cgs32_dots_dev(int64_t n, const double* __restri
         }
         __syncthreads();
     }
+}
+
+__device__ __forceinline__ void cgs32_dots_dev(int64_t n, const double* __restrict__ w, const float* __restrict__ V,
+                                               int64_t ldv, int nvec, int vec4, double* partials, unsigned* counter,
+                                               double* coeff) {
+    cgs32_dots_part(n, w, V, ldv, nvec, vec4, partials);
     if (!last_block_arrived(counter)) return;
-    for (int v = wid; v < nvec; v += RT / 32) {
-        double r = 0.0;
-        for (int b = lane; b < (int)gridDim.x; b += 32) r += __ldcg(partials + (int64_t)b * nvec + v);
-        r = ct_warp_sum(r);
-        if (lane == 0) coeff[v] = r;
-    }
+    cgs_coeffs(partials, nvec, coeff);
     if (threadIdx.x == 0) *counter = 0u;
 }
 
-__device__ __forceinline__ void cgs32_update_dev(int64_t n, double* __restrict__ w, const float* __restrict__ V,
-                                                 int64_t ldv, int nvec, int vec4, const double* coeff,
-                                                 double* partials, unsigned* counter, double* scalars, int* flags,
-                                                 int j, double thr, int second, double ratio64) {
-    __shared__ double sm[32];
+__device__ __forceinline__ double cgs32_update_part(int64_t n, double* __restrict__ w, const float* __restrict__ V, int64_t ldv,
+                                                 int nvec, int vec4, const double* coeff) {
     __shared__ float c[CT_MAX_KRYLOV];
     for (int v = threadIdx.x; v < nvec; v += RT) c[v] = (float)coeff[v];
     __syncthreads();
@@ -551,6 +571,15 @@ __device__ __forceinline__ void cgs32_update_dev(int64_t n, double* __restrict__
             nn = fma(x, x, nn);
         }
     }
+    return nn;
+}
+
+__device__ __forceinline__ void cgs32_update_dev(int64_t n, double* __restrict__ w, const float* __restrict__ V,
+                                                 int64_t ldv, int nvec, int vec4, const double* coeff,
+                                                 double* partials, unsigned* counter, double* scalars, int* flags,
+                                                 int j, double thr, int second, double ratio64) {
+    __shared__ double sm[32];
+    double nn = cgs32_update_part(n, w, V, ldv, nvec, vec4, coeff);
     nn = ct_block_sum<RT>(nn, sm);
     if (threadIdx.x == 0) partials[blockIdx.x] = nn;
     if (!last_block_arrived(counter)) return;
@@ -587,16 +616,8 @@ __device__ __forceinline__ void cgs32_update_dev(int64_t n, double* __restrict__
     }
 }
 
-// alpha_j = <v_j, w> -> scalars[SC_ALPHA + j]: block partials over 16-byte loads, then
-// the block that arrives last sums them in block order (the same fixed-order sum as a
-// separate one-block finisher, without its launch)
-__global__ void __launch_bounds__(RT) lanczos_alpha_kernel(int64_t n, const double* __restrict__ vj,
-                                                           const double* __restrict__ w, double* partials,
-                                                           unsigned* counter, double* scalars, int j,
-                                                           const int* skip) {
-    ct_pdl();
-    if (ct_skip(skip)) return;
-    __shared__ double sm[32];
+// <v_j, w> over this thread's elements
+__device__ __forceinline__ double alpha_part(int64_t n, const double* vj, const double* w) {
     double acc = 0.0;
     const int64_t stride = (int64_t)gridDim.x * RT;
     const int64_t start = (int64_t)blockIdx.x * RT + threadIdx.x;
@@ -613,6 +634,20 @@ __global__ void __launch_bounds__(RT) lanczos_alpha_kernel(int64_t n, const doub
     } else {
         for (int64_t i = start; i < n; i += stride) acc = fma(vj[i], w[i], acc);
     }
+    return acc;
+}
+
+// alpha_j = <v_j, w> -> scalars[SC_ALPHA + j]: block partials over 16-byte loads, then
+// the block that arrives last sums them in block order (the same fixed-order sum as a
+// separate one-block finisher, without its launch)
+__global__ void __launch_bounds__(RT) lanczos_alpha_kernel(int64_t n, const double* __restrict__ vj,
+                                                           const double* __restrict__ w, double* partials,
+                                                           unsigned* counter, double* scalars, int j,
+                                                           const int* skip) {
+    ct_pdl();
+    if (ct_skip(skip)) return;
+    __shared__ double sm[32];
+    double acc = alpha_part(n, vj, w);
     acc = ct_block_sum<RT>(acc, sm);
     if (threadIdx.x == 0) partials[blockIdx.x] = acc;
     if (!last_block_arrived(counter)) return;
@@ -723,6 +758,142 @@ __global__ void lanczos_next32_kernel(int64_t n, const double* w, double* vnext,
             vnext32[i] = (float)v;
         }
     }
+}
+
+// ---- one Lanczos step's vector work in one launch (short vectors) --------------------
+// alpha, the recurrence, the Gram-Schmidt pass with its gated second pass, beta and the next
+// vector, as the kernels above do them: up to STEP_MAXG blocks are one cluster, whose barrier
+// takes the place of the launches and of the last block's arrival.  What bounds a short step is
+// the chain of launches (seven of 4 to 5 us in the mixed form, four in the others) and of block
+// sums, not the vectors.  The grid, each thread's elements and every sum's order are those of the
+// separate kernels, so the results are the same bits; each block forms the totals itself.
+// Vectors past 32768 elements (16 blocks) need more SMs.  Measured: Lanczos at chi 32, 20 steps,
+// 837 us with separate launches, 725 here; the 16-site Heisenberg run, chi 64, mixed, 162 ms
+// and 141.5.
+constexpr int STEP_MAXG = 16;
+struct LanczosStep {
+    int64_t n, ldv;
+    double *w, *vnext;
+    const double *vj, *vjm1, *V;
+    const float* V32;
+    float* vnext32;
+    double *partials, *scalars;
+    int* flags;
+    const int* skip;
+    double thr, ratio64;
+    int j, vec2, vec4;
+};
+
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// sum over the grid of per-thread values, in every thread; slot: gridDim.x doubles used once
+__device__ __forceinline__ double grid_total(double v, double* slot, double* sm) {
+    v = ct_block_sum<RT>(v, sm);
+    if (threadIdx.x == 0) slot[blockIdx.x] = v;
+    cluster_barrier();
+    const int lane = threadIdx.x & 31;
+    return ct_warp_sum(lane < (int)gridDim.x ? __ldcg(slot + lane) : 0.0);
+}
+
+// f(element) for this thread's elements under the unit-element mapping of the kernels above
+template <typename F>
+__device__ __forceinline__ void own_elements(int64_t n, int unit, F f) {
+    for (int64_t i = (int64_t)blockIdx.x * RT + threadIdx.x; i < n / unit; i += (int64_t)gridDim.x * RT)
+        for (int e = 0; e < unit; ++e) f(i * unit + e);
+}
+
+// MODE 0: the reference recurrence, 1: reorthogonalised in FP64, 2: against the FP32 copy
+template <int MODE>
+__global__ void __launch_bounds__(RT) lanczos_step_kernel(LanczosStep q) {
+    ct_pdl();
+    if (ct_skip(q.skip)) return;
+    __shared__ double sm[32], coeff[CT_MAX_KRYLOV], bs[2];
+    const int j = q.j, nvec = j + 1, lane = threadIdx.x & 31;
+    const bool writer = blockIdx.x == 0 && threadIdx.x == 0;
+    // one region of the partials per sum, so that none is overwritten while it is read
+    double *p_alpha = q.partials, *p_beta = p_alpha + STEP_MAXG, *p_beta2 = p_beta + STEP_MAXG,
+           *p_dots = p_beta2 + STEP_MAXG, *p_dots2 = p_dots + STEP_MAXG * 64;
+    static_assert(3 * STEP_MAXG + 2 * STEP_MAXG * 64 <= CT_NPARTIALS, "partials of a fused step");
+    const double alpha = grid_total(alpha_part(q.n, q.vj, q.w), p_alpha, sm);
+    if (writer) q.scalars[SC_ALPHA + j] = alpha;
+    const double bprev = j > 0 ? q.scalars[SC_BETA + j - 1] : 0.0;
+    // beta = sqrt(s) and 1 / beta; true (in every thread) on a breakdown
+    auto beta = [&](double s) -> bool {
+        if (threadIdx.x < 32) {
+            const double b = ct_fp64::sqrt_rn(s), inv = ct_fp64::div_rn(1.0, b);
+            if (threadIdx.x == 0) {
+                bs[0] = b;
+                bs[1] = inv;
+            }
+        }
+        __syncthreads();
+        if (bs[0] < q.thr) {
+            if (writer) {
+                q.flags[FL_NUMITER] = j + 1;
+                q.flags[FL_STOP] = 1;
+            }
+            return true;
+        }
+        if (writer) q.scalars[SC_BETA + j] = bs[0];
+        return false;
+    };
+    int unit = 1;
+    if (MODE == 0) {
+        const bool v2 = aligned16(q.w) && aligned16(q.vj) && (!q.vjm1 || aligned16(q.vjm1));
+        if (beta(grid_total(recurrence<true>(q.n, q.w, q.vj, q.vjm1, alpha, bprev), p_beta, sm))) return;
+        const double inv = bs[1];
+        own_elements(q.n, v2 ? 2 : 1, [&](int64_t e) { q.vnext[e] = q.w[e] * inv; });
+        if (v2 && (q.n & 1) && writer) q.vnext[q.n - 1] = q.w[q.n - 1] * inv;
+        return;
+    }
+    unit = MODE == 2 ? (q.vec4 ? 4 : 1) : (q.vec2 ? 2 : 1);
+    own_elements(q.n, unit, [&](int64_t e) {
+        double x = q.w[e] - alpha * q.vj[e];
+        if (q.vjm1) x -= bprev * q.vjm1[e];
+        q.w[e] = x;
+    });
+    if (MODE == 2) cgs32_dots_part(q.n, q.w, q.V32, q.ldv, nvec, q.vec4, p_dots);
+    else cgs_dots_part(q.n, q.w, q.V, q.ldv, nvec, q.vec2, p_dots);
+    cluster_barrier();
+    cgs_coeffs(p_dots, nvec, coeff);
+    __syncthreads();
+    const double s = grid_total(MODE == 2 ? cgs32_update_part(q.n, q.w, q.V32, q.ldv, nvec, q.vec4, coeff)
+                                          : cgs_update_part(q.n, q.w, q.V, q.ldv, nvec, q.vec2, coeff),
+                                p_beta, sm);
+    bool stop = beta(s);
+    if (MODE == 2) {
+        // the gate of the second pass (cgs32_update_dev)
+        const double c0 = lane < nvec ? coeff[lane] : 0.0, c1 = lane + 32 < nvec ? coeff[lane + 32] : 0.0;
+        const double cc = ct_warp_sum(c0 * c0) + ct_warp_sum(c1 * c1);
+        const bool big = cc > 1e-2 * s, huge = cc > q.ratio64 * q.ratio64 * s;
+        if (writer) {
+            q.flags[FL_REDO] = (big && !huge) ? 1 : 0;
+            q.flags[FL_REDO64] = huge ? 1 : 0;
+        }
+        if (stop) return;
+        if (huge || big) {
+            __threadfence();   // (the FP64 pass reads w under another mapping)
+            if (huge) cgs_dots_part(q.n, q.w, q.V, q.ldv, nvec, q.vec2, p_dots2);
+            else cgs32_dots_part(q.n, q.w, q.V32, q.ldv, nvec, q.vec4, p_dots2);
+            cluster_barrier();
+            cgs_coeffs(p_dots2, nvec, coeff);
+            __syncthreads();
+            stop = beta(grid_total(huge ? cgs_update_part(q.n, q.w, q.V, q.ldv, nvec, q.vec2, coeff)
+                                        : cgs32_update_part(q.n, q.w, q.V32, q.ldv, nvec, q.vec4, coeff),
+                                   p_beta2, sm));
+            if (huge) unit = q.vec2 ? 2 : 1;
+        }
+    }
+    if (stop) return;
+    const double inv = bs[1];
+    own_elements(q.n, unit, [&](int64_t e) {
+        const double v = q.w[e] * inv;
+        q.vnext[e] = v;
+        if (MODE == 2) q.vnext32[e] = (float)v;
+    });
 }
 
 __global__ void f64_to_f32_copy_kernel(int64_t n, const double* x, float* y, const int* skip) {
@@ -1283,6 +1454,54 @@ int ct_lanczos_reorth_redo(ct_handle* h, int64_t n, double* w, const double* V, 
                                                     counter, h->d_scalars, h->d_flags, j, beta_threshold, skip);
     ct_note_launch();
     CT_LAUNCH_CHECK(h);
+    return CT_OK;
+}
+
+// Whether ct_lanczos_step takes vectors of n elements.
+bool ct_lanczos_step_fits(ct_handle* h, int64_t n) { return grid_for(h, n) <= STEP_MAXG; }
+
+// Everything of Lanczos step j after w = H v_j up to v_{j+1} (see lanczos_step_kernel).  V32
+// (mixed form, reorthogonalised) and reorth choose the form.
+int ct_lanczos_step(ct_handle* h, int64_t n, double* w, double* V, float* V32, int j, bool reorth, double beta_threshold,
+                    double ratio64, const int* skip) {
+    if (reorth && j + 1 > 64) return CT_ERR_UNSUPPORTED;
+    LanczosStep q{};
+    q.n = q.ldv = n;
+    q.w = w;
+    q.V = V;
+    q.V32 = V32;
+    q.vj = V + (int64_t)j * n;
+    q.vjm1 = j > 0 ? V + (int64_t)(j - 1) * n : nullptr;
+    q.vnext = V + (int64_t)(j + 1) * n;
+    q.vnext32 = V32 ? V32 + (int64_t)(j + 1) * n : nullptr;
+    q.partials = h->d_partials;
+    q.scalars = h->d_scalars;
+    q.flags = h->d_flags;
+    q.skip = skip;
+    q.thr = beta_threshold;
+    q.ratio64 = ratio64;
+    q.j = j;
+    q.vec2 = ((n & 1) == 0 && aligned16(w) && aligned16(V)) ? 1 : 0;
+    q.vec4 = ((n & 3) == 0 && aligned16(w) && V32 && aligned16(V32)) ? 1 : 0;
+    auto* f = !reorth ? lanczos_step_kernel<0> : V32 ? lanczos_step_kernel<2> : lanczos_step_kernel<1>;
+    static int attr_dev = -1;
+    if (attr_dev != h->device) {
+        for (auto* k : {lanczos_step_kernel<0>, lanczos_step_kernel<1>, lanczos_step_kernel<2>})
+            CT_CUDA(h, cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        attr_dev = h->device;
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid_for(h, n));
+    cfg.blockDim = dim3(RT);
+    cfg.stream = h->stream;
+    cudaLaunchAttribute at[2]{};
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // (as ct_launch)
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim = {cfg.gridDim.x, 1, 1};
+    cfg.attrs = at;
+    cfg.numAttrs = 2;
+    CT_CUDA(h, cudaLaunchKernelEx(&cfg, f, q)); ct_note_launch();
     return CT_OK;
 }
 
