@@ -186,19 +186,25 @@ __device__ __forceinline__ double recurrence(int64_t n, double* w, const double*
         double2* w2 = reinterpret_cast<double2*>(w);
         const double2* a2 = reinterpret_cast<const double2*>(vj);
         const double2* c2 = reinterpret_cast<const double2*>(vjm1);
-        for (int64_t i = (int64_t)blockIdx.x * RT + threadIdx.x; i < n2; i += stride) {
-            double2 x = w2[i];
-            const double2 v = a2[i];
+        int64_t i = (int64_t)blockIdx.x * RT + threadIdx.x;
+        auto one = [&](double2 x, const double2& v, const double2& u, int64_t at) {
             x.x -= a * v.x;
             x.y -= a * v.y;
             if (vjm1) {
-                const double2 u = c2[i];
                 x.x -= b * u.x;
                 x.y -= b * u.y;
             }
-            w2[i] = x;
+            w2[at] = x;
             if (NORM) acc = fma(x.x, x.x, fma(x.y, x.y, acc));
+        };
+        const double2 zero = make_double2(0.0, 0.0);
+        for (; i + stride < n2; i += 2 * stride) {   // the loads of two in flight (w is written)
+            const double2 x0 = w2[i], x1 = w2[i + stride], v0 = a2[i], v1 = a2[i + stride];
+            const double2 u0 = vjm1 ? c2[i] : zero, u1 = vjm1 ? c2[i + stride] : zero;
+            one(x0, v0, u0, i);
+            one(x1, v1, u1, i + stride);
         }
+        if (i < n2) one(w2[i], a2[i], vjm1 ? c2[i] : zero, i);
         if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
             double x = w[n - 1] - a * vj[n - 1];
             if (vjm1) x -= b * vjm1[n - 1];
@@ -465,7 +471,7 @@ __device__ __forceinline__ void cgs32_dots_group(int64_t n, const double* __rest
         const double2* w2 = reinterpret_cast<const double2*>(w);
         for (int64_t i = (int64_t)blockIdx.x * RT + threadIdx.x; i < n4; i += stride) {
             const double2 wa = w2[2 * i], wb = w2[2 * i + 1];
-            const float w0 = (float)wa.x, w1 = (float)wa.y, w2f = (float)wb.x, w3 = (float)wb.y;
+            const float w0 = ct_d2f(wa.x), w1 = ct_d2f(wa.y), w2f = ct_d2f(wb.x), w3 = ct_d2f(wb.y);
 #pragma unroll
             for (int k = 0; k < NV; ++k) {
                 const float4 a = reinterpret_cast<const float4*>(x + (int64_t)k * ldv)[i];
@@ -474,7 +480,7 @@ __device__ __forceinline__ void cgs32_dots_group(int64_t n, const double* __rest
         }
     } else {
         for (int64_t i = (int64_t)blockIdx.x * RT + threadIdx.x; i < n; i += stride) {
-            const float wi = (float)w[i];
+            const float wi = ct_d2f(w[i]);
 #pragma unroll
             for (int k = 0; k < NV; ++k) acc[k] = fmaf(x[(int64_t)k * ldv + i], wi, acc[k]);
         }
@@ -544,20 +550,28 @@ __device__ __forceinline__ double cgs32_update_part(int64_t n, double* __restric
         const int64_t n4 = n / 4;
         double2* w2 = reinterpret_cast<double2*>(w);
         for (int64_t i = (int64_t)blockIdx.x * RT + threadIdx.x; i < n4; i += stride) {
+            double2 xa = w2[2 * i], xb = w2[2 * i + 1];
             float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (int v = 0; v < nvec; ++v) {
-                const float4 a = reinterpret_cast<const float4*>(V + (int64_t)v * ldv)[i];
-                const float cv = c[v];
+            auto add = [&](const float4& a, float cv) {
                 s.x = fmaf(cv, a.x, s.x);
                 s.y = fmaf(cv, a.y, s.y);
                 s.z = fmaf(cv, a.z, s.z);
                 s.w = fmaf(cv, a.w, s.w);
+            };
+            auto row = [&](int v) { return reinterpret_cast<const float4*>(V + (int64_t)v * ldv)[i]; };
+            int v = 0;
+            for (; v + 8 <= nvec; v += 8) {   // eight loads in flight
+                float4 a[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) a[u] = row(v + u);
+#pragma unroll
+                for (int u = 0; u < 8; ++u) add(a[u], c[v + u]);
             }
-            double2 xa = w2[2 * i], xb = w2[2 * i + 1];
-            xa.x -= (double)s.x;
-            xa.y -= (double)s.y;
-            xb.x -= (double)s.z;
-            xb.y -= (double)s.w;
+            for (; v < nvec; ++v) add(row(v), c[v]);
+            xa.x -= ct_f2d(s.x);
+            xa.y -= ct_f2d(s.y);
+            xb.x -= ct_f2d(s.z);
+            xb.y -= ct_f2d(s.w);
             w2[2 * i] = xa;
             w2[2 * i + 1] = xb;
             nn = fma(xa.x, xa.x, fma(xa.y, xa.y, fma(xb.x, xb.x, fma(xb.y, xb.y, nn))));
@@ -566,7 +580,7 @@ __device__ __forceinline__ double cgs32_update_part(int64_t n, double* __restric
         for (int64_t i = (int64_t)blockIdx.x * RT + threadIdx.x; i < n; i += stride) {
             float s = 0.f;
             for (int v = 0; v < nvec; ++v) s = fmaf(c[v], V[(int64_t)v * ldv + i], s);
-            const double x = w[i] - (double)s;
+            const double x = w[i] - ct_f2d(s);
             w[i] = x;
             nn = fma(x, x, nn);
         }
@@ -744,7 +758,7 @@ __global__ void lanczos_next32_kernel(int64_t n, const double* w, double* vnext,
             const double2 x = w2[i];
             const double2 v = make_double2(x.x * inv, x.y * inv);
             v2[i] = v;
-            f2[i] = make_float2((float)v.x, (float)v.y);
+            f2[i] = make_float2(ct_d2f(v.x), ct_d2f(v.y));
         }
         if ((n & 1) && blockIdx.x == 0 && threadIdx.x == 0) {
             const double v = w[n - 1] * inv;
@@ -755,7 +769,7 @@ __global__ void lanczos_next32_kernel(int64_t n, const double* w, double* vnext,
         for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
             const double v = w[i] * inv;
             vnext[i] = v;
-            vnext32[i] = (float)v;
+            vnext32[i] = ct_d2f(v);
         }
     }
 }
@@ -892,7 +906,7 @@ __global__ void __launch_bounds__(RT) lanczos_step_kernel(LanczosStep q) {
     own_elements(q.n, unit, [&](int64_t e) {
         const double v = q.w[e] * inv;
         q.vnext[e] = v;
-        if (MODE == 2) q.vnext32[e] = (float)v;
+        if (MODE == 2) q.vnext32[e] = ct_d2f(v);
     });
 }
 
@@ -900,7 +914,7 @@ __global__ void f64_to_f32_copy_kernel(int64_t n, const double* x, float* y, con
     ct_pdl();
     if (ct_skip(skip)) return;
     for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        y[i] = (float)x[i];
+        y[i] = ct_d2f(x[i]);
 }
 
 // Ritz vector: out = sum_{i < numiter} c_i V[i]
