@@ -1,8 +1,8 @@
 // Persistent one-sided Jacobi: all round-robin rounds of all sweeps in one
 // cooperative launch.  Every CTA walks the pairs of a round (k = blockIdx.x,
-// += gridDim.x), then waits at a grid barrier; after each sweep every CTA reads
-// the sweep's rotation flag and leaves together when it is zero.  The barrier
-// spins at most 2 s (then sets the status word and aborts), and cooperative
+// += gridDim.x), each pair waiting for its two vectors; after each sweep all meet at a
+// grid barrier, read the sweep's rotation flag and leave together when it is zero.  The
+// waits spin at most 2 s (then sets the status word and aborts), and cooperative
 // launch refuses grids that cannot be co-resident, so no wait is unbounded.
 //
 // What bounds it.  A warp issues one FP64 instruction every 64 cycles on this part
@@ -35,7 +35,47 @@ struct Sync {
     int* rot;          // [MAX_SWEEPS] nonzero: the sweep rotated; zeroed before launch
     int* sweeps;       // out: sweeps run
     int* status;
+    unsigned* ver;     // [vectors] rounds completed of each, zeroed before the launch; null: a grid
+                       // barrier after every round
 };
+
+// A round needs its vectors from two pairs of the round before, so within a sweep a pair waits
+// for those alone: every vector has a count of completed rounds (a grid barrier of 128 CTAs takes
+// ~2300 cycles after the stores, a release and an acquire ~1000, and no pair waits for the
+// slowest).  The counts a pair waits for at round r (base: rounds of the sweeps before): r, or
+// r - 1 of the vector that had no partner in the round before (odd numbers of vectors; pair 0).
+__device__ __forceinline__ unsigned vec_expected(unsigned base, int r, int v, bool odd) {
+    return base + (unsigned)r - (odd && v == r - 1 ? 1u : 0u);
+}
+// by one warp: true when both counts are there, false when the launch gives up
+__device__ __forceinline__ bool vec_wait(const Sync& s, int p, unsigned ep, int q, unsigned eq) {
+    const int lane = threadIdx.x & 31;
+    const unsigned* at = s.ver + (lane == 0 ? p : q);
+    const unsigned want = lane == 0 ? ep : eq;
+    const unsigned long long t0 = gtime();
+    for (;;) {
+        bool ready = true, give_up = false;
+        if (lane < 2) {
+            unsigned v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(at) : "memory");
+            ready = (int)(v - want) >= 0;
+            if (!ready) {
+                give_up = *(volatile int*)s.abort_flag != 0;
+                if (!give_up && gtime() - t0 > 2000000000ull) {
+                    atomicExch(s.abort_flag, 1);
+                    ct_set_status(s.status, CT_ERR_CUDA);
+                    give_up = true;
+                }
+            }
+        }
+        if (__any_sync(0xffffffffu, give_up)) return false;
+        if (__all_sync(0xffffffffu, ready)) return true;
+    }
+}
+// by one thread per vector, after a barrier of the threads that wrote it
+__device__ __forceinline__ void vec_done(const Sync& s, int v, unsigned count) {
+    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(s.ver + v), "r"(count) : "memory");
+}
 
 // target: arrivals expected so far (per thread, starting at 0).  Data that crosses the
 // barrier is read with __ldcg (the L1 of another SM may hold an old copy).
@@ -151,7 +191,7 @@ __global__ void __launch_bounds__(NT) jacobi_coop_kernel(T* X, int64_t len, T* Q
     ct_pdl();
     __shared__ double sm[24];
     __shared__ double rot_cs, rot_sn;
-    __shared__ int do_rot;
+    __shared__ int do_rot, live;
     const int P = (int)(nvec + (nvec & 1));
     const double floor = floor_rel * (*frob2);
     const int tid = threadIdx.x;
@@ -166,6 +206,19 @@ __global__ void __launch_bounds__(NT) jacobi_coop_kernel(T* X, int64_t len, T* Q
                 int p, q;
                 pair_index(P, r, k, p, q);
                 if (p >= nvec || q >= nvec) continue;
+                const unsigned base = (unsigned)(sweep * (P - 1));
+                if (s.ver && r > 0) {
+                    if (tid < 32) {
+                        const bool odd = nvec & 1;
+                        const bool there = vec_wait(s, p, vec_expected(base, r, p, odd), q, vec_expected(base, r, q, odd));
+                        if (tid == 0) live = there;
+                    }
+                    __syncthreads();
+                    if (!live) {
+                        ok = false;
+                        break;
+                    }
+                }
                 T* xp = X + (int64_t)p * len;
                 T* xq = X + (int64_t)q * len;
                 T* qp = Q + (int64_t)p * nvec;
@@ -233,8 +286,9 @@ __global__ void __launch_bounds__(NT) jacobi_coop_kernel(T* X, int64_t len, T* Q
                     }
                 }
                 __syncthreads();
+                if (s.ver && tid < 2) vec_done(s, tid ? q : p, base + (unsigned)r + 1);
             }
-            ok = grid_barrier(s, target);
+            if (ok && (!s.ver || r == P - 2)) ok = grid_barrier(s, target);
         }
         if (!ok) break;
         last_rot = __ldcg(s.rot + sweep) != 0;
@@ -251,7 +305,13 @@ __global__ void __launch_bounds__(NT) jacobi_coop_kernel(T* X, int64_t len, T* Q
 
 // Barrier and sweep scratch of a launch in d_flags: [16] count, [18] abort, [19] sweeps,
 // [32 .. 32 + max_sweeps) rotation flags; zeroed on the stream.
-inline int reset_sync(ct_handle* h, int max_sweeps, Sync& s) {
+// The vectors' counts are in d_partials, where they fit.
+inline int reset_sync(ct_handle* h, int max_sweeps, int64_t nvec, Sync& s) {
+    s.ver = nullptr;
+    if (nvec > 0 && nvec <= 2 * (int64_t)CT_NPARTIALS) {
+        s.ver = (unsigned*)h->d_partials;
+        CT_CUDA(h, cudaMemsetAsync(s.ver, 0, (size_t)nvec * sizeof(unsigned), h->stream));
+    }
     int* base = h->d_flags;
     CT_CUDA(h, cudaMemsetAsync(base + 16, 0, (16 + max_sweeps) * sizeof(int), h->stream));
     s.count = (unsigned*)(base + 16);
@@ -271,7 +331,7 @@ int run(ct_handle* h, T* X, int64_t len, T* Q, int64_t nvec, double tol, double 
         return CT_OK;
     }
     Sync s;
-    CT_TRY(reset_sync(h, MAX_SWEEPS, s));
+    CT_TRY(reset_sync(h, MAX_SWEEPS, nvec, s));
     static int occ_dev = -1, occ = 0;
     if (occ_dev != h->device) {
         CT_CUDA(h, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, jacobi_coop_kernel<T>, NT, 0));

@@ -366,7 +366,7 @@ static int svd_qr_jacobi(ct_handle* h, Arena& ar, const double* M, int64_t m, in
         if (grid > need) grid = need;
         if (grid < 1) grid = 1;
         ct_jacobi::Sync sy;
-        CT_TRY(ct_jacobi::reset_sync(h, 0, sy));
+        CT_TRY(ct_jacobi::reset_sync(h, 0, 0, sy));
         void* args[] = {&T, &len, &nvec, (void*)&k, &refl, &sy};
         CT_CUDA(h, cudaLaunchCooperativeKernel((const void*)qr_coop_kernel, dim3((unsigned)grid), dim3(QR_NT), args,
                                                smem, h->stream));

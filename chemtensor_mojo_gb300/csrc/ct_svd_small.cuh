@@ -9,7 +9,9 @@
 // one-warp dot product: lane l sums elements l, l + 32, ...), then all four the rotation.
 //   * up to 96 vectors: one cluster of up to 16 CTAs with one to three teams each and the
 //     hardware cluster barrier (~900 cycles with the stores before it);
-//   * more: one team per CTA and the grid barrier (~2300 cycles for 128 CTAs).
+//   * more: one team per CTA, every pair waiting for its two vectors alone (vec_wait), with a
+//     grid barrier per sweep.
+// (One launch per form, us: 64 vectors 3855 as a cluster and 4178 as a grid, 96 7383 and 7342.)
 // The rotations and their order are those of the one-CTA form, operation for operation, so
 // the factors come out the same to the last bit (the signs of singular vectors included,
 // which depend on the path: without QR preconditioning a change of 1e-16 flips some).
@@ -51,6 +53,7 @@ __global__ void __launch_bounds__(CLUSTER ? TEAM * MAX_TEAMS : TEAM) svd_small_k
     __shared__ double dots[MAX_TEAMS][3];
     __shared__ double rot_s[MAX_TEAMS][2];
     __shared__ int go_s[MAX_TEAMS];
+    __shared__ int live;
     const int lane = threadIdx.x & 31;
     // warps spread over the CTAs first, so that fewer tasks than warps still use every SM
     const int w = (int)(threadIdx.x >> 5) * (int)gridDim.x + (int)blockIdx.x;
@@ -86,7 +89,9 @@ __global__ void __launch_bounds__(CLUSTER ? TEAM * MAX_TEAMS : TEAM) svd_small_k
     for (int i = lane; i < nvec; i += 32) f2 += __ldcg(a.nsq + i);
     const double floor = EPS * EPS * ct_warp_sum(f2);
 
-    const int team = (int)threadIdx.x / TEAM, tt = (int)threadIdx.x % TEAM, tw = tt >> 5;
+    // (the roles of a team's warps start one SM quarter later in each team, so that two teams'
+    // rotations, a chain of FP64 instructions in one warp, do not share a quarter)
+    const int team = (int)threadIdx.x / TEAM, tt = (int)threadIdx.x % TEAM, tw = ((tt >> 5) + 4 - team) & 3;
     const int gt = team * (int)gridDim.x + (int)blockIdx.x;
     const int teams = (int)(blockDim.x / TEAM) * (int)gridDim.x;
     // Q's elements start half a team later than X's: up to 64 of each are rotated side by side
@@ -100,6 +105,19 @@ __global__ void __launch_bounds__(CLUSTER ? TEAM * MAX_TEAMS : TEAM) svd_small_k
                 int p, q;
                 ct_jacobi::pair_index(P, r, pr, p, q);
                 if (p >= nvec || q >= nvec) continue;   // the same for the whole team
+                const unsigned base = (unsigned)(sweep * (P - 1));
+                if constexpr (!CLUSTER) {   // (one team per CTA)
+                    if (a.s.ver && r > 0) {
+                        if (tt < 32) {
+                            const bool odd = nvec & 1;
+                            const bool there = ct_jacobi::vec_wait(a.s, p, ct_jacobi::vec_expected(base, r, p, odd), q,
+                                                                   ct_jacobi::vec_expected(base, r, q, odd));
+                            if (tt == 0) live = there;
+                        }
+                        team_sync(team);
+                        if (!live) return;
+                    }
+                }
                 double* xp = a.X + (int64_t)p * len;
                 double* xq = a.X + (int64_t)q * len;
                 double* qp = a.Q + (int64_t)p * nvec;
@@ -149,9 +167,10 @@ __global__ void __launch_bounds__(CLUSTER ? TEAM * MAX_TEAMS : TEAM) svd_small_k
                     }
                 }
                 team_sync(team);
-                if (!go_s[team]) continue;
+                const bool go = go_s[team];
                 const double cs = rot_s[team][0], sn = rot_s[team][1];
-                if constexpr (E > 0) {
+                if (!go) {
+                } else if constexpr (E > 0) {
 #pragma unroll
                     for (int e = 0; e < E; ++e) {
                         const int i = e * TEAM + tt, iq = e * TEAM + tq;
@@ -178,8 +197,16 @@ __global__ void __launch_bounds__(CLUSTER ? TEAM * MAX_TEAMS : TEAM) svd_small_k
                         qq[i] = ct_jacobi::rot_y(cs, sn, u, v);
                     }
                 }
+                if constexpr (!CLUSTER) {
+                    if (a.s.ver) {
+                        team_sync(team);
+                        if (tt < 2) ct_jacobi::vec_done(a.s, tt ? q : p, base + (unsigned)r + 1);
+                    }
+                }
             }
-            if (!barrier()) return;
+            if (CLUSTER || !a.s.ver || r == P - 2) {
+                if (!barrier()) return;
+            }
         }
         // every CTA reads the same word: nothing writes rot[sweep] after the last barrier
         converged = __ldcg(a.s.rot + sweep) == 0;
@@ -223,7 +250,7 @@ int launch(ct_handle* h, Args& a, int ctas, int teams) {
 // Jacobi of the vectors of M (nvec >= 2): X, Q and nsq in the fields set by the caller; the
 // sweeps run go to d_flags[19].
 inline int run(ct_handle* h, Args& a) {
-    CT_TRY(ct_jacobi::reset_sync(h, MAX_SWEEPS, a.s));
+    CT_TRY(ct_jacobi::reset_sync(h, MAX_SWEEPS, a.nvec, a.s));
     a.max_sweeps = (h->svd_max_sweeps > 0 && h->svd_max_sweeps < MAX_SWEEPS) ? h->svd_max_sweeps : MAX_SWEEPS;
     const int pairs = (a.nvec + 1) / 2;
     const int big = a.len > a.nvec ? a.len : a.nvec;
