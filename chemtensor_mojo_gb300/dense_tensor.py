@@ -25,6 +25,12 @@ import torch
 from . import _lib
 from ._lib import check
 
+# The current stream's handle without the Stream object that torch.cuda.current_stream makes: an
+# H_eff apply at chi 16 is bound by the host (34 us a call with it, numpy's product of the shape
+# and ctypes objects for pointers; 20 us without).
+_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None) or (
+    lambda device: torch.cuda.current_stream(device).cuda_stream)
+
 _ctx_lock = threading.Lock()
 _contexts = {}
 
@@ -48,7 +54,7 @@ class DeviceContext:
         self._bound = self._torch_stream()
 
     def _torch_stream(self) -> int:
-        s = torch.cuda.current_stream(self.device).cuda_stream
+        s = _raw_stream(self.device)
         return s if s != 0 else 1  # 1 = cudaStreamLegacy (torch's default stream)
 
     def bind(self) -> "DeviceContext":
@@ -99,8 +105,9 @@ def get_context(device: int | None = None) -> DeviceContext:
         return ctx
 
 
-def _ptr(t: torch.Tensor) -> C.c_void_p:
-    return C.c_void_p(t.data_ptr())
+def _ptr(t: torch.Tensor) -> int:
+    """Device address for a void* argument (the library's functions have their argtypes)."""
+    return t.data_ptr()
 
 
 def compute_row_major_strides(shape: Sequence[int]) -> List[int]:
@@ -116,11 +123,14 @@ class DenseTensor:
     def __init__(self, storage: torch.Tensor, shape: Sequence[int]):
         if storage.dtype != torch.float64 or not storage.is_cuda:
             raise TypeError("DenseTensor storage must be a CUDA float64 tensor")
-        n = int(np.prod(shape)) if len(shape) else 1
-        if storage.numel() < n:
-            raise ValueError("storage smaller than shape")
-        self.storage = storage.reshape(-1)[:n] if storage.numel() != n else storage.reshape(-1)
         self.shape = [int(s) for s in shape]
+        n = math.prod(self.shape)
+        have = storage.numel()
+        if have < n:
+            raise ValueError("storage smaller than shape")
+        if storage.dim() != 1:
+            storage = storage.reshape(-1)
+        self.storage = storage[:n] if have != n else storage
 
     # -- views and properties ------------------------------------------------
     @property
