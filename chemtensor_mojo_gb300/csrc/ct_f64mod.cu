@@ -657,11 +657,13 @@ int fm_map(ct_handle* h, CUtensorMap* m, const FmSrc& s, int box_rows) {
 }  // namespace
 
 // Whether an FP64-form product goes to the tensor cores.  Estimated times in us: the SIMT
-// kernel at 85% of the FP64 pipe (2 multiply-adds per clock and SM, 1.9 GHz); here 14 us of
-// launches and latencies, the residues (written and read once) and the tensor-core products.
-// Taken when at least a fifth shorter.  Only when the scratch is there or can be had: within the
-// handle's workspace limit, outside a stream capture, and with the memory available; otherwise
-// the SIMT kernel, as before.
+// kernel at 85% of the FP64 pipe (2 multiply-adds per clock and SM, 1.9 GHz); here 12 us of
+// launches and latencies, tile items at 1.2 us plus 0.16 us per 64 of K on each SM, and operands
+// and residues written and read at 4 TB/s.  Measured (us, SIMT / here): 128x384x128 16.6 / 17.9 and
+// 128x256x128 12.9 / 13.9 stay, 512x128x128 20.6 / 17.0, 640x128x128 24.0 / 18.7, 256x256x128
+// 20.5 / 19.2 and 256x256x256 36.9 / 20.0 go.  Only when the scratch is there or can be had: within
+// the handle's workspace limit, outside a stream capture, and with the memory available;
+// otherwise the SIMT kernel, as before.
 bool ct_f64_route(ct_handle* h, int64_t M, int64_t N, int64_t K) {
     if (M <= 0 || N <= 0 || K <= 0 || K > ((int64_t)1 << 20) || !ct_fp64_tc_enabled(h, M, N, K)) return false;
     const FmPlan q = fm_plan(M, N, K);
@@ -670,7 +672,7 @@ bool ct_f64_route(ct_handle* h, int64_t M, int64_t N, int64_t K) {
     const double simt = (double)M * (double)N * (double)K / (0.85 * 2.0 * h->num_sms * 1900.0);
     const double items = (double)ct_cdiv(q.tiles * MODS, h->num_sms) * (1.2 + 0.16 * (double)(q.ldk / FM_BK));
     const double traffic = ((double)(M + N) * (double)q.ldk * 4.0 * MODS + (double)M * (double)q.ldn * 2.0 * MODS) / 4.0e6;
-    if (14.0 + items + traffic > 0.8 * simt) return false;
+    if (12.0 + items + traffic > simt) return false;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess) {
         (void)cudaGetLastError();
