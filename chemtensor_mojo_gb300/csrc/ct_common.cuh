@@ -310,6 +310,7 @@ int ct_apply_mpo_launch(ct_handle* h, const double* A, const double* W, double* 
 // vector kernels (ct_vec.cu)
 int ct_reduce_dot(ct_handle* h, int64_t n, const double* x, const double* y, double* d_out,
                   const int* skip);
+int ct_partial_nrm2sq(ct_handle* h, int64_t n, const double* x, int* np);
 int ct_reduce_nrm2sq(ct_handle* h, int64_t n, const double* x, double* d_out, const int* skip);
 int ct_scale_by_inv_sqrt(ct_handle* h, int64_t n, const double* x, double* y,
                          const double* d_nsq, const int* skip, int zero_code);

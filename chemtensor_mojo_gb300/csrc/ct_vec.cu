@@ -1300,6 +1300,14 @@ int ct_reduce_nrm2sq(ct_handle* h, int64_t n, const double* x, double* d_out, co
     return CT_OK;
 }
 
+// the first half of ct_reduce_nrm2sq: *np partial sums of squares in d_partials
+int ct_partial_nrm2sq(ct_handle* h, int64_t n, const double* x, int* np) {
+    *np = grid_for(h, n);
+    ct_launch(h, partial_kernel<1>, *np, RT, 0, n, x, nullptr, h->d_partials, nullptr); ct_note_launch();
+    CT_LAUNCH_CHECK(h);
+    return CT_OK;
+}
+
 int ct_scale_by_inv_sqrt(ct_handle* h, int64_t n, const double* x, double* y, const double* d_nsq,
                          const int* skip, int zero_code) {
     ct_launch(h, scale_inv_sqrt_kernel, elem_grid(h, n), 256, 0, n, x, y, d_nsq, skip, h->d_status, zero_code); ct_note_launch();
