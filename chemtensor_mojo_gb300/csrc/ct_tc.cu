@@ -638,6 +638,73 @@ __device__ __forceinline__ unsigned tc_arrive(unsigned long long* p, unsigned ep
 }
 
 
+// One thread's HC sums of row m, columns from n0 on, to C.
+template <int HC>
+__device__ __forceinline__ void tc_store_sums(const TcEpi& epi, const float (&sum)[HC], int64_t m, int n0, int M, int N) {
+    if (m >= M) return;
+    if (epi.trans) {
+        // element (m, n) to C[n][m]: for each n the warp's 32 rows are 32 consecutive words
+#pragma unroll
+        for (int j = 0; j < HC; ++j) {
+            const int64_t n = (int64_t)n0 + j;
+            if (n >= N) break;
+            const int64_t a = n * epi.sCm0 + m;
+            if (epi.out_fp64) {
+                double* Cd = (double*)epi.C;
+                double v = epi.alpha * (double)sum[j];
+                if (epi.beta != 0.0) v = fma(epi.beta, Cd[a], v);
+                Cd[a] = v;
+            } else {
+                ((float*)epi.C)[a] = (float)epi.alpha * sum[j];
+            }
+        }
+        return;
+    }
+    const int64_t rbase = (m / epi.M0) * epi.sCm1 + (m % epi.M0) * epi.sCm0;
+#pragma unroll
+    for (int cc = 0; cc < HC; cc += 16) {
+        const int64_t nb = (int64_t)n0 + cc;
+        if (epi.vec && nb + 16 <= N) {
+            if (epi.out_fp64) {
+                double2* Cd = (double2*)((double*)epi.C + rbase + nb);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    double2 o;
+                    o.x = epi.alpha * (double)sum[cc + 2 * j];
+                    o.y = epi.alpha * (double)sum[cc + 2 * j + 1];
+                    if (epi.beta != 0.0) {
+                        const double2 c0 = Cd[j];
+                        o.x = fma(epi.beta, c0.x, o.x);
+                        o.y = fma(epi.beta, c0.y, o.y);
+                    }
+                    Cd[j] = o;
+                }
+            } else {
+                float4* Cf = (float4*)((float*)epi.C + rbase + nb);
+                const float a = (float)epi.alpha;
+#pragma unroll
+                for (int j = 0; j < 4; ++j)
+                    Cf[j] = make_float4(a * sum[cc + 4 * j], a * sum[cc + 4 * j + 1], a * sum[cc + 4 * j + 2],
+                                        a * sum[cc + 4 * j + 3]);
+            }
+            continue;
+        }
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            const int64_t n = nb + j;
+            if (n >= N) break;
+            if (epi.out_fp64) {
+                double* Cd = (double*)epi.C + rbase;
+                double v = epi.alpha * (double)sum[cc + j];
+                if (epi.beta != 0.0) v = fma(epi.beta, Cd[n], v);
+                Cd[n] = v;
+            } else {
+                ((float*)epi.C)[rbase + n] = (float)epi.alpha * sum[cc + j];
+            }
+        }
+    }
+}
+
 // Registers: each SM sub-partition holds 16K of them; 10 warps put 3 on some
 // sub-partitions (168 per thread), 18 warps put 5 (96 per thread, enough for 32
 // sums and 32 loaded columns).
@@ -865,70 +932,7 @@ __global__ void __launch_bounds__(tc_chunk_threads(BN), 1)
                 }
             }
             const int m0 = (w.t / tiles_n) * TC_BM;
-            const int n0 = (w.t % tiles_n) * BN + hf * HC;
-            const int64_t m = (int64_t)m0 + row;
-            if (m >= M) continue;
-            if (epi.trans) {
-                // element (m, n) to C[n][m]: for each n the warp's 32 rows are 32 consecutive words
-#pragma unroll
-                for (int j = 0; j < HC; ++j) {
-                    const int64_t n = (int64_t)n0 + j;
-                    if (n >= N) break;
-                    const int64_t a = n * epi.sCm0 + m;
-                    if (epi.out_fp64) {
-                        double* Cd = (double*)epi.C;
-                        double v = epi.alpha * (double)sum[j];
-                        if (epi.beta != 0.0) v = fma(epi.beta, Cd[a], v);
-                        Cd[a] = v;
-                    } else {
-                        ((float*)epi.C)[a] = (float)epi.alpha * sum[j];
-                    }
-                }
-                continue;
-            }
-            const int64_t rbase = (m / epi.M0) * epi.sCm1 + (m % epi.M0) * epi.sCm0;
-#pragma unroll
-            for (int cc = 0; cc < HC; cc += 16) {
-                const int64_t nb = (int64_t)n0 + cc;
-                if (epi.vec && nb + 16 <= N) {
-                    if (epi.out_fp64) {
-                        double2* Cd = (double2*)((double*)epi.C + rbase + nb);
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            double2 o;
-                            o.x = epi.alpha * (double)sum[cc + 2 * j];
-                            o.y = epi.alpha * (double)sum[cc + 2 * j + 1];
-                            if (epi.beta != 0.0) {
-                                const double2 c0 = Cd[j];
-                                o.x = fma(epi.beta, c0.x, o.x);
-                                o.y = fma(epi.beta, c0.y, o.y);
-                            }
-                            Cd[j] = o;
-                        }
-                    } else {
-                        float4* Cf = (float4*)((float*)epi.C + rbase + nb);
-                        const float a = (float)epi.alpha;
-#pragma unroll
-                        for (int j = 0; j < 4; ++j)
-                            Cf[j] = make_float4(a * sum[cc + 4 * j], a * sum[cc + 4 * j + 1], a * sum[cc + 4 * j + 2],
-                                                a * sum[cc + 4 * j + 3]);
-                    }
-                    continue;
-                }
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const int64_t n = nb + j;
-                    if (n >= N) break;
-                    if (epi.out_fp64) {
-                        double* Cd = (double*)epi.C + rbase;
-                        double v = epi.alpha * (double)sum[cc + j];
-                        if (epi.beta != 0.0) v = fma(epi.beta, Cd[n], v);
-                        Cd[n] = v;
-                    } else {
-                        ((float*)epi.C)[rbase + n] = (float)epi.alpha * sum[cc + j];
-                    }
-                }
-            }
+            tc_store_sums<HC>(epi, sum, (int64_t)m0 + row, (w.t % tiles_n) * BN + hf * HC, M, N);
         }
     }
     ct_pdl_next();
@@ -936,6 +940,207 @@ __global__ void __launch_bounds__(tc_chunk_threads(BN), 1)
     if (warp == 1) {
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS)
+                     : "memory");
+    }
+}
+
+// The chunked kernel for whole tiles by pairs of CTAs (cta_group::2): a cluster of two takes 256
+// rows x BN columns, each CTA its 128 rows of A, its half of B's columns and its 128 rows of the
+// accumulator; the first CTA issues the MMAs for both.  A CTA then loads 2 x (16 KB + BN x 64
+// bytes) per k-block instead of 2 x (16 KB + BN x 128): the transfer from L2 bounds the one-CTA
+// kernel (tensor pipe 65% active at 224 columns; 88 KB per k-block arrive at 41 bytes per clock
+// and SM, where the MMAs take 1344 of the 2150 clocks; neither deeper pipelines of half k-blocks nor
+// keeping A in the collector changed that).  Same MMAs, chunks and sums per element, so the same
+// bits.  4096 x 1024 x 4096: 132.8 us with one CTA per tile, 110.5 here (311 TFLOP/s); H_eff at chi
+// 1024 450 and 419.
+template <int BN>
+struct TcPairSmem {
+    static constexpr int A_BYTES = TC_BM * TC_BK * 4;
+    static constexpr int B_BYTES = BN / 2 * TC_BK * 4;
+    static constexpr int STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES;
+    static constexpr int STAGES = (227 * 1024 - 1280) / STAGE_BYTES;
+    static constexpr int TILE_BYTES = STAGES * STAGE_BYTES;
+    static constexpr int TOTAL = TILE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+};
+
+template <int BN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(tc_chunk_threads(BN), 1)
+    tc_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmAh, const __grid_constant__ CUtensorMap tmAl,
+                        const __grid_constant__ CUtensorMap tmBh, const __grid_constant__ CUtensorMap tmBl, int M,
+                        int N, int Kpad, int kc, TcEpi epi, int ptiles, const int* skip, int* status) {
+    ct_pdl();
+    using L = TcPairSmem<BN>;
+    constexpr int STAGES = L::STAGES;
+    constexpr int EPW = tc_chunk_epw(BN);
+    constexpr int HC = BN / EPW;   // columns per epilogue warp
+    constexpr int NB = 512 / BN;   // chunk accumulators in TMEM (all 512 columns)
+    constexpr uint32_t TMEM_COLS = tc_pow2_cols(NB * BN);
+    if (ct_skip(skip)) return;
+    extern __shared__ uint8_t tc_smem_raw[];
+    uint8_t* smem = tc_smem_raw + ((1024u - (smem_u32(tc_smem_raw) & 1023u)) & 1023u);
+    uint64_t* full = (uint64_t*)(smem + L::TILE_BYTES);   // the first CTA's: both CTAs' loads
+    uint64_t* empty = full + STAGES;
+    uint64_t* acc_full = empty + STAGES;
+    uint64_t* acc_empty = acc_full + NB;                  // the first CTA's: both CTAs' epilogues
+    uint32_t* tmem_slot = (uint32_t*)(acc_empty + NB);
+    volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int rank = (int)cluster_rank();
+    const int tiles_n = (N + BN - 1) / BN;
+    const int nkb = Kpad / TC_BK;
+    const int c = blockIdx.x / 2, G = gridDim.x / 2;
+
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < STAGES; ++s) {
+            mbar_init(&full[s], 1);
+            mbar_init(&empty[s], 1);
+        }
+        for (int b = 0; b < NB; ++b) {
+            mbar_init(&acc_full[b], 1);
+            mbar_init(&acc_empty[b], 2 * 4 * EPW);
+        }
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                     "r"(TMEM_COLS)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    cluster_sync_all();   // both CTAs' barriers and accumulators are there
+    tc_fence_after();
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int g = 0;
+            bool ok = true;
+            for (int t = c; ok && t < ptiles; t += G) {
+                const int m0 = (2 * (t / tiles_n) + rank) * TC_BM, n0 = (t % tiles_n) * BN + rank * (BN / 2);
+                for (int kb = 0; kb < nkb; ++kb, ++g) {
+                    const int s = g % STAGES;
+                    const uint32_t ph = (uint32_t)(g / STAGES) & 1u;
+                    if (g >= STAGES && !mbar_wait(&empty[s], ph ^ 1u, abort_flag)) {
+                        *abort_flag = 1;
+                        ct_set_status(status, CT_ERR_CUDA);
+                        ok = false;
+                        break;
+                    }
+                    uint8_t* st = smem + s * L::STAGE_BYTES;
+                    if (rank == 0) mbar_expect_tx(&full[s], 2 * L::STAGE_BYTES);
+                    const uint32_t bar = smem_peer(&full[s], 0);
+                    const int x = kb * TC_BK;
+                    tma_load_2d_pair(st, &tmAh, x, m0, bar);
+                    tma_load_2d_pair(st + L::A_BYTES, &tmAl, x, m0, bar);
+                    tma_load_2d_pair(st + 2 * L::A_BYTES, &tmBh, x, n0, bar);
+                    tma_load_2d_pair(st + 2 * L::A_BYTES + L::B_BYTES, &tmBl, x, n0, bar);
+                }
+            }
+            // the last arrivals on this CTA's empty barriers, before it may exit
+            for (int q = g > STAGES ? g - STAGES : 0; ok && q < g; ++q) {
+                if (!mbar_wait(&empty[q % STAGES], (uint32_t)(q / STAGES) & 1u, abort_flag)) {
+                    *abort_flag = 1;
+                    ct_set_status(status, CT_ERR_CUDA);
+                    ok = false;
+                }
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0 && rank == 0) {
+            constexpr uint32_t idesc = idesc_tf32(2 * TC_BM, BN);
+            int g = 0, gc = 0;
+            bool ok = true;
+            for (int t = c; ok && t < ptiles; t += G) {
+                for (int kb0 = 0; kb0 < nkb && ok; kb0 += kc, ++gc) {
+                    const int b = gc % NB, u = gc / NB;
+                    if (u > 0 && !mbar_wait(&acc_empty[b], (uint32_t)((u - 1) & 1), abort_flag)) {
+                        *abort_flag = 1;
+                        ct_set_status(status, CT_ERR_CUDA);
+                        ok = false;
+                        break;
+                    }
+                    tc_fence_after();
+                    const uint32_t dt = tmem + (uint32_t)(b * BN);
+                    const int kb1 = kb0 + kc < nkb ? kb0 + kc : nkb;
+                    for (int kb = kb0; kb < kb1; ++kb, ++g) {
+                        const int s = g % STAGES;
+                        const uint32_t ph = (uint32_t)(g / STAGES) & 1u;
+                        if (!mbar_wait(&full[s], ph, abort_flag)) {
+                            *abort_flag = 1;
+                            ct_set_status(status, CT_ERR_CUDA);
+                            ok = false;
+                            break;
+                        }
+                        tc_fence_after();
+                        const uint32_t a_hi = smem_u32(smem + s * L::STAGE_BYTES);
+                        const uint32_t a_lo = a_hi + L::A_BYTES;
+                        const uint32_t b_hi = a_hi + 2 * L::A_BYTES;
+                        const uint32_t b_lo = b_hi + L::B_BYTES;
+#pragma unroll
+                        for (int kk = 0; kk < TC_BK / 8; ++kk) {
+                            const uint32_t off = kk * 32;
+                            const uint32_t acc0 = (kb > kb0 || kk > 0) ? 1u : 0u;
+                            mma_tf32_pair(dt, sw128_desc(a_lo + off), sw128_desc(b_hi + off), idesc, acc0);
+                            mma_tf32_pair(dt, sw128_desc(a_hi + off), sw128_desc(b_lo + off), idesc, 1u);
+                            mma_tf32_pair(dt, sw128_desc(a_hi + off), sw128_desc(b_hi + off), idesc, 1u);
+                        }
+                        mma_commit_pair(&empty[s]);
+                    }
+                    if (ok) mma_commit_pair(&acc_full[b]);
+                }
+            }
+        }
+    } else {
+        const int q = warp & 3;              // TMEM lane quadrant of this warp
+        const int hf = (warp - 2) >> 2;      // column group of the tile
+        const int row = q * 32 + lane;
+        float sum[HC];
+        int gc = 0;
+        bool ok = true;
+        for (int t = c; ok && t < ptiles; t += G) {
+#pragma unroll
+            for (int j = 0; j < HC; ++j) sum[j] = 0.f;
+            for (int kb0 = 0; kb0 < nkb; kb0 += kc, ++gc) {
+                const int b = gc % NB, u = gc / NB;
+                if (!mbar_wait(&acc_full[b], (uint32_t)(u & 1), abort_flag)) {
+                    *abort_flag = 1;
+                    ct_set_status(status, CT_ERR_CUDA);
+                    ok = false;
+                    break;
+                }
+                __syncwarp();
+                tc_fence_after();
+                const uint32_t tq = tmem + (uint32_t)(b * BN + hf * HC) + ((uint32_t)(q * 32) << 16);
+                constexpr int LB = HC >= 96 ? (HC % 32 == 0 ? 32 : 16) : HC;   // (as the one-CTA kernel)
+#pragma unroll
+                for (int cc = 0; cc < HC; cc += LB) {
+                    uint32_t r[LB];
+#pragma unroll
+                    for (int q8 = 0; q8 < LB; q8 += 8)
+                        tmem_ld8_nowait(tq + (uint32_t)(cc + q8), *reinterpret_cast<uint32_t(*)[8]>(&r[q8]));
+                    tmem_wait_ld();
+#pragma unroll
+                    for (int j = 0; j < LB; ++j) sum[cc + j] += __uint_as_float(r[j]);
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive_peer(smem_peer(&acc_empty[b], 0));
+            }
+            if (!ok) break;
+            const int m0 = (2 * (t / tiles_n) + rank) * TC_BM;
+            tc_store_sums<HC>(epi, sum, (int64_t)m0 + row, (t % tiles_n) * BN + hf * HC, M, N);
+        }
+    }
+    __syncthreads();
+    tc_fence_before();
+    cluster_sync_all();   // neither CTA's barriers or accumulators are used any more
+    if (warp == 1) {
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS)
                      : "memory");
     }
 }
@@ -1646,6 +1851,29 @@ int tc_gemm_run(ct_handle* h, const SplitOperand& A, const SplitOperand& B, int6
             hy.part = h->tc_hy_part;
             hy.cnt = h->tc_hy_cnt;
             grid = hy.tiles_dp > 0 ? h->num_sms : hy.gsk;
+        }
+        // Whole tiles in pairs of rows, wide and at least 1024 deep: the paired kernel.  (us, one CTA /
+        // pairs: 4096x1024xK in 224-wide tiles K 256 12.5 / 12.6, 512 19.1 / 18.8, 1024 32.5 / 31.0,
+        // 2048 70.7 / 59.6, 4096 132.8 / 110.5; 4864x1024xK in 256-wide ones 16.8 / 17.4, 23.8 / 24.1,
+        // 38.6 / 38.0, 83.7 / 70.4, 154 / 128; 192-wide 5120x2048x1024 87.5 / 92.6, 128-wide
+        // 3072x768x3840 87.1 / 88.0.)
+        constexpr bool wide = BN >= 224;
+        if (wide && hy.gsk == 0 && ct_cdiv(M, TC_BM) % 2 == 0 && A.ldk >= 32 * TC_BK && h->num_sms % 2 == 0) {
+            constexpr int PBN = wide ? BN : 224;   // (the others are not instantiated)
+            using LP = TcPairSmem<PBN>;
+            static int pair_dev = -1;
+            if (pair_dev != h->device) {
+                CT_CUDA(h, cudaFuncSetAttribute(tc_gemm_pair_kernel<PBN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                LP::TOTAL));
+                pair_dev = h->device;
+            }
+            CT_TRY(make_map(h, &tb_h, B.hi, B.rows, B.ldk, BN / 2));
+            CT_TRY(make_map(h, &tb_l, B.lo, B.rows, B.ldk, BN / 2));
+            const int64_t ptiles = tiles / 2, pairs = std::min<int64_t>(ptiles, h->num_sms / 2);
+            ct_launch(h, tc_gemm_pair_kernel<PBN>, (unsigned)(2 * pairs), tc_chunk_threads(PBN), LP::TOTAL, ta_h, ta_l, tb_h,
+                      tb_l, (int)M, (int)N, (int)A.ldk, kc, epi, (int)ptiles, skip, h->d_status); ct_note_launch();
+            CT_LAUNCH_CHECK(h);
+            return CT_OK;
         }
         ct_launch(h, tc_gemm_chunk_kernel<BN, STAGES>, (unsigned)grid, tc_chunk_threads(BN), L::TOTAL, 
             ta_h, ta_l, tb_h, tb_l, (int)M, (int)N, (int)A.ldk, kc, epi, hy, skip, h->d_status);
