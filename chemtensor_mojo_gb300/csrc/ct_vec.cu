@@ -368,6 +368,22 @@ __device__ __forceinline__ void cgs_dots_part(int64_t n, const double* __restric
 // the blocks
 __device__ __forceinline__ void cgs_coeffs(const double* partials, int nvec, double* coeff) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    if (gridDim.x <= 32 && nvec <= 64) {   // (short vectors: all loads first)
+        double r[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int v = wid + k * (RT / 32);
+            r[k] = v < nvec && lane < (int)gridDim.x ? __ldcg(partials + (int64_t)lane * nvec + v) : 0.0;
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int v = wid + k * (RT / 32);
+            if (v >= nvec) break;
+            const double t = ct_warp_sum(r[k]);
+            if (lane == 0) coeff[v] = t;
+        }
+        return;
+    }
     for (int v = wid; v < nvec; v += RT / 32) {
         double r = 0.0;
         for (int b = lane; b < (int)gridDim.x; b += 32) r += __ldcg(partials + (int64_t)b * nvec + v);
@@ -782,8 +798,8 @@ __global__ void lanczos_next32_kernel(int64_t n, const double* w, double* vnext,
 // sums, not the vectors.  The grid, each thread's elements and every sum's order are those of the
 // separate kernels, so the results are the same bits; each block forms the totals itself.
 // Vectors past 32768 elements (16 blocks) need more SMs.  Measured: Lanczos at chi 32, 20 steps,
-// 837 us with separate launches, 725 here; the 16-site Heisenberg run, chi 64, mixed, 162 ms
-// and 141.5.
+// 837 us with separate launches, 701 here; the 16-site Heisenberg run, chi 64, mixed, 162 ms
+// and 135.
 constexpr int STEP_MAXG = 16;
 struct LanczosStep {
     int64_t n, ldv;
@@ -812,11 +828,32 @@ __device__ __forceinline__ double grid_total(double v, double* slot, double* sm)
     return ct_warp_sum(lane < (int)gridDim.x ? __ldcg(slot + lane) : 0.0);
 }
 
-// f(element) for this thread's elements under the unit-element mapping of the kernels above
-template <typename F>
-__device__ __forceinline__ void own_elements(int64_t n, int unit, F f) {
-    for (int64_t i = (int64_t)blockIdx.x * RT + threadIdx.x; i < n / unit; i += (int64_t)gridDim.x * RT)
-        for (int e = 0; e < unit; ++e) f(i * unit + e);
+// store(element, load(element)) for this thread's elements under the UNIT-element mapping of the
+// kernels above, eight elements' loads before their stores (a step of 16384 elements has eight per
+// thread: one memory latency instead of eight)
+template <int UNIT, typename L, typename S>
+__device__ __forceinline__ void own_elements_u(int64_t n, L load, S store) {
+    constexpr int B = 8 / UNIT;
+    const int64_t m = n / UNIT, stride = (int64_t)gridDim.x * RT;
+    for (int64_t i = (int64_t)blockIdx.x * RT + threadIdx.x; i < m; i += B * stride) {
+        double v[8];
+#pragma unroll
+        for (int b = 0; b < B; ++b)
+#pragma unroll
+            for (int e = 0; e < UNIT; ++e)
+                if (i + b * stride < m) v[b * UNIT + e] = load((i + b * stride) * UNIT + e);
+#pragma unroll
+        for (int b = 0; b < B; ++b)
+#pragma unroll
+            for (int e = 0; e < UNIT; ++e)
+                if (i + b * stride < m) store((i + b * stride) * UNIT + e, v[b * UNIT + e]);
+    }
+}
+template <typename L, typename S>
+__device__ __forceinline__ void own_elements(int64_t n, int unit, L load, S store) {
+    if (unit == 4) own_elements_u<4>(n, load, store);
+    else if (unit == 2) own_elements_u<2>(n, load, store);
+    else own_elements_u<1>(n, load, store);
 }
 
 // MODE 0: the reference recurrence, 1: reorthogonalised in FP64, 2: against the FP32 copy
@@ -859,16 +896,19 @@ __global__ void __launch_bounds__(RT) lanczos_step_kernel(LanczosStep q) {
         const bool v2 = aligned16(q.w) && aligned16(q.vj) && (!q.vjm1 || aligned16(q.vjm1));
         if (beta(grid_total(recurrence<true>(q.n, q.w, q.vj, q.vjm1, alpha, bprev), p_beta, sm))) return;
         const double inv = bs[1];
-        own_elements(q.n, v2 ? 2 : 1, [&](int64_t e) { q.vnext[e] = q.w[e] * inv; });
+        own_elements(q.n, v2 ? 2 : 1, [&](int64_t e) { return q.w[e] * inv; },
+                     [&](int64_t e, double v) { q.vnext[e] = v; });
         if (v2 && (q.n & 1) && writer) q.vnext[q.n - 1] = q.w[q.n - 1] * inv;
         return;
     }
     unit = MODE == 2 ? (q.vec4 ? 4 : 1) : (q.vec2 ? 2 : 1);
-    own_elements(q.n, unit, [&](int64_t e) {
-        double x = q.w[e] - alpha * q.vj[e];
-        if (q.vjm1) x -= bprev * q.vjm1[e];
-        q.w[e] = x;
-    });
+    own_elements(q.n, unit,
+                 [&](int64_t e) {
+                     double x = q.w[e] - alpha * q.vj[e];
+                     if (q.vjm1) x -= bprev * q.vjm1[e];
+                     return x;
+                 },
+                 [&](int64_t e, double x) { q.w[e] = x; });
     if (MODE == 2) cgs32_dots_part(q.n, q.w, q.V32, q.ldv, nvec, q.vec4, p_dots);
     else cgs_dots_part(q.n, q.w, q.V, q.ldv, nvec, q.vec2, p_dots);
     cluster_barrier();
@@ -903,11 +943,11 @@ __global__ void __launch_bounds__(RT) lanczos_step_kernel(LanczosStep q) {
     }
     if (stop) return;
     const double inv = bs[1];
-    own_elements(q.n, unit, [&](int64_t e) {
-        const double v = q.w[e] * inv;
-        q.vnext[e] = v;
-        if (MODE == 2) q.vnext32[e] = ct_d2f(v);
-    });
+    own_elements(q.n, unit, [&](int64_t e) { return q.w[e] * inv; },
+                 [&](int64_t e, double v) {
+                     q.vnext[e] = v;
+                     if (MODE == 2) q.vnext32[e] = ct_d2f(v);
+                 });
 }
 
 __global__ void f64_to_f32_copy_kernel(int64_t n, const double* x, float* y, const int* skip) {
