@@ -1643,6 +1643,7 @@ int make_map(ct_handle* h, CUtensorMap* m, const float* base, int64_t rows, int6
 // with a 2-stage ring (80 / 96 KB stages; 192 in the chunked kernel only).  The wide tile reads
 // 25% fewer operand bytes from shared memory and L2 per MMA flop; the narrow one leaves smaller
 // partial waves.  CTDMRG_TC_BN=128, 192 or 256 forces one; otherwise tc_pick_bn chooses per shape.
+constexpr int GEMM_STAGES_64 = 4;
 constexpr int GEMM_STAGES_N = 3;
 constexpr int GEMM_STAGES_W = 2;
 
@@ -1832,8 +1833,8 @@ int tc_gemm_run(ct_handle* h, const SplitOperand& A, const SplitOperand& B, int6
     }
     const int64_t tiles = ct_cdiv(N, BN) * ct_cdiv(M, TC_BM);
     const int kc = tc_kchunk();
-    if ((BN == 192 || BN == 224) && !(tc_use_persistent() && kc > 0 && !tc_use_stream_k())) {
-        ct_seterr(h, "128 x 192 and 128 x 224 tiles exist only in the chunked kernel");
+    if ((BN == 64 || BN == 192 || BN == 224) && !(tc_use_persistent() && kc > 0 && !tc_use_stream_k())) {
+        ct_seterr(h, "128 x 64, 128 x 192 and 128 x 224 tiles exist only in the chunked kernel");
         return CT_ERR_UNSUPPORTED;
     }
     if (tc_use_persistent() && kc > 0 && !tc_use_stream_k()) {
@@ -1969,7 +1970,14 @@ int tc_gemm_launch(ct_handle* h, const SplitOperand& A, const SplitOperand& B, i
         Mr = N;
         Nr = M;
     }
-    const int rc = bn == 256 ? tc_gemm_run<256, GEMM_STAGES_W>(h, *opA, *opB, Mr, Nr, e, skip)
+    // 128-wide tiles that leave half of the SMs idle: as many 64-wide ones (each element's chunks and
+    // their order are the same).  Measured (us, 128 / 64 wide): 256x64x320 10.0 / 9.7,
+    // 320x256x64 6.6 / 5.0, 640x160x800 22.6 / 20.4, 512x1024x1024 26.8 / 24.2, 3376x163x1152
+    // 36.1 / 30.3.
+    const bool narrow = bn == 128 && ch.chunked && !tc_bn_mode() &&
+                        ct_cdiv(Mr, TC_BM) * ct_cdiv(Nr, 64) <= h->num_sms;
+    const int rc = narrow ? tc_gemm_run<64, GEMM_STAGES_64>(h, *opA, *opB, Mr, Nr, e, skip)
+                 : bn == 256 ? tc_gemm_run<256, GEMM_STAGES_W>(h, *opA, *opB, Mr, Nr, e, skip)
                  : bn == 224 ? tc_gemm_run<224, GEMM_STAGES_W>(h, *opA, *opB, Mr, Nr, e, skip)
                  : bn == 192 ? tc_gemm_run<192, GEMM_STAGES_W>(h, *opA, *opB, Mr, Nr, e, skip)
                              : tc_gemm_run<128, GEMM_STAGES_N>(h, *opA, *opB, Mr, Nr, e, skip);
