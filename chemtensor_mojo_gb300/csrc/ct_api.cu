@@ -49,9 +49,8 @@ int ct_reserve(ct_handle* h, size_t bytes) {
 }
 
 static int check_status(ct_handle* h) {
-    int st = 0;
-    CT_CUDA(h, cudaMemcpyAsync(&st, h->d_status, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    CT_CUDA(h, cudaStreamSynchronize(h->stream));
+    CT_TRY(ct_readback(h));
+    const int st = ct_host(h, h->d_status);
     if (st != 0) {
         CT_CUDA(h, cudaMemsetAsync(h->d_status, 0, sizeof(int), h->stream));
         if (h->err.empty()) ct_seterr(h, "device status %d", st);
@@ -138,13 +137,15 @@ int ct_create(int device, void* stream, ct_handle** out) {
         }
         h->own_stream = true;
     }
-    bool ok = cudaMalloc((void**)&h->d_status, sizeof(int)) == cudaSuccess &&
-              cudaMalloc((void**)&h->d_scalars, CT_NSCALARS * sizeof(double)) == cudaSuccess &&
+    bool ok = cudaMalloc((void**)&h->d_small, CT_SMALL_BYTES) == cudaSuccess &&
               cudaMalloc((void**)&h->d_partials, CT_NPARTIALS * sizeof(double)) == cudaSuccess &&
-              cudaMalloc((void**)&h->d_flags, CT_NFLAGS * sizeof(int)) == cudaSuccess;
-    if (ok) ok = cudaMemset(h->d_status, 0, sizeof(int)) == cudaSuccess &&
-                 cudaMemset(h->d_flags, 0, CT_NFLAGS * sizeof(int)) == cudaSuccess &&
-                 cudaMemset(h->d_scalars, 0, CT_NSCALARS * sizeof(double)) == cudaSuccess;
+              cudaMallocHost((void**)&h->pin, 2 * CT_SMALL_BYTES) == cudaSuccess;
+    if (ok) {
+        h->d_status = (int*)(h->d_small + CT_SMALL_STATUS);
+        h->d_scalars = (double*)(h->d_small + CT_SMALL_SCALARS);
+        h->d_flags = (int*)(h->d_small + CT_SMALL_FLAGS);
+        ok = cudaMemset(h->d_small, 0, CT_SMALL_BYTES) == cudaSuccess;
+    }
     if (!ok) {
         ct_destroy(h);
         return CT_ERR_OOM;
@@ -168,10 +169,9 @@ int ct_destroy(ct_handle* h) {
     cudaFree(h->tc_sk_flag);
     cudaFree(h->tc_hy_part);
     cudaFree(h->tc_hy_cnt);
-    cudaFree(h->d_status);
-    cudaFree(h->d_scalars);
+    cudaFree(h->d_small);
     cudaFree(h->d_partials);
-    cudaFree(h->d_flags);
+    if (h->pin) cudaFreeHost(h->pin);
     if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
     delete h;
     return CT_OK;
@@ -518,17 +518,12 @@ int ct_lanczos2(ct_handle* h, int prec, const double* theta_in, double* theta_ou
     LanczosResult res;
     CT_TRY(ct_lanczos_run(h, ar, prec, theta_in, theta_out, L, R, W1, W2, Dl, d, Dr, wL, wM, wR, max_iter, tol,
                           max_rotations, reorth, &res));
-    int nk = 0;
-    CT_CUDA(h, cudaMemcpyAsync(energy_host, res.d_energy, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    CT_CUDA(h, cudaMemcpyAsync(&nk, res.d_numiter, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    if (alpha_host)
-        CT_CUDA(h, cudaMemcpyAsync(alpha_host, h->d_scalars + SC_ALPHA, max_iter * sizeof(double),
-                                   cudaMemcpyDeviceToHost, h->stream));
-    if (beta_host && max_iter > 1)
-        CT_CUDA(h, cudaMemcpyAsync(beta_host, h->d_scalars + SC_BETA, (max_iter - 1) * sizeof(double),
-                                   cudaMemcpyDeviceToHost, h->stream));
-    CT_TRY(check_status(h));
-    if (numiter_host) *numiter_host = nk;
+    const int rc = check_status(h);   // (reads back)
+    *energy_host = ct_host(h, res.d_energy);
+    for (int i = 0; alpha_host && i < max_iter; ++i) alpha_host[i] = ct_host(h, h->d_scalars + SC_ALPHA + i);
+    for (int i = 0; beta_host && i < max_iter - 1; ++i) beta_host[i] = ct_host(h, h->d_scalars + SC_BETA + i);
+    if (rc != CT_OK) return rc;
+    if (numiter_host) *numiter_host = ct_host(h, res.d_numiter);
     return CT_OK;
 }
 
@@ -598,13 +593,13 @@ int ct_svd_split(ct_handle* h, int prec, const double* theta, int64_t Dl, int64_
     // |theta|^2 in FP64 on the device (dmrg.mojo:176)
     CT_TRY(ct_reduce_nrm2sq(h, m * n, theta, h->d_scalars + SC_THETA_NSQ, nullptr));
     CT_TRY(ct_check_finite(h, h->d_scalars + SC_THETA_NSQ, nullptr));
-    double tn = 0.0;
-    CT_CUDA(h, cudaMemcpyAsync(&tn, h->d_scalars + SC_THETA_NSQ, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
+    CT_TRY(ct_readback_later(h));
     SvdOut o;
     CT_TRY(ct_split_run(h, ar, prec, theta, m, n, chi_max, eps_trunc, mode, A_out, B_out, S_out,
                         h->d_scalars + SC_THETA_NSQ, &o));
     CT_TRY(check_status(h));
     *chi_host = o.chi;
+    const double tn = ct_host(h, h->d_scalars + SC_THETA_NSQ, 1);
     if (discarded_host) *discarded_host = (tn > 0.0) ? (tn - o.sum_s2_kept) / tn : 0.0;
     return CT_OK;
 }

@@ -53,6 +53,9 @@ struct ct_handle {
     size_t oz_ws_bytes = 0;
     void* fm_ws = nullptr;   // residues of the FP64-form tensor-core GEMM (ct_f64mod.cu)
     size_t fm_ws_bytes = 0;
+    // status word, scalars and flags in one allocation, and two pinned copies of it (ct_readback)
+    uint8_t* d_small = nullptr;
+    uint8_t* pin = nullptr;
     bool fm_captured = false;        // fm_ws is in a captured graph
     std::vector<void*> fm_kept;      // outgrown buffers of captured graphs, freed with the handle
     // allocation-free mode (the stack handle of ct_heff2_apply_noalloc): the
@@ -163,6 +166,30 @@ void ct_launch(ct_handle* h, void (*kernel)(P...), dim3 grid, dim3 block, size_t
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);   // (CT_LAUNCH_CHECK reads the error)
+}
+
+// What the host reads after a solve or a split (status, scalars, flags) comes over in one copy to
+// pinned memory and one synchronisation: a copy to pageable memory each cost about 9 us, five of
+// them the end of a Lanczos run.  ct_readback waits; ct_readback_later's values (slot 1) are there
+// after the next synchronisation of the stream.
+constexpr size_t CT_SMALL_STATUS = 0, CT_SMALL_SCALARS = 256, CT_SMALL_FLAGS = CT_SMALL_SCALARS + CT_NSCALARS * sizeof(double),
+                 CT_SMALL_BYTES = CT_SMALL_FLAGS + CT_NFLAGS * sizeof(int);
+static inline int ct_readback_later(ct_handle* h, int slot = 1) {
+    CT_CUDA(h, cudaMemcpyAsync(h->pin + slot * CT_SMALL_BYTES, h->d_small, CT_SMALL_BYTES, cudaMemcpyDeviceToHost, h->stream));
+    return CT_OK;
+}
+static inline int ct_readback(ct_handle* h) {
+    const int rc = ct_readback_later(h, 0);
+    if (rc != CT_OK) return rc;
+    CT_CUDA(h, cudaStreamSynchronize(h->stream));
+    return CT_OK;
+}
+// the copy of a word of that allocation
+template <typename T>
+static inline T ct_host(const ct_handle* h, const T* device, int slot = 0) {
+    T v;
+    memcpy(&v, h->pin + slot * CT_SMALL_BYTES + ((const uint8_t*)device - h->d_small), sizeof(T));
+    return v;
 }
 
 static inline int64_t ct_cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }

@@ -209,15 +209,7 @@ int ct_dmrg_two_site(ct_handle* h, const ct_dmrg_params* P, int N, int d, const 
         // split (dmrg.mojo:143-252): |theta|^2 then SVD
         CT_TRY(ct_reduce_nrm2sq(h, m * n, th_opt.p, h->d_scalars + SC_THETA_NSQ, nullptr));
         CT_TRY(ct_check_finite(h, h->d_scalars + SC_THETA_NSQ, nullptr));
-        struct {
-            double e;
-            double tn;
-            int nk;
-        } hb{};
-        CT_CUDA(h, cudaMemcpyAsync(&hb.e, h->d_scalars + SC_ENERGY, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-        CT_CUDA(h, cudaMemcpyAsync(&hb.tn, h->d_scalars + SC_THETA_NSQ, sizeof(double), cudaMemcpyDeviceToHost,
-                                   h->stream));
-        CT_CUDA(h, cudaMemcpyAsync(&hb.nk, h->d_flags + FL_NUMITER, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
+        CT_TRY(ct_readback_later(h));   // energy, |theta|^2 and the Lanczos steps, read after the bond's end
         const int64_t chi_bound = std::min<int64_t>(std::min(m, n), P->chi_max);
         if (Dl * d * chi_bound > site_capacity[i] || chi_bound * d * Dr > site_capacity[i + 1] ||
             chi_bound > cap[i + 1]) {
@@ -403,9 +395,14 @@ int ct_dmrg_two_site(ct_handle* h, const ct_dmrg_params* P, int N, int d, const 
             }
         }
         CT_CUDA(h, cudaEventRecord(ev_e.b, h->stream));
-        CT_CUDA(h, cudaStreamSynchronize(h->stream));
-        int dst = 0;
-        CT_CUDA(h, cudaMemcpy(&dst, h->d_status, sizeof(int), cudaMemcpyDeviceToHost));
+        CT_TRY(ct_readback(h));
+        const int dst = ct_host(h, h->d_status);
+        const struct {
+            double e;
+            double tn;
+            int nk;
+        } hb{ct_host(h, h->d_scalars + SC_ENERGY, 1), ct_host(h, h->d_scalars + SC_THETA_NSQ, 1),
+             ct_host(h, h->d_flags + FL_NUMITER, 1)};
         if (dst != 0) {
             cudaMemset(h->d_status, 0, sizeof(int));
             ct_seterr(h, "bond %d: device status %d", i, dst);

@@ -347,9 +347,8 @@ int run(ct_handle* h, T* X, int64_t len, T* Q, int64_t nvec, double tol, double 
     CT_CUDA(h, cudaLaunchCooperativeKernel((const void*)jacobi_coop_kernel<T>, dim3((unsigned)grid), dim3(NT), args,
                                            0, h->stream));
     ct_note_launch();
-    int sw = 0;
-    CT_CUDA(h, cudaMemcpyAsync(&sw, s.sweeps, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    CT_CUDA(h, cudaStreamSynchronize(h->stream));
+    CT_TRY(ct_readback(h));
+    const int sw = ct_host(h, s.sweeps);
     h->last_svd_sweeps = sw;
     h->total_svd_sweeps += sw;
     if (sweeps_host) *sweeps_host = sw;

@@ -483,23 +483,16 @@ static int svd_run_geometry(ct_handle* h, Arena& ar, const double* M, int64_t m,
     ct_launch(h, svd_rank_kernel, (unsigned)ct_cdiv(nv * 32, 256), 256, 0, sig, nv, perm); ct_note_launch();
     ct_launch(h, svd_trunc_kernel, 1, 32, 0, sig, perm, k, chi_max, eps_trunc, h->d_scalars, h->d_flags); ct_note_launch();
     CT_LAUNCH_CHECK(h);
-    int chi = 0;
-    double sums[2];
-    CT_CUDA(h, cudaMemcpyAsync(&chi, h->d_flags + FL_CHI, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    CT_CUDA(h, cudaMemcpyAsync(sums, h->d_scalars + SC_TMP0, 2 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    CT_CUDA(h, cudaMemcpyAsync(min_kept, h->d_scalars + SC_SVD_MINKEPT, sizeof(double), cudaMemcpyDeviceToHost,
-                               h->stream));
-    int small_sweeps = 0;
-    if (small_run)
-        CT_CUDA(h, cudaMemcpyAsync(&small_sweeps, h->d_flags + 19, sizeof(int), cudaMemcpyDeviceToHost,
-                                   h->stream));
-    CT_CUDA(h, cudaStreamSynchronize(h->stream));
+    CT_TRY(ct_readback(h));
+    const int chi = ct_host(h, h->d_flags + FL_CHI);
+    const double sums[2] = {ct_host(h, h->d_scalars + SC_TMP0), ct_host(h, h->d_scalars + SC_TMP0 + 1)};
+    *min_kept = ct_host(h, h->d_scalars + SC_SVD_MINKEPT);
     if (small_run) {
+        const int small_sweeps = ct_host(h, h->d_flags + 19);
         h->last_svd_sweeps = small_sweeps;
         h->total_svd_sweeps += small_sweeps;
     }
-    int st = 0;
-    CT_CUDA(h, cudaMemcpy(&st, h->d_status, sizeof(int), cudaMemcpyDeviceToHost));
+    const int st = ct_host(h, h->d_status);
     if (st != 0) {
         CT_CUDA(h, cudaMemset(h->d_status, 0, sizeof(int)));
         ct_seterr(h, "device SVD reported status %d", st);

@@ -301,11 +301,9 @@ int ct_svd_mixed_run(ct_handle* h, Arena& ar, const double* M, int64_t m, int64_
     ct_launch(h, rank_desc_kernel, (unsigned)ct_cdiv(c, 256), 256, 0, sig, c, perm); ct_note_launch();
     ct_launch(h, trunc_kernel, 1, 32, 0, sig, perm, c, k, eps_trunc, d_total, h->d_scalars, h->d_flags); ct_note_launch();
     CT_LAUNCH_CHECK(h);
-    int chi = 0;
-    double sums[2];
-    CT_CUDA(h, cudaMemcpyAsync(&chi, h->d_flags + FL_CHI, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    CT_CUDA(h, cudaMemcpyAsync(sums, h->d_scalars + SC_TMP0, 2 * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    CT_CUDA(h, cudaStreamSynchronize(h->stream));
+    CT_TRY(ct_readback(h));
+    const int chi = ct_host(h, h->d_flags + FL_CHI);
+    const double sums[2] = {ct_host(h, h->d_scalars + SC_TMP0), ct_host(h, h->d_scalars + SC_TMP0 + 1)};
     if (eps_trunc > 0.0 && sums[0] > 0.0 &&
         (chi < c || (sums[0] - sums[1]) / sums[0] <= 2.0 * eps_trunc + 1e-9)) {
         ar.off = entry;

@@ -464,9 +464,8 @@ int orth_correct(ct_handle* h, Arena& ar, const double* Q, double* out, int64_t 
         ct_launch(h, orth_correction_kernel, grid_n(h, c * c), 256, 0, ob.G, ob.cp, c, ob.Linv, d_emax);
         ct_note_launch();
         CT_LAUNCH_CHECK(h);
-        unsigned long long bits = 0;
-        CT_CUDA(h, cudaMemcpyAsync(&bits, d_emax, sizeof(bits), cudaMemcpyDeviceToHost, h->stream));
-        CT_CUDA(h, cudaStreamSynchronize(h->stream));
+        CT_TRY(ct_readback(h));
+        const unsigned long long bits = ct_host(h, d_emax);
         double emax;
         memcpy(&emax, &bits, sizeof(emax));
         if (step == 0) {
@@ -527,8 +526,8 @@ int orth_rows(ct_handle* h, Arena& ar, double* Z, double* W, int64_t c, int64_t 
         CT_TRY(chol_inv(h, ob.G, ob.Linv, cp, cp, ob.S, d_minpiv + pass, d_fail, mk, 0));
         CT_TRY(fac_gemm(h, c, len, c, ob.Linv, cp, src, len, 0, dst, len, 1.0, 0.0, 2));
         if (pass == 0 && complete) {
-            CT_CUDA(h, cudaMemcpyAsync(&nrep, d_count, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-            CT_CUDA(h, cudaStreamSynchronize(h->stream));
+            CT_TRY(ct_readback(h));
+            nrep = ct_host(h, d_count);
             if (nrep > 0) {
                 const unsigned g = (unsigned)std::min<int64_t>(nrep, (int64_t)h->num_sms * 4);
                 ct_launch(h, replace_rows_kernel, g, 256, 0, dst, len, ob.defrows, d_count, (int)cp, seed);
@@ -642,14 +641,10 @@ int split_attempt(ct_handle* h, Arena& ar, const SplitBufs& sb, const double* M,
     CT_TRY(ct_tc_gemm(h, ar, 0, 0, m, n, c, -1.0, Aout, c, Bout, n, 1.0, sb.R, n));
     ar.off = mark;
     CT_TRY(ct_reduce_nrm2sq(h, m * n, sb.R, h->d_scalars + SC_TMP1, nullptr));
-    double host[2];
-    unsigned long long piv[2];
-    int fail = 0;
-    CT_CUDA(h, cudaMemcpyAsync(host, d_total, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    CT_CUDA(h, cudaMemcpyAsync(host + 1, h->d_scalars + SC_TMP1, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
-    CT_CUDA(h, cudaMemcpyAsync(piv, d_piv, sizeof(piv), cudaMemcpyDeviceToHost, h->stream));
-    CT_CUDA(h, cudaMemcpyAsync(&fail, d_fail, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    CT_CUDA(h, cudaStreamSynchronize(h->stream));
+    CT_TRY(ct_readback(h));
+    const double host[2] = {ct_host(h, d_total), ct_host(h, h->d_scalars + SC_TMP1)};
+    const unsigned long long piv[2] = {ct_host(h, d_piv), ct_host(h, d_piv + 1)};
+    const int fail = ct_host(h, d_fail);
     double piv1, piv2;
     memcpy(&piv1, &piv[0], 8);
     memcpy(&piv2, &piv[1], 8);
@@ -767,9 +762,8 @@ int ct_qr_run(ct_handle* h, Arena& ar, const double* A, int64_t m, int64_t n, do
     CT_LAUNCH_CHECK(h);
     ct_launch(h, zero_strict_lower_kernel, grid_n(h, k * n), 256, 0, R, k, n); ct_note_launch();
     CT_LAUNCH_CHECK(h);
-    int fail = 0;
-    CT_CUDA(h, cudaMemcpyAsync(&fail, d_fail, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
-    CT_CUDA(h, cudaStreamSynchronize(h->stream));
+    CT_TRY(ct_readback(h));
+    const int fail = ct_host(h, d_fail);
     if (completed) *completed = nrep;
     if (fail) {
         ct_seterr(h, "ct_qr: the Cholesky factorisation met a non-finite pivot");
