@@ -114,6 +114,25 @@ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
     e = __fadd_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fsub_rn(b, bb));
 }
 
+// The epilogue's FP64 operations issue at one per 64 clocks and SM quarter, and a CTA has one
+// tile's columns to finish after its last MMA: conversions, scalings and products by 1 as FP64
+// instructions took 17 us of a launch (30.6 us at K = 64, 19.7 with the integer forms below).
+// (double)x of a sum of slice products (normal, zero, infinite or NaN: the slices' products
+// are multiples of 2^-63).
+__device__ __forceinline__ double oz_f2d(float x) {
+    const unsigned u = __float_as_uint(x), a = u & 0x7fffffffu;
+    unsigned w = (a >> 3) + (896u << 20);
+    if (a >= 0x7f800000u) w |= 0x7ff00000u;
+    if (a == 0) w = 0;
+    return __hiloint2double((int)(w | (u & 0x80000000u)), (int)(u << 29));
+}
+// x 2^e
+__device__ __forceinline__ double oz_scale(double x, int e) {
+    const int hi = __double2hiint(x), f = (hi >> 20) & 0x7ff;
+    if ((unsigned)(f - 1) < 2046u && (unsigned)(f + e - 1) < 2046u) return __hiloint2double(hi + (e << 20), __double2loint(x));
+    return scalbn(x, e);
+}
+
 struct OzEpi {
     double* C;       // row m at (m / M0) * s1 + (m % M0) * s0, columns contiguous
     int64_t M0, s1, s0;
@@ -306,8 +325,9 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                     }
 #pragma unroll
                     for (int j = 0; j < OZ_HH; ++j) {
-                        acc[half * OZ_HH + j] += (double)hi[j];
-                        acc[half * OZ_HH + j] += (double)lo[j];
+                        const double h = oz_f2d(hi[j]);
+                        acc[half * OZ_HH + j] = kb0 == 0 ? h : acc[half * OZ_HH + j] + h;
+                        acc[half * OZ_HH + j] += oz_f2d(lo[j]);
                     }
                 }
             }
@@ -317,12 +337,15 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
             const int64_t m = (int64_t)m0 + row;
             if (m >= M) continue;
             const int em = epi.ea[m];
+            const bool one = epi.alpha == 1.0, minus = epi.alpha == -1.0;
             double* Cr = epi.C + (m / epi.M0) * epi.s1 + (m % epi.M0) * epi.s0;
 #pragma unroll
             for (int j = 0; j < OZ_HC; ++j) {
                 const int64_t n = (int64_t)n0 + j;
                 if (n >= N) break;
-                double r = epi.alpha * scalbn(acc[j], em + epi.eb[n]);
+                double r = oz_scale(acc[j], em + epi.eb[n]);
+                if (minus) r = -r;
+                else if (!one) r *= epi.alpha;
                 if (epi.beta != 0.0) r = fma(epi.beta, Cr[n], r);
                 Cr[n] = r;
             }
