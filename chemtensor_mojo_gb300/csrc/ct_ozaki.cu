@@ -35,7 +35,8 @@
 // Kernel: one CTA per SM walks 128 x 64 tiles (consecutive CTAs share the A
 // rows, which stay in L2); warp 0 issues TMA loads (64-byte swizzle, 32 BF16
 // of K per row, all 8 slices of A and of B per stage, 2 stages), one thread of
-// warp 1 issues the 72 MMAs (M128 N64 K16) of a K-block, and 8 epilogue warps
+// warp 1 issues the 54 MMAs of a K-block (M128 K16; 12 of up to N256 for the exact levels,
+// 42 of N64 for the others), and 8 epilogue warps
 // (two per TMEM lane quadrant, 32 columns each) read the six accumulators of a
 // 512-wide chunk (384 TMEM columns, one buffer: the MMAs of the next chunk wait
 // only for the reads, ~1 us against ~20 us of MMAs) and add them in FP64.
