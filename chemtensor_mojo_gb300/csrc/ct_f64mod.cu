@@ -166,19 +166,11 @@ constexpr int FM_PK = 64;    // columns per block of the residue kernel
 constexpr int FM_XK = 256;   // columns per block of the exponent kernel
 constexpr int FM_ZERO = -0x40000000;
 
-// Exponents of both operands' rows over FM_XK columns (part: 2^e > max |x[r][k]| >= 2^(e - 1),
-// FM_ZERO without a non-zero, FM_NONFINITE).  Blocks (x, y): 8 rows, x in [0, nba) operand A's,
-// columns [y FM_XK, +FM_XK); every thread has its 8 loads in flight at once (with whole rows per
-// block, the memory latency five times over and too few blocks: 12.5 us instead of 4 for the
-// H_eff products of chi 256).  sk == 1: a warp per row; else threads along the rows, which are
-// contiguous then.
-__global__ void __launch_bounds__(256) fm_rowexp_kernel(FmSrc a, FmSrc b, int nba, const int* skip) {
-    ct_pdl();
-    if (ct_skip(skip)) return;
-    __shared__ unsigned long long part[8][FM_PR];
-    const bool first = (int)blockIdx.x < nba;
-    const FmSrc& x = first ? a : b;
-    const int64_t r0 = (int64_t)(first ? blockIdx.x : blockIdx.x - nba) * FM_PR, k0 = (int64_t)blockIdx.y * FM_XK;
+// Exponents of 8 rows from r0 on over the FM_XK columns from k0 on (2^e > max |x| >= 2^(e - 1),
+// FM_ZERO without a non-zero, FM_NONFINITE): true in one thread per row r0 + *row, with *e.
+// sk == 1: a warp per row; else threads along the rows, which are contiguous then.
+__device__ __forceinline__ bool fm_piece_exponent(const FmSrc& x, int64_t r0, int64_t k0,
+                                                  unsigned long long (&part)[8][FM_PR], int* row, int* e) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     // largest magnitude of each row, as bit patterns (their integer order is the order; a NaN
     // or infinity exceeds every finite value)
@@ -205,16 +197,32 @@ __global__ void __launch_bounds__(256) fm_rowexp_kernel(FmSrc a, FmSrc b, int nb
     if (!along) {
         if (lane < FM_PR) part[warp][lane] = m;
         __syncthreads();
-        if (tid >= FM_PR) return;
+        if (tid >= FM_PR) return false;
 #pragma unroll
         for (int i = 0; i < 8; ++i) m = part[i][tid] > m ? part[i][tid] : m;
     } else if (lane != 0) {
-        return;
+        return false;
     }
-    if (r >= x.R) return;
+    if (r >= x.R) return false;
     const int field = (int)(m >> 52);
-    const int e = field == 0x7ff ? FM_NONFINITE : field ? field - 1022 : m ? -1010 - __clzll((long long)m) : FM_ZERO;
-    x.part[(int64_t)blockIdx.y * x.R + r] = e;
+    *e = field == 0x7ff ? FM_NONFINITE : field ? field - 1022 : m ? -1010 - __clzll((long long)m) : FM_ZERO;
+    *row = (int)(r - r0);
+    return true;
+}
+
+// Exponents of both operands' rows by pieces of FM_XK columns (part), for K beyond one piece.
+// Blocks (x, y): 8 rows, x in [0, nba) operand A's, columns [y FM_XK, +FM_XK); every thread has
+// its 8 loads in flight at once (with whole rows per block, the memory latency five times over
+// and too few blocks: 12.5 us instead of 4 for the H_eff products of chi 256).
+__global__ void __launch_bounds__(256) fm_rowexp_kernel(FmSrc a, FmSrc b, int nba, const int* skip) {
+    ct_pdl();
+    if (ct_skip(skip)) return;
+    __shared__ unsigned long long part[8][FM_PR];
+    const bool first = (int)blockIdx.x < nba;
+    const FmSrc& x = first ? a : b;
+    const int64_t r0 = (int64_t)(first ? blockIdx.x : blockIdx.x - nba) * FM_PR, k0 = (int64_t)blockIdx.y * FM_XK;
+    int row, e;
+    if (fm_piece_exponent(x, r0, k0, part, &row, &e)) x.part[(int64_t)blockIdx.y * x.R + r0 + row] = e;
 }
 
 
@@ -264,10 +272,22 @@ __global__ void __launch_bounds__(256) fm_residue_kernel(FmSrc a, FmSrc b, int n
         v0 = tile[2 * lane][warp];
         v1 = tile[2 * lane + 1][warp];
     }
+    __shared__ unsigned long long part[8][FM_PR];
+    __shared__ int es[FM_PR];
+    const bool own = x.K <= FM_XK;   // one piece: found here, 8 more loads per thread and a launch less
+    if (own) {
+        int row, pe;
+        if (fm_piece_exponent(x, r0, 0, part, &row, &pe)) es[row] = pe;
+        __syncthreads();
+    }
     if (r0 + warp >= x.R) return;
-    int e = FM_ZERO;   // the row's exponent from its pieces'
-    for (int64_t c = lane; c * FM_XK < x.K; c += 32) e = max(e, x.part[c * x.R + r0 + warp]);
-    e = __reduce_max_sync(0xffffffffu, e);
+    int e = FM_ZERO;   // the row's exponent, or the largest of its pieces'
+    if (own) {
+        e = es[warp];
+    } else {
+        for (int64_t c = lane; c * FM_XK < x.K; c += 32) e = max(e, x.part[c * x.R + r0 + warp]);
+        e = __reduce_max_sync(0xffffffffu, e);
+    }
     if (e == FM_ZERO) e = 0;
     if (blockIdx.y == 0 && lane == 0) x.ex[r0 + warp] = e;
     const unsigned long long u0 = fm_fixed(v0, e, bits), u1 = fm_fixed(v1, e, bits);
@@ -726,7 +746,9 @@ int ct_f64_gemm(ct_handle* h, int64_t M, int64_t N, int64_t K, const OzMat& A, c
     const int nba = (int)ct_cdiv(M, FM_PR);
     const dim3 grid((unsigned)(nba + ct_cdiv(N, FM_PR)), (unsigned)ct_cdiv(q.ldk, FM_PK));
     if (grid.y > 65535) return CT_ERR_UNSUPPORTED;
-    ct_launch(h, fm_rowexp_kernel, dim3(grid.x, (unsigned)ct_cdiv(K, FM_XK)), 256, 0, a, b, nba, skip); ct_note_launch();
+    if (K > FM_XK) {
+        ct_launch(h, fm_rowexp_kernel, dim3(grid.x, (unsigned)ct_cdiv(K, FM_XK)), 256, 0, a, b, nba, skip); ct_note_launch();
+    }
     ct_launch(h, fm_residue_kernel, grid, 256, 0, a, b, nba, bits, t.mod, skip); ct_note_launch();
     const int64_t items = q.tiles * MODS;
     const int64_t ctas = items < h->num_sms ? items : h->num_sms;
