@@ -141,6 +141,11 @@ __global__ void __launch_bounds__(SP_NT) gemm_f64_spread_kernel(GemmDesc g, int 
     const int64_t m0 = (int64_t)blockIdx.y * SP_M, n0 = (int64_t)blockIdx.x * SP_N;
     const int64_t mt = m0 / TRI * TRI;
     if (g.tri == 1 && n0 / TRI * TRI >= mt + TRI) return;   // the whole cluster
+    // the first CTA's shared memory may be written once it has started: everyone arrives here, and
+    // waits before its store (the K loop covers the latency; a piece without any K comes there at once)
+    namespace cg = cooperative_groups;
+    cg::cluster_group cl = cg::this_cluster();
+    if (clustered) (void)cl.barrier_arrive();
     int64_t kend = (g.tri == 2 && mt + TRI < g.K) ? mt + TRI : g.K;
     int64_t kbeg = 0;
     if (g.ksplit > 1) {
@@ -202,8 +207,7 @@ __global__ void __launch_bounds__(SP_NT) gemm_f64_spread_kernel(GemmDesc g, int 
     const int64_t gm = m0 + ty, gn = n0 + tx;
     if (g.ksplit > 1) {
         if (clustered) {
-            namespace cg = cooperative_groups;
-            cg::cluster_group cl = cg::this_cluster();
+            cl.barrier_wait();
             *cl.map_shared_rank(&piece[ks][tid], 0) = acc;
             cl.sync();
             if (ks != 0) return;
