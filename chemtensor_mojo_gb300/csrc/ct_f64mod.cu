@@ -1,32 +1,50 @@
-// FP64-form GEMM on the BF16 tensor cores by residues (no rounding but the operands').
+// FP64-form GEMM on the BF16 tensor cores by residues, with FP64 accuracy of every element.
 //
 // C[M,N] = sum_k A[m,k] B[n,k] with FP64 A, B and C, for the contraction chains of the FP64
 // form.  The scheme is that of K. Ozaki, Y. Uchino and T. Imamura, Ozaki Scheme II: a
 // GEMM-oriented emulation of floating-point matrix multiplication using an integer modular
-// technique (arXiv:2504.08009, 2025), here on tcgen05 kind::f16 with BF16 operands:
-//   * every row of A and of B is scaled by a power of two and rounded to integers of b bits,
-//     |X| <= 2^b (b = 62, less only beyond K = 2^15: the moduli hold 2 K 2^(2b) < P);
+// technique (arXiv:2504.08009, 2025), here on tcgen05 kind::f16, with a correction for the
+// operands' rounding and a test of each element:
+//   * every row of A and of B is scaled by a power of two, to a' and b' below 1, and rounded to
+//     integers of b bits (b = 58 at K = 256, less for larger K: the moduli hold 2 K 2^(2b) < P);
 //   * for each of MODS pairwise coprime moduli m_i <= 256 the residues of A and B (at most
 //     128 in magnitude, exact in BF16) are multiplied: a product is at most 2^14, so 1024 of K
 //     add up exactly in the FP32 accumulator, which the epilogue reduces modulo m_i;
 //   * the Chinese remainder theorem gives the integer product sum, below P / 2 = prod m_i / 2
-//     in magnitude, exactly; it is rounded to FP64 once and scaled back.
-// The only error is the operands' rounding, 2^-(b + 1) of each row's largest entry, and the
-// final one.  Relative error against exact products, N(0,1) operands, 1024^3: 4.7e-17 (half an
-// ulp), the SIMT kernel's 1.1e-15.  (16 moduli, b = 57, are 12% cheaper, but rows and columns
-// graded in opposite directions, exp(-8 k / K) against exp(8 k / K), then lose to the SIMT
-// kernel: 2.6e-15 against 3e-16 at 256^3.)
+//     in magnitude, exactly;
+//   * what the rounding took from a' and b', da and db (at most half a unit), comes back as a
+//     pair of FP16 products, sum_k a' db and sum_k da b', to 2^-11 of each term;
+//   * both are added as integers and rounded to FP64 once.
 //
-// What bounds it.  MODS products of full-size tensor-core tiles per FP64 product (the sliced
+// Accuracy.  The integers are relative to a row's largest entry, so what is left of the error,
+// 2^-(b + 12) T with T = sum_k |a'| [db != 0] + [da != 0] |b'|, may exceed what FP64 FMAs leave of an
+// element whose S = sum_k |a'| |b'| is small (one operand falls along k and the other rises; rows of
+// an identity).  So each element is tested for 2^-(b + 12) T <= 16 2^-53 S: one more BF16 product, of
+// x = |a'| - theta [da != 0] and y = |b'| - theta [db != 0] with theta = 2^(37 - b), is S - theta T +
+// theta^2 n, n <= K the number of k where neither is exact, and has to be theta^2 K at least.  It is
+// exactly zero where no k has both, as between the blocks of a block-sparse operand (x and y of a
+// non-zero entry are kept from zero): such an element passes if its product is zero too.  The
+// others are computed as FP64 dot products, by a warp each; when they are more than an eighth of
+// all, the whole product by FP64 FMAs in the order of k, as without this route.
+// Every element is thus within 16.5 2^-53 S and the final rounding (worst case; FP64 FMAs: K 2^-53 S).
+// Measured, 256^3, N(0,1) operands with A falling and B rising along k by a factor f, largest error
+// in units of 2^-53 S (here, with the final rounding / FP64 FMAs): f = 1 below 0.001 / 4.0, 1e2 0.22 /
+// 4.3, 1e4 0.41 / 4.0, 1e5 0.45 / 3.6, 1e6 1.1 / 4.4, beyond that it is the FMA path.  (18 moduli
+// alone, b = 62, without correction and test: 2e-14 of an element at f = 1e6, 1.5e-8 at 1e12.)
+// When the FMA path is taken the products here are lost: 256^3 54 us (40 without this route), 512^3
+// 264 (231), 1024^3 1827 (1743); thin and deep, where that one would split K, 128 x 128 x 2048 224 (64).
+//
+// What bounds it.  MODS + 3 products of full-size tensor-core tiles per FP64 product (the sliced
 // scheme of ct_ozaki.cu forms 36 to 45, on 64-wide tiles that its eight accumulators leave);
 // for small products the four launches.  FP64 arithmetic issues at 1/64 of the FP32 rate
 // here, so the residues, the reduction and the reconstruction are integer and FP32 work.
 //
-// A row with an infinity or a NaN has no scale: its elements of C are computed as plain FP64
+// A row with an infinity or a NaN has no scale: its elements of C are computed as FP64
 // dot products from the operands, so non-finite values go where an FP64 GEMM takes them.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 #include <math.h>
 
 #include <algorithm>
@@ -38,8 +56,10 @@ PFN_cuTensorMapEncodeTiled_v12000 ct_tma_encoder();
 
 namespace {
 
-constexpr int MODS = 18;
-constexpr int GROUPS = MODS / 3;                        // reconstructed three moduli at a time
+constexpr int MODS = 16;
+constexpr int GROUPS = MODS / 2;                        // reconstructed two moduli at a time
+// planes of an operand: the residues; a' and da of A beside db and b' of B; x or y of the test
+constexpr int PL_CORR = MODS, PL_TEST = MODS + 2, PLANES = MODS + 3;
 constexpr int FM_BM = 128;
 constexpr int FM_BN = 128;
 constexpr int FM_BK = 64;                               // BF16 of K per 128-byte row
@@ -53,10 +73,10 @@ constexpr int FM_A_BYTES = FM_BM * FM_BK * 2;           // 16 KB
 constexpr int FM_STAGE = FM_A_BYTES + FM_BN * FM_BK * 2;
 constexpr int FM_SMEM = FM_STAGES * FM_STAGE + 1024 /*align*/ + 256 /*barriers*/;
 constexpr int FM_NONFINITE = 0x40000000;                // exponent of a row with an infinity or a NaN
-constexpr int LIMBS = 5;                                // 32-bit limbs of P (141 bits) and of the sums
+constexpr int LIMBS = 4;                                // 32-bit limbs of P (125 bits) and of the sums
 
-// pairwise coprime, at most 256: P = 2^140.6
-constexpr int kMod[MODS] = {256, 253, 251, 249, 247, 245, 241, 239, 233, 229, 227, 223, 211, 199, 197, 193, 191, 181};
+// pairwise coprime, at most 256: P = 2^125.5
+constexpr int kMod[MODS] = {256, 253, 251, 249, 247, 245, 241, 239, 233, 229, 227, 223, 211, 199, 197, 193};
 
 // Constants of one modulus: m, 1 / m, 2^(13 i) modulo m for i = 1 .. 4 and the inverse of P / m
 // modulo m (symmetric residues: at most m / 2 in magnitude).
@@ -66,11 +86,11 @@ struct ModConst {
 struct ModTable {
     ModConst c[MODS];
 };
-// Reconstruction constants.  Group g holds the moduli 3g .. 3g + 2, G = their product: co[j] = G /
+// Reconstruction constants.  Group g holds the moduli 2g and 2g + 1, G = their product: co[j] = G /
 // m_j, w = P / G, rcp = round(2^40 / G); bias = 128 sum_i P / m_i, subtracted because the stored
 // t_i are offset by 128.
 struct CrtTable {
-    unsigned co[GROUPS][3];
+    unsigned co[GROUPS][2];
     unsigned w[GROUPS][LIMBS];
     unsigned rcp[GROUPS];
     unsigned P[LIMBS];
@@ -112,20 +132,20 @@ Tables make_tables() {
     q.P[0] = 1;
     for (int m : kMod) mul(q.P, (unsigned)m);
     for (int g = 0; g < GROUPS; ++g) {
-        const unsigned G = (unsigned)kMod[3 * g] * (unsigned)kMod[3 * g + 1] * (unsigned)kMod[3 * g + 2];
+        const unsigned G = (unsigned)kMod[2 * g] * (unsigned)kMod[2 * g + 1];
         unsigned cosum = 0;
-        for (int j = 0; j < 3; ++j) {
-            q.co[g][j] = G / (unsigned)kMod[3 * g + j];
+        for (int j = 0; j < 2; ++j) {
+            q.co[g][j] = G / (unsigned)kMod[2 * g + j];
             cosum += q.co[g][j];
         }
         q.w[g][0] = 1;
         for (int i = 0; i < MODS; ++i)
-            if (i / 3 != g) mul(q.w[g], (unsigned)kMod[i]);
+            if (i / 2 != g) mul(q.w[g], (unsigned)kMod[i]);
         q.rcp[g] = (unsigned)(((1ull << 40) + G / 2) / G);
         q.rbias += 128ll * cosum * q.rcp[g];
         unsigned x[LIMBS];
         for (int l = 0; l < LIMBS; ++l) x[l] = q.w[g][l];
-        mul(x, 128u * cosum);   // < 2^27
+        mul(x, 128u * cosum);
         unsigned long long carry = 0;
         for (int l = 0; l < LIMBS; ++l) {
             carry += (unsigned long long)q.bias[l] + x[l];
@@ -145,11 +165,11 @@ int bits_for(int64_t K) {
     double lp = 0.0;
     for (int m : kMod) lp += log2((double)m);
     const int b = (int)floor((lp - 1.03 - log2((double)K)) / 2.0);
-    return b < 62 ? b : 62;
+    return b < 59 ? b : 59;   // (five digits of 13 bits)
 }
 
 // Element (r, k) of an operand: p[(r / R0) * s1 + (r % R0) * s0 + k * sk], r < R, k < K; its
-// residues are stored [MODS][R][ldk] as BF16 (columns K..ldk-1 zero), exponents in ex[R].
+// planes are stored [PLANES][R][ldk], 16 bits each (columns K..ldk-1 zero), exponents in ex[R].
 struct FmSrc {
     const double* p;
     int64_t R, K, R0, s1, s0, sk;
@@ -226,27 +246,53 @@ __global__ void __launch_bounds__(256) fm_rowexp_kernel(FmSrc a, FmSrc b, int nb
 }
 
 
-// |v| 2^(bits - e) rounded to an integer (e: the row's exponent), 0 in a non-finite row
-__device__ __forceinline__ unsigned long long fm_fixed(double v, int e, int bits) {
-    const unsigned long long u = (unsigned long long)__double_as_longlong(v);
-    int ev = (int)((u >> 52) & 0x7FF);
-    unsigned long long m = u & ((1ull << 52) - 1);
+// |v| 2^(bits - e) = u + d, u rounded to an integer, d to 2^-23 (e: the row's exponent; 0 in a
+// non-finite row); whether d is not zero
+__device__ __forceinline__ bool fm_fixed(double v, int e, int bits, unsigned long long& u, float& d) {
+    const unsigned long long w = (unsigned long long)__double_as_longlong(v);
+    int ev = (int)((w >> 52) & 0x7FF);
+    unsigned long long m = w & ((1ull << 52) - 1);
     if (ev == 0) ev = 1;           // subnormal (or zero: m = 0)
     else m |= 1ull << 52;
+    u = 0;
+    d = 0.0f;
+    if (e == FM_NONFINITE || m == 0) return false;
     // v = m 2^(ev - 1075); the shift is at most bits - 53
-    const int sh = ev - 1075 - e + bits;
-    if (e == FM_NONFINITE) return 0;
-    if (sh >= 0) return m << sh;
-    return sh > -63 ? (m + (1ull << (-sh - 1))) >> (-sh) : 0;
+    const int s = -(ev - 1075 - e + bits);
+    if (s <= 0) {
+        u = m << -s;
+        return false;
+    }
+    unsigned x;    // |d| = x 2^ex, x below 2^23
+    int ex;
+    bool down = false;
+    if (s < 64) {
+        u = (m + (1ull << (s - 1))) >> s;
+        const long long rem = (long long)(m - (u << s));
+        if (rem == 0) return false;
+        down = rem < 0;
+        const unsigned long long a = (unsigned long long)(down ? -rem : rem);
+        x = (unsigned)(s > 23 ? a >> (s - 23) : a);
+        ex = s > 23 ? -23 : -s;
+    } else {       // u = 0
+        x = (unsigned)(m >> 30);
+        ex = 30 - s;
+    }
+    if (ex > -120) {
+        d = (__uint_as_float(0x4B000000u | x) - 8388608.0f) * __uint_as_float((unsigned)(127 + ex) << 23);
+        if (down) d = -d;
+    }
+    return true;
 }
 
 // The residues of both operands in one launch: a block takes FM_PR rows x FM_PK columns, a warp
 // a row, a lane two columns.  sk == 1: read along k; else through a shared-memory tile, read
 // along the rows.
-__global__ void __launch_bounds__(256) fm_residue_kernel(FmSrc a, FmSrc b, int nba, int bits, const ModTable tab,
-                                                         const int* skip) {
+__global__ void __launch_bounds__(256) fm_residue_kernel(FmSrc a, FmSrc b, int nba, int bits, float theta,
+                                                         const ModTable tab, unsigned* failed, const int* skip) {
     ct_pdl();
     if (ct_skip(skip)) return;
+    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *failed = 0;
     __shared__ double tile[FM_PK][FM_PR + 1];
     const bool first = (int)blockIdx.x < nba;
     const FmSrc& x = first ? a : b;
@@ -290,7 +336,10 @@ __global__ void __launch_bounds__(256) fm_residue_kernel(FmSrc a, FmSrc b, int n
     }
     if (e == FM_ZERO) e = 0;
     if (blockIdx.y == 0 && lane == 0) x.ex[r0 + warp] = e;
-    const unsigned long long u0 = fm_fixed(v0, e, bits), u1 = fm_fixed(v1, e, bits);
+    unsigned long long u0, u1;
+    float r0f, r1f;
+    const bool inx0 = fm_fixed(v0, e, bits, u0, r0f), inx1 = fm_fixed(v1, e, bits, u1, r1f);
+    const bool neg0 = __double2hiint(v0) < 0, neg1 = __double2hiint(v1) < 0;
     // five 13-bit digits of each as floats with the value's sign (a digit in the low bits of
     // 2^23 + digit)
     float d[2][5];
@@ -298,8 +347,8 @@ __global__ void __launch_bounds__(256) fm_residue_kernel(FmSrc a, FmSrc b, int n
     for (int i = 0; i < 5; ++i) {
         const float x0 = __uint_as_float(0x4B000000u | ((unsigned)(u0 >> (13 * i)) & 8191u)) - 8388608.0f;
         const float x1 = __uint_as_float(0x4B000000u | ((unsigned)(u1 >> (13 * i)) & 8191u)) - 8388608.0f;
-        d[0][i] = __double2hiint(v0) < 0 ? -x0 : x0;
-        d[1][i] = __double2hiint(v1) < 0 ? -x1 : x1;
+        d[0][i] = neg0 ? -x0 : x0;
+        d[1][i] = neg1 ? -x1 : x1;
     }
     const int64_t plane = x.R * x.ldk;
     __nv_bfloat16* out = x.res + (r0 + warp) * x.ldk + k;
@@ -320,11 +369,32 @@ __global__ void __launch_bounds__(256) fm_residue_kernel(FmSrc a, FmSrc b, int n
         }
         *reinterpret_cast<uint32_t*>(out + i * plane) = __byte_perm(f[0], f[1], 0x7632);
     }
+    // a' and da, both times 2^15 (FP16 reaches down to 2^-29 of the row's largest, or of a unit)
+    const float unit = __uint_as_float((unsigned)(127 + 15 - bits) << 23);   // 2^(15 - bits)
+    float hv[2];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        float t = d[q][4];
+#pragma unroll
+        for (int j = 3; j >= 0; --j) t = fmaf(t, 8192.0f, d[q][j]);
+        hv[q] = t * unit;
+    }
+    const __half2 main2 = __floats2half2_rn(hv[0], hv[1]);
+    const __half2 rest2 = __floats2half2_rn((neg0 ? -r0f : r0f) * 32768.0f, (neg1 ? -r1f : r1f) * 32768.0f);
+    *reinterpret_cast<__half2*>(out + PL_CORR * plane) = first ? main2 : rest2;
+    *reinterpret_cast<__half2*>(out + (PL_CORR + 1) * plane) = first ? rest2 : main2;
+    // the test's x or y, in BF16 by its upper half; not zero in a non-zero entry
+    float g[2] = {fabsf(hv[0]) * 0x1p-15f, fabsf(hv[1]) * 0x1p-15f};
+    if (inx0) g[0] -= theta;
+    if (inx1) g[1] -= theta;
+    if (g[0] == 0.0f && (inx0 || u0)) g[0] = 0x1p-40f;
+    if (g[1] == 0.0f && (inx1 || u1)) g[1] = 0x1p-40f;
+    *reinterpret_cast<uint32_t*>(out + PL_TEST * plane) = __byte_perm(__float_as_uint(g[0]), __float_as_uint(g[1]), 0x7632);
 }
 
-// kind::f16 instruction descriptor: D f32, A and B bf16, both K-major.
-__host__ __device__ constexpr uint32_t fm_idesc(int M, int N) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+// kind::f16 instruction descriptor: D f32, A and B both bf16 (type 1) or both f16 (0), K-major.
+__host__ __device__ constexpr uint32_t fm_idesc(int M, int N, uint32_t type) {
+    return (1u << 4) | (type << 7) | (type << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 __device__ __forceinline__ void fm_mma(uint32_t dtm, uint64_t ad, uint64_t bd, uint32_t idesc, uint32_t acc) {
     asm volatile(
@@ -336,20 +406,26 @@ __device__ __forceinline__ void fm_mma(uint32_t dtm, uint64_t ad, uint64_t bd, u
 }
 
 struct FmOut {
-    unsigned char* r;    // [MODS][M][ldn]: t_i + 128 of C (ldn a multiple of FM_BN)
+    unsigned char* r;    // [MODS + 1][M][ldn]: t_i + 128 of C, then the test's answer (ldn a multiple of FM_BN)
+    float* corr;         // [2][M][ldn]: the corrections times 2^30
+    unsigned* failed;    // number of elements that fail the test
+    float limit;         // theta^2 K
     int64_t ldn;
 };
+constexpr unsigned FM_PASS = 0, FM_FAIL = 1, FM_NONE = 2;   // the test's answer (FM_NONE: exactly zero)
 
-// The MODS residue products: one CTA per SM walks (modulus, tile) items; warp 0 issues TMA
+// The products of all planes: one CTA per SM walks (plane, tile) items; warp 0 issues TMA
 // loads (128-byte swizzle, 4 stages of 32 KB), one thread of warp 1 the MMAs (M128 N128 K16),
 // 16 epilogue warps (four per TMEM lane quadrant, 32 columns each) take a chunk's accumulator
 // (512 / 128 of them in TMEM), reduce it modulo m in FP32 (x - m rint(x / m), exact below
-// 2^24), add the chunks and store t = r (P / m)^-1 mod m, the reconstruction's factor.  Every wait is bounded (2 s), after which the kernel sets the
-// status word, releases TMEM and returns.
+// 2^24), add the chunks and store t = r (P / m)^-1 mod m, the reconstruction's factor.  The
+// correction's chunks are added up as they are; so are the test's, which is answered in a byte.
+// Every wait is bounded (2 s), after which the kernel sets the status word, releases TMEM and
+// returns.
 __global__ void __launch_bounds__(FM_THREADS, 1)
     fm_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB, int M, int N,
                    int Kpad, FmOut out, const ModTable tab, const int* skip, int* status) {
-    ct_pdl();
+    ct_pdl_wait();
     if (ct_skip(skip)) return;
     extern __shared__ uint8_t fm_smem_raw[];
     uint8_t* smem = fm_smem_raw + ((1024u - (smem_u32(fm_smem_raw) & 1023u)) & 1023u);
@@ -363,7 +439,7 @@ __global__ void __launch_bounds__(FM_THREADS, 1)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int tiles_n = (N + FM_BN - 1) / FM_BN;
     const int tiles = tiles_n * ((M + FM_BM - 1) / FM_BM);
-    const int items = tiles * MODS;
+    const int items = tiles * PLANES;
     const int nkb = Kpad / FM_BK;
 
     if (threadIdx.x == 0) {
@@ -394,8 +470,8 @@ __global__ void __launch_bounds__(FM_THREADS, 1)
             int g = 0;
             bool ok = true;
             for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
-                const int mod = it / tiles, t = it % tiles;
-                const int ya = mod * M + (t / tiles_n) * FM_BM, yb = mod * N + (t % tiles_n) * FM_BN;
+                const int pl = it / tiles, t = it % tiles;
+                const int ya = pl * M + (t / tiles_n) * FM_BM, yb = pl * N + (t % tiles_n) * FM_BN;
                 for (int kb = 0; kb < nkb; ++kb, ++g) {
                     const int s = g % FM_STAGES;
                     const uint32_t ph = (uint32_t)(g / FM_STAGES) & 1u;
@@ -414,10 +490,11 @@ __global__ void __launch_bounds__(FM_THREADS, 1)
         }
     } else if (warp == 1) {
         if (lane == 0) {
-            constexpr uint32_t idesc = fm_idesc(FM_BM, FM_BN);
             int g = 0, gc = 0;
             bool ok = true;
             for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
+                const int pl = it / tiles;
+                const uint32_t idesc = fm_idesc(FM_BM, FM_BN, pl == PL_CORR || pl == PL_CORR + 1 ? 0u : 1u);
                 for (int kb0 = 0; kb0 < nkb && ok; kb0 += FM_KCH, ++gc) {
                     const int b = gc % FM_NB, u = gc / FM_NB;
                     if (u > 0 && !mbar_wait(&acc_empty[b], (uint32_t)((u - 1) & 1), abort_flag)) {
@@ -458,8 +535,8 @@ __global__ void __launch_bounds__(FM_THREADS, 1)
         int gc = 0;
         bool ok = true;
         for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
-            const int mod = it / tiles, t = it % tiles;
-            const float m = tab.c[mod].mf, rcp = tab.c[mod].rcp, inv = tab.c[mod].inv;
+            const int pl = it / tiles, t = it % tiles, mod = pl < MODS ? pl : 0;
+            const float m = tab.c[mod].mf, rcp = pl < MODS ? tab.c[mod].rcp : 0.0f, inv = tab.c[mod].inv;
             float sum[FM_HC];
 #pragma unroll
             for (int j = 0; j < FM_HC; ++j) sum[j] = 0.f;
@@ -485,13 +562,40 @@ __global__ void __launch_bounds__(FM_THREADS, 1)
 #pragma unroll
                 for (int j = 0; j < FM_HC; ++j) {
                     const float x = __uint_as_float(r[j]);
-                    const float k = __fsub_rn(__fadd_rn(__fmul_rn(x, rcp), RND), RND);
+                    const float k = __fsub_rn(__fadd_rn(__fmul_rn(x, rcp), RND), RND);   // (rcp 0: x as it is)
                     sum[j] += fmaf(-k, m, x);
                 }
             }
             if (!ok) break;
             const int64_t mr = (int64_t)(t / tiles_n) * FM_BM + row;
+            const int nc = (t % tiles_n) * FM_BN + hf * FM_HC;
+            if (pl == PL_TEST) {
+                int fails = 0;
+                uint32_t w[FM_HC / 4];
+#pragma unroll
+                for (int j = 0; j < FM_HC; ++j) {
+                    const uint32_t v = sum[j] >= out.limit ? FM_PASS : sum[j] == 0.0f ? FM_NONE : FM_FAIL;
+                    w[j / 4] = j % 4 ? w[j / 4] | v << (8 * (j % 4)) : v;
+                    fails += v == FM_FAIL && mr < M && nc + j < N;
+                }
+                fails = __reduce_add_sync(0xffffffffu, fails);
+                if (lane == 0 && fails) atomicAdd(out.failed, (unsigned)fails);
+                if (mr < M) {
+                    unsigned char* o = out.r + ((int64_t)MODS * M + mr) * out.ldn + nc;
+#pragma unroll
+                    for (int j = 0; j < FM_HC / 16; ++j)
+                        reinterpret_cast<uint4*>(o)[j] = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+                }
+                continue;
+            }
             if (mr >= M) continue;
+            if (pl >= PL_CORR) {
+                float4* o = reinterpret_cast<float4*>(out.corr + ((int64_t)(pl - PL_CORR) * M + mr) * out.ldn + nc);
+#pragma unroll
+                for (int j = 0; j < FM_HC / 4; ++j)
+                    o[j] = make_float4(sum[4 * j], sum[4 * j + 1], sum[4 * j + 2], sum[4 * j + 3]);
+                continue;
+            }
             // reduced once more, times the inverse (below 2^14), reduced, offset by 128 and packed, one
             // byte per element (t is at most m / 2 in magnitude; 128 occurs for m = 256 only,
             // where 256 wraps to 0, that is -128)
@@ -509,7 +613,7 @@ __global__ void __launch_bounds__(FM_THREADS, 1)
                 }
                 w[j4] = __byte_perm(__byte_perm(v[0], v[1], 0x0040), __byte_perm(v[2], v[3], 0x0040), 0x5410);
             }
-            unsigned char* o = out.r + ((int64_t)mod * M + mr) * out.ldn + (t % tiles_n) * FM_BN + hf * FM_HC;
+            unsigned char* o = out.r + ((int64_t)mod * M + mr) * out.ldn + nc;
 #pragma unroll
             for (int j = 0; j < FM_HC / 16; ++j)
                 reinterpret_cast<uint4*>(o)[j] = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
@@ -520,6 +624,9 @@ __global__ void __launch_bounds__(FM_THREADS, 1)
         tc_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
     }
+    // (earlier, the reconstruction's blocks would crowd on the SMs that are free first: 256^3 20.2 us for
+    // the whole product, 15.5 so)
+    ct_pdl_next();
 }
 
 struct FmC {
@@ -527,47 +634,120 @@ struct FmC {
     int64_t M0, s1, s0;
 };
 
-// C from its residues: S = sum t_i P / m_i - k P with k = rint(sum t_i / m_i), then
-// S 2^(ea + eb - 2 bits) rounded to FP64.  Three moduli at a time, u = sum t_j G / m_j (below
-// 2^26), so that the multi-word sums have six terms.  A thread takes four columns of a row.
-__global__ void __launch_bounds__(256) fm_crt_kernel(FmOut in, int M, int N, FmSrc a, FmSrc b, FmC c, int bits,
-                                                     const CrtTable tab, const int* skip) {
+// The whole product by FP64 FMAs, added in the order of k: 8 x 16 tiles dealt to the blocks, an
+// element per thread (FMAs of a warp issue at one per 64 clocks whatever a thread holds, see
+// gemm_f64_spread_kernel), the next 32 of K loaded while these are multiplied.
+constexpr int FM_CRT = 128;   // threads of the reconstruction: two rows of 128 columns
+__device__ void fm_fma_product(const FmSrc& a, const FmSrc& b, const FmC& c, int M, int N) {
+    constexpr int TM = 8, TN = 16, BK = 32, NA = TM * BK / FM_CRT, NB = TN * BK / FM_CRT;
+    __shared__ double As[BK][TM + 1], Bs[BK][TN + 1];
+    const int tid = threadIdx.x, tx = tid % TN, ty = tid / TN;
+    const int64_t tiles_n = (N + TN - 1) / TN, tiles = tiles_n * ((M + TM - 1) / TM);
+    const int64_t blocks = (int64_t)gridDim.x * gridDim.y;
+    for (int64_t t = (int64_t)blockIdx.y * gridDim.x + blockIdx.x; t < tiles; t += blocks) {
+        const int64_t m0 = t / tiles_n * TM, n0 = t % tiles_n * TN;
+        // a thread's elements of an operand's block: read along k, or along the rows
+        int ra[NA], ka[NA], rb[NB], kb[NB];
+        const double *pa[NA], *pb[NB];
+#pragma unroll
+        for (int i = 0; i < NA; ++i) {
+            const int e = tid + FM_CRT * i;
+            ra[i] = a.sk == 1 ? e / BK : e % TM;
+            ka[i] = a.sk == 1 ? e % BK : e / TM;
+            pa[i] = m0 + ra[i] < M ? a.p + a.row(m0 + ra[i]) + ka[i] * a.sk : nullptr;
+        }
+#pragma unroll
+        for (int i = 0; i < NB; ++i) {
+            const int e = tid + FM_CRT * i;
+            rb[i] = b.sk == 1 ? e / BK : e % TN;
+            kb[i] = b.sk == 1 ? e % BK : e / TN;
+            pb[i] = n0 + rb[i] < N ? b.p + b.row(n0 + rb[i]) + kb[i] * b.sk : nullptr;
+        }
+        double xa[NA], xb[NB];
+        auto load = [&](int64_t k0) {
+#pragma unroll
+            for (int i = 0; i < NA; ++i) {
+                xa[i] = pa[i] && k0 + ka[i] < a.K ? *pa[i] : 0.0;
+                if (pa[i]) pa[i] += BK * a.sk;
+            }
+#pragma unroll
+            for (int i = 0; i < NB; ++i) {
+                xb[i] = pb[i] && k0 + kb[i] < a.K ? *pb[i] : 0.0;
+                if (pb[i]) pb[i] += BK * b.sk;
+            }
+        };
+        double acc = 0.0;
+        load(0);
+        for (int64_t k0 = 0; k0 < a.K; k0 += BK) {
+            __syncthreads();
+#pragma unroll
+            for (int i = 0; i < NA; ++i) As[ka[i]][ra[i]] = xa[i];
+#pragma unroll
+            for (int i = 0; i < NB; ++i) Bs[kb[i]][rb[i]] = xb[i];
+            __syncthreads();
+            if (k0 + BK < a.K) load(k0 + BK);
+            const int kn = a.K - k0 < BK ? (int)(a.K - k0) : BK;
+#pragma unroll 1
+            for (int kk = 0; kk < kn; kk += 8)
+#pragma unroll
+                for (int u = 0; u < 8; ++u) acc = fma(As[kk + u][ty], Bs[kk + u][tx], acc);   // (zeros from kn on)
+        }
+        const int64_t m = m0 + ty, n = n0 + tx;
+        if (m < M && n < N) c.p[(m / c.M0) * c.s1 + (m % c.M0) * c.s0 + n] = acc;
+    }
+}
+
+// C from its residues: S = sum t_i P / m_i - k P with k = rint(sum t_i / m_i), plus the correction,
+// then times 2^(ea + eb - 2 bits) and rounded to FP64.  Two moduli at a time, u = sum t_j G / m_j (below
+// 2^17), so that the multi-word sums have eight terms.  A thread takes two columns of a row; the
+// elements that fail the test, or have no scale, are FP64 dot products by the warp.  Above
+// `most` of them the blocks compute the whole product instead.
+__global__ void __launch_bounds__(FM_CRT) fm_crt_kernel(FmOut in, int M, int N, FmSrc a, FmSrc b, FmC c, int bits,
+                                                     unsigned most, const CrtTable tab, const int* skip) {
     ct_pdl();
     if (ct_skip(skip)) return;
-    const int64_t n0 = 4 * ((int64_t)blockIdx.x * 64 + (threadIdx.x & 63));
-    const int64_t m = (int64_t)blockIdx.y * 4 + (threadIdx.x >> 6);
-    if (m >= M || n0 >= N) return;
+    if (__ldcg(in.failed) > most) {
+        fm_fma_product(a, b, c, M, N);
+        return;
+    }
+    const int lane = threadIdx.x & 31;
+    const int64_t n0 = 2 * ((int64_t)blockIdx.y * 64 + (threadIdx.x & 63));
+    const int64_t m = (int64_t)blockIdx.x * (FM_CRT / 64) + (threadIdx.x >> 6);   // the same for a warp
+    if (m >= M) return;
     const int em = a.ex[m];
-    uint32_t r4[MODS];
+    uint32_t r2[MODS], t2 = 0;
+    float2 cr = make_float2(0.0f, 0.0f);
 #pragma unroll
-    for (int i = 0; i < MODS; ++i)
-        r4[i] = *reinterpret_cast<const uint32_t*>(in.r + ((int64_t)i * M + m) * in.ldn + n0);
+    for (int i = 0; i < MODS; ++i) r2[i] = 0;
+    if (n0 < N) {
+#pragma unroll
+        for (int i = 0; i < MODS; ++i)
+            r2[i] = *reinterpret_cast<const uint16_t*>(in.r + ((int64_t)i * M + m) * in.ldn + n0);
+        t2 = *reinterpret_cast<const uint16_t*>(in.r + ((int64_t)MODS * M + m) * in.ldn + n0);
+        const float2 q = *reinterpret_cast<const float2*>(in.corr + m * in.ldn + n0);
+        const float2 w = *reinterpret_cast<const float2*>(in.corr + ((int64_t)M + m) * in.ldn + n0);
+        cr = make_float2(q.x + w.x, q.y + w.y);
+    }
     double* Cr = c.p + (m / c.M0) * c.s1 + (m % c.M0) * c.s0;
 #pragma unroll 1
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < 2; ++j) {
         const int64_t n = n0 + j;
-        if (n >= N) break;
-        const int en = b.ex[n];
-        if (em == FM_NONFINITE || en == FM_NONFINITE) {
-            double v = 0.0;
-            const double* pa = a.p + a.row(m);
-            const double* pb = b.p + b.row(n);
-            for (int64_t k = 0; k < a.K; ++k) v = fma(pa[k * a.sk], pb[k * b.sk], v);
-            Cr[n] = v;
-            continue;
-        }
-        unsigned long long acc[LIMBS] = {0, 0, 0, 0, 0};
+        const bool live = n < N;
+        const int en = live ? b.ex[n] : 0;
+        const unsigned answer = (t2 >> (8 * j)) & 0xffu;
+        const float corr = j == 0 ? cr.x : cr.y;
+        unsigned long long acc[LIMBS] = {};
         long long frac = -tab.rbias;
 #pragma unroll
         for (int g = 0; g < GROUPS; ++g) {
             unsigned u = 0;
 #pragma unroll
-            for (int i = 0; i < 3; ++i) u += ((r4[3 * g + i] >> (8 * j)) & 0xffu) * tab.co[g][i];
+            for (int i = 0; i < 2; ++i) u += ((r2[2 * g + i] >> (8 * j)) & 0xffu) * tab.co[g][i];
             frac += (long long)((unsigned long long)u * tab.rcp[g]);
 #pragma unroll
             for (int l = 0; l < LIMBS; ++l) acc[l] += (unsigned long long)u * tab.w[g][l];
         }
-        // (2^40 / G to half a unit: an error below 2^-12 of the fraction)
+        // (2^40 / G to half a unit: an error below 2^-20 of the fraction)
         const int kk = (int)((frac + (1ll << 39)) >> 40);
         // S = sum - bias - kk P as a two's complement number of LIMBS limbs
         unsigned s[LIMBS];
@@ -579,31 +759,26 @@ __global__ void __launch_bounds__(256) fm_crt_kernel(FmOut in, int M, int N, FmS
             s[l] = (unsigned)v;
             carry = (v >> 32) + (long long)(acc[l] >> 32);
         }
-        const bool neg = (s[LIMBS - 1] >> 31) != 0;
-        if (neg) {
-            unsigned cy = 1;
-#pragma unroll
-            for (int l = 0; l < LIMBS; ++l) {
-                const unsigned v = ~s[l];
-                s[l] = v + cy;
-                cy = (cy && s[l] == 0) ? 1 : 0;
-            }
+        unsigned long long hi = ((unsigned long long)s[3] << 32) | s[2], lo = ((unsigned long long)s[1] << 32) | s[0];
+        bool redo = em == FM_NONFINITE || en == FM_NONFINITE || answer == FM_FAIL ||
+                    (answer == FM_NONE && ((hi | lo) != 0 || corr != 0.0f));
+        {   // the correction, an integer of 2^-40 units, times 2^bits
+            const long long ci = __float2ll_rn(corr * 1024.0f);
+            const unsigned long long l = (unsigned long long)ci << (bits - 40);
+            lo += l;
+            hi += (unsigned long long)(ci >> (104 - bits)) + (lo < l ? 1 : 0);
         }
-        // magnitude (below 2^140) left-aligned in (hi, lo) and a sticky bit; the leading bit is worth
-        // 2^top
-        unsigned long long hi = ((unsigned long long)s[4] << 32) | s[3], lo = ((unsigned long long)s[2] << 32) | s[1];
-        unsigned below = s[0];
-        int top = 159;
+        const bool neg = (hi >> 63) != 0;
+        if (neg) {
+            lo = ~lo + 1;
+            hi = ~hi + (lo == 0 ? 1 : 0);
+        }
+        // magnitude (below 2^126) left-aligned in (hi, lo); the leading bit is worth 2^top
+        int top = 127;
         if (hi == 0) {
             hi = lo;
-            lo = (unsigned long long)below << 32;
-            below = 0;
+            lo = 0;
             top -= 64;
-            if (hi == 0) {
-                hi = lo;
-                lo = 0;
-                top -= 64;
-            }
         }
         double v = 0.0;
         if (hi != 0) {
@@ -616,13 +791,32 @@ __global__ void __launch_bounds__(256) fm_crt_kernel(FmOut in, int M, int N, FmS
             // 53 bits kept, round to nearest even
             unsigned long long f = hi >> 11;
             const unsigned long long rem = hi & 0x7ff;
-            f += (rem > 0x400 || (rem == 0x400 && ((lo | below) != 0 || (f & 1)))) ? 1 : 0;
+            f += (rem > 0x400 || (rem == 0x400 && (lo != 0 || (f & 1)))) ? 1 : 0;
             const int e = em + en - 2 * bits, ex = 1023 + top + e;   // exponent field of f's leading bit
             if (ex < 1 || ex > 2045) v = scalbn(neg ? -(double)f : (double)f, top - 52 + e);
             else v = __longlong_as_double((long long)((((unsigned long long)(ex - 1) << 52) + f) |
                                                       ((unsigned long long)neg << 63)));
         }
-        Cr[n] = v;
+        for (unsigned mask = __ballot_sync(0xffffffffu, live && redo); mask; mask &= mask - 1) {
+            const int src = __ffs(mask) - 1;
+            const double* pa = a.p + a.row(m);
+            const double* pb = b.p + b.row(__shfl_sync(0xffffffffu, n, src));
+            double dot = 0.0;
+            for (int64_t k0 = lane; k0 < a.K; k0 += 256) {   // (eight loads of each in flight)
+                double x[8], y[8];
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int64_t k = k0 + 32 * i;
+                    x[i] = k < a.K ? pa[k * a.sk] : 0.0;
+                    y[i] = k < a.K ? pb[k * b.sk] : 0.0;
+                }
+#pragma unroll
+                for (int i = 0; i < 8; ++i) dot = fma(x[i], y[i], dot);
+            }
+            dot = ct_warp_sum(dot);
+            if (lane == src) v = dot;
+        }
+        if (live) Cr[n] = v;
     }
 }
 
@@ -635,8 +829,8 @@ FmPlan fm_plan(int64_t M, int64_t N, int64_t K) {
     q.ldk = ct_round_up(K, FM_BK);
     q.ldn = ct_round_up(N, FM_BN);
     q.tiles = ct_cdiv(M, FM_BM) * ct_cdiv(N, FM_BN);
-    q.bytes = ct_bytes(MODS * M * q.ldk, 2) + ct_bytes(MODS * N * q.ldk, 2) + ct_bytes(MODS * M * q.ldn, 1) +
-              ct_bytes(M, 4) + ct_bytes(N, 4) + ct_bytes(ct_cdiv(K, FM_XK) * M, 4) + ct_bytes(ct_cdiv(K, FM_XK) * N, 4);
+    q.bytes = ct_bytes(PLANES * M * q.ldk, 2) + ct_bytes(PLANES * N * q.ldk, 2) + ct_bytes((MODS + 1) * M * q.ldn, 1) +
+              ct_bytes(2 * M * q.ldn, 4) + ct_bytes(1, 4) + ct_bytes(M, 4) + ct_bytes(N, 4) + ct_bytes(ct_cdiv(K, FM_XK) * M, 4) + ct_bytes(ct_cdiv(K, FM_XK) * N, 4);
     return q;
 }
 
@@ -660,7 +854,7 @@ int fm_map(ct_handle* h, CUtensorMap* m, const FmSrc& s, int box_rows) {
         ct_seterr(h, "TMA operand misaligned (base %p, ldk %lld)", (const void*)s.res, (long long)s.ldk);
         return CT_ERR_INVALID;
     }
-    cuuint64_t dims[2] = {(cuuint64_t)s.ldk, (cuuint64_t)(MODS * s.R)};
+    cuuint64_t dims[2] = {(cuuint64_t)s.ldk, (cuuint64_t)(PLANES * s.R)};
     cuuint64_t strides[1] = {(cuuint64_t)(s.ldk * 2)};
     cuuint32_t box[2] = {(cuuint32_t)FM_BK, (cuuint32_t)box_rows};
     cuuint32_t estr[2] = {1, 1};
@@ -677,22 +871,22 @@ int fm_map(ct_handle* h, CUtensorMap* m, const FmSrc& s, int box_rows) {
 }  // namespace
 
 // Whether an FP64-form product goes to the tensor cores.  Estimated times in us: the SIMT
-// kernel at 85% of the FP64 pipe (2 multiply-adds per clock and SM, 1.9 GHz); here 12 us of
+// kernel at 85% of the FP64 pipe (2 multiply-adds per clock and SM, 1.9 GHz); here 11 us of
 // launches and latencies, tile items at 1.2 us plus 0.16 us per 64 of K on each SM, and operands
-// and residues written and read at 4 TB/s.  Measured (us, SIMT / here): 128x384x128 16.6 / 17.9 and
-// 128x256x128 12.9 / 13.9 stay, 512x128x128 20.6 / 17.0, 640x128x128 24.0 / 18.7, 256x256x128
-// 20.5 / 19.2 and 256x256x256 36.9 / 20.0 go.  Only when the scratch is there or can be had: within
-// the handle's workspace limit, outside a stream capture, and with the memory available;
-// otherwise the SIMT kernel, as before.
+// and residues written and read at 4 TB/s.  Measured (us, SIMT / here): 96x288x96 12.4 / 13.3,
+// 128x256x128 12.9 / 12.2 and 128x384x128 16.9 / 14.7 stay, 128x512x128 20.7 / 14.0, 640x128x128
+// 23.8 / 15.0, 256x256x128 20.9 / 13.7 and 256x256x256 36.9 / 15.5 go.  Only when the scratch is
+// there or can be had: within the handle's workspace limit, outside a stream capture, and with the
+// memory available; otherwise the SIMT kernel, as before.
 bool ct_f64_route(ct_handle* h, int64_t M, int64_t N, int64_t K) {
     if (M <= 0 || N <= 0 || K <= 0 || K > ((int64_t)1 << 20) || !ct_fp64_tc_enabled(h, M, N, K)) return false;
     const FmPlan q = fm_plan(M, N, K);
-    if (MODS * M > (1ll << 30) || MODS * N > (1ll << 30) || q.tiles * MODS > (1ll << 30) || ct_cdiv(M, 4) > 65535)
+    if (PLANES * M > (1ll << 30) || PLANES * N > (1ll << 30) || q.tiles * PLANES > (1ll << 30) || ct_cdiv(N, 128) > 65535)
         return false;
     const double simt = (double)M * (double)N * (double)K / (0.85 * 2.0 * h->num_sms * 1900.0);
-    const double items = (double)ct_cdiv(q.tiles * MODS, h->num_sms) * (1.2 + 0.16 * (double)(q.ldk / FM_BK));
-    const double traffic = ((double)(M + N) * (double)q.ldk * 4.0 * MODS + (double)M * (double)q.ldn * 2.0 * MODS) / 4.0e6;
-    if (12.0 + items + traffic > simt) return false;
+    const double items = (double)ct_cdiv(q.tiles * PLANES, h->num_sms) * (1.2 + 0.16 * (double)(q.ldk / FM_BK));
+    const double traffic = ((double)(M + N) * (double)q.ldk * 4.0 * PLANES + (double)M * (double)q.ldn * 2.0 * (MODS + 9)) / 4.0e6;
+    if (11.0 + items + traffic > simt) return false;
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess) {
         (void)cudaGetLastError();
@@ -721,11 +915,17 @@ int ct_f64_gemm(ct_handle* h, int64_t M, int64_t N, int64_t K, const OzMat& A, c
     CT_TRY(fm_workspace(h, q.bytes));
     uint8_t* p = (uint8_t*)h->fm_ws;
     FmSrc a{A.p, M, K, A.R0 > 0 ? A.R0 : M, A.s1, A.s0, A.sk, (__nv_bfloat16*)p, nullptr, nullptr, q.ldk};
-    p += ct_bytes(MODS * M * q.ldk, 2);
+    p += ct_bytes(PLANES * M * q.ldk, 2);
     FmSrc b{B.p, N, K, B.R0 > 0 ? B.R0 : N, B.s1, B.s0, B.sk, (__nv_bfloat16*)p, nullptr, nullptr, q.ldk};
-    p += ct_bytes(MODS * N * q.ldk, 2);
-    FmOut o{(unsigned char*)p, q.ldn};
-    p += ct_bytes(MODS * M * q.ldn, 1);
+    p += ct_bytes(PLANES * N * q.ldk, 2);
+    const int bits = bits_for(K);
+    const float theta = ldexpf(1.0f, 37 - bits);
+    FmOut o{(unsigned char*)p, nullptr, nullptr, theta * theta * (float)K * 1.01f, q.ldn};
+    p += ct_bytes((MODS + 1) * M * q.ldn, 1);
+    o.corr = (float*)p;
+    p += ct_bytes(2 * M * q.ldn, 4);
+    o.failed = (unsigned*)p;
+    p += ct_bytes(1, 4);
     a.ex = (int*)p;
     p += ct_bytes(M, 4);
     b.ex = (int*)p;
@@ -742,21 +942,21 @@ int ct_f64_gemm(ct_handle* h, int64_t M, int64_t N, int64_t K, const OzMat& A, c
         attr_dev = h->device;
     }
     const Tables& t = tables();
-    const int bits = bits_for(K);
     const int nba = (int)ct_cdiv(M, FM_PR);
     const dim3 grid((unsigned)(nba + ct_cdiv(N, FM_PR)), (unsigned)ct_cdiv(q.ldk, FM_PK));
     if (grid.y > 65535) return CT_ERR_UNSUPPORTED;
     if (K > FM_XK) {
         ct_launch(h, fm_rowexp_kernel, dim3(grid.x, (unsigned)ct_cdiv(K, FM_XK)), 256, 0, a, b, nba, skip); ct_note_launch();
     }
-    ct_launch(h, fm_residue_kernel, grid, 256, 0, a, b, nba, bits, t.mod, skip); ct_note_launch();
-    const int64_t items = q.tiles * MODS;
+    ct_launch(h, fm_residue_kernel, grid, 256, 0, a, b, nba, bits, theta, t.mod, o.failed, skip); ct_note_launch();
+    const int64_t items = q.tiles * PLANES;
     const int64_t ctas = items < h->num_sms ? items : h->num_sms;
     ct_launch(h, fm_gemm_kernel, (unsigned)ctas, FM_THREADS, FM_SMEM, ta, tb, (int)M, (int)N, (int)q.ldk, o, t.mod, skip,
                                                                        h->d_status); ct_note_launch();
     const FmC c{Cout.p, Cout.M0 > 0 ? Cout.M0 : M, Cout.s1, Cout.s0};
-    ct_launch(h, fm_crt_kernel, dim3((unsigned)ct_cdiv(N, 256), (unsigned)ct_cdiv(M, 4)), 256, 0, 
-        o, (int)M, (int)N, a, b, c, bits, t.crt, skip); ct_note_launch();
+    const unsigned most = (unsigned)std::min<int64_t>(M * N / 8, 0x7fffffff);
+    ct_launch(h, fm_crt_kernel, dim3((unsigned)ct_cdiv(M, FM_CRT / 64), (unsigned)ct_cdiv(N, 128)), FM_CRT, 0,
+              o, (int)M, (int)N, a, b, c, bits, most, t.crt, skip); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }

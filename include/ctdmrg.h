@@ -18,10 +18,12 @@
  * Precision forms (ct_prec):
  *   CT_PREC_FP64    plain form, FP64 everywhere.  The contractions of H_eff,
  *                   the environments, theta and the gradients form products
- *                   that are large enough exactly, modulo 18 small integers on
- *                   the BF16 tensor cores, from operands rounded to 2^-63 of
- *                   each row's largest entry, and round them to FP64 once
- *                   (CTDMRG_FP64_TC=0 keeps them on FP64 FMAs).
+ *                   that are large enough modulo 16 small integers on the
+ *                   tensor cores.  Every element is tested on the device for
+ *                   the accuracy of FP64 FMAs (an error within 16.5 2^-53 of
+ *                   sum_k |a_k b_k|, in practice below 2 2^-53) and formed by
+ *                   them where it fails, so graded operands lose nothing
+ *                   (CTDMRG_FP64_TC=0 keeps all of them on FP64 FMAs).
  *   CT_PREC_TF32X3  contractions on tcgen05 tensor cores in TF32 with
  *                   3xTF32 split compensation and FP32 accumulation; all
  *                   storage, Lanczos, eigensolve, SVD and reductions FP64.
