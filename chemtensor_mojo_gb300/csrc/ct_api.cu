@@ -26,18 +26,21 @@ void ct_seterr(ct_handle* h, const char* fmt, ...) {
 int ct_reserve(ct_handle* h, size_t bytes) {
     if (bytes <= h->ws_cap) return CT_OK;
     size_t want = bytes + bytes / 4 + (1u << 20);
-    if (h->ws_limit && want > h->ws_limit) want = bytes;
+    // (what a captured graph holds is the graph's: it does not count against the limit)
+    const size_t residues = h->fm_captured ? 0 : h->fm_ws_bytes;
+    if (h->ws_limit && want + residues > h->ws_limit) want = bytes;
     if (h->ws_limit && want > h->ws_limit) {
         ct_seterr(h, "workspace of %zu bytes exceeds the limit of %zu bytes", bytes, h->ws_limit);
         return CT_ERR_OOM;
     }
+    if (h->ws_limit && want + residues > h->ws_limit) (void)ct_release_residues(h);
     if (h->ws) {
         CT_CUDA(h, cudaStreamSynchronize(h->stream));
         CT_CUDA(h, cudaFree(h->ws));
         h->ws = nullptr;
         h->ws_cap = 0;
     }
-    cudaError_t e = cudaMalloc((void**)&h->ws, want);
+    cudaError_t e = ct_malloc(h, (void**)&h->ws, want);
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
         h->ws = nullptr;
@@ -213,7 +216,7 @@ int ct_get_status(ct_handle* h, int* status_out) {
 int ct_workspace_bytes(ct_handle* h, int64_t* bytes_out) {
     CT_NULLCHK(h, h);
     CT_NULLCHK(h, bytes_out);
-    *bytes_out = (int64_t)h->ws_cap;
+    *bytes_out = (int64_t)(h->ws_cap + h->fm_ws_bytes + h->fm_kept_bytes);
     return CT_OK;
 }
 
@@ -228,6 +231,7 @@ int ct_set_workspace_limit(ct_handle* h, int64_t bytes) {
     CT_NULLCHK(h, h);
     if (bytes < 0) return CT_ERR_INVALID;
     h->ws_limit = (size_t)bytes;
+    if (bytes > 0 && h->ws_cap + h->fm_ws_bytes > (size_t)bytes) (void)ct_release_residues(h);
     return CT_OK;
 }
 

@@ -58,6 +58,7 @@ struct ct_handle {
     uint8_t* pin = nullptr;
     bool fm_captured = false;        // fm_ws is in a captured graph
     std::vector<void*> fm_kept;      // outgrown buffers of captured graphs, freed with the handle
+    size_t fm_kept_bytes = 0;
     // allocation-free mode (the stack handle of ct_heff2_apply_noalloc): the
     // launchers never call cudaMalloc; split-K partials come from the fixed
     // region below, and K is split only as far as that region holds
@@ -150,6 +151,28 @@ static inline void ct_note_launch() { g_ct_launches.fetch_add(1, std::memory_ord
         int s_ = (x);              \
         if (s_ != CT_OK) return s_; \
     } while (0)
+
+// Frees the residue products' scratch (ct_f64mod.cu) unless a graph may replay on it: it is the
+// first to go where memory or the workspace limit is short.  False when there was none to free.
+static inline bool ct_release_residues(ct_handle* h) {
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    if (!h->fm_ws || h->fm_captured || cudaStreamIsCapturing(h->stream, &cs) != cudaSuccess ||
+        cs != cudaStreamCaptureStatusNone || cudaStreamSynchronize(h->stream) != cudaSuccess)
+        return false;
+    (void)cudaFree(h->fm_ws);
+    h->fm_ws = nullptr;
+    h->fm_ws_bytes = 0;
+    return true;
+}
+// cudaMalloc that takes that scratch back before it gives up
+static inline cudaError_t ct_malloc(ct_handle* h, void** p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        (void)cudaGetLastError();
+        if (ct_release_residues(h)) e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
 
 #define CT_LAUNCH_CHECK(h) CT_CUDA(h, cudaGetLastError())
 

@@ -114,14 +114,14 @@ int ct_dmrg_two_site(ct_handle* h, const ct_dmrg_params* P, int N, int d, const 
     std::vector<DevBuf> Lenv(N + 1), Renv(N + 1);
     for (int k = 0; k <= N; ++k) {
         const size_t n = (size_t)(mpo_dims[k] * cap[k] * cap[k]);
-        CT_CUDA(h, cudaMalloc((void**)&Lenv[k].p, n * sizeof(double)));
-        CT_CUDA(h, cudaMalloc((void**)&Renv[k].p, n * sizeof(double)));
+        CT_CUDA(h, ct_malloc(h, (void**)&Lenv[k].p, n * sizeof(double)));
+        CT_CUDA(h, ct_malloc(h, (void**)&Renv[k].p, n * sizeof(double)));
     }
     int64_t th_cap = 1;
     for (int i = 0; i + 2 <= N; ++i) th_cap = std::max<int64_t>(th_cap, cap[i] * d * d * cap[i + 2]);
     DevBuf th, th_opt;
-    CT_CUDA(h, cudaMalloc((void**)&th.p, (size_t)th_cap * sizeof(double)));
-    CT_CUDA(h, cudaMalloc((void**)&th_opt.p, (size_t)th_cap * sizeof(double)));
+    CT_CUDA(h, ct_malloc(h, (void**)&th.p, (size_t)th_cap * sizeof(double)));
+    CT_CUDA(h, ct_malloc(h, (void**)&th_opt.p, (size_t)th_cap * sizeof(double)));
 
     // mixed form: rotations of the last split per (bond, direction), FP32, to
     // warm-start the next sweep's Jacobi at the same bond
@@ -235,7 +235,7 @@ int ct_dmrg_two_site(ct_handle* h, const ct_dmrg_params* P, int N, int d, const 
                     if (own.p) cudaFree(own.p);
                     own.p = nullptr;
                     own.cap = 0;
-                    CT_CUDA(h, cudaMalloc((void**)&own.p, (size_t)(c * own_len) * sizeof(double)));
+                    CT_CUDA(h, ct_malloc(h, (void**)&own.p, (size_t)(c * own_len) * sizeof(double)));
                     own.cap = c * own_len;
                 }
                 own.len = own.c = -1;
@@ -311,7 +311,7 @@ int ct_dmrg_two_site(ct_handle* h, const ct_dmrg_params* P, int N, int d, const 
                 if (c.cap < nv * nv) {
                     if (c.p) cudaFree(c.p);
                     c.p = nullptr;
-                    CT_CUDA(h, cudaMalloc((void**)&c.p, (size_t)(nv * nv) * sizeof(float)));
+                    CT_CUDA(h, ct_malloc(h, (void**)&c.p, (size_t)(nv * nv) * sizeof(float)));
                     c.cap = nv * nv;
                     c.m = c.n = -1;
                 }
@@ -474,8 +474,8 @@ int ct_mps_right_normalize(ct_handle* h, int N, int d, int64_t* bd, double* cons
         maxm = std::max<int64_t>(maxm, bd[i]);
     }
     DevBuf US, tmp;
-    CT_CUDA(h, cudaMalloc((void**)&US.p, (size_t)(maxm * maxm) * sizeof(double)));
-    CT_CUDA(h, cudaMalloc((void**)&tmp.p, (size_t)maxel * sizeof(double)));
+    CT_CUDA(h, ct_malloc(h, (void**)&US.p, (size_t)(maxm * maxm) * sizeof(double)));
+    CT_CUDA(h, ct_malloc(h, (void**)&tmp.p, (size_t)maxel * sizeof(double)));
     for (int i = N - 1; i >= 1; --i) {
         const int64_t Dl = bd[i], Dr = bd[i + 1];
         const int64_t m = Dl, n = d * Dr;
@@ -527,9 +527,9 @@ int ct_mps_expectation(ct_handle* h, int prec, int N, int d, const int64_t* mpo_
     int64_t cap = 1;
     for (int k = 0; k <= N; ++k) cap = std::max<int64_t>(cap, std::max<int64_t>(mpo_dims[k], 1) * bd[k] * bd[k]);
     DevBuf e0, e1, Wid;
-    CT_CUDA(h, cudaMalloc((void**)&e0.p, (size_t)cap * sizeof(double)));
-    CT_CUDA(h, cudaMalloc((void**)&e1.p, (size_t)cap * sizeof(double)));
-    CT_CUDA(h, cudaMalloc((void**)&Wid.p, (size_t)(d * d) * sizeof(double)));
+    CT_CUDA(h, ct_malloc(h, (void**)&e0.p, (size_t)cap * sizeof(double)));
+    CT_CUDA(h, ct_malloc(h, (void**)&e1.p, (size_t)cap * sizeof(double)));
+    CT_CUDA(h, ct_malloc(h, (void**)&Wid.p, (size_t)(d * d) * sizeof(double)));
     std::vector<double> idh((size_t)(d * d), 0.0);
     for (int s = 0; s < d; ++s) idh[(size_t)(s * d + s)] = 1.0;
     CT_CUDA(h, cudaMemcpyAsync(Wid.p, idh.data(), idh.size() * sizeof(double), cudaMemcpyHostToDevice, h->stream));
@@ -581,8 +581,8 @@ int ct_mps_expectation2(ct_handle* h, int prec, int N, int d, const int64_t* mpo
     for (int k = 0; k <= N; ++k)
         cap = std::max<int64_t>(cap, (mpo_sites ? mpo_dims[k] : 1) * bra_dims[k] * ket_dims[k]);
     DevBuf e0, e1;
-    CT_CUDA(h, cudaMalloc((void**)&e0.p, (size_t)cap * sizeof(double)));
-    CT_CUDA(h, cudaMalloc((void**)&e1.p, (size_t)cap * sizeof(double)));
+    CT_CUDA(h, ct_malloc(h, (void**)&e0.p, (size_t)cap * sizeof(double)));
+    CT_CUDA(h, ct_malloc(h, (void**)&e1.p, (size_t)cap * sizeof(double)));
     double* a = e0.p;
     double* b = e1.p;
     const int64_t w0 = mpo_sites ? mpo_dims[0] : 1;

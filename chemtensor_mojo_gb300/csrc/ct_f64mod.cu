@@ -834,16 +834,30 @@ FmPlan fm_plan(int64_t M, int64_t N, int64_t K) {
     return q;
 }
 
+// Room for `bytes`, with a quarter to spare for growing bonds where the limit and the memory allow it.
 int fm_workspace(ct_handle* h, size_t bytes) {
     if (h->fm_ws_bytes >= bytes) return CT_OK;
     CT_CUDA(h, cudaStreamSynchronize(h->stream));
-    if (h->fm_ws && h->fm_captured) h->fm_kept.push_back(h->fm_ws);   // graphs may replay on it
-    else if (h->fm_ws) cudaFree(h->fm_ws);
+    if (h->fm_ws && h->fm_captured) {   // graphs may replay on it
+        h->fm_kept.push_back(h->fm_ws);
+        h->fm_kept_bytes += h->fm_ws_bytes;
+    } else if (h->fm_ws) {
+        cudaFree(h->fm_ws);
+    }
     h->fm_captured = false;
     h->fm_ws = nullptr;
     h->fm_ws_bytes = 0;
-    CT_CUDA(h, cudaMalloc(&h->fm_ws, bytes));
-    h->fm_ws_bytes = bytes;
+    size_t want = bytes + bytes / 4;
+    if (h->ws_limit && h->ws_cap + want > h->ws_limit) want = bytes;
+    cudaError_t e = cudaMalloc(&h->fm_ws, want);
+    if (e != cudaSuccess && want > bytes) {
+        (void)cudaGetLastError();
+        want = bytes;
+        e = cudaMalloc(&h->fm_ws, want);
+    }
+    if (e != cudaSuccess) h->fm_ws = nullptr;
+    CT_CUDA(h, e);
+    h->fm_ws_bytes = want;
     return CT_OK;
 }
 
@@ -876,8 +890,9 @@ int fm_map(ct_handle* h, CUtensorMap* m, const FmSrc& s, int box_rows) {
 // and residues written and read at 4 TB/s.  Measured (us, SIMT / here): 96x288x96 12.4 / 13.3,
 // 128x256x128 12.9 / 12.2 and 128x384x128 16.9 / 14.7 stay, 128x512x128 20.7 / 14.0, 640x128x128
 // 23.8 / 15.0, 256x256x128 20.9 / 13.7 and 256x256x256 36.9 / 15.5 go.  Only when the scratch is
-// there or can be had: within the handle's workspace limit, outside a stream capture, and with the
-// memory available; otherwise the SIMT kernel, as before.
+// there or can be had: within the handle's workspace limit, beside the arena as it is, outside a
+// stream capture, and with the memory available; otherwise the SIMT kernel.  (So a handle with a limit may compute a product either
+// way, to the same accuracy, as its arena has grown: the arena comes first.)
 bool ct_f64_route(ct_handle* h, int64_t M, int64_t N, int64_t K) {
     if (M <= 0 || N <= 0 || K <= 0 || K > ((int64_t)1 << 20) || !ct_fp64_tc_enabled(h, M, N, K)) return false;
     const FmPlan q = fm_plan(M, N, K);
@@ -912,7 +927,10 @@ bool ct_f64_route(ct_handle* h, int64_t M, int64_t N, int64_t K) {
 int ct_f64_gemm(ct_handle* h, int64_t M, int64_t N, int64_t K, const OzMat& A, const OzMat& B, const OzOut& Cout,
                 const int* skip) {
     const FmPlan q = fm_plan(M, N, K);
-    CT_TRY(fm_workspace(h, q.bytes));
+    if (h->fm_ws_bytes < q.bytes) {
+        ct_seterr(h, "ct_f64_gemm: no scratch for %lld x %lld x %lld", (long long)M, (long long)N, (long long)K);
+        return CT_ERR_OOM;
+    }
     uint8_t* p = (uint8_t*)h->fm_ws;
     FmSrc a{A.p, M, K, A.R0 > 0 ? A.R0 : M, A.s1, A.s0, A.sk, (__nv_bfloat16*)p, nullptr, nullptr, q.ldk};
     p += ct_bytes(PLANES * M * q.ldk, 2);

@@ -334,7 +334,7 @@ int ct_gemm_f64_launch(ct_handle* h, const GemmDesc& g) {
                 if (h->splitk) cudaFree(h->splitk);
                 h->splitk = nullptr;
                 h->splitk_cap = 0;
-                CT_CUDA(h, cudaMalloc((void**)&h->splitk, need * sizeof(double)));
+                CT_CUDA(h, ct_malloc(h, (void**)&h->splitk, need * sizeof(double)));
                 h->splitk_cap = need;
             }
             gg.ksplit = ks;

@@ -180,7 +180,7 @@ int ct_energy_grad(ct_handle* h, int prec, int N, int d, const int64_t* mpo_dims
     const size_t o_R[4] = {reserve(maxh), reserve(maxh), reserve(maxn), reserve(maxn)};
     const size_t o_hA = reserve(maxsite), o_nA = reserve(maxsite), o_id = reserve((size_t)(d * d)), o_sc = reserve(2),
                  o_ex = reserve(2 * (size_t)(N + 1)), o_cum = reserve(2 * (size_t)(N + 1));
-    CT_CUDA(h, cudaMalloc((void**)&all.p, used * sizeof(double)));
+    CT_CUDA(h, ct_malloc(h, (void**)&all.p, used * sizeof(double)));
     struct Part {
         double* p;
     };

@@ -542,7 +542,7 @@ static int oz_workspace(ct_handle* h, size_t bytes, void** ws) {
         if (h->oz_ws) cudaFree(h->oz_ws);
         h->oz_ws = nullptr;
         h->oz_ws_bytes = 0;
-        CT_CUDA(h, cudaMalloc(&h->oz_ws, bytes));
+        CT_CUDA(h, ct_malloc(h, (void**)&h->oz_ws, bytes));
         h->oz_ws_bytes = bytes;
     }
     *ws = h->oz_ws;

@@ -1733,14 +1733,14 @@ int tc_hybrid_scratch(ct_handle* h, int64_t part_floats, int64_t cnt_n) {
         cudaFree(h->tc_hy_part);
         h->tc_hy_part = nullptr;
         h->tc_hy_part_floats = 0;
-        CT_CUDA(h, cudaMalloc((void**)&h->tc_hy_part, (size_t)part_floats * sizeof(float)));
+        CT_CUDA(h, ct_malloc(h, (void**)&h->tc_hy_part, (size_t)part_floats * sizeof(float)));
         h->tc_hy_part_floats = part_floats;
     }
     if (h->tc_hy_cnt_n < cnt_n) {
         cudaFree(h->tc_hy_cnt);
         h->tc_hy_cnt = nullptr;
         h->tc_hy_cnt_n = 0;
-        CT_CUDA(h, cudaMalloc((void**)&h->tc_hy_cnt, (size_t)cnt_n * sizeof(unsigned long long)));
+        CT_CUDA(h, ct_malloc(h, (void**)&h->tc_hy_cnt, (size_t)cnt_n * sizeof(unsigned long long)));
         CT_CUDA(h, cudaMemsetAsync(h->tc_hy_cnt, 0, (size_t)cnt_n * sizeof(unsigned long long), h->stream));
         h->tc_hy_cnt_n = cnt_n;
     }
@@ -1895,8 +1895,8 @@ int tc_gemm_run(ct_handle* h, const SplitOperand& A, const SplitOperand& B, int6
                 h->tc_sk_part = nullptr;
                 h->tc_sk_flag = nullptr;
                 h->tc_sk_floats = 0;
-                CT_CUDA(h, cudaMalloc((void**)&h->tc_sk_part, need * sizeof(float)));
-                CT_CUDA(h, cudaMalloc((void**)&h->tc_sk_flag, (size_t)h->num_sms * 4 * sizeof(int)));
+                CT_CUDA(h, ct_malloc(h, (void**)&h->tc_sk_part, need * sizeof(float)));
+                CT_CUDA(h, ct_malloc(h, (void**)&h->tc_sk_flag, (size_t)h->num_sms * 4 * sizeof(int)));
                 h->tc_sk_floats = (int64_t)need;
             }
             CT_CUDA(h, cudaMemsetAsync(h->tc_sk_flag, 0, (size_t)grid * 4 * sizeof(int), h->stream));

@@ -80,11 +80,15 @@ CT_API const char* ct_last_error(ct_handle* h);
 CT_API int ct_version(void);
 /* number of kernels this library has launched in the process (all handles) */
 CT_API int64_t ct_launch_count(void);
-/* bytes of handle-owned scratch currently reserved */
+/* bytes of handle-owned scratch currently reserved: the arena and the scratch of the FP64-form
+ * products on the tensor cores (with what captured graphs hold of it) */
 CT_API int ct_workspace_bytes(ct_handle* h, int64_t* bytes_out);
 /* Jacobi sweeps of the last SVD split on this handle and the running total */
 CT_API int ct_svd_sweeps(ct_handle* h, int* last_host, int64_t* total_host);
-/* cap on handle-owned scratch in bytes (0 = unlimited); growth beyond it -> CT_ERR_OOM */
+/* cap on handle-owned scratch in bytes (0 = unlimited); growth beyond it -> CT_ERR_OOM.
+ * FP64-form products on the tensor cores take their scratch from what the arena leaves of
+ * it, give it back when the arena grows or the cap is lowered, and run on FP64 FMAs where
+ * it is too small (same accuracy, other last bits).  Scratch in a captured graph stays. */
 CT_API int ct_set_workspace_limit(ct_handle* h, int64_t bytes);
 /* cap on the one-sided Jacobi sweeps of every SVD on this handle (0 = the
  * built-in caps, 60 for one-CTA problems and 48 for the cooperative kernel;
