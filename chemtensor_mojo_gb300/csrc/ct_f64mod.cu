@@ -835,10 +835,12 @@ FmPlan fm_plan(int64_t M, int64_t N, int64_t K) {
 }
 
 // Room for `bytes`, with a quarter to spare for growing bonds where the limit and the memory allow it.
-int fm_workspace(ct_handle* h, size_t bytes) {
+// Under a capture the new buffer is allocated too (in the thread's relaxed mode), so that a captured
+// call computes as the same call does outside; nothing is waited for or freed then.
+int fm_workspace(ct_handle* h, size_t bytes, bool capturing) {
     if (h->fm_ws_bytes >= bytes) return CT_OK;
-    CT_CUDA(h, cudaStreamSynchronize(h->stream));
-    if (h->fm_ws && h->fm_captured) {   // graphs may replay on it
+    if (!capturing) CT_CUDA(h, cudaStreamSynchronize(h->stream));
+    if (h->fm_ws && (h->fm_captured || capturing)) {   // graphs or launched kernels may run on it
         h->fm_kept.push_back(h->fm_ws);
         h->fm_kept_bytes += h->fm_ws_bytes;
     } else if (h->fm_ws) {
@@ -849,12 +851,15 @@ int fm_workspace(ct_handle* h, size_t bytes) {
     h->fm_ws_bytes = 0;
     size_t want = bytes + bytes / 4;
     if (h->ws_limit && h->ws_cap + want > h->ws_limit) want = bytes;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    if (capturing) CT_CUDA(h, cudaThreadExchangeStreamCaptureMode(&mode));
     cudaError_t e = cudaMalloc(&h->fm_ws, want);
     if (e != cudaSuccess && want > bytes) {
         (void)cudaGetLastError();
         want = bytes;
         e = cudaMalloc(&h->fm_ws, want);
     }
+    if (capturing) CT_CUDA(h, cudaThreadExchangeStreamCaptureMode(&mode));
     if (e != cudaSuccess) h->fm_ws = nullptr;
     CT_CUDA(h, e);
     h->fm_ws_bytes = want;
@@ -890,8 +895,8 @@ int fm_map(ct_handle* h, CUtensorMap* m, const FmSrc& s, int box_rows) {
 // and residues written and read at 4 TB/s.  Measured (us, SIMT / here): 96x288x96 12.4 / 13.3,
 // 128x256x128 12.9 / 12.2 and 128x384x128 16.9 / 14.7 stay, 128x512x128 20.7 / 14.0, 640x128x128
 // 23.8 / 15.0, 256x256x128 20.9 / 13.7 and 256x256x256 36.9 / 15.5 go.  Only when the scratch is
-// there or can be had: within the handle's workspace limit, beside the arena as it is, outside a
-// stream capture, and with the memory available; otherwise the SIMT kernel.  (So a handle with a limit may compute a product either
+// there or can be had: within the handle's workspace limit, beside the arena as it is, and with the
+// memory available; otherwise the SIMT kernel.  (So a handle with a limit may compute a product either
 // way, to the same accuracy, as its arena has grown: the arena comes first.)
 bool ct_f64_route(ct_handle* h, int64_t M, int64_t N, int64_t K) {
     if (M <= 0 || N <= 0 || K <= 0 || K > ((int64_t)1 << 20) || !ct_fp64_tc_enabled(h, M, N, K)) return false;
@@ -912,13 +917,14 @@ bool ct_f64_route(ct_handle* h, int64_t M, int64_t N, int64_t K) {
         h->fm_captured |= capturing;
         return true;
     }
-    if (capturing || (h->ws_limit && h->ws_cap + q.bytes > h->ws_limit)) return false;
+    if (h->ws_limit && h->ws_cap + q.bytes > h->ws_limit) return false;
     const std::string keep = h->err;
-    if (fm_workspace(h, q.bytes) != CT_OK) {
+    if (fm_workspace(h, q.bytes, capturing) != CT_OK) {
         (void)cudaGetLastError();
         h->err = keep;
         return false;
     }
+    h->fm_captured |= capturing;
     return true;
 }
 

@@ -1,10 +1,11 @@
 """Scratch of the FP64-form products on the tensor cores: reported, kept within the workspace limit
-beside the arena, given back, grown in few steps.
+beside the arena, given back, grown in few steps, and the same products with and without a capture.
 
 Small-integer operands: the products are exact on either path.
 """
 import numpy as np
 import pytest
+import torch
 
 pytestmark = pytest.mark.gpu
 
@@ -73,3 +74,27 @@ def test_growing_bonds_grow_the_scratch_in_few_steps():
         _theta(ctx, 2 * (k // 2), 2 * (k // 2), k)
         sizes.add(ctx.workspace_bytes())
     assert len(sizes) <= 8                           # 4.3 times as much in steps of a quarter
+
+
+@pytest.mark.parametrize("D", [160])
+def test_captured_apply_without_scratch_computes_as_the_eager_one(D):
+    import chemtensor_mojo_gb300 as ct
+    gen = torch.Generator(device="cuda").manual_seed(D)
+    rnd = lambda *s: ct.DenseTensor(torch.randn(s, dtype=torch.float64, device="cuda", generator=gen), list(s))  # noqa: E731
+    th, L, R, W = rnd(D, 2, 2, D), rnd(5, D, D), rnd(5, D, D), ct.MPOSite(rnd(5, 2, 2, 5))
+    ref = ct.apply_two_site_heff(th, L, R, W, W, ct.DeviceContext(0)).storage.clone()
+    ctx = ct.DeviceContext(0)
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        ct.apply_two_site_heff(th, L, R, W, W, ctx, prec="tf32x3")   # the arena alone
+        s.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=s):
+            out = ct.apply_two_site_heff(th, L, R, W, W, ctx).storage
+        for n in (512, 768):                         # eager products outgrow the graph's scratch (no arena here)
+            _theta(ctx, n, n, n)
+            out.fill_(float("nan"))
+            graph.replay()
+            s.synchronize()
+            assert torch.equal(out, ref)
