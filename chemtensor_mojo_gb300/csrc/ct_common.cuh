@@ -6,8 +6,11 @@
 #include <stdint.h>
 #include <stdio.h>
 #include <string.h>
+#include <stdlib.h>
 #include <atomic>
+#include <map>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/ctdmrg.h"
@@ -76,6 +79,7 @@ struct ct_handle {
     unsigned long long* tc_hy_cnt = nullptr;
     int64_t tc_hy_cnt_n = 0;
     unsigned tc_hy_epoch = 0;       // tag of the last launch (never 0 once used)
+    std::map<std::pair<const void*, unsigned>, bool> clusters;   // ct_cluster_fits's answers
     // tensor-core path state
     bool tc_checked = false;
     bool tc_ok = false;
@@ -189,6 +193,34 @@ void ct_launch(ct_handle* h, void (*kernel)(P...), dim3 grid, dim3 block, size_t
     cfg.attrs = &at;
     cfg.numAttrs = 1;
     (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);   // (CT_LAUNCH_CHECK reads the error)
+}
+
+// Whether clusters of `ctas` CTAs of this kernel (no dynamic shared memory) can run where the handle
+// does: more than 8 are not portable, and a part of a device may not have the SMs together.
+// CTDMRG_MAX_CLUSTER=n caps them (0: not even one of one CTA), read on every call.
+template <typename... P>
+bool ct_cluster_fits(ct_handle* h, void (*kernel)(P...), unsigned ctas, unsigned threads) {
+    const char* e = getenv("CTDMRG_MAX_CLUSTER");
+    if (e && (int)ctas > atoi(e)) return false;
+    if (ctas <= 1) return true;
+    const auto key = std::make_pair((const void*)kernel, ctas);
+    const auto it = h->clusters.find(key);
+    if (it != h->clusters.end()) return it->second;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(threads);
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = ctas;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    const bool fits = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                      cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) == cudaSuccess && n > 0;
+    if (!fits) (void)cudaGetLastError();
+    h->clusters[key] = fits;
+    return fits;
 }
 
 // What the host reads after a solve or a split (status, scalars, flags) comes over in one copy to
@@ -391,7 +423,7 @@ int ct_lanczos_reorth_pass32(ct_handle* h, int64_t n, double* w, const float* V3
                              double beta_threshold, const int* skip, double ratio64);
 int ct_lanczos_reorth_redo(ct_handle* h, int64_t n, double* w, const double* V, const float* V32, int64_t ldv, int j,
                            double beta_threshold, const int* skip);
-bool ct_lanczos_step_fits(ct_handle* h, int64_t n);
+bool ct_lanczos_step_fits(ct_handle* h, int64_t n, bool reorth, bool v32);
 int ct_lanczos_step(ct_handle* h, int64_t n, double* w, double* V, float* V32, int j, bool reorth, double beta_threshold,
                     double ratio64, const int* skip);
 int ct_lanczos_next32(ct_handle* h, int64_t n, const double* w, double* vnext, float* vnext32, int j,

@@ -314,7 +314,7 @@ int ct_lanczos_run(ct_handle* h, Arena& ar, int prec, const double* theta_in, do
     // algorithmic FLOPs of one apply (the reference's four contractions)
     const double heff_flops = 2.0 * (double)Dl * wL * d * d * Dr * Dl + 2.0 * (double)Dl * d * Dr * wL * d * d * wM +
                               2.0 * (double)Dl * Dr * d * wM * d * d * wR + 2.0 * (double)Dl * d * d * Dr * wR * Dr;
-    const bool short_step = ct_lanczos_step_fits(h, N);
+    const bool short_step = ct_lanczos_step_fits(h, N, reorth != 0, V32 != nullptr);
     for (int j = 0; j < max_iter - 1; ++j) {
         double* vj = V + (int64_t)j * N;
         const double* vjm1 = (j > 0) ? V + (int64_t)(j - 1) * N : nullptr;

@@ -221,12 +221,6 @@ template <int E, bool CLUSTER>
 int launch(ct_handle* h, Args& a, int ctas, int teams) {
     const dim3 block((unsigned)(TEAM * teams));
     if (CLUSTER) {
-        static int attr_dev = -1;
-        if (attr_dev != h->device) {
-            CT_CUDA(h, cudaFuncSetAttribute(svd_small_kernel<E, CLUSTER>, cudaFuncAttributeNonPortableClusterSizeAllowed,
-                                            1));
-            attr_dev = h->device;
-        }
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3((unsigned)ctas);
         cfg.blockDim = block;
@@ -240,8 +234,12 @@ int launch(ct_handle* h, Args& a, int ctas, int teams) {
         CT_CUDA(h, cudaLaunchKernelEx(&cfg, svd_small_kernel<E, CLUSTER>, a));
     } else {
         void* args[] = {&a};
-        CT_CUDA(h, cudaLaunchCooperativeKernel((const void*)svd_small_kernel<E, CLUSTER>, dim3((unsigned)ctas), block,
-                                               args, 0, h->stream));
+        cudaError_t e;
+        do {   // (fewer CTAs where the handle has not the whole device)
+            e = cudaLaunchCooperativeKernel((const void*)svd_small_kernel<E, CLUSTER>, dim3((unsigned)ctas), block, args, 0,
+                                            h->stream);
+        } while (e == cudaErrorCooperativeLaunchTooLarge && cudaGetLastError() == e && (ctas /= 2) > 0);
+        CT_CUDA(h, e);
     }
     ct_note_launch();
     return CT_OK;
@@ -257,7 +255,12 @@ inline int run(ct_handle* h, Args& a) {
     if (a.nvec <= CLUSTER_MAX) {
         int ctas = 1;
         while (ctas < pairs && ctas < CLUSTER_CTAS) ctas *= 2;
-        const int teams = (pairs + ctas - 1) / ctas;
+        // the largest cluster that can run here; the rotations are the same in any
+        const auto kernel = big <= TEAM       ? svd_small_kernel<1, true>
+                            : big <= 2 * TEAM ? svd_small_kernel<2, true>
+                                              : svd_small_kernel<0, true>;
+        while (ctas > 1 && !ct_cluster_fits(h, kernel, (unsigned)ctas, TEAM * MAX_TEAMS)) ctas /= 2;
+        const int teams = std::min((pairs + ctas - 1) / ctas, MAX_TEAMS);
         if (big <= TEAM) return launch<1, true>(h, a, ctas, teams);
         if (big <= 2 * TEAM) return launch<2, true>(h, a, ctas, teams);
         return launch<0, true>(h, a, ctas, teams);

@@ -1519,8 +1519,18 @@ int ct_lanczos_reorth_redo(ct_handle* h, int64_t n, double* w, const double* V, 
     return CT_OK;
 }
 
-// Whether ct_lanczos_step takes vectors of n elements.
-bool ct_lanczos_step_fits(ct_handle* h, int64_t n) { return grid_for(h, n) <= STEP_MAXG; }
+// The form of a step: reorth and the FP32 copy of the basis (mixed form).
+using StepKernel = void (*)(LanczosStep);
+static StepKernel step_kernel(bool reorth, bool v32) {
+    return !reorth ? lanczos_step_kernel<0> : v32 ? lanczos_step_kernel<2> : lanczos_step_kernel<1>;
+}
+
+// Whether ct_lanczos_step takes vectors of n elements: up to STEP_MAXG blocks, as one cluster that can
+// run here.  The separate launches otherwise, to the same bits.
+bool ct_lanczos_step_fits(ct_handle* h, int64_t n, bool reorth, bool v32) {
+    const int g = grid_for(h, n);
+    return g <= STEP_MAXG && ct_cluster_fits(h, step_kernel(reorth, v32), (unsigned)g, RT);
+}
 
 // Everything of Lanczos step j after w = H v_j up to v_{j+1} (see lanczos_step_kernel).  V32
 // (mixed form, reorthogonalised) and reorth choose the form.
@@ -1545,13 +1555,7 @@ int ct_lanczos_step(ct_handle* h, int64_t n, double* w, double* V, float* V32, i
     q.j = j;
     q.vec2 = ((n & 1) == 0 && aligned16(w) && aligned16(V)) ? 1 : 0;
     q.vec4 = ((n & 3) == 0 && aligned16(w) && V32 && aligned16(V32)) ? 1 : 0;
-    auto* f = !reorth ? lanczos_step_kernel<0> : V32 ? lanczos_step_kernel<2> : lanczos_step_kernel<1>;
-    static int attr_dev = -1;
-    if (attr_dev != h->device) {
-        for (auto* k : {lanczos_step_kernel<0>, lanczos_step_kernel<1>, lanczos_step_kernel<2>})
-            CT_CUDA(h, cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        attr_dev = h->device;
-    }
+    const StepKernel f = step_kernel(reorth, V32 != nullptr);   // (ct_lanczos_step_fits allowed the size)
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)grid_for(h, n));
     cfg.blockDim = dim3(RT);
