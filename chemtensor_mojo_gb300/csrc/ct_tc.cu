@@ -1812,6 +1812,15 @@ struct SplitOperand {
     int64_t rows = 0, ldk = 0;
 };
 
+// Whole tiles in pairs of rows, wide and at least 1024 deep: the paired kernel.  (us, one CTA /
+// pairs: 4096x1024xK in 224-wide tiles K 256 12.5 / 12.6, 512 19.1 / 18.8, 1024 32.5 / 31.0,
+// 2048 70.7 / 59.6, 4096 132.8 / 110.5; 4864x1024xK in 256-wide ones 16.8 / 17.4, 23.8 / 24.1,
+// 38.6 / 38.0, 83.7 / 70.4, 154 / 128; 192-wide 5120x2048x1024 87.5 / 92.6, 128-wide
+// 3072x768x3840 87.1 / 88.0.)
+constexpr bool tc_pairs(int bn, int64_t gsk, int64_t rows, int64_t ldk, int num_sms) {
+    return bn >= 224 && gsk == 0 && (rows + TC_BM - 1) / TC_BM % 2 == 0 && ldk >= 32 * TC_BK && num_sms % 2 == 0;
+}
+
 template <int BN, int STAGES>
 int tc_gemm_run(ct_handle* h, const SplitOperand& A, const SplitOperand& B, int64_t M, int64_t N,
                 const TcEpi& epi, const int* skip) {
@@ -1853,14 +1862,8 @@ int tc_gemm_run(ct_handle* h, const SplitOperand& A, const SplitOperand& B, int6
             hy.cnt = h->tc_hy_cnt;
             grid = hy.tiles_dp > 0 ? h->num_sms : hy.gsk;
         }
-        // Whole tiles in pairs of rows, wide and at least 1024 deep: the paired kernel.  (us, one CTA /
-        // pairs: 4096x1024xK in 224-wide tiles K 256 12.5 / 12.6, 512 19.1 / 18.8, 1024 32.5 / 31.0,
-        // 2048 70.7 / 59.6, 4096 132.8 / 110.5; 4864x1024xK in 256-wide ones 16.8 / 17.4, 23.8 / 24.1,
-        // 38.6 / 38.0, 83.7 / 70.4, 154 / 128; 192-wide 5120x2048x1024 87.5 / 92.6, 128-wide
-        // 3072x768x3840 87.1 / 88.0.)
-        constexpr bool wide = BN >= 224;
-        if (wide && hy.gsk == 0 && ct_cdiv(M, TC_BM) % 2 == 0 && A.ldk >= 32 * TC_BK && h->num_sms % 2 == 0) {
-            constexpr int PBN = wide ? BN : 224;   // (the others are not instantiated)
+        if (tc_pairs(BN, hy.gsk, M, A.ldk, h->num_sms)) {
+            constexpr int PBN = BN >= 224 ? BN : 224;   // (the others are not instantiated)
             using LP = TcPairSmem<PBN>;
             static int pair_dev = -1;
             if (pair_dev != h->device) {
@@ -1944,6 +1947,14 @@ TcChoice tc_choose(int num_sms, bool no_alloc, int64_t M, int64_t N, int64_t ldk
     return c;
 }
 
+// 128-wide tiles that leave half of the SMs idle: as many 64-wide ones (each element's chunks and
+// their order are the same).  Measured (us, 128 / 64 wide): 256x64x320 10.0 / 9.7,
+// 320x256x64 6.6 / 5.0, 640x160x800 22.6 / 20.4, 512x1024x1024 26.8 / 24.2, 3376x163x1152
+// 36.1 / 30.3.  rows, cols: as the tiles see them (transposed or not).
+bool tc_narrow(const TcChoice& c, int64_t rows, int64_t cols, int num_sms) {
+    return c.bn == 128 && c.chunked && !tc_bn_mode() && ct_cdiv(rows, TC_BM) * ct_cdiv(cols, 64) <= num_sms;
+}
+
 int tc_gemm_launch(ct_handle* h, const SplitOperand& A, const SplitOperand& B, int64_t M, int64_t N,
                    const TcEpi& epi, const int* skip) {
     if (A.ldk != B.ldk) return CT_ERR_SHAPE;
@@ -1970,13 +1981,7 @@ int tc_gemm_launch(ct_handle* h, const SplitOperand& A, const SplitOperand& B, i
         Mr = N;
         Nr = M;
     }
-    // 128-wide tiles that leave half of the SMs idle: as many 64-wide ones (each element's chunks and
-    // their order are the same).  Measured (us, 128 / 64 wide): 256x64x320 10.0 / 9.7,
-    // 320x256x64 6.6 / 5.0, 640x160x800 22.6 / 20.4, 512x1024x1024 26.8 / 24.2, 3376x163x1152
-    // 36.1 / 30.3.
-    const bool narrow = bn == 128 && ch.chunked && !tc_bn_mode() &&
-                        ct_cdiv(Mr, TC_BM) * ct_cdiv(Nr, 64) <= h->num_sms;
-    const int rc = narrow ? tc_gemm_run<64, GEMM_STAGES_64>(h, *opA, *opB, Mr, Nr, e, skip)
+    const int rc = tc_narrow(ch, Mr, Nr, h->num_sms) ? tc_gemm_run<64, GEMM_STAGES_64>(h, *opA, *opB, Mr, Nr, e, skip)
                  : bn == 256 ? tc_gemm_run<256, GEMM_STAGES_W>(h, *opA, *opB, Mr, Nr, e, skip)
                  : bn == 224 ? tc_gemm_run<224, GEMM_STAGES_W>(h, *opA, *opB, Mr, Nr, e, skip)
                  : bn == 192 ? tc_gemm_run<192, GEMM_STAGES_W>(h, *opA, *opB, Mr, Nr, e, skip)
@@ -2413,6 +2418,20 @@ extern "C" CT_API int ct_tc_gemm_plan(int64_t m, int64_t n, int64_t k, int num_s
     out[5] = hy.units;
     out[6] = hy.maxp;
     out[7] = ldk / TC_BK;
+    return CT_OK;
+}
+
+// What the plan's product is launched as.
+extern "C" CT_API int ct_tc_gemm_form(int64_t m, int64_t n, int64_t k, int num_sms, int64_t* out) {
+    int64_t plan[8];
+    CT_TRY(ct_tc_gemm_plan(m, n, k, num_sms, plan));
+    const int64_t ldk = ct_round_up(k, TC_BK), Mr = plan[1] ? n : m, Nr = plan[1] ? m : n;
+    const TcChoice c = tc_choose(num_sms, false, m, n, ldk, true);
+    const bool narrow = tc_narrow(c, Mr, Nr, num_sms), pairs = c.chunked && tc_pairs(c.bn, plan[4], Mr, ldk, num_sms);
+    const int64_t tiles = narrow ? ct_cdiv(Nr, 64) * ct_cdiv(Mr, TC_BM) : plan[2];
+    out[0] = narrow ? 64 : c.bn;
+    out[1] = pairs ? 2 : 1;
+    out[2] = tc_use_persistent() ? (pairs ? 2 * std::min<int64_t>(tiles / 2, num_sms / 2) : std::min<int64_t>(tiles, num_sms)) : tiles;
     return CT_OK;
 }
 

@@ -354,9 +354,12 @@ CT_API int ct_tc_gemm_time(ct_handle* h, int64_t m, int64_t n, int64_t k, int re
  * 224 or 256), out[1] 1 when C^T = B A^T is computed instead, out[2] tiles,
  * out[3] whole tiles of the hybrid schedule, out[4] CTAs sharing the stream-K
  * k-blocks (0: no stream-K part), out[5] stream-K k-blocks, out[6] most pieces
- * of one stream-K tile, out[7] k-blocks (32 of K) per tile.  (128-wide tiles
- * are halved at launch while the halves still fit the SMs in one wave.) */
+ * of one stream-K tile, out[7] k-blocks (32 of K) per tile.                */
 CT_API int ct_tc_gemm_plan(int64_t m, int64_t n, int64_t k, int num_sms, int64_t* out);
+/* What that plan is launched as: out[0] the width of the tiles (64 where
+ * 128-wide ones are halved because the halves still fit the SMs in one wave),
+ * out[1] CTAs per tile (2: pairs on 256-row tiles), out[2] CTAs in all.     */
+CT_API int ct_tc_gemm_form(int64_t m, int64_t n, int64_t k, int num_sms, int64_t* out);
 
 /* Live timing of the tensor-core GEMM inside real work (no reference
  * counterpart).  ct_kernel_timing(h, 1) resets the totals and makes every
