@@ -487,6 +487,7 @@ __global__ void __launch_bounds__(FM_THREADS, 1)
                     tma_load_2d(st + FM_A_BYTES, &tmB, kb * FM_BK, yb, &full[s]);
                 }
             }
+            drain_loads(full, FM_STAGES, g);
         }
     } else if (warp == 1) {
         if (lane == 0) {

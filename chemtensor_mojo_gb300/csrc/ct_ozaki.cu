@@ -210,6 +210,7 @@ __global__ void __launch_bounds__(OZ_THREADS, 1)
                     }
                 }
             }
+            drain_loads(full, OZ_STAGES, g);
         }
     } else if (warp == 1) {
         if (lane == 0) {
