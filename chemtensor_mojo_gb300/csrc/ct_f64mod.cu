@@ -25,11 +25,11 @@
 // exactly zero where no k has both, as between the blocks of a block-sparse operand (x and y of a
 // non-zero entry are kept from zero): such an element passes if its product is zero too.  The
 // others are computed as FP64 dot products, by a warp each; when they are more than an eighth of
-// all, the whole product by FP64 FMAs in the order of k, as without this route.
+// all, the whole product by FP64 FMAs.
 // Every element is thus within 16.5 2^-53 S and the final rounding (worst case; FP64 FMAs: K 2^-53 S).
 // Measured, 256^3, N(0,1) operands with A falling and B rising along k by a factor f, largest error
 // in units of 2^-53 S (here, with the final rounding / FP64 FMAs): f = 1 below 0.001 / 4.0, 1e2 0.22 /
-// 4.3, 1e4 0.41 / 4.0, 1e5 0.45 / 3.6, 1e6 1.1 / 4.4, beyond that it is the FMA path.  (18 moduli
+// 4.3, 1e4 0.41 / 4.0, 1e5 0.45 / 3.6, 1e6 1.1 / 4.4, 1e7 and more, on FMAs, 1.2 / 4.4.  (18 moduli
 // alone, b = 62, without correction and test: 2e-14 of an element at f = 1e6, 1.5e-8 at 1e12.)
 // When the FMA path is taken the products here are lost: 256^3 54 us (40 without this route), 512^3
 // 264 (231), 1024^3 1827 (1743); thin and deep, where that one would split K, 128 x 128 x 2048 224 (64).
@@ -635,9 +635,10 @@ struct FmC {
     int64_t M0, s1, s0;
 };
 
-// The whole product by FP64 FMAs, added in the order of k: 8 x 16 tiles dealt to the blocks, an
-// element per thread (FMAs of a warp issue at one per 64 clocks whatever a thread holds, see
-// gemm_f64_spread_kernel), the next 32 of K loaded while these are multiplied.
+// The whole product by FP64 FMAs, the sums of 32 of K added in the order of k (so that no error is
+// above that of K pieces): 8 x 16 tiles dealt to the blocks, an element per thread (FMAs of a warp
+// issue at one per 64 clocks whatever a thread holds, see gemm_f64_spread_kernel), the next 32 of K
+// loaded while these are multiplied.
 constexpr int FM_CRT = 128;   // threads of the reconstruction: two rows of 128 columns
 __device__ void fm_fma_product(const FmSrc& a, const FmSrc& b, const FmC& c, int M, int N) {
     constexpr int TM = 8, TN = 16, BK = 32, NA = TM * BK / FM_CRT, NB = TN * BK / FM_CRT;
@@ -688,10 +689,12 @@ __device__ void fm_fma_product(const FmSrc& a, const FmSrc& b, const FmC& c, int
             __syncthreads();
             if (k0 + BK < a.K) load(k0 + BK);
             const int kn = a.K - k0 < BK ? (int)(a.K - k0) : BK;
+            double part = 0.0;
 #pragma unroll 1
             for (int kk = 0; kk < kn; kk += 8)
 #pragma unroll
-                for (int u = 0; u < 8; ++u) acc = fma(As[kk + u][ty], Bs[kk + u][tx], acc);   // (zeros from kn on)
+                for (int u = 0; u < 8; ++u) part = fma(As[kk + u][ty], Bs[kk + u][tx], part);   // (zeros from kn on)
+            acc += part;
         }
         const int64_t m = m0 + ty, n = n0 + tx;
         if (m < M && n < N) c.p[(m / c.M0) * c.s1 + (m % c.M0) * c.s0 + n] = acc;

@@ -117,7 +117,7 @@ def test_deep_products(ctx, k):
         check(ctx, A / g, B * g[:, None])
 
 
-GAUGES = [1e4, 1e8, 1e12]
+GAUGES = [1e4, 1e6, 1e8, 1e12]
 
 
 # a gauge between the environment and the site (or theta), entries of H_eff and of both updates
