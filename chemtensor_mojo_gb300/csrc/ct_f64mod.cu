@@ -31,8 +31,9 @@
 // in units of 2^-53 S (here, with the final rounding / FP64 FMAs): f = 1 below 0.001 / 4.0, 1e2 0.22 /
 // 4.3, 1e4 0.41 / 4.0, 1e5 0.45 / 3.6, 1e6 1.1 / 4.4, 1e7 and more, on FMAs, 1.2 / 4.4.  (18 moduli
 // alone, b = 62, without correction and test: 2e-14 of an element at f = 1e6, 1.5e-8 at 1e12.)
-// When the FMA path is taken the products here are lost: 256^3 54 us (40 without this route), 512^3
-// 264 (231), 1024^3 1827 (1743); thin and deep, where that one would split K, 128 x 128 x 2048 224 (64).
+// When the FMA path is taken the products here are lost: 256^3 56 us (41 without this route), 512^3
+// 272 (231), 1024^3 1892 (1744), 2048^3 14.8 ms (14.3); thin and deep, where the FMA kernel splits K,
+// 128 x 128 x 2048 228 (64; K in a cluster here, 109, costs every other product 0.5 to 2 us).
 //
 // What bounds it.  MODS + 3 products of full-size tensor-core tiles per FP64 product (the sliced
 // scheme of ct_ozaki.cu forms 36 to 45, on 64-wide tiles that its eight accumulators leave);

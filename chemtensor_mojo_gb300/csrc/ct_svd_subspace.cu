@@ -222,7 +222,8 @@ __device__ __forceinline__ void chol_pivot(double p, int j, double* pv, long lon
 // pivot's eleven dependent ones take 700 clocks a step, the rows' multiply-adds 1100 on
 // three quarters.  The pivot has a quarter of the SM to itself (the row warps are those
 // with warp % 4 != 0): beside two row warps each of its instructions waits its turn,
-// which set the step (75 us a leaf so, 68 here).
+// which set the step (75 us a leaf so, 68 here).  A step takes about 2100 clocks in all: what the two
+// do not account for, the barrier and the shared-memory latencies around it, was not isolated.
 __global__ void __launch_bounds__(CH_THREADS) chol_diag_kernel(double* G, double* Linv, int64_t ld,
                                                         unsigned long long* minpiv, int* fail, int* defrows,
                                                         int* defcount, int64_t row0, double floor) {

@@ -952,9 +952,9 @@ __global__ void __launch_bounds__(tc_chunk_threads(BN), 1)
 // rows x BN columns, each CTA its 128 rows of A, its half of B's columns and its 128 rows of the
 // accumulator; the first CTA issues the MMAs for both.  A CTA then loads 2 x (16 KB + BN x 64
 // bytes) per k-block instead of 2 x (16 KB + BN x 128): the transfer from L2 bounds the one-CTA
-// kernel (tensor pipe 65% active at 224 columns; 88 KB per k-block arrive at 41 bytes per clock
-// and SM, where the MMAs take 1344 of the 2150 clocks; neither deeper pipelines of half k-blocks nor
-// keeping A in the collector changed that).  Same MMAs, chunks and sums per element, so the same
+// kernel (tensor pipe 68% active at 224 columns; 88 KB per k-block arrive at 42 bytes per clock
+// and SM, where the MMAs take 1344 of about 2100 clocks; neither deeper pipelines of half k-blocks nor
+// keeping A in the collector changed that; in pairs it is active 71% at K = 1024, 82% at 5120).  Same MMAs, chunks and sums per element, so the same
 // bits.  4096 x 1024 x 4096: 132.8 us with one CTA per tile, 110.5 here (311 TFLOP/s); H_eff at chi
 // 1024 450 and 419.
 template <int BN>
