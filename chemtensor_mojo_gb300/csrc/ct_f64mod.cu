@@ -24,16 +24,14 @@
 // theta^2 n, n <= K the number of k where neither is exact, and has to be theta^2 K at least.  It is
 // exactly zero where no k has both, as between the blocks of a block-sparse operand (x and y of a
 // non-zero entry are kept from zero): such an element passes if its product is zero too.  The
-// others are computed as FP64 dot products, by a warp each; when they are more than an eighth of
-// all, the whole product by FP64 FMAs.
+// others are computed as FP64 dot products.
 // Every element is thus within 16.5 2^-53 S and the final rounding (worst case; FP64 FMAs: K 2^-53 S).
 // Measured, 256^3, N(0,1) operands with A falling and B rising along k by a factor f, largest error
 // in units of 2^-53 S (here, with the final rounding / FP64 FMAs): f = 1 below 0.001 / 4.0, 1e2 0.22 /
-// 4.3, 1e4 0.41 / 4.0, 1e5 0.45 / 3.6, 1e6 1.1 / 4.4, 1e7 and more, on FMAs, 1.2 / 4.4.  (18 moduli
-// alone, b = 62, without correction and test: 2e-14 of an element at f = 1e6, 1.5e-8 at 1e12.)
-// When the FMA path is taken the products here are lost: 256^3 56 us (41 without this route), 512^3
-// 272 (231), 1024^3 1892 (1744), 2048^3 14.8 ms (14.3); thin and deep, where the FMA kernel splits K,
-// 128 x 128 x 2048 228 (64; K in a cluster here, 109, costs every other product 0.5 to 2 us).
+// 4.3, 1e4 0.41 / 4.0, 1e5 0.45 / 3.6, 1e6 1.1 / 4.4, 1e7 2.3 / 4.4, then all dot products, 1.2 / 4.4.  (18
+// moduli alone, b = 62, without correction and test: 2e-14 of an element at f = 1e6, 1.5e-8 at 1e12.)
+// Dot products of all elements, after the products here (us, and the FMA kernel without this route):
+// 256^3 55 (41), 512^3 293 (231), 1280 x 1024 x 256 648 (780), 1024 x 256 x 1280 724 (570).
 //
 // What bounds it.  MODS + 3 products of full-size tensor-core tiles per FP64 product (the sliced
 // scheme of ct_ozaki.cu forms 36 to 45, on 64-wide tiles that its eight accumulators leave);
@@ -290,10 +288,9 @@ __device__ __forceinline__ bool fm_fixed(double v, int e, int bits, unsigned lon
 // a row, a lane two columns.  sk == 1: read along k; else through a shared-memory tile, read
 // along the rows.
 __global__ void __launch_bounds__(256) fm_residue_kernel(FmSrc a, FmSrc b, int nba, int bits, float theta,
-                                                         const ModTable tab, unsigned* failed, const int* skip) {
+                                                         const ModTable tab, const int* skip) {
     ct_pdl();
     if (ct_skip(skip)) return;
-    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) *failed = 0;
     __shared__ double tile[FM_PK][FM_PR + 1];
     const bool first = (int)blockIdx.x < nba;
     const FmSrc& x = first ? a : b;
@@ -409,7 +406,6 @@ __device__ __forceinline__ void fm_mma(uint32_t dtm, uint64_t ad, uint64_t bd, u
 struct FmOut {
     unsigned char* r;    // [MODS + 1][M][ldn]: t_i + 128 of C, then the test's answer (ldn a multiple of FM_BN)
     float* corr;         // [2][M][ldn]: the corrections times 2^30
-    unsigned* failed;    // number of elements that fail the test
     float limit;         // theta^2 K
     int64_t ldn;
 };
@@ -572,16 +568,12 @@ __global__ void __launch_bounds__(FM_THREADS, 1)
             const int64_t mr = (int64_t)(t / tiles_n) * FM_BM + row;
             const int nc = (t % tiles_n) * FM_BN + hf * FM_HC;
             if (pl == PL_TEST) {
-                int fails = 0;
                 uint32_t w[FM_HC / 4];
 #pragma unroll
                 for (int j = 0; j < FM_HC; ++j) {
                     const uint32_t v = sum[j] >= out.limit ? FM_PASS : sum[j] == 0.0f ? FM_NONE : FM_FAIL;
                     w[j / 4] = j % 4 ? w[j / 4] | v << (8 * (j % 4)) : v;
-                    fails += v == FM_FAIL && mr < M && nc + j < N;
                 }
-                fails = __reduce_add_sync(0xffffffffu, fails);
-                if (lane == 0 && fails) atomicAdd(out.failed, (unsigned)fails);
                 if (mr < M) {
                     unsigned char* o = out.r + ((int64_t)MODS * M + mr) * out.ldn + nc;
 #pragma unroll
@@ -636,86 +628,66 @@ struct FmC {
     int64_t M0, s1, s0;
 };
 
-// The whole product by FP64 FMAs, the sums of 32 of K added in the order of k (so that no error is
-// above that of K pieces): 8 x 16 tiles dealt to the blocks, an element per thread (FMAs of a warp
-// issue at one per 64 clocks whatever a thread holds, see gemm_f64_spread_kernel), the next 32 of K
-// loaded while these are multiplied.
 constexpr int FM_CRT = 128;   // threads of the reconstruction: two rows of 128 columns
-__device__ void fm_fma_product(const FmSrc& a, const FmSrc& b, const FmC& c, int M, int N) {
-    constexpr int TM = 8, TN = 16, BK = 32, NA = TM * BK / FM_CRT, NB = TN * BK / FM_CRT;
-    __shared__ double As[BK][TM + 1], Bs[BK][TN + 1];
-    const int tid = threadIdx.x, tx = tid % TN, ty = tid / TN;
-    const int64_t tiles_n = (N + TN - 1) / TN, tiles = tiles_n * ((M + TM - 1) / TM);
-    const int64_t blocks = (int64_t)gridDim.x * gridDim.y;
-    for (int64_t t = (int64_t)blockIdx.y * gridDim.x + blockIdx.x; t < tiles; t += blocks) {
-        const int64_t m0 = t / tiles_n * TM, n0 = t % tiles_n * TN;
-        // a thread's elements of an operand's block: read along k, or along the rows
-        int ra[NA], ka[NA], rb[NB], kb[NB];
-        const double *pa[NA], *pb[NB];
+
+// FP64 dot products of row m of A with the rows n of B of the lanes in `mask`, v in the others.  A few
+// are formed one after another by the warp, more by their lanes, at the rate of the FP64 pipe, in sums
+// of 32.  (1280 x 1024 x 256 with 3% of the elements failing, in whole rows: 205 us by the warp alone, 117 so.)
+__device__ __forceinline__ double fm_dots(const FmSrc& a, const FmSrc& b, int64_t m, int64_t n, unsigned mask, double v) {
+    const int lane = threadIdx.x & 31;
+    const double* pa = a.p + a.row(m);
+    if (__popc(mask) > 6) {
+        if ((mask >> lane) & 1) {
+            const double* pb = b.p + b.row(n);
+            v = 0.0;
+            for (int64_t k0 = 0; k0 < a.K; k0 += 32) {
+                double part = 0.0;
 #pragma unroll
-        for (int i = 0; i < NA; ++i) {
-            const int e = tid + FM_CRT * i;
-            ra[i] = a.sk == 1 ? e / BK : e % TM;
-            ka[i] = a.sk == 1 ? e % BK : e / TM;
-            pa[i] = m0 + ra[i] < M ? a.p + a.row(m0 + ra[i]) + ka[i] * a.sk : nullptr;
-        }
+                for (int h = 0; h < 32; h += 8) {   // (eight loads of each in flight)
+                    double x[8], y[8];
 #pragma unroll
-        for (int i = 0; i < NB; ++i) {
-            const int e = tid + FM_CRT * i;
-            rb[i] = b.sk == 1 ? e / BK : e % TN;
-            kb[i] = b.sk == 1 ? e % BK : e / TN;
-            pb[i] = n0 + rb[i] < N ? b.p + b.row(n0 + rb[i]) + kb[i] * b.sk : nullptr;
-        }
-        double xa[NA], xb[NB];
-        auto load = [&](int64_t k0) {
+                    for (int i = 0; i < 8; ++i) {
+                        const int64_t k = k0 + h + i;
+                        x[i] = k < a.K ? pa[k * a.sk] : 0.0;
+                        y[i] = k < a.K ? pb[k * b.sk] : 0.0;
+                    }
 #pragma unroll
-            for (int i = 0; i < NA; ++i) {
-                xa[i] = pa[i] && k0 + ka[i] < a.K ? *pa[i] : 0.0;
-                if (pa[i]) pa[i] += BK * a.sk;
+                    for (int i = 0; i < 8; ++i) part = fma(x[i], y[i], part);
+                }
+                v += part;
             }
-#pragma unroll
-            for (int i = 0; i < NB; ++i) {
-                xb[i] = pb[i] && k0 + kb[i] < a.K ? *pb[i] : 0.0;
-                if (pb[i]) pb[i] += BK * b.sk;
-            }
-        };
-        double acc = 0.0;
-        load(0);
-        for (int64_t k0 = 0; k0 < a.K; k0 += BK) {
-            __syncthreads();
-#pragma unroll
-            for (int i = 0; i < NA; ++i) As[ka[i]][ra[i]] = xa[i];
-#pragma unroll
-            for (int i = 0; i < NB; ++i) Bs[kb[i]][rb[i]] = xb[i];
-            __syncthreads();
-            if (k0 + BK < a.K) load(k0 + BK);
-            const int kn = a.K - k0 < BK ? (int)(a.K - k0) : BK;
-            double part = 0.0;
-#pragma unroll 1
-            for (int kk = 0; kk < kn; kk += 8)
-#pragma unroll
-                for (int u = 0; u < 8; ++u) part = fma(As[kk + u][ty], Bs[kk + u][tx], part);   // (zeros from kn on)
-            acc += part;
         }
-        const int64_t m = m0 + ty, n = n0 + tx;
-        if (m < M && n < N) c.p[(m / c.M0) * c.s1 + (m % c.M0) * c.s0 + n] = acc;
+        return v;
     }
+    for (; mask; mask &= mask - 1) {
+        const int src = __ffs(mask) - 1;
+        const double* pb = b.p + b.row(__shfl_sync(0xffffffffu, n, src));
+        double dot = 0.0;
+        for (int64_t k0 = lane; k0 < a.K; k0 += 256) {
+            double x[8], y[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const int64_t k = k0 + 32 * i;
+                x[i] = k < a.K ? pa[k * a.sk] : 0.0;
+                y[i] = k < a.K ? pb[k * b.sk] : 0.0;
+            }
+#pragma unroll
+            for (int i = 0; i < 8; ++i) dot = fma(x[i], y[i], dot);
+        }
+        dot = ct_warp_sum(dot);
+        if (lane == src) v = dot;
+    }
+    return v;
 }
 
 // C from its residues: S = sum t_i P / m_i - k P with k = rint(sum t_i / m_i), plus the correction,
 // then times 2^(ea + eb - 2 bits) and rounded to FP64.  Two moduli at a time, u = sum t_j G / m_j (below
 // 2^17), so that the multi-word sums have eight terms.  A thread takes two columns of a row; the
-// elements that fail the test, or have no scale, are FP64 dot products by the warp.  Above
-// `most` of them the blocks compute the whole product instead.
-__global__ void __launch_bounds__(FM_CRT) fm_crt_kernel(FmOut in, int M, int N, FmSrc a, FmSrc b, FmC c, int bits,
-                                                     unsigned most, const CrtTable tab, const int* skip) {
+// elements that fail the test, or have no scale, are FP64 dot products.
+__global__ void __launch_bounds__(FM_CRT, 6) fm_crt_kernel(FmOut in, int M, int N, FmSrc a, FmSrc b, FmC c, int bits,
+                                                     const CrtTable tab, const int* skip) {
     ct_pdl();
     if (ct_skip(skip)) return;
-    if (__ldcg(in.failed) > most) {
-        fm_fma_product(a, b, c, M, N);
-        return;
-    }
-    const int lane = threadIdx.x & 31;
     const int64_t n0 = 2 * ((int64_t)blockIdx.y * 64 + (threadIdx.x & 63));
     const int64_t m = (int64_t)blockIdx.x * (FM_CRT / 64) + (threadIdx.x >> 6);   // the same for a warp
     if (m >= M) return;
@@ -734,6 +706,7 @@ __global__ void __launch_bounds__(FM_CRT) fm_crt_kernel(FmOut in, int M, int N, 
         cr = make_float2(q.x + w.x, q.y + w.y);
     }
     double* Cr = c.p + (m / c.M0) * c.s1 + (m % c.M0) * c.s0;
+    unsigned redo = 0;   // bit j: column n0 + j
 #pragma unroll 1
     for (int j = 0; j < 2; ++j) {
         const int64_t n = n0 + j;
@@ -765,8 +738,8 @@ __global__ void __launch_bounds__(FM_CRT) fm_crt_kernel(FmOut in, int M, int N, 
             carry = (v >> 32) + (long long)(acc[l] >> 32);
         }
         unsigned long long hi = ((unsigned long long)s[3] << 32) | s[2], lo = ((unsigned long long)s[1] << 32) | s[0];
-        bool redo = em == FM_NONFINITE || en == FM_NONFINITE || answer == FM_FAIL ||
-                    (answer == FM_NONE && ((hi | lo) != 0 || corr != 0.0f));
+        const bool bad = em == FM_NONFINITE || en == FM_NONFINITE || answer == FM_FAIL ||
+                         (answer == FM_NONE && ((hi | lo) != 0 || corr != 0.0f));
         {   // the correction, an integer of 2^-40 units, times 2^bits
             const long long ci = __float2ll_rn(corr * 1024.0f);
             const unsigned long long l = (unsigned long long)ci << (bits - 40);
@@ -802,26 +775,18 @@ __global__ void __launch_bounds__(FM_CRT) fm_crt_kernel(FmOut in, int M, int N, 
             else v = __longlong_as_double((long long)((((unsigned long long)(ex - 1) << 52) + f) |
                                                       ((unsigned long long)neg << 63)));
         }
-        for (unsigned mask = __ballot_sync(0xffffffffu, live && redo); mask; mask &= mask - 1) {
-            const int src = __ffs(mask) - 1;
-            const double* pa = a.p + a.row(m);
-            const double* pb = b.p + b.row(__shfl_sync(0xffffffffu, n, src));
-            double dot = 0.0;
-            for (int64_t k0 = lane; k0 < a.K; k0 += 256) {   // (eight loads of each in flight)
-                double x[8], y[8];
-#pragma unroll
-                for (int i = 0; i < 8; ++i) {
-                    const int64_t k = k0 + 32 * i;
-                    x[i] = k < a.K ? pa[k * a.sk] : 0.0;
-                    y[i] = k < a.K ? pb[k * b.sk] : 0.0;
-                }
-#pragma unroll
-                for (int i = 0; i < 8; ++i) dot = fma(x[i], y[i], dot);
-            }
-            dot = ct_warp_sum(dot);
-            if (lane == src) v = dot;
-        }
-        if (live) Cr[n] = v;
+        if (live && bad) redo |= 1u << j;
+        else if (live) Cr[n] = v;
+    }
+    // (apart from the loop above, whose code and registers stay few)
+    if (!__any_sync(0xffffffffu, redo != 0)) return;
+#pragma unroll 1
+    for (int j = 0; j < 2; ++j) {
+        const bool mine = (redo >> j) & 1;
+        const unsigned mask = __ballot_sync(0xffffffffu, mine);
+        if (mask == 0) continue;
+        const double v = fm_dots(a, b, m, mine ? n0 + j : 0, mask, 0.0);
+        if (mine) Cr[n0 + j] = v;
     }
 }
 
@@ -835,7 +800,7 @@ FmPlan fm_plan(int64_t M, int64_t N, int64_t K) {
     q.ldn = ct_round_up(N, FM_BN);
     q.tiles = ct_cdiv(M, FM_BM) * ct_cdiv(N, FM_BN);
     q.bytes = ct_bytes(PLANES * M * q.ldk, 2) + ct_bytes(PLANES * N * q.ldk, 2) + ct_bytes((MODS + 1) * M * q.ldn, 1) +
-              ct_bytes(2 * M * q.ldn, 4) + ct_bytes(1, 4) + ct_bytes(M, 4) + ct_bytes(N, 4) + ct_bytes(ct_cdiv(K, FM_XK) * M, 4) + ct_bytes(ct_cdiv(K, FM_XK) * N, 4);
+              ct_bytes(2 * M * q.ldn, 4) + ct_bytes(M, 4) + ct_bytes(N, 4) + ct_bytes(ct_cdiv(K, FM_XK) * M, 4) + ct_bytes(ct_cdiv(K, FM_XK) * N, 4);
     return q;
 }
 
@@ -949,12 +914,10 @@ int ct_f64_gemm(ct_handle* h, int64_t M, int64_t N, int64_t K, const OzMat& A, c
     p += ct_bytes(PLANES * N * q.ldk, 2);
     const int bits = bits_for(K);
     const float theta = ldexpf(1.0f, 37 - bits);
-    FmOut o{(unsigned char*)p, nullptr, nullptr, theta * theta * (float)K * 1.01f, q.ldn};
+    FmOut o{(unsigned char*)p, nullptr, theta * theta * (float)K * 1.01f, q.ldn};
     p += ct_bytes((MODS + 1) * M * q.ldn, 1);
     o.corr = (float*)p;
     p += ct_bytes(2 * M * q.ldn, 4);
-    o.failed = (unsigned*)p;
-    p += ct_bytes(1, 4);
     a.ex = (int*)p;
     p += ct_bytes(M, 4);
     b.ex = (int*)p;
@@ -968,6 +931,9 @@ int ct_f64_gemm(ct_handle* h, int64_t M, int64_t N, int64_t K, const OzMat& A, c
     static int attr_dev = -1;
     if (attr_dev != h->device) {
         CT_CUDA(h, cudaFuncSetAttribute(fm_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FM_SMEM));
+        // the product kernel's share of the L1: an SM that changes it between the two loses time (256^3
+        // 17.3 us without, 14.9 so)
+        CT_CUDA(h, cudaFuncSetAttribute(fm_crt_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 60));
         attr_dev = h->device;
     }
     const Tables& t = tables();
@@ -977,15 +943,14 @@ int ct_f64_gemm(ct_handle* h, int64_t M, int64_t N, int64_t K, const OzMat& A, c
     if (K > FM_XK) {
         ct_launch(h, fm_rowexp_kernel, dim3(grid.x, (unsigned)ct_cdiv(K, FM_XK)), 256, 0, a, b, nba, skip); ct_note_launch();
     }
-    ct_launch(h, fm_residue_kernel, grid, 256, 0, a, b, nba, bits, theta, t.mod, o.failed, skip); ct_note_launch();
+    ct_launch(h, fm_residue_kernel, grid, 256, 0, a, b, nba, bits, theta, t.mod, skip); ct_note_launch();
     const int64_t items = q.tiles * PLANES;
     const int64_t ctas = items < h->num_sms ? items : h->num_sms;
     ct_launch(h, fm_gemm_kernel, (unsigned)ctas, FM_THREADS, FM_SMEM, ta, tb, (int)M, (int)N, (int)q.ldk, o, t.mod, skip,
                                                                        h->d_status); ct_note_launch();
     const FmC c{Cout.p, Cout.M0 > 0 ? Cout.M0 : M, Cout.s1, Cout.s0};
-    const unsigned most = (unsigned)std::min<int64_t>(M * N / 8, 0x7fffffff);
     ct_launch(h, fm_crt_kernel, dim3((unsigned)ct_cdiv(M, FM_CRT / 64), (unsigned)ct_cdiv(N, 128)), FM_CRT, 0,
-              o, (int)M, (int)N, a, b, c, bits, most, t.crt, skip); ct_note_launch();
+              o, (int)M, (int)N, a, b, c, bits, t.crt, skip); ct_note_launch();
     CT_LAUNCH_CHECK(h);
     return CT_OK;
 }

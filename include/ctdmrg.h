@@ -21,7 +21,7 @@
  *                   that are large enough modulo 16 small integers on the
  *                   tensor cores.  Every element is tested on the device for
  *                   the accuracy of FP64 FMAs (an error within 16.5 2^-53 of
- *                   sum_k |a_k b_k|, in practice below 2 2^-53) and formed by
+ *                   sum_k |a_k b_k|, in practice below 3 2^-53) and formed by
  *                   them where it fails, so graded operands lose nothing
  *                   (CTDMRG_FP64_TC=0 keeps all of them on FP64 FMAs).
  *   CT_PREC_TF32X3  contractions on tcgen05 tensor cores in TF32 with
