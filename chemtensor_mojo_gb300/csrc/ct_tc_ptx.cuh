@@ -55,12 +55,14 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
 
 // A producer's last act: its loads have arrived (`issued` of them, one barrier per stage), so that none
 // writes to shared memory after the CTA has gone.  Its consumers have waited for them unless a wait was
-// given up; then up to 0.1 s here.
+// given up; then up to 0.05 s a load here.
 __device__ __forceinline__ void drain_loads(uint64_t* full, int stages, int issued) {
-    const unsigned long long t0 = gtimer();
-    for (int q = issued > stages ? issued - stages : 0; q < issued; ++q)
-        while (!mbar_try_wait(&full[q % stages], (uint32_t)(q / stages) & 1u) && gtimer() - t0 < 100000000ull) {
+    for (int q = issued > stages ? issued - stages : 0; q < issued; ++q) {
+        if (mbar_try_wait(&full[q % stages], (uint32_t)(q / stages) & 1u)) continue;
+        const unsigned long long t0 = gtimer();
+        while (!mbar_try_wait(&full[q % stages], (uint32_t)(q / stages) & 1u) && gtimer() - t0 < 50000000ull) {
         }
+    }
 }
 
 __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* tm, int x, int y, uint64_t* bar) {
